@@ -12,21 +12,29 @@
 // This replaces the reference's emulation of the recipe, dequantise -> descale -> bf16 matmul
 // (alto/kernels/fp4/mxfp4/mxfp_linear.py:337-356, mxfp_grouped_gemm/cg_backward.py:668-690).
 //
-// One CTA (768 threads = six warpgroups, persistent over 128 x 128 output tiles):
-//   warpgroup 0   warp 0: producer - per stage (128 bytes of K = two chunks) two tiled TMA loads and the
-//                 bulk copies of the stage's scale tiles; warp 1: MMA issuer - two tcgen05.mma per chunk
-//                 into one of three 128-column chunk accumulators in tensor memory, then a commit to that
-//                 accumulator's "full" barrier; warp 2: waits on the shared-memory barriers for the MMA issuer
-//                 and releases it once per CHUNK through a named barrier; warp 3 idle;
-//   warpgroup 1   scale transfer shared memory -> tensor memory (as in the plain kernel);
-//   warpgroups 2-5  fold + epilogue: sixteen warps, four per tensor-memory lane quarter, each 32 rows x 32
-//                 columns of the tile in 32 registers per thread.  Per chunk a warp reads its slice of the
-//                 chunk accumulator (one tcgen05.ld), gives the accumulator back, and adds
-//                 P * (1/fa[row]) * (1/fb[col]) with packed fp32x2 arithmetic; the column factors of the
-//                 chunk pass through a small per-warp shared-memory buffer.  After the last chunk the
+// One CTA (512 threads = four warpgroups, persistent over 128 x 256 output tiles, each two halves of 128
+// columns that share the A operand):
+//   warpgroup 0   warp 0: producer - per stage (128 bytes of K = two chunks) three tiled TMA loads and the
+//                 bulk copies of the stage's scale tiles; warps 1 and 3: MMA issuers of the two halves - two
+//                 tcgen05.mma per chunk into one of three 128-column chunk accumulators in tensor memory, then
+//                 a commit to that accumulator's "full" barrier; warp 2 idle;
+//   warpgroup 1   scale transfer shared memory -> tensor memory (as in the plain kernel), and the macro
+//                 factors: the codes of the tile's rows (and columns) for the next stage's two chunks are read
+//                 a stage ahead and their reciprocals left in a shared-memory ring;
+//   warpgroups 2-3  fold + epilogue of one half each: four warps, one per tensor-memory lane quarter, 32 rows
+//                 x 128 columns in 128 registers per thread.  A chunk is read in four pieces of 32 columns,
+//                 and one piece is always on its way from tensor memory while another is folded:
+//                 acc += P * (1/fa[row]) * (1/fb[col]) in packed fp32x2 arithmetic.  After the last chunk the
 //                 registers are scaled, converted, staged and TMA-stored.
-// The warpgroups re-divide the register file with setmaxnreg (768 threads x 80 at launch -> 48 for the
-// small roles, 96 for the fold warps; the two must balance exactly, see CfgMacro).
+//
+// What bounds it: the hand-over of the chunk accumulators between the MMAs and the fold (three fit beside the
+// scales), then the fold itself, 64 (128 with per-column factors) packed operations of two cycles per scheduler
+// and 128 x 128 x 128 block whose MMAs take 128 cycles, then the shared-memory port: with 128 x 128 tiles, whose
+// operands are 17 KB of loads per block against 13 here, loading alone took 284 cycles per block.
+// Measured at 8192 x 4096 x 14336, one factor per tile of B / one per column: 476 / 694 us; with 128 x 128
+// tiles, sixteen fold warps of 32 columns that each looked up their factors, and one issuer: 572 / 924 us.
+// The warpgroups re-divide the register file with setmaxnreg (512 threads x 128 at launch -> 40 for the
+// small roles, 216 for the fold warps; the two must balance exactly, see CfgMacro).
 // Rows grouped by expert (`group_expert`) and K ranges per batch entry (`k_offs`) work as in the
 // plain kernel; every K range starts on a multiple of 128 elements, so chunks never straddle one.
 #pragma once
@@ -43,68 +51,51 @@ struct MacroGemmArgs {
   GemmArgs g;
   MacroSide ma, mb;
   float out_scale;
-#ifdef ALTOB200_GEMM_PROFILE
-  unsigned long long* prof;  // [gridDim.x][4 roles][8] clock sums of a -DALTOB200_GEMM_PROFILE build
-#endif
 };
 
-// Clock accounting of a profiling build: PROF_NOW() reads the SM clock, PROF_ADD(slot, t0) adds the
-// cycles since t0 to a per-thread counter; both vanish from the default build.
-#ifdef ALTOB200_GEMM_PROFILE
-#define PROF_DECL unsigned long long prof_c[8] = {0, 0, 0, 0, 0, 0, 0, 0}
-#define PROF_NOW() clock64()
-#define PROF_ADD(slot, t0) prof_c[slot] += (unsigned long long)(clock64() - (t0))
-#define PROF_FLUSH(role)                                                                   \
-  if (margs.prof != nullptr)                                                               \
-    for (int i_ = 0; i_ < 8; ++i_) margs.prof[((size_t)blockIdx.x * 4 + (role)) * 8 + i_] = prof_c[i_]
-// event trace of CTA 0: clock of event k of step idx (< 128) of a role, after the per-CTA sums
-#define PROF_TRACE(role, idx, k)                                                            \
-  if (margs.prof != nullptr && blockIdx.x == 0 && (idx) < 128u)                              \
-  margs.prof[(size_t)gridDim.x * 32 + (((role) * 128 + (idx)) * 4 + (k))] = (unsigned long long)clock64()
-#else
-#define PROF_TRACE(role, idx, k)
-#define PROF_DECL
-#define PROF_NOW() 0
-#define PROF_ADD(slot, t0) (void)(t0)
-#define PROF_FLUSH(role)
-#endif
-
-constexpr int NUM_THREADS_MACRO = 768;
+constexpr int NUM_THREADS_MACRO = 512;
 
 struct CfgMacro {
-  static constexpr int BN = 128;
+  static constexpr int HN = 128;                                // columns of a half (one chunk accumulator)
+  static constexpr int BN = 2 * HN;
   static constexpr int SF_TILES = Kind<KIND_MXF4>::SF_TILES;
   static constexpr int A_BYTES = BM * STAGE_K_BYTES;
-  static constexpr int B_BYTES = BN * STAGE_K_BYTES;
-  static constexpr int SFA_BYTES = SF_TILES * 512;
-  static constexpr int SFB_BYTES = SF_TILES * 512;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;
+  static constexpr int B_BYTES = HN * STAGE_K_BYTES;            // per half
+  static constexpr int SF_BYTES = SF_TILES * 512;               // per 128 rows of either operand
+  static constexpr int SF_OFF = A_BYTES + 2 * B_BYTES;          // scales of A, of B's first and second half
+  static constexpr int STAGE_BYTES = SF_OFF + 3 * SF_BYTES;
   static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 128-byte swizzle atom aligned");
-  static constexpr int SF_COLS_A = SF_TILES * 4;
-  static constexpr int SF_COLS_B = SF_TILES * 4;
-  static constexpr int STAGES = 4;
+  static constexpr int SF_COLS = SF_TILES * 4;                  // tensor-memory columns of SF_BYTES
+  static constexpr int STAGES = 3;
   static constexpr int P_BUFS = 3;                              // chunk accumulators in tensor memory
-  static constexpr int FOLD_WARPS = 16;                         // four per tensor-memory lane quarter, 32 columns each
-  static constexpr int FOLD_COLS = BN / (FOLD_WARPS / 4);
-  static constexpr int EPI_WARP_BYTES = 4096;                   // bf16: two buffers of 32 rows x 64 bytes; fp32: one of 32 x 128
+  static constexpr int FOLD_WARPS = 8;                          // four per half
+  static constexpr int EPI_UNIT = 2048;                         // 16 rows x 128 bytes
+  static constexpr int EPI_WARP_BYTES = 2 * EPI_UNIT;
   static constexpr int EPI_BYTES = FOLD_WARPS * EPI_WARP_BYTES;
-  static constexpr int FB_BYTES = FOLD_WARPS * 2 * FOLD_COLS * 4;  // two buffers of 32 column factors per warp
+  // Ring of reciprocal factors, per chunk 128 rows and 256 columns (B_UNIFORM: the products of both, 128 rows
+  // per half).  No barrier guards its reuse: a slot is rewritten FAC_STAGES stages after its last use, once
+  // that stage's operands have landed, so the MMAs of the stage STAGES earlier are done, and with them (see
+  // the issuers) both halves have read out every chunk up to two before - at least one after the slot's own,
+  // which has therefore been folded.
+  static constexpr int FAC_STAGES = 8;
+  static constexpr int FAC_STRIDE = BM + BN + 4;                // floats per chunk; + 4 spreads the banks
+  static constexpr int FAC_BYTES = 2 * FAC_STAGES * FAC_STRIDE * 4;
+  static_assert(FAC_STAGES >= STAGES + 3, "factors are overwritten while they are in use");
   static constexpr int RCP_BYTES = 256 * 4;                     // 1 / factor for every code
-  static constexpr int TMEM_SF_BASE = P_BUFS * BN;
-  static constexpr int TMEM_COLS_USED = TMEM_SF_BASE + STAGES * (SF_COLS_A + SF_COLS_B);
+  static constexpr int TMEM_SF_BASE = P_BUFS * HN;
+  static constexpr int TMEM_COLS_USED = TMEM_SF_BASE + STAGES * 3 * SF_COLS;
   static_assert(TMEM_COLS_USED <= 512, "tensor memory budget");
-  static constexpr int NUM_BARS = 3 * STAGES + 2 * P_BUFS;
+  static constexpr int NUM_BARS = 3 * STAGES + 4 * P_BUFS;
   static constexpr int SMEM_BYTES =
-      STAGES * STAGE_BYTES + EPI_BYTES + FB_BYTES + RCP_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+      STAGES * STAGE_BYTES + EPI_BYTES + FAC_BYTES + RCP_BYTES + 1024 /*align*/ + 512 /*barriers*/;
   static_assert(NUM_BARS * 8 + 16 <= 512, "barrier area");
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
-  // Registers per thread after the warpgroups have re-divided the file.  The CTA is launched with 80
-  // registers per thread (65536 / 768 rounded down to a multiple of 8, what ptxas reports for this
-  // kernel); setmaxnreg.inc can only take what setmaxnreg.dec has released INSIDE the CTA and blocks
-  // for ever otherwise, so the two must balance exactly: 2 x 128 x 48 + 4 x 128 x 96 = 768 x 80.
-  static constexpr int REGS_LAUNCH = 80;
-  static constexpr int REGS_SMALL = 48, REGS_FOLD = 96;
-  static_assert(2 * 128 * REGS_SMALL + (FOLD_WARPS / 4) * 128 * REGS_FOLD == NUM_THREADS_MACRO * REGS_LAUNCH,
+  // Registers per thread after the warpgroups have re-divided the file.  The CTA is launched with 128
+  // registers per thread (65536 / 512); setmaxnreg.inc can only take what setmaxnreg.dec has released
+  // INSIDE the CTA and blocks for ever otherwise, so the two must balance exactly.
+  static constexpr int REGS_LAUNCH = 128;
+  static constexpr int REGS_SMALL = 40, REGS_FOLD = 216;
+  static_assert(2 * 128 * REGS_SMALL + 2 * 128 * REGS_FOLD == NUM_THREADS_MACRO * REGS_LAUNCH,
                 "setmaxnreg budget must balance");
   static_assert(NUM_THREADS_MACRO == (8 + FOLD_WARPS) * 32, "role layout");
 };
@@ -116,6 +107,7 @@ struct MacroTile {
   int64_t chunk0;
   int n_chunks;
   int expert;
+  int halves;       // 1 when the tile's second half lies outside the matrix
 };
 
 __device__ __forceinline__ MacroTile decode_macro_tile(const GemmArgs& args, int64_t tile, int64_t tiles_m,
@@ -137,75 +129,117 @@ __device__ __forceinline__ MacroTile decode_macro_tile(const GemmArgs& args, int
     if (args.num_experts > 0 && !m.t.skip) m.expert = __ldg(args.group_expert + m.t.mb);
   }
   m.n_chunks = bytes > 0 ? (int)((bytes + 63) / 64) : 0;
+  m.halves = args.N - m.t.nb * CfgMacro::BN > CfgMacro::HN ? 2 : 1;
   return m;
 }
 
-// acc += P * (ra * fb[col]) for the 32 columns of one chunk that a fold warp owns (P: raw tensor-memory
-// words of this thread's row)
-__device__ __forceinline__ void fold_cols(float2 (&acc)[16], const uint32_t (&p)[32], float ra, const float* fb,
-                                          bool b_uniform, float rb_uniform) {
-  if (b_uniform) {
-    const float g = __fmul_rn(ra, rb_uniform);
-    const float2 g2 = make_float2(g, g);
+// One piece of a chunk accumulator: 32 columns of a warp's 32 rows, as two tensor-memory loads of 16 rows in
+// the 16 x 256-bit layout.  A lane gets, per group of eight columns, columns 2 (lane % 4) and + 1 of rows
+// lane / 4 and + 8 of each load: four rows and eight columns of the piece, so that it needs twelve factors,
+// where the layout of one row per lane needs 33 and the broadcast of the column factors out of shared memory
+// (128 bytes per register and warp) took longer than the multiply-adds.
+struct Piece {
+  uint32_t r[32];   // [row half 2][column group 4][row 2][column 2]
+};
+__device__ __forceinline__ void tc_ld_piece(uint32_t taddr, Piece& p) {
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      acc[j] = __ffma2_rn(make_float2(u2f(p[2 * j]), u2f(p[2 * j + 1])), g2, acc[j]);
-  } else {
-    const float2 ra2 = make_float2(ra, ra);
+  for (int h = 0; h < 2; ++h) {
+    uint32_t* r = p.r + 16 * h;
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr + ((uint32_t)(16 * h) << 16))
+        : "memory");
+  }
+}
+// tcgen05.wait::ld that the values in p depend on: nothing that uses them can move above it
+__device__ __forceinline__ void tc_wait_piece(Piece& p) {
+#define ALTOB200_RW8(o) "+r"(p.r[o]), "+r"(p.r[o + 1]), "+r"(p.r[o + 2]), "+r"(p.r[o + 3]), "+r"(p.r[o + 4]), \
+                        "+r"(p.r[o + 5]), "+r"(p.r[o + 6]), "+r"(p.r[o + 7])
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : ALTOB200_RW8(0), ALTOB200_RW8(8), ALTOB200_RW8(16), ALTOB200_RW8(24)
+               :
+               : "memory");
+#undef ALTOB200_RW8
+}
+// acc += P * ra[row] * fb[col]; B_UNIFORM: one B factor for the half and chunk, already multiplied into ra.
+// `acc` and `p` are laid out alike; fb points at this lane's first column.
+template <bool B_UNIFORM>
+__device__ __forceinline__ void fold_piece(float2* acc, const Piece& p, const float (&ra)[4], const float* fb) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float4 f = *reinterpret_cast<const float4*>(fb + 4 * j);
-      const float2 g0 = __fmul2_rn(ra2, make_float2(f.x, f.y));
-      const float2 g1 = __fmul2_rn(ra2, make_float2(f.z, f.w));
-      acc[2 * j] = __ffma2_rn(make_float2(u2f(p[4 * j]), u2f(p[4 * j + 1])), g0, acc[2 * j]);
-      acc[2 * j + 1] = __ffma2_rn(make_float2(u2f(p[4 * j + 2]), u2f(p[4 * j + 3])), g1, acc[2 * j + 1]);
+  for (int g = 0; g < 4; ++g) {
+    float2 f = make_float2(1.0f, 1.0f);
+    if (!B_UNIFORM) f = *reinterpret_cast<const float2*>(fb + 8 * g);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {   // row half q / 2, row 8 (q % 2)
+      const int i = (q >> 1) * 8 + g * 2 + (q & 1);
+      float2 w = make_float2(ra[q], ra[q]);
+      if (!B_UNIFORM) w = __fmul2_rn(w, f);
+      acc[i] = __ffma2_rn(make_float2(u2f(p.r[2 * i]), u2f(p.r[2 * i + 1])), w, acc[i]);
     }
   }
 }
 
+// One look at a barrier's phase, without waiting.
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// B_UNIFORM: B's macro blocks are 128 x 128 tiles (one factor per half and chunk), else per column.
+template <bool B_UNIFORM>
 __global__ void __launch_bounds__(NUM_THREADS_MACRO, 1)
 gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_d, const MacroGemmArgs margs) {
   using C = CfgMacro;
-  constexpr int BN = C::BN;
+  constexpr int HN = C::HN;
   const GemmArgs& args = margs.g;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* epi = smem + C::STAGES * C::STAGE_BYTES;
-  float* fb_all = reinterpret_cast<float*>(epi + C::EPI_BYTES);
-  float* rcp_tab = reinterpret_cast<float*>(epi + C::EPI_BYTES + C::FB_BYTES);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(epi + C::EPI_BYTES + C::FB_BYTES + C::RCP_BYTES);
+  float* fac = reinterpret_cast<float*>(epi + C::EPI_BYTES);
+  float* rcp_tab = reinterpret_cast<float*>(epi + C::EPI_BYTES + C::FAC_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(epi + C::EPI_BYTES + C::FAC_BYTES + C::RCP_BYTES);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + C::STAGES;
   uint64_t* sf_full = bars + 2 * C::STAGES;
-  uint64_t* p_full = bars + 3 * C::STAGES;
-  uint64_t* p_empty = p_full + C::P_BUFS;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_empty + C::P_BUFS);
+  uint64_t* p_full = bars + 3 * C::STAGES;        // [half][chunk % P_BUFS]
+  uint64_t* p_empty = p_full + 2 * C::P_BUFS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_empty + 2 * C::P_BUFS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t tiles_m = (args.M + BM - 1) / BM;
-  const int64_t tiles_n = (args.N + BN - 1) / BN;
+  const int64_t tiles_n = (args.N + C::BN - 1) / C::BN;
   const int64_t n_tiles = tiles_m * tiles_n * (args.k_offs != nullptr ? args.num_batches : 1);
   const int k_stages = (int)((args.k_bytes + STAGE_K_BYTES - 1) / STAGE_K_BYTES);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+      mbar_init(&empty_bar[s], 2);
       mbar_init(&sf_full[s], 4);
     }
-    for (int p = 0; p < C::P_BUFS; ++p) {
+    for (int p = 0; p < 2 * C::P_BUFS; ++p) {
       mbar_init(&p_full[p], 1);
-      mbar_init(&p_empty[p], C::FOLD_WARPS);
+      mbar_init(&p_empty[p], C::FOLD_WARPS / 2);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // scale staging starts from zero: a ragged last stage never feeds uninitialised scale bytes
   for (int s = 0; s < C::STAGES; ++s) {
-    uint32_t* z = reinterpret_cast<uint32_t*>(smem + s * C::STAGE_BYTES + C::A_BYTES + C::B_BYTES);
-    for (int i = threadIdx.x; i < (C::SFA_BYTES + C::SFB_BYTES) / 4; i += NUM_THREADS_MACRO) z[i] = 0u;
+    uint32_t* z = reinterpret_cast<uint32_t*>(smem + s * C::STAGE_BYTES + C::SF_OFF);
+    for (int i = threadIdx.x; i < 3 * C::SF_BYTES / 4; i += NUM_THREADS_MACRO) z[i] = 0u;
   }
   // 1 / factor(code), factor = 1 + code / 256 (exact), correctly rounded
   if (threadIdx.x < 256) rcp_tab[threadIdx.x] = __frcp_rn(u2f((threadIdx.x << 15) + (127u << 23)));
@@ -234,8 +268,6 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const bool elected = elect_one();
       uint32_t it = 0;
       bool alive = true;
-      PROF_DECL;
-      const long long t_all = PROF_NOW();
       for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
         const MacroTile mt = decode_macro_tile(args, tile, tiles_m, tiles_n, k_stages);
         const TileInfo& ti = mt.t;
@@ -243,290 +275,294 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         const int64_t mb = ti.mb, nb = ti.nb;
         for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
           const int s = it % C::STAGES;
-          const long long t0 = PROF_NOW();
           alive = __all_sync(0xFFFFFFFFu,
                              mbar_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1, abort_flag, 21, args.wait_ns));
           if (!alive) break;
-          PROF_ADD(1, t0);
-          if (lane == 0) { PROF_TRACE(0, it, 0); }
           uint8_t* st = smem + s * C::STAGE_BYTES;
           const int64_t cb0 = ti.sf_tile0 + (int64_t)ks * C::SF_TILES;
           int64_t sf_tiles = args.nct - cb0;
           if (sf_tiles > C::SF_TILES) sf_tiles = C::SF_TILES;
           const uint32_t sf_bytes = (uint32_t)sf_tiles * 512u;
           const int32_t kx = (int32_t)(ti.k_byte0 + (int64_t)ks * STAGE_K_BYTES);
-          if (ALTOB200_DBG(args, 4) && it >= (uint32_t)C::STAGES) {
-            if (elected) mbar_arrive(&full_bar[s]);
-            continue;
-          }
           if (elected) {
-            mbar_expect_tx(&full_bar[s], C::A_BYTES + C::B_BYTES + 2 * sf_bytes);
+            const uint32_t n_b = (uint32_t)mt.halves;
+            mbar_expect_tx(&full_bar[s], C::A_BYTES + sf_bytes + n_b * (C::B_BYTES + sf_bytes));
             tma_load_2d(st, &tmap_a, kx, (int32_t)(mb * BM), &full_bar[s]);
-            tma_load_2d(st + C::A_BYTES, &tmap_b, kx, (int32_t)ti.b_row0, &full_bar[s]);
-            bulk_load(st + C::A_BYTES + C::B_BYTES, args.sfa + (mb * args.nct + cb0) * 512, sf_bytes, &full_bar[s]);
-            bulk_load(st + C::A_BYTES + C::B_BYTES + C::SFA_BYTES, ti.sfb + (nb * args.nct + cb0) * 512, sf_bytes,
-                      &full_bar[s]);
+            bulk_load(st + C::SF_OFF, args.sfa + (mb * args.nct + cb0) * 512, sf_bytes, &full_bar[s]);
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+              if (h < n_b) {
+                tma_load_2d(st + C::A_BYTES + h * C::B_BYTES, &tmap_b, kx, (int32_t)(ti.b_row0 + h * HN), &full_bar[s]);
+                bulk_load(st + C::SF_OFF + (1 + h) * C::SF_BYTES, ti.sfb + ((nb * 2 + h) * args.nct + cb0) * 512, sf_bytes,
+                          &full_bar[s]);
+              }
+            }
           }
         }
       }
-      PROF_ADD(0, t_all);
-      if (lane == 0) { PROF_FLUSH(0); }
-    } else if (warp == 1) {
-      // ------------------------------ MMA issuer ------------------------------
-      // Never waits on a shared-memory barrier itself (such a wait between two tcgen05.mma costs ~150
-      // cycles during which the tensor pipe idles): warp 2 waits and meets this warp at named barrier
-      // 1 + stage.
+    } else if (warp == 1 || warp == 3) {
+      // ------------------------------ MMA issuers ------------------------------
+      // One per half: a tcgen05.mma does not run ahead of its thread's other instructions, so while one
+      // issuer waits for its barriers (~150 cycles even when they are complete) the other one's MMAs keep the
+      // tensor pipe busy.
+      // Chunk n of half h goes to accumulator (2 n + h) % 3, which held chunk n - 2 of half 1 (h = 0) or
+      // chunk n - 1 of half 0 (h = 1); the barriers count the chunks of one half, so that whoever waits on
+      // one has waited for all its earlier phases.  A half outside the matrix runs the protocol without MMAs.
+      static_assert(C::P_BUFS == 3, "order of the accumulators");
       const bool elected = elect_one();
-      uint32_t it = 0, pc = 0;
+      const int h = warp >> 1;
+      uint32_t it = 0, n = 0;         // stages and chunks so far
       bool alive = true;
       const uint32_t smem_base = smem_u32(smem);
-      PROF_DECL;
-      const long long t_all = PROF_NOW();
+      uint64_t* const my_full = p_full + h * C::P_BUFS;
+      uint64_t* const other_empty = p_empty + (h ^ 1) * C::P_BUFS;
+      const uint32_t back = h == 0 ? 2u : 1u;
       for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
         const MacroTile mt = decode_macro_tile(args, tile, tiles_m, tiles_n, k_stages);
         const TileInfo& ti = mt.t;
         if (ti.skip) continue;
+        const bool mine = h < mt.halves;
         for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
           const int n_mma = (ks == ti.k_stages - 1) ? ti.last_mmas : 4;
           const int s = it % C::STAGES;
-          const uint32_t st4 = (smem_base + (uint32_t)s * C::STAGE_BYTES) >> 4;
-          const uint32_t sfa_t = tmem_base + C::TMEM_SF_BASE + s * (C::SF_COLS_A + C::SF_COLS_B);
-          const uint32_t sfb_t = sfa_t + C::SF_COLS_A;
-          const uint32_t a_lo = st4 | 0x10000u;
-          const uint32_t b_lo = a_lo + (C::A_BYTES >> 4);
-          // The issuer is released per chunk (two MMAs), not per stage: a stage holds two chunks and only
-          // three chunk accumulators exist, so a release per stage would wait for the fold of the previous
-          // stage's FIRST chunk and leave one chunk of overlap instead of three.
+          const uint32_t sfa_t = tmem_base + C::TMEM_SF_BASE + s * 3 * C::SF_COLS;
+          const uint32_t sfb_t = sfa_t + (1 + h) * C::SF_COLS;
+          const uint32_t a_lo = ((smem_base + (uint32_t)s * C::STAGE_BYTES) >> 4) | 0x10000u;
+          const uint32_t b_lo = a_lo + ((C::A_BYTES + h * C::B_BYTES) >> 4);
+          // operands and scales of the stage are in place
+          bool ok = mbar_wait(&sf_full[s], (it / C::STAGES) & 1, abort_flag, 25, args.wait_ns);
+          ok = ok && mbar_wait(&full_bar[s], (it / C::STAGES) & 1, abort_flag, 23, args.wait_ns);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (2 * h >= n_mma) break;
-            const long long t0 = PROF_NOW();
-            // operands and scales of the stage are in place and this chunk's accumulator is drained
-            if (named_barrier_or(1 + 2 * s + h, 64, false)) { alive = false; break; }
-            PROF_ADD(1, t0);
-            tc_fence_after();
-            const uint32_t buf = pc % C::P_BUFS;
-            if (elected) {
-#pragma unroll
-              for (int j = 2 * h; j < 2 * h + 2; ++j) {
-                if (j < n_mma)
-                  tc_mma<KIND_MXF4>(tmem_base + buf * BN, desc_of(DESC_SW128_HI, a_lo + 2 * j),
-                                    desc_of(DESC_SW128_HI, b_lo + 2 * j), args.idesc[j], (uint32_t)(j & 1),
-                                    sfa_t + h * 4, sfb_t + h * 4);
-              }
-              tc_commit(&p_full[buf]);
-              if (2 * h + 2 >= n_mma) tc_commit(&empty_bar[s]);
+          for (int c = 0; c < 2; ++c) {
+            if (2 * c >= n_mma) break;
+            // the chunk's accumulator is drained
+            if (n >= back) {
+              const uint32_t m = n - back;
+              ok = ok && mbar_wait(&other_empty[m % C::P_BUFS], (m / C::P_BUFS) & 1, abort_flag, 22, args.wait_ns);
             }
-            __syncwarp();
-            ++pc;
+            alive = __all_sync(0xFFFFFFFFu, ok);
+            if (!alive) break;
+            tc_fence_after();
+            if (elected) {
+              if (mine) {
+                const uint32_t acc_t = tmem_base + ((2 * n + (uint32_t)h) % C::P_BUFS) * HN;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                  if (2 * c + j < n_mma)
+                    tc_mma<KIND_MXF4>(acc_t, desc_of(DESC_SW128_HI, a_lo + 4 * c + 2 * j),
+                                      desc_of(DESC_SW128_HI, b_lo + 4 * c + 2 * j), args.idesc[j], (uint32_t)j,
+                                      sfa_t + c * 4, sfb_t + c * 4);
+                }
+              }
+              tc_commit(&my_full[n % C::P_BUFS]);
+            }
+            ++n;
           }
           if (!alive) break;
-        }
-      }
-      PROF_ADD(0, t_all);
-      if (lane == 0) { PROF_FLUSH(1); }
-    } else if (warp == 2) {
-      // ------------------------------ wait warp ------------------------------
-      uint32_t it = 0, pc = 0;
-      bool alive = true;
-      for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
-        const MacroTile mt = decode_macro_tile(args, tile, tiles_m, tiles_n, k_stages);
-        const TileInfo& ti = mt.t;
-        if (ti.skip) continue;
-        for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
-          const int n_mma = (ks == ti.k_stages - 1) ? ti.last_mmas : 4;
-          const int n_chunks = (n_mma + 1) >> 1;
-          const int s = it % C::STAGES;
-          bool ok = mbar_wait(&full_bar[s], (it / C::STAGES) & 1, abort_flag, 23, args.wait_ns);
-          ok = ok && mbar_wait(&sf_full[s], (it / C::STAGES) & 1, abort_flag, 25, args.wait_ns);
-          for (int c = 0; c < n_chunks && alive; ++c, ++pc) {
-            ok = ok && mbar_wait(&p_empty[pc % C::P_BUFS], ((pc / C::P_BUFS) & 1) ^ 1, abort_flag, 22, args.wait_ns);
-            const bool failed = !__all_sync(0xFFFFFFFFu, ok);
-            if (named_barrier_or(1 + 2 * s + c, 64, failed)) alive = false;
-          }
-          if (!alive) break;
+          if (elected) tc_commit(&empty_bar[s]);   // both issuers
+          __syncwarp();
         }
       }
     }
   } else if (warp < 8) {
-    // ------------------------------ scale transfer ------------------------------
+    // ------------------------------ scale transfer and macro factors ------------------------------
     setmaxnreg_dec<C::REGS_SMALL>();
-    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const int quad = warp & 3;
+    const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
+    // factors: lane = (row of sixteen, chunk of the stage); the warp serves 32 rows of A and 64 columns of B
+    const int fc = lane & 1, fr = lane >> 1;
     uint32_t it = 0;
     bool alive = true;
-    PROF_DECL;
-    const long long t_all = PROF_NOW();
     for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
       const MacroTile mt = decode_macro_tile(args, tile, tiles_m, tiles_n, k_stages);
       const TileInfo& ti = mt.t;
       if (ti.skip) continue;
+      const int64_t m0 = ti.mb * BM, n0 = ti.nb * C::BN;
+      const uint8_t* pa = margs.ma.codes + (mt.chunk0 + fc) * margs.ma.chunk_stride +
+                          (m0 >> margs.ma.shift) * margs.ma.row_stride;
+      const uint8_t* pb = margs.mb.codes + (int64_t)mt.expert * margs.mb.expert_stride +
+                          (mt.chunk0 + fc) * margs.mb.chunk_stride + (n0 >> margs.mb.shift) * margs.mb.row_stride;
+      // offsets of the lane's rows from the tile's first (a row beyond the matrix reads the last one): they
+      // stay below 256 * 2^24, the chunks of the longest K the host accepts
+      constexpr int NB = B_UNIFORM ? 2 : 4;
+      uint32_t off_a[2], off_b[NB];
+      const uint32_t m_last = (uint32_t)(args.M - m0 < BM ? args.M - m0 : BM) - 1u;
+      const uint32_t n_last = (uint32_t)(args.N - n0 < C::BN ? args.N - n0 : C::BN) - 1u;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t r = (uint32_t)(quad * 32 + 16 * i + fr);
+        off_a[i] = ((r < m_last ? r : m_last) >> margs.ma.shift) * (uint32_t)margs.ma.row_stride;
+      }
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        const uint32_t r = (uint32_t)(B_UNIFORM ? HN * i : quad * 64 + 16 * i + fr);
+        off_b[i] = ((r < n_last ? r : n_last) >> (B_UNIFORM ? 7 : 0)) * (uint32_t)margs.mb.row_stride;
+      }
+      uint32_t ca[2], cb[NB];
+      auto load_codes = [&](int ks) {
+        const bool have = 2 * ks + fc < mt.n_chunks;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) ca[i] = have ? __ldg(pa + off_a[i]) : 0u;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) cb[i] = have ? __ldg(pb + off_b[i]) : 0u;
+        pa += 2 * margs.ma.chunk_stride;
+        pb += 2 * margs.mb.chunk_stride;
+      };
+      load_codes(0);
       for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
         const int s = it % C::STAGES;
-        const long long t0 = PROF_NOW();
         if (!mbar_wait(&full_bar[s], (it / C::STAGES) & 1, abort_flag, 26, args.wait_ns)) { alive = false; break; }
-        PROF_ADD(1, t0);
-        if (warp == 4 && lane == 0) { PROF_TRACE(2, it, 0); }
-        const uint8_t* sf = smem + s * C::STAGE_BYTES + C::A_BYTES + C::B_BYTES + lane * 16;
-        const uint32_t sfa_t = tmem_base + lane_base + C::TMEM_SF_BASE + s * (C::SF_COLS_A + C::SF_COLS_B);
-        const uint32_t sfb_t = sfa_t + C::SF_COLS_A;
-        if (!(ALTOB200_DBG(args, 1) && it > 0)) {
+        const uint8_t* sf = smem + s * C::STAGE_BYTES + C::SF_OFF + lane * 16;
+        const uint32_t sf_t = tmem_base + lane_base + C::TMEM_SF_BASE + s * 3 * C::SF_COLS;
 #pragma unroll
-          for (int t = 0; t < C::SF_TILES; ++t) {
-            const uint4 a = *reinterpret_cast<const uint4*>(sf + t * 512);
-            tc_st4(sfa_t + t * 4, a.x, a.y, a.z, a.w);
-            const uint4 b = *reinterpret_cast<const uint4*>(sf + C::SFA_BYTES + t * 512);
-            tc_st4(sfb_t + t * 4, b.x, b.y, b.z, b.w);
-          }
-          tc_wait_st();
+        for (int t = 0; t < 3 * C::SF_TILES; ++t) {
+          const uint4 a = *reinterpret_cast<const uint4*>(sf + t * 512);
+          tc_st4(sf_t + t * 4, a.x, a.y, a.z, a.w);
         }
+        float* dst = fac + (2 * (it % C::FAC_STAGES) + fc) * C::FAC_STRIDE + fr;
+        if (B_UNIFORM) {
+          const float rb0 = rcp_tab[cb[0]], rb1 = rcp_tab[cb[1]];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const float ra = rcp_tab[ca[i]];
+            dst[quad * 32 + 16 * i] = __fmul_rn(ra, rb0);
+            dst[HN + quad * 32 + 16 * i] = __fmul_rn(ra, rb1);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) dst[quad * 32 + 16 * i] = rcp_tab[ca[i]];
+#pragma unroll
+          for (int i = 0; i < NB; ++i) dst[BM + quad * 64 + 16 * i] = rcp_tab[cb[i]];
+        }
+        tc_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sf_full[s]);
-        if (warp == 4 && lane == 0) { PROF_TRACE(2, it, 1); }
+        if (ks + 1 < ti.k_stages) load_codes(ks + 1);
       }
     }
-    PROF_ADD(0, t_all);
-    if (warp == 4 && lane == 0) { PROF_FLUSH(2); }
   } else {
     // ------------------------------ fold + epilogue ------------------------------
-    // Sixteen warps, four per tensor-memory lane quarter, each 32 rows x 32 columns of the tile.  What
-    // bounds the fold is the latency of the tensor-memory load (a warp has one in flight and waits for
-    // it), so the chunk is spread over as many warps as the register file carries: 64 KB per chunk are
-    // in flight at once, and the four warps of a scheduler cover each other's waits.
     setmaxnreg_inc<C::REGS_FOLD>();
-    constexpr int FC = C::FOLD_COLS;
     const int quad = warp & 3;                        // tensor-memory lane quarter this warp may read
-    const int cq = (warp - 8) >> 2;                   // columns [32 cq, 32 cq + 32) of the tile
-    const int fold_idx = warp - 8;
-    uint8_t* epi_warp = epi + fold_idx * C::EPI_WARP_BYTES;
-    float* fb_warp = fb_all + fold_idx * (2 * FC);
-    const bool b_uniform = margs.mb.shift >= 7;       // one B factor per 128-column tile and chunk
+    const int half = (warp - 8) >> 2;                 // columns [128 half, 128 half + 128) of the tile
+    uint8_t* epi_warp = epi + (warp - 8) * C::EPI_WARP_BYTES;
     const bool out_bf16 = args.out_bf16 != 0;
-    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + cq * FC;
-    uint32_t pc = 0, store_it = 0;
-    uint32_t p_buf = 0, p_phase = 0;                  // position in the ring of chunk accumulators, its phase
+    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
+    // this lane's first row and column factor in a chunk's slot
+    const float* fac_a = fac + (B_UNIFORM ? half * HN : 0) + quad * 32 + (lane >> 2);
+    const float* fac_b = fac + BM + half * HN + 2 * (lane & 3);
+    uint64_t* const my_full = p_full + half * C::P_BUFS;
+    uint64_t* const my_empty = p_empty + half * C::P_BUFS;
+    uint32_t store_it = 0, it = 0, n = 0;             // store units, stages and chunks so far
     bool alive = true;
-    PROF_DECL;
-    const long long t_all = PROF_NOW();
     for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
       const MacroTile mt = decode_macro_tile(args, tile, tiles_m, tiles_n, k_stages);
       const TileInfo& ti = mt.t;
-      float2 acc[FC / 2];
-#pragma unroll
-      for (int j = 0; j < FC / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
-      if (!ti.skip) {
-        // factor codes of this thread's row of A and of the column of B this lane stages
-        int64_t m = ti.mb * BM + quad * 32 + lane;
-        if (m >= args.M) m = args.M - 1;
-        int64_t n0 = ti.nb * BN + cq * FC + lane;
-        if (n0 >= args.N) n0 = args.N - 1;
-        const uint8_t* pa = margs.ma.codes + (m >> margs.ma.shift) * margs.ma.row_stride +
-                            mt.chunk0 * margs.ma.chunk_stride;
-        const uint8_t* pb = margs.mb.codes + (int64_t)mt.expert * margs.mb.expert_stride +
-                            mt.chunk0 * margs.mb.chunk_stride + (n0 >> margs.mb.shift) * margs.mb.row_stride;
-        const int nch = mt.n_chunks;
-        uint32_t ca = __ldg(pa), cb = __ldg(pb);
-        uint32_t p[FC];   // chunk accumulator words of this thread's row
-        // The loop body is what bounds the kernel (instruction issue of sixteen of these warps), so the
-        // ring position and its phase are carried instead of divided out, the code pointers advance by
-        // their strides, and the two barrier addresses are 32-bit shared-memory addresses.
-        const int64_t sa = margs.ma.chunk_stride, sb = margs.mb.chunk_stride;
-        for (int c = 0; c < nch; ++c) {
-          if (ALTOB200_DBG(args, 256)) continue;
-          long long t0 = PROF_NOW();
-          alive = mbar_wait(&p_full[p_buf], p_phase, abort_flag, 24, args.wait_ns);
-          PROF_ADD(2, t0);
-          if (!alive) break;
-          tc_fence_after();
-          if (warp == 8 && lane == 0) { PROF_TRACE(3, pc, 0); }
-          tc_ld32(t_row + p_buf * BN, p);
-          // under the load: this chunk's factors, the next chunk's codes
-          t0 = PROF_NOW();
-          const float ra = rcp_tab[ca], rb = rcp_tab[cb];
-          pa += sa;
-          pb += sb;
-          if (c + 1 < nch) {
-            ca = __ldg(pa);
-            cb = __ldg(pb);
-          }
-          float* fb = fb_warp + (c & 1) * FC;
-          if (!b_uniform) {
-            fb[lane] = rb;
-            __syncwarp();
-          }
-          PROF_ADD(6, t0);
-          t0 = PROF_NOW();
-          tc_wait_ld();                 // the chunk has left tensor memory
-          PROF_ADD(1, t0);
-          t0 = PROF_NOW();
-          tc_fence_before();
+      const int nch = ti.skip ? 0 : mt.n_chunks;
+      const uint32_t n_end = n + (uint32_t)nch, n0 = n, it0 = it;
+      it += ti.skip ? 0u : (uint32_t)ti.k_stages;
+      if (half >= mt.halves) {                        // nothing to read, only the hand-over
+        for (; n < n_end && alive; ++n) {
+          alive = mbar_wait(&my_full[n % C::P_BUFS], (n / C::P_BUFS) & 1, abort_flag, 24, args.wait_ns);
           __syncwarp();
-          if (lane == 0) mbar_arrive(&p_empty[p_buf]);
-          if (warp == 8 && lane == 0) { PROF_TRACE(3, pc, 1); }
-          ++pc;
-          if (++p_buf == C::P_BUFS) {
-            p_buf = 0;
-            p_phase ^= 1u;
+          if (alive && lane == 0) mbar_arrive(&my_empty[n % C::P_BUFS]);
+        }
+        continue;
+      }
+      float2 acc[64];                                 // [piece 4][Piece]
+#pragma unroll
+      for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
+      if (nch > 0) {
+        Piece p0, p1;                                 // one arrives while the other is folded
+        alive = mbar_wait(&my_full[n % C::P_BUFS], (n / C::P_BUFS) & 1, abort_flag, 24, args.wait_ns);
+        if (!alive) break;
+        uint32_t t_acc = t_row + ((2 * n + (uint32_t)half) % C::P_BUFS) * HN;
+        tc_fence_after();
+        tc_ld_piece(t_acc, p0);
+        while (n < n_end) {
+          const uint32_t c = n - n0;
+          const uint32_t slot = (2 * ((it0 + (c >> 1)) % C::FAC_STAGES) + (c & 1)) * C::FAC_STRIDE;
+          const float* fb = fac_b + slot;
+          float ra[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) ra[q] = fac_a[slot + 8 * q];
+          uint64_t* const gone = &my_empty[n % C::P_BUFS];
+          ++n;
+          uint64_t* const next = &my_full[n % C::P_BUFS];
+          // the next chunk's barrier is looked at here, where the answer has time to arrive (a wait on a
+          // barrier that is already complete costs ~150 cycles when the code depends on it at once)
+          const bool ready = __all_sync(0xFFFFFFFFu, mbar_test(next, (n / C::P_BUFS) & 1));
+          tc_wait_piece(p0);
+          tc_ld_piece(t_acc + 32, p1);
+          fold_piece<B_UNIFORM>(acc, p0, ra, fb);
+          tc_wait_piece(p1);
+          tc_ld_piece(t_acc + 64, p0);
+          fold_piece<B_UNIFORM>(acc + 16, p1, ra, fb + 32);
+          tc_wait_piece(p0);
+          tc_ld_piece(t_acc + 96, p1);
+          fold_piece<B_UNIFORM>(acc + 32, p0, ra, fb + 64);
+          tc_wait_piece(p1);              // the chunk has left tensor memory (a warp-wide wait)
+          tc_fence_before();
+          if (lane == 0) mbar_arrive(gone);
+          if (n < n_end) {
+            if (!ready) {
+              alive = mbar_wait(next, (n / C::P_BUFS) & 1, abort_flag, 24, args.wait_ns);
+              if (!alive) break;
+            }
+            t_acc = t_row + ((2 * n + (uint32_t)half) % C::P_BUFS) * HN;
+            tc_fence_after();
+            tc_ld_piece(t_acc, p0);
           }
-          PROF_ADD(7, t0);
-          if (ALTOB200_DBG(args, 64)) continue;   // profiling builds only: chunks are handed straight back
-          t0 = PROF_NOW();
-          fold_cols(acc, p, ra, fb, b_uniform, rb);
-          PROF_ADD(3, t0);
+          fold_piece<B_UNIFORM>(acc + 48, p1, ra, fb + 96);
         }
         if (!alive) break;
       }
-      // ---- epilogue of the tile: this warp's 32 rows x 32 columns ----
-      const long long t_epi = PROF_NOW();
+      // ---- epilogue of the tile: this warp's 32 rows x 128 columns, in units of 16 rows x 128 bytes ----
       const float os = margs.out_scale;
       const int64_t row0 = ti.mb * BM + quad * 32;
-      const int64_t col0 = ti.nb * BN + cq * FC;
-      uint32_t buf;
-      if (out_bf16) {
-        // 64-byte rows (64-byte swizzle: chunk index ^ bits 1-2 of the row), two buffers
-        if (lane == 0) bulk_wait_read<1>();  // the store issued two tiles ago has finished reading this buffer
-        __syncwarp();
-        buf = (store_it & 1u) * 2048u;
-        const uint32_t row = smem_u32(epi_warp) + buf + (uint32_t)lane * 64u;
-        const uint32_t sw = (uint32_t)((lane >> 1) & 3);
+      const int64_t col0 = ti.nb * C::BN + half * HN;
+      const int lr = lane >> 2, lc = lane & 3;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t o[4];
+      for (int q = 0; q < 4; ++q) {
+        if (out_bf16 && (q & 1) != 0) continue;
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float2 v = acc[4 * j + q];
-            const __nv_bfloat162 p2 = __floats2bfloat162_rn(__fmul_rn(v.x, os), __fmul_rn(v.y, os));
-            o[q] = *reinterpret_cast<const uint32_t*>(&p2);
+        for (int rh = 0; rh < 2; ++rh) {
+          if (lane == 0) bulk_wait_read<1>();  // the store issued two units ago has finished reading this buffer
+          __syncwarp();
+          uint8_t* unit = epi_warp + (store_it & 1u) * C::EPI_UNIT;
+          const uint32_t base = smem_u32(unit);
+#pragma unroll
+          for (int g = 0; g < 8; ++g) {                 // column groups of eight: 16 bytes of bf16, 32 of fp32
+            if (!out_bf16 && g >= 4) continue;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {               // row lr + 8 e of the unit
+              const int piece = (q + (g >> 2)) & 3;     // (& 3: the unreachable fp32 case stays inside acc)
+              const float2 v = acc[piece * 16 + rh * 8 + (g & 3) * 2 + e];
+              const uint32_t row = (uint32_t)(lr + 8 * e);
+              const float x = __fmul_rn(v.x, os), y = __fmul_rn(v.y, os);
+              if (out_bf16) {
+                const __nv_bfloat162 p2 = __floats2bfloat162_rn(x, y);
+                st_shared_u32(base + row * 128u + ((((uint32_t)g) ^ (row & 7u)) << 4) + lc * 4u,
+                              *reinterpret_cast<const uint32_t*>(&p2));
+              } else {
+                const uint32_t chunk = (uint32_t)(2 * g) + (uint32_t)(lc >> 1);
+                st_shared_v2(base + row * 128u + ((chunk ^ (row & 7u)) << 4) + (lc & 1) * 8u, f2u(x), f2u(y));
+              }
+            }
           }
-          st_shared_v4(row + ((((uint32_t)j) ^ sw) << 4), o[0], o[1], o[2], o[3]);
-        }
-      } else {
-        // 128-byte rows (128-byte swizzle), one buffer
-        if (lane == 0) bulk_wait_read<0>();
-        __syncwarp();
-        buf = 0u;
-        const uint32_t row = smem_u32(epi_warp) + (uint32_t)lane * 128u;
-        const uint32_t sw = (uint32_t)(lane & 7);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 v0 = acc[2 * j], v1 = acc[2 * j + 1];
-          st_shared_v4(row + ((((uint32_t)j) ^ sw) << 4), f2u(__fmul_rn(v0.x, os)), f2u(__fmul_rn(v0.y, os)),
-                       f2u(__fmul_rn(v1.x, os)), f2u(__fmul_rn(v1.y, os)));
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          const int64_t col = col0 + 32 * q, r0 = row0 + 16 * rh;
+          if (lane == 0) {
+            if (r0 < args.M && col < args.N) tma_store_3d(unit, &tmap_d, (int32_t)col, (int32_t)r0, ti.batch);
+            bulk_commit();  // one group per unit, empty or not: the waits above count groups
+          }
+          ++store_it;
         }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) {
-        if (row0 < args.M && col0 < args.N)
-          tma_store_3d(epi_warp + buf, &tmap_d, (int32_t)col0, (int32_t)row0, ti.batch);
-        bulk_commit();  // one group per tile, empty or not: the waits above count groups
-      }
-      ++store_it;
-      PROF_ADD(5, t_epi);
     }
     if (lane == 0) bulk_wait_all();
-    PROF_ADD(0, t_all);
-    if (warp == 8 && lane == 0) { PROF_FLUSH(3); }
   }
 
   // ------------------------------ teardown ------------------------------

@@ -239,6 +239,13 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t a) {
+  asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(a) : "memory");
+}
+__device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t a, uint32_t b) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
@@ -1269,13 +1276,13 @@ static EncodeTiledFn get_encode_fn() {
 // the 128-byte swizzle, or x 64 bytes with the 64-byte swizzle (epilogues whose column share is not
 // a multiple of 128 bytes).  The batch coordinate keeps a ragged tile of one batch entry out of the next.
 static int make_tmap_out(CUtensorMap* m, void* base, int64_t batches, int64_t M, int64_t N, int64_t ldd, bool bf16,
-                         int row_bytes = 128) {
+                         int row_bytes = 128, int box_rows = 32) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return ALTOB200_ECUDA;
   const int esz = bf16 ? 2 : 4;
   cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)batches};
   cuuint64_t strides[2] = {(cuuint64_t)(ldd * esz), (cuuint64_t)(M * ldd * esz)};
-  cuuint32_t box[3] = {(cuuint32_t)(row_bytes / esz), 32u, 1u};
+  cuuint32_t box[3] = {(cuuint32_t)(row_bytes / esz), (cuuint32_t)box_rows, 1u};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -1537,14 +1544,16 @@ static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N,
 static int launch_gemm_macro(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td,
                              const MacroGemmArgs& margs, cudaStream_t st) {
   using C = CfgMacro;
-  static std::atomic<int> attr_set[MAX_DEVICES];
-  const int rc = ensure_smem_attr(gemm_macro_kernel, C::SMEM_BYTES, attr_set);
+  const bool b_uniform = margs.mb.shift >= 7;   // one B factor per column tile and chunk
+  auto kernel = b_uniform ? gemm_macro_kernel<true> : gemm_macro_kernel<false>;
+  static std::atomic<int> attr_set[2][MAX_DEVICES];
+  const int rc = ensure_smem_attr(kernel, C::SMEM_BYTES, attr_set[b_uniform ? 1 : 0]);
   if (rc != ALTOB200_OK) return rc;
   const GemmArgs& a = margs.g;
   const int64_t tiles = ceil_div(a.M, BM) * ceil_div(a.N, C::BN) * (a.k_offs != nullptr ? a.num_batches : 1);
   int64_t grid = sm_count_gemm();
   if (grid > tiles) grid = tiles;
-  (void)launch_after(gemm_macro_kernel, dim3((unsigned)grid), dim3(NUM_THREADS_MACRO), C::SMEM_BYTES, st, ta, tb, td, margs);
+  (void)launch_after(kernel, dim3((unsigned)grid), dim3(NUM_THREADS_MACRO), C::SMEM_BYTES, st, ta, tb, td, margs);
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }
 
@@ -1575,11 +1584,9 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   CUtensorMap ta, tb, td;
   int rc = make_tmap(&ta, a_codes, M, k_bytes, BM);
   if (rc != ALTOB200_OK) return rc;
-  rc = make_tmap(&tb, b_codes, b_rows, k_bytes, CfgMacro::BN);
+  rc = make_tmap(&tb, b_codes, b_rows, k_bytes, CfgMacro::HN);
   if (rc != ALTOB200_OK) return rc;
-  // a fold warp stores 32 columns per row: 64 bytes of bf16 (64-byte swizzle) or 128 bytes of fp32
-  rc = make_tmap_out(&td, d, k_offs != nullptr ? num_experts : 1, M, N, ldd, out_dtype == ALTOB200_DT_BF16,
-                     out_dtype == ALTOB200_DT_BF16 ? 64 : 128);
+  rc = make_tmap_out(&td, d, k_offs != nullptr ? num_experts : 1, M, N, ldd, out_dtype == ALTOB200_DT_BF16, 128, 16);
   if (rc != ALTOB200_OK) return rc;
 
   MacroGemmArgs m;
@@ -1601,7 +1608,7 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   }
   g.wait_ns = wait_limit_ns();
   for (int j = 0; j < 4; ++j)
-    g.idesc[j] = make_idesc(KIND_MXF4, ALTOB200_FMT_MXFP4, ALTOB200_FMT_MXFP4, BM, CfgMacro::BN, (j & 1) * 2);
+    g.idesc[j] = make_idesc(KIND_MXF4, ALTOB200_FMT_MXFP4, ALTOB200_FMT_MXFP4, BM, CfgMacro::HN, (j & 1) * 2);
 #ifdef ALTOB200_GEMM_PROFILE
   {
     const char* e = getenv("ALTOB200_GEMM_DEBUG");
@@ -1613,12 +1620,6 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   m.mb.codes = b_macro->codes; m.mb.row_stride = b_macro->row_stride; m.mb.chunk_stride = b_macro->chunk_stride;
   m.mb.expert_stride = row_groups ? b_macro->expert_stride : 0; m.mb.shift = b_macro->row_shift;
   m.out_scale = out_scale;
-#ifdef ALTOB200_GEMM_PROFILE
-  {
-    const char* e = getenv("ALTOB200_MACRO_PROF_PTR");  // device address of the clock table, set by the probe script
-    m.prof = e ? reinterpret_cast<unsigned long long*>(strtoull(e, nullptr, 0)) : nullptr;
-  }
-#endif
   return launch_gemm_macro(ta, tb, td, m, (cudaStream_t)stream);
 }
 
