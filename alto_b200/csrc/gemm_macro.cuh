@@ -22,7 +22,7 @@
 //                 factors: the codes of the tile's rows (and columns) for the next stage's two chunks are read
 //                 a stage ahead and their reciprocals left in a shared-memory ring;
 //   warpgroups 2-3  fold + epilogue of one half each: four warps, one per tensor-memory lane quarter, 32 rows
-//                 x 128 columns in 128 registers per thread.  A chunk is read in four pieces of 32 columns,
+//                 x 128 columns in 128 registers per thread.  A chunk is read in eight pieces of 16 columns,
 //                 and one piece is always on its way from tensor memory while another is folded:
 //                 acc += P * (1/fa[row]) * (1/fb[col]) in packed fp32x2 arithmetic.  After the last chunk the
 //                 registers are scaled, converted, staged and TMA-stored.
@@ -31,10 +31,12 @@
 // scales), then the fold itself, 64 (128 with per-column factors) packed operations of two cycles per scheduler
 // and 128 x 128 x 128 block whose MMAs take 128 cycles, then the shared-memory port: with 128 x 128 tiles, whose
 // operands are 17 KB of loads per block against 13 here, loading alone took 284 cycles per block.
-// Measured at 8192 x 4096 x 14336, one factor per tile of B / one per column: 476 / 694 us; with 128 x 128
+// Measured at 8192 x 4096 x 14336, one factor per tile of B / one per column: 455 / 571 us; with 128 x 128
 // tiles, sixteen fold warps of 32 columns that each looked up their factors, and one issuer: 572 / 924 us.
-// The warpgroups re-divide the register file with setmaxnreg (512 threads x 128 at launch -> 40 for the
-// small roles, 216 for the fold warps; the two must balance exactly, see CfgMacro).
+// (Pieces of 32 columns: 449 / 631 us - a few spilled registers more in the chunk loop, local memory that this
+// kernel's small L1 does not hold.)
+// The warpgroups re-divide the register file with setmaxnreg (512 threads x 128 at launch -> 56 for the
+// small roles, 200 for the fold warps; the two must balance exactly, see CfgMacro).
 // Rows grouped by expert (`group_expert`) and K ranges per batch entry (`k_offs`) work as in the
 // plain kernel; every K range starts on a multiple of 128 elements, so chunks never straddle one.
 #pragma once
@@ -94,7 +96,7 @@ struct CfgMacro {
   // registers per thread (65536 / 512); setmaxnreg.inc can only take what setmaxnreg.dec has released
   // INSIDE the CTA and blocks for ever otherwise, so the two must balance exactly.
   static constexpr int REGS_LAUNCH = 128;
-  static constexpr int REGS_SMALL = 40, REGS_FOLD = 216;
+  static constexpr int REGS_SMALL = 56, REGS_FOLD = 200;
   static_assert(2 * 128 * REGS_SMALL + 2 * 128 * REGS_FOLD == NUM_THREADS_MACRO * REGS_LAUNCH,
                 "setmaxnreg budget must balance");
   static_assert(NUM_THREADS_MACRO == (8 + FOLD_WARPS) * 32, "role layout");
@@ -133,23 +135,22 @@ __device__ __forceinline__ MacroTile decode_macro_tile(const GemmArgs& args, int
   return m;
 }
 
-// One piece of a chunk accumulator: 32 columns of a warp's 32 rows, as two tensor-memory loads of 16 rows in
+// One piece of a chunk accumulator: 16 columns of a warp's 32 rows, as two tensor-memory loads of 16 rows in
 // the 16 x 256-bit layout.  A lane gets, per group of eight columns, columns 2 (lane % 4) and + 1 of rows
-// lane / 4 and + 8 of each load: four rows and eight columns of the piece, so that it needs twelve factors,
-// where the layout of one row per lane needs 33 and the broadcast of the column factors out of shared memory
+// lane / 4 and + 8 of each load: four rows and four columns of the piece, so that it needs eight factors,
+// where the layout of one row per lane needs 17 and the broadcast of the column factors out of shared memory
 // (128 bytes per register and warp) took longer than the multiply-adds.
 struct Piece {
-  uint32_t r[32];   // [row half 2][column group 4][row 2][column 2]
+  uint32_t r[16];   // [row half 2][column group 2][row 2][column 2]
 };
 __device__ __forceinline__ void tc_ld_piece(uint32_t taddr, Piece& p) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    uint32_t* r = p.r + 16 * h;
+    uint32_t* r = p.r + 8 * h;
     asm volatile(
-        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        "tcgen05.ld.sync.aligned.16x256b.x2.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
         : "r"(taddr + ((uint32_t)(16 * h) << 16))
         : "memory");
   }
@@ -159,40 +160,54 @@ __device__ __forceinline__ void tc_wait_piece(Piece& p) {
 #define ALTOB200_RW8(o) "+r"(p.r[o]), "+r"(p.r[o + 1]), "+r"(p.r[o + 2]), "+r"(p.r[o + 3]), "+r"(p.r[o + 4]), \
                         "+r"(p.r[o + 5]), "+r"(p.r[o + 6]), "+r"(p.r[o + 7])
   asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : ALTOB200_RW8(0), ALTOB200_RW8(8), ALTOB200_RW8(16), ALTOB200_RW8(24)
+               : ALTOB200_RW8(0), ALTOB200_RW8(8)
                :
                : "memory");
 #undef ALTOB200_RW8
 }
-// acc += P * ra[row] * fb[col]; B_UNIFORM: one B factor for the half and chunk, already multiplied into ra.
-// `acc` and `p` are laid out alike; fb points at this lane's first column.
-template <bool B_UNIFORM>
-__device__ __forceinline__ void fold_piece(float2* acc, const Piece& p, const float (&ra)[4], const float* fb) {
-#pragma unroll
-  for (int g = 0; g < 4; ++g) {
-    float2 f = make_float2(1.0f, 1.0f);
-    if (!B_UNIFORM) f = *reinterpret_cast<const float2*>(fb + 8 * g);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {   // row half q / 2, row 8 (q % 2)
-      const int i = (q >> 1) * 8 + g * 2 + (q & 1);
-      float2 w = make_float2(ra[q], ra[q]);
-      if (!B_UNIFORM) w = __fmul2_rn(w, f);
-      acc[i] = __ffma2_rn(make_float2(u2f(p.r[2 * i]), u2f(p.r[2 * i + 1])), w, acc[i]);
-    }
-  }
+__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float2 ld_shared_f32x2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint64_t* generic_bar(uint32_t addr) {
+  return reinterpret_cast<uint64_t*>(__cvta_shared_to_generic(addr));
 }
 
 // One look at a barrier's phase, without waiting.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
+}
+
+// acc += P * ra[row] * fb[col]; B_UNIFORM: one B factor for the half and chunk, already multiplied into ra.
+// `acc` and `p` are laid out alike; fb: shared-memory address of this lane's first column factor.
+template <bool B_UNIFORM>
+__device__ __forceinline__ void fold_piece(float2* acc, const Piece& p, const float (&ra)[4], uint32_t fb) {
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    float2 f = make_float2(1.0f, 1.0f);
+    if (!B_UNIFORM) f = ld_shared_f32x2(fb + 32 * g);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {   // row half q / 2, row 8 (q % 2)
+      const int i = (q >> 1) * 4 + g * 2 + (q & 1);
+      float2 w = make_float2(ra[q], ra[q]);
+      if (!B_UNIFORM) w = __fmul2_rn(w, f);
+      acc[i] = __ffma2_rn(make_float2(u2f(p.r[2 * i]), u2f(p.r[2 * i + 1])), w, acc[i]);
+    }
+  }
 }
 
 // B_UNIFORM: B's macro blocks are 128 x 128 tiles (one factor per half and chunk), else per column.
@@ -444,84 +459,114 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   } else {
     // ------------------------------ fold + epilogue ------------------------------
     setmaxnreg_inc<C::REGS_FOLD>();
+    // Of the 200 registers, 160 are accumulators and pieces in flight: what else lives across the chunk loop is
+    // kept in 32 bits (shared-memory addresses, tile numbers; the output of 2^31 tiles would not fit any memory).
     const int quad = warp & 3;                        // tensor-memory lane quarter this warp may read
     const int half = (warp - 8) >> 2;                 // columns [128 half, 128 half + 128) of the tile
-    uint8_t* epi_warp = epi + (warp - 8) * C::EPI_WARP_BYTES;
-    const bool out_bf16 = args.out_bf16 != 0;
     const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
     // this lane's first row and column factor in a chunk's slot
-    const float* fac_a = fac + (B_UNIFORM ? half * HN : 0) + quad * 32 + (lane >> 2);
-    const float* fac_b = fac + BM + half * HN + 2 * (lane & 3);
-    uint64_t* const my_full = p_full + half * C::P_BUFS;
-    uint64_t* const my_empty = p_empty + half * C::P_BUFS;
-    uint32_t store_it = 0, it = 0, n = 0;             // store units, stages and chunks so far
+    const uint32_t fac_a = smem_u32(fac) + 4u * (uint32_t)((B_UNIFORM ? half * HN : 0) + quad * 32 + (lane >> 2));
+    const uint32_t fac_b = smem_u32(fac) + 4u * (uint32_t)(BM + half * HN + 2 * (lane & 3));
+    const uint32_t my_full = smem_u32(p_full + half * C::P_BUFS), my_empty = smem_u32(p_empty + half * C::P_BUFS);
+    uint32_t store_it = 0;                            // store units so far
+    uint32_t slot = 0;                                // byte offset of the chunk's factors, always of an even slot at a tile's start
+    // ring positions of the half's next chunk: its barriers (n % 3), their phase, its accumulator ((2 n + half) % 3)
+    uint32_t ring = 0, phase = 0, acc_i = (uint32_t)half;
+    constexpr uint32_t SLOT_BYTES = C::FAC_STRIDE * 4, SLOTS_END = 2 * C::FAC_STAGES * SLOT_BYTES;
     bool alive = true;
-    for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
-      const MacroTile mt = decode_macro_tile(args, tile, tiles_m, tiles_n, k_stages);
-      const TileInfo& ti = mt.t;
-      const int nch = ti.skip ? 0 : mt.n_chunks;
-      const uint32_t n_end = n + (uint32_t)nch, n0 = n, it0 = it;
-      it += ti.skip ? 0u : (uint32_t)ti.k_stages;
-      if (half >= mt.halves) {                        // nothing to read, only the hand-over
-        for (; n < n_end && alive; ++n) {
-          alive = mbar_wait(&my_full[n % C::P_BUFS], (n / C::P_BUFS) & 1, abort_flag, 24, args.wait_ns);
-          __syncwarp();
-          if (alive && lane == 0) mbar_arrive(&my_empty[n % C::P_BUFS]);
-        }
-        continue;
+    for (int tile = (int)blockIdx.x; tile < (int)n_tiles && alive; tile += (int)gridDim.x) {
+      int left, row0, col0, batch;                    // chunks left, this warp's part of the output
+      bool mine;
+      {
+        const MacroTile mt = decode_macro_tile(args, tile, tiles_m, tiles_n, k_stages);
+        left = mt.t.skip ? 0 : mt.n_chunks;
+        mine = half < mt.halves;
+        row0 = (int)mt.t.mb * BM + quad * 32;
+        col0 = (int)mt.t.nb * C::BN + half * HN;
+        batch = mt.t.batch;
       }
-      float2 acc[64];                                 // [piece 4][Piece]
+      auto step = [&]() {
+        if (++ring == C::P_BUFS) {
+          ring = 0;
+          phase ^= 1u;
+        }
+        acc_i = acc_i == 0u ? 2u : acc_i - 1u;        // + 2 mod 3
+        slot = slot + SLOT_BYTES == SLOTS_END ? 0u : slot + SLOT_BYTES;
+      };
+      float2 acc[64];                                 // [piece 8][Piece]
 #pragma unroll
       for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
-      if (nch > 0) {
-        Piece p0, p1;                                 // one arrives while the other is folded
-        alive = mbar_wait(&my_full[n % C::P_BUFS], (n / C::P_BUFS) & 1, abort_flag, 24, args.wait_ns);
+      const bool odd = (left & 1) != 0;
+      if (left > 0) {
+        alive = mbar_wait(generic_bar(my_full + 8 * ring), phase, abort_flag, 24, args.wait_ns);
         if (!alive) break;
-        uint32_t t_acc = t_row + ((2 * n + (uint32_t)half) % C::P_BUFS) * HN;
+      }
+      if (!mine) {                                    // nothing to read, only the hand-over
+        while (left > 0 && alive) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(generic_bar(my_empty + 8 * ring));
+          step();
+          if (--left > 0) alive = mbar_wait(generic_bar(my_full + 8 * ring), phase, abort_flag, 24, args.wait_ns);
+        }
+      } else if (left > 0) {
+        Piece p0, p1;                                 // one arrives while the other is folded
+        uint32_t t_acc = t_row + acc_i * HN;
         tc_fence_after();
         tc_ld_piece(t_acc, p0);
-        while (n < n_end) {
-          const uint32_t c = n - n0;
-          const uint32_t slot = (2 * ((it0 + (c >> 1)) % C::FAC_STAGES) + (c & 1)) * C::FAC_STRIDE;
-          const float* fb = fac_b + slot;
+        while (true) {
+          const uint32_t fb = fac_b + slot;
           float ra[4];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) ra[q] = fac_a[slot + 8 * q];
-          uint64_t* const gone = &my_empty[n % C::P_BUFS];
-          ++n;
-          uint64_t* const next = &my_full[n % C::P_BUFS];
+          for (int q = 0; q < 4; ++q) ra[q] = ld_shared_f32(fac_a + slot + 32 * q);
+          const uint32_t gone = my_empty + 8 * ring;
+          step();
           // the next chunk's barrier is looked at here, where the answer has time to arrive (a wait on a
           // barrier that is already complete costs ~150 cycles when the code depends on it at once)
-          const bool ready = __all_sync(0xFFFFFFFFu, mbar_test(next, (n / C::P_BUFS) & 1));
+          const bool ready = __all_sync(0xFFFFFFFFu, mbar_test(my_full + 8 * ring, phase));
           tc_wait_piece(p0);
-          tc_ld_piece(t_acc + 32, p1);
-          fold_piece<B_UNIFORM>(acc, p0, ra, fb);
+          tc_ld_piece(t_acc + 16, p1);
+          fold_piece<B_UNIFORM>(acc + 0, p0, ra, fb + 0);
+          tc_wait_piece(p1);
+          tc_ld_piece(t_acc + 32, p0);
+          fold_piece<B_UNIFORM>(acc + 8, p1, ra, fb + 64);
+          tc_wait_piece(p0);
+          tc_ld_piece(t_acc + 48, p1);
+          fold_piece<B_UNIFORM>(acc + 16, p0, ra, fb + 128);
           tc_wait_piece(p1);
           tc_ld_piece(t_acc + 64, p0);
-          fold_piece<B_UNIFORM>(acc + 16, p1, ra, fb + 32);
+          fold_piece<B_UNIFORM>(acc + 24, p1, ra, fb + 192);
           tc_wait_piece(p0);
-          tc_ld_piece(t_acc + 96, p1);
-          fold_piece<B_UNIFORM>(acc + 32, p0, ra, fb + 64);
+          tc_ld_piece(t_acc + 80, p1);
+          fold_piece<B_UNIFORM>(acc + 32, p0, ra, fb + 256);
+          tc_wait_piece(p1);
+          tc_ld_piece(t_acc + 96, p0);
+          fold_piece<B_UNIFORM>(acc + 40, p1, ra, fb + 320);
+          tc_wait_piece(p0);
+          tc_ld_piece(t_acc + 112, p1);
+          fold_piece<B_UNIFORM>(acc + 48, p0, ra, fb + 384);
           tc_wait_piece(p1);              // the chunk has left tensor memory (a warp-wide wait)
           tc_fence_before();
-          if (lane == 0) mbar_arrive(gone);
-          if (n < n_end) {
+          if (lane == 0) mbar_arrive(generic_bar(gone));
+          if (--left > 0) {
             if (!ready) {
-              alive = mbar_wait(next, (n / C::P_BUFS) & 1, abort_flag, 24, args.wait_ns);
+              alive = mbar_wait(generic_bar(my_full + 8 * ring), phase, abort_flag, 24, args.wait_ns);
               if (!alive) break;
             }
-            t_acc = t_row + ((2 * n + (uint32_t)half) % C::P_BUFS) * HN;
+            t_acc = t_row + acc_i * HN;
             tc_fence_after();
             tc_ld_piece(t_acc, p0);
           }
-          fold_piece<B_UNIFORM>(acc + 48, p1, ra, fb + 96);
+          fold_piece<B_UNIFORM>(acc + 56, p1, ra, fb + 448);
+          if (left == 0) break;
         }
-        if (!alive) break;
       }
+      if (!alive) break;
+      if (odd) slot = slot + SLOT_BYTES == SLOTS_END ? 0u : slot + SLOT_BYTES;   // a stage has two slots
+      if (!mine) continue;
       // ---- epilogue of the tile: this warp's 32 rows x 128 columns, in units of 16 rows x 128 bytes ----
       const float os = margs.out_scale;
-      const int64_t row0 = ti.mb * BM + quad * 32;
-      const int64_t col0 = ti.nb * C::BN + half * HN;
+      const bool out_bf16 = args.out_bf16 != 0;
+      uint8_t* epi_warp = epi + (warp - 8) * C::EPI_WARP_BYTES;
       const int lr = lane >> 2, lc = lane & 3;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -537,8 +582,8 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             if (!out_bf16 && g >= 4) continue;
 #pragma unroll
             for (int e = 0; e < 2; ++e) {               // row lr + 8 e of the unit
-              const int piece = (q + (g >> 2)) & 3;     // (& 3: the unreachable fp32 case stays inside acc)
-              const float2 v = acc[piece * 16 + rh * 8 + (g & 3) * 2 + e];
+              const int cg = (q * 4 + g) & 15;          // (& 15: the unreachable fp32 case stays inside acc)
+              const float2 v = acc[(cg >> 1) * 8 + rh * 4 + (cg & 1) * 2 + e];
               const uint32_t row = (uint32_t)(lr + 8 * e);
               const float x = __fmul_rn(v.x, os), y = __fmul_rn(v.y, os);
               if (out_bf16) {
@@ -553,9 +598,9 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
-          const int64_t col = col0 + 32 * q, r0 = row0 + 16 * rh;
+          const int col = col0 + 32 * q, r0 = row0 + 16 * rh;
           if (lane == 0) {
-            if (r0 < args.M && col < args.N) tma_store_3d(unit, &tmap_d, (int32_t)col, (int32_t)r0, ti.batch);
+            if (r0 < args.M && col < args.N) tma_store_3d(unit, &tmap_d, col, r0, batch);
             bulk_commit();  // one group per unit, empty or not: the waits above count groups
           }
           ++store_it;
