@@ -140,7 +140,8 @@ __device__ __forceinline__ void nvfp4_block_scale(float amax, bool use_outer, fl
 // with r = RN(1/q) returns the correctly rounded quotient (checked exhaustively over all
 // 2^7 numerator and 2^23 denominator mantissas); it needs q and the quotient to stay away
 // from the subnormal range, which callers guarantee by testing q once per block
-// (`div_fast_ok`).  The sign of x is copied so that -0.0 keeps its sign bit as IEEE
+// (`div_fast_ok`).  Written with e negated - e = fma(y, q, -x), y' = fma(-r, e, y), the same roundings -
+// it also keeps the sign of a zero x (y is that zero, and an exact e is +0, so -r * e is -0), as IEEE
 // division does (the reference ORs that sign into the code, triton_fp4_ops.py:40-41,90-92).
 // ---------------------------------------------------------------------------------------
 __device__ __forceinline__ bool div_fast_ok(float q) {
@@ -149,15 +150,8 @@ __device__ __forceinline__ bool div_fast_ok(float q) {
 }
 __device__ __forceinline__ float div_bf16_num(float x, float q, float r) {
   const float y = __fmul_rn(x, r);
-  const float e = __fmaf_rn(-y, q, x);
-  const float y2 = __fmaf_rn(e, r, y);
-  return u2f((f2u(y2) & 0x7FFFFFFFu) | (f2u(x) & 0x80000000u));
-}
-// The same quotient up to the sign of a zero (for callers that take the sign from x).
-__device__ __forceinline__ float div_bf16_num_mag(float x, float q, float r) {
-  const float y = __fmul_rn(x, r);
-  const float e = __fmaf_rn(-y, q, x);
-  return __fmaf_rn(e, r, y);
+  const float e = __fmaf_rn(y, q, -x);
+  return __fmaf_rn(-r, e, y);
 }
 
 // x / 6 for a normal x whose quotient and residual stay normal (callers keep |x| in [2^-91, 2^120) or
@@ -185,42 +179,72 @@ __device__ __forceinline__ uint32_t e2m1x2_rtn_hw(float v0, float v1) {
       : "f"(v1), "f"(v0));
   return (uint32_t)r;
 }
+// Eight floats -> four bytes, element 0 in the lowest nibble: the converters write into the bytes of one
+// register, nothing is shifted or merged.
+__device__ __forceinline__ uint32_t e2m1x8_rtn_hw(const float* v) {
+  uint32_t r;
+  asm("{\n\t.reg .b8 t0, t1, t2, t3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 t0, %2, %1;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 t1, %4, %3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 t2, %6, %5;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 t3, %8, %7;\n\t"
+      "mov.b32 %0, {t0, t1, t2, t3};\n\t}"
+      : "=r"(r)
+      : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
+  return r;
+}
 
 // ---------------------------------------------------------------------------------------
 // E2M1 encode with stochastic rounding from 32 random bits.  Restatement of
 //   alto/kernels/fp4/fp4_common/triton_fp4_ops.py:26-93 with USE_SR=True.
 // ---------------------------------------------------------------------------------------
-// Arranged for instruction count (the stochastic-rounding quantizers are bound by instruction
-// issue, not by memory).  The reference rounds the normal range [1, 6) by adding 22 random bits
-// below the kept mantissa bit and truncating; in the E2M1-subnormal range [0, 1), with 2a = k + frac,
-// it compares the random word with uint32(a * fp32(2^33 - 2)) for a < 0.5 and with
-// uint32((2a - 1) * fp32(2^32 - 1)) otherwise; both constants round to powers of two in fp32, so
-// both thresholds are trunc(frac * 2^32) and the code is k + [rnd <= threshold].
-// `v` is the scaled value up to the sign of a zero; the sign
-// bit of the code is taken from `sign_bits` (the bits of the unscaled element: scales are positive).
+// The reference rounds the normal range [1, 6) by adding 22 random bits below the kept mantissa bit and
+// truncating; in the E2M1-subnormal range [0, 1), with 2a = k + frac, it compares the random word with
+// uint32(a * fp32(2^33 - 2)) for a < 0.5 and with uint32((2a - 1) * fp32(2^32 - 1)) otherwise; both
+// constants round to powers of two in fp32, so both thresholds are trunc(frac * 2^32) and the code is
+// k + [rnd <= threshold].
+//
+// The general form (any v; the quantizers use it for blocks that hold an infinity or a NaN, or whose scale
+// rules out the reciprocal division).  `v` is the scaled value up to the sign of a zero; the sign bit of the
+// code is taken from `sign_bits` (the bits of the unscaled element: scales are positive).
 // With a = min(|v|, 6):
 //   normal range   code = (bits(a) + (rnd & (2^22 - 1)) - (126 << 23)) >> 22: the carry out of the low
 //                  22 mantissa bits rounds up, and 6.0 itself maps to 7, so saturation needs no
 //                  separate test;
 //   a < 1          with T = trunc(a * 2^33) = k * 2^32 + threshold (k = [a >= 0.5]),
-//                  code = hi32(T + 1 + ~rnd) = k + [rnd <= threshold].
+//                  code = T.hi + [T.lo >= rnd].
 // A NaN saturates to 7 (the reference's code for a NaN element is an accident of its payload).
-// COMPARE selects how the sub-one threshold is evaluated (same value): the 64-bit carry form above, or
-// T.hi + [T.lo >= rnd]; the row-wise kernel is faster with the compare, the column-wise one with the carry.
-template <bool COMPARE = false>
 __device__ __forceinline__ uint32_t e2m1_sr_code(float v, uint32_t sign_bits, uint32_t rnd) {
   const float a = fminf(fabsf(v), 6.0f);
   const uint32_t ab = f2u(a);
   const uint32_t cn = (ab + (rnd & 0x3FFFFFu) - (126u << 23)) >> 22;
   const uint64_t t = __float2ull_rz(__fmul_rn(a, 8589934592.0f));
-  // hi32(T + 1 + ~rnd) = hi32(T + 2^32 - rnd) = T.hi + [T.lo >= rnd]
-  const uint32_t cd = COMPARE ? (uint32_t)(t >> 32) + ((uint32_t)t >= rnd ? 1u : 0u)
-                              : (uint32_t)((t + 1ull + (uint64_t)(~rnd)) >> 32);
-  const uint32_t mag = a < 1.0f ? cd : cn;
-  // sign into bit 3 with one shift and one multiply-add (disjoint bits): the ALU pipe is the busy one
-  uint32_t r;
-  asm("mad.lo.u32 %0, %1, 8, %2;" : "=r"(r) : "r"(sign_bits >> 31), "r"(mag));
-  return r;
+  const uint32_t cd = (uint32_t)(t >> 32) + ((uint32_t)t >= rnd ? 1u : 0u);
+  return ((sign_bits >> 31) << 3) | (a < 1.0f ? cd : cn);
+}
+
+// The same for finite v whose zeros carry their sign, as the VALUE of the code (which the hardware converter
+// then packs with its neighbours), without selects, shifts or integer conversions of v - the quantizers are
+// bound by the integer pipe, whose compares, selects, shifts and permutes take two cycles a warp and its
+// 64-bit float conversion eight:
+//   a < 1    [rnd <= threshold] is a >= rnd * 2^-33 (plus 0.5 when k = 1), and since a and a - 0.5 are fp32
+//            numbers, rnd may first be rounded UP to fp32.  With t = RZ(a - u), u = RU(rnd) * 2^-33, whose
+//            rounding towards zero never moves it across 0 or 0.5, the value is (floor(2t) + 1) / 2: the
+//            round-down multiply-add with 1.5 * 2^23 is floor(2t), and saturating the rest at 1 makes it 1 for
+//            every a >= 1 (u <= 0.5, so t >= 0.5 there);
+//   a >= 1   (bits(v) + 22 random bits) with the low bits cut is the rounded value; what it exceeds 1 by is
+//            added (saturated at 8, which the converter saturates to 6); below 1 there is no excess.
+// Bit for bit the code of e2m1_sr_code.
+__device__ __forceinline__ float e2m1_sr_value(float v, uint32_t rnd) {
+  const float u = __uint2float_ru(rnd);
+  const float t = __fmaf_rz(u, -1.16415321826934814453125e-10f, fabsf(v));
+  const float g = __fmaf_rd(t, 2.0f, 12582912.0f);
+  float below, above;
+  asm("fma.rn.sat.f32 %0, %1, 0f3F000000, %2;" : "=f"(below) : "f"(g), "f"(-6291455.5f));
+  const uint32_t n = (f2u(v) + (rnd & 0x3FFFFFu)) & 0x7FC00000u;
+  asm("fma.rn.sat.f32 %0, %1, 0f3E000000, 0fBE000000;" : "=f"(above) : "f"(u2f(n)));
+  const float w = __fmaf_rn(above, 8.0f, below);
+  return u2f(f2u(w) | (f2u(v) & 0x80000000u));
 }
 
 // E2M1 decode to fp32 (alto/kernels/fp4/fp4_common/triton_fp4_ops.py:100-132).

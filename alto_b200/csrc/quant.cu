@@ -97,7 +97,7 @@ __device__ __forceinline__ BlockScale make_block_scale(uint32_t amax_abs_bits, c
     // (exact, see div_bf16_num and div_by_6); everything else divides
     const uint32_t e8 = amax_abs_bits >> 7;
     if (IN_BF16 && (amax_abs_bits == 0u || (e8 >= 97u && e8 < 187u)) && (!os.use || os.fast)) {
-      const float t = os.use ? div_bf16_num_mag(amax, os.v, os.r) : amax;
+      const float t = os.use ? div_bf16_num(amax, os.v, os.r) : amax;
       nvfp4_block_scale_from_raw(div_by_6(t), os.use, os.v, &s.plain, &s.q, &s.byte);
     } else {
       nvfp4_block_scale(amax, os.use, os.v, &s.plain, &s.q, &s.byte);
@@ -186,14 +186,9 @@ __device__ __forceinline__ uint32_t merge_shifted(uint32_t x, int sh, uint32_t a
 // The scaled element up to the sign of a zero (the stochastic-rounding encoder takes the sign from x).
 template <int FMT, bool IN_BF16, bool FAST>
 __device__ __forceinline__ float scale_elem_mag(float x, const BlockScale& s) {
-  if (!FAST) return __fdiv_rn(x, s.q);
-  if (Fmt<FMT>::MX) return __fmul_rn(x, s.r);
-  return div_bf16_num_mag(x, s.q, s.r);
+  return scale_elem<FMT, IN_BF16, FAST>(x, s);
 }
 
-// Two elements of two different blocks divided by their block scales at once (reciprocal forms only;
-// magnitudes up to the sign of a zero, as scale_elem_mag): x * r for the power-of-two scales of the MX
-// formats, else y = x r, e = fma(y, -q, x), y + e r - the three roundings of div_bf16_num_mag per element.
 template <int FMT>
 __device__ __forceinline__ float2 scale_pair_mag(float2 x, const BlockScale& s0, const BlockScale& s1) {
   const float2 r = make_float2(s0.r, s1.r);
@@ -203,16 +198,30 @@ __device__ __forceinline__ float2 scale_pair_mag(float2 x, const BlockScale& s0,
   return __ffma2_rn(e, r, y);
 }
 
-// Scale and quantise 2 elements into one FP4 byte (x0 in the low nibble).
+// Eight elements of one block scaled and quantised into four FP4 bytes (element 0 in the lowest nibble).
+// SR words: r0[j] for element 2j, r1[j] for element 2j + 1; FAST also means that the elements are finite.
 template <int FMT, bool IN_BF16, int ROUND, bool FAST>
-__device__ __forceinline__ uint32_t fp4_pair(float x0, float x1, const BlockScale& s, uint32_t r0, uint32_t r1) {
-  if (ROUND == ALTOB200_ROUND_RTN)
-    return e2m1x2_rtn_hw(scale_elem<FMT, IN_BF16, FAST>(x0, s), scale_elem<FMT, IN_BF16, FAST>(x1, s));
-  // codes are merged with multiply-adds (disjoint bits: adding is or-ing): the integer ALU is the
-  // busiest pipe of these kernels and the multiply-add pipe has room
-  const uint32_t c0 = e2m1_sr_code<true>(scale_elem_mag<FMT, IN_BF16, FAST>(x0, s), f2u(x0), r0);
-  const uint32_t c1 = e2m1_sr_code<true>(scale_elem_mag<FMT, IN_BF16, FAST>(x1, s), f2u(x1), r1);
-  return merge_shifted(c1, 4, c0);
+__device__ __forceinline__ uint32_t fp4_octet(const float* x, const BlockScale& s, const uint32_t* r0, const uint32_t* r1) {
+  float q[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) q[j] = scale_elem<FMT, IN_BF16, FAST>(x[j], s);
+  if (ROUND == ALTOB200_ROUND_RTN) return e2m1x8_rtn_hw(q);
+  if (FAST) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) q[j] = e2m1_sr_value(q[j], (j & 1) ? r1[j >> 1] : r0[j >> 1]);
+    return e2m1x8_rtn_hw(q);
+  }
+  uint32_t word = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    word = merge_shifted(e2m1_sr_code(q[j], f2u(x[j]), (j & 1) ? r1[j >> 1] : r0[j >> 1]), 4 * j, word);
+  return word;
+}
+
+// Whether a block may take the reciprocal forms: with stochastic rounding only without infinities and NaNs.
+template <bool IN_BF16, int ROUND>
+__device__ __forceinline__ bool block_fast(const BlockScale& s, uint32_t amax_abs_bits) {
+  return s.fast && (ROUND == ALTOB200_ROUND_RTN || amax_abs_bits < (IN_BF16 ? 0x7F80u : 0x7F800000u));
 }
 
 // Runs body(std::true_type) when every lane of the warp may use the reciprocal forms, else
@@ -238,6 +247,10 @@ __device__ __forceinline__ void divmod_fast(int64_t t, int64_t d, int64_t* q, in
 
 __device__ __forceinline__ uint32_t absmax_bf16x2(uint32_t acc, uint32_t w) {
   return __vmaxu2(acc, w & 0x7FFF7FFFu);
+}
+// maximum over two words at once (one three-input instruction)
+__device__ __forceinline__ uint32_t absmax2_bf16x2(uint32_t acc, uint32_t w0, uint32_t w1) {
+  return __vimax3_u16x2(acc, w0 & 0x7FFF7FFFu, w1 & 0x7FFF7FFFu);
 }
 __device__ __forceinline__ uint32_t fold_bf16x2(uint32_t acc) {
   const uint32_t lo = acc & 0xFFFFu, hi = acc >> 16;
@@ -315,6 +328,8 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
     }
     const int64_t kb = (chunk << 9) / F::B + lane / LPB;  // scale column of this lane
     const bool holder = col_ok && (lane % LPB == 0);
+    static_assert(ROW_R == 4, "the packed scales are transposed four rows at a time");
+    uint32_t scale_bytes = 0;   // byte i: scale of row i
 
 #pragma unroll
     for (int i = 0; i < ROW_R; ++i) {
@@ -363,7 +378,7 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
         uint32_t acc = 0;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          acc = absmax_bf16x2(acc, w[j]);
+          if (j & 1) acc = absmax2_bf16x2(acc, w[j - 1], w[j]);
           v[2 * j] = bf16lo_to_f32(w[j]);
           v[2 * j + 1] = bf16hi_to_f32(w[j]);
         }
@@ -408,16 +423,11 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
       }
 
       // ---- encode and store ----
-      with_uniform_fast(s.fast, [&](auto fast_tag) {
+      with_uniform_fast(block_fast<IN_BF16, ROUND>(s, amax_bits), [&](auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
         if (F::FP4) {
-          uint32_t lo = 0, hi = 0;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            lo = merge_shifted(fp4_pair<FMT, IN_BF16, ROUND, FAST>(v[2 * j], v[2 * j + 1], s, r0[j], r1[j]), 8 * j, lo);
-            hi = merge_shifted(fp4_pair<FMT, IN_BF16, ROUND, FAST>(v[8 + 2 * j], v[9 + 2 * j], s, r0[4 + j], r1[4 + j]),
-                               8 * j, hi);
-          }
+          const uint32_t lo = fp4_octet<FMT, IN_BF16, ROUND, FAST>(v, s, r0, r1);
+          const uint32_t hi = fp4_octet<FMT, IN_BF16, ROUND, FAST>(v + 8, s, r0 + 4, r1 + 4);
           if (active) *reinterpret_cast<uint2*>(a.codes + row * half_cols + (col >> 1)) = make_uint2(lo, hi);
         } else {
           uint32_t o[4];
@@ -437,13 +447,19 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
         if (F::MX) reinterpret_cast<uint8_t*>(a.scale_plain)[row * nkb + kb] = (uint8_t)s.byte;
         else reinterpret_cast<float*>(a.scale_plain)[row * nkb + kb] = s.plain;
       }
-      if (a.scale_packed != nullptr) {
-        uint32_t word = (holder && row < a.rows) ? s.byte : 0u;
-        word |= __shfl_down_sync(0xFFFFFFFFu, word, LPB) << 8;
-        word |= __shfl_down_sync(0xFFFFFFFFu, word, 2 * LPB) << 16;
-        if ((lane % (4 * LPB) == 0) && (kb < a.ncol_tiles * 4) && row < a.rows)
-          *reinterpret_cast<uint32_t*>(a.scale_packed + packed_scale_offset(row, kb, a.ncol_tiles)) = word;
-      }
+      scale_bytes = merge_shifted((holder && row < a.rows) ? s.byte : 0u, 8 * i, scale_bytes);
+    }
+    // ---- packed scales: four lanes hold four rows of four scale columns each; a 4 x 4 byte transpose in two
+    // exchanges leaves each of them one row's word (a word is four scale columns of one row) ----
+    if (a.scale_packed != nullptr) {
+      const int h = (lane / LPB) & 3;
+      uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, scale_bytes, 2 * LPB);
+      scale_bytes = __byte_perm(scale_bytes, o, (h & 2) ? 0x3276 : 0x5410);
+      o = __shfl_xor_sync(0xFFFFFFFFu, scale_bytes, LPB);
+      scale_bytes = __byte_perm(scale_bytes, o, (h & 1) ? 0x3715 : 0x6240);
+      const int64_t kb4 = kb - h;
+      if (lane % LPB == 0 && kb4 < a.ncol_tiles * 4 && row0 + h < a.rows)
+        *reinterpret_cast<uint32_t*>(a.scale_packed + packed_scale_offset(row0 + h, kb4, a.ncol_tiles)) = scale_bytes;
     }
   }
 }
@@ -964,7 +980,7 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       raw[i] = ok ? __ldg(reinterpret_cast<const uint4*>(src + i * pitch)) : make_uint4(0u, 0u, 0u, 0u);
-      acc = absmax_bf16x2(absmax_bf16x2(absmax_bf16x2(absmax_bf16x2(acc, raw[i].x), raw[i].y), raw[i].z), raw[i].w);
+      acc = absmax2_bf16x2(absmax2_bf16x2(acc, raw[i].x, raw[i].y), raw[i].z, raw[i].w);
     }
     amax_bits = fold_bf16x2(acc);
     if (stats) {
@@ -1021,7 +1037,7 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
 
   // ---- encode row by row, K packing ----
   uint32_t kw[F::FP4 ? 16 : 32];  // FP4: one word per row (8 codes); FP8: two words per row (8 bytes)
-  with_uniform_fast(s.fast, [&](auto fast_tag) {
+  with_uniform_fast(block_fast<IN_BF16, ROUND>(s, amax_bits), [&](auto fast_tag) {
     constexpr bool FAST = decltype(fast_tag)::value;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -1063,18 +1079,13 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
           ro = __ldg(reinterpret_cast<const uint4*>(a.rand_bits + plane + rr * pitch + pp));
         }
         const uint32_t e4[4] = {re.x, re.y, re.z, re.w}, o4[4] = {ro.x, ro.y, ro.z, ro.w};
-        uint32_t word = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          word = merge_shifted(fp4_pair<FMT, IN_BF16, ROUND, FAST>(v[2 * j], v[2 * j + 1], s, e4[j], o4[j]), 8 * j, word);
-        kw[i] = word;
+        kw[i] = fp4_octet<FMT, IN_BF16, ROUND, FAST>(v, s, e4, o4);
         if (ok) *reinterpret_cast<uint32_t*>(a.codes_k + (rows_before + row0 + i) * (a.cols >> 1) + (col0 >> 1)) = kw[i];
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = scale_elem<FMT, IN_BF16, FAST>(v[j], s);
         if (F::FP4) {
-          kw[i] = e2m1x2_rtn_hw(v[0], v[1]) | (e2m1x2_rtn_hw(v[2], v[3]) << 8) | (e2m1x2_rtn_hw(v[4], v[5]) << 16) |
-                  (e2m1x2_rtn_hw(v[6], v[7]) << 24);
+          kw[i] = e2m1x8_rtn_hw(v);
           if (ok) *reinterpret_cast<uint32_t*>(a.codes_k + (rows_before + row0 + i) * (a.cols >> 1) + (col0 >> 1)) = kw[i];
         } else {
           kw[2 * i] = fp8x2_rtn_hw<F::E5M2>(v[0], v[1]) | (fp8x2_rtn_hw<F::E5M2>(v[2], v[3]) << 16);
