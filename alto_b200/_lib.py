@@ -24,7 +24,7 @@ LIB_PATH = _PKG / "libaltob200.so"
 FMT_NVFP4, FMT_MXFP4, FMT_MXFP8_E4M3, FMT_MXFP8_E5M2 = 0, 1, 2, 3
 DT_BF16, DT_F32 = 0, 1
 SCALE_PLAIN, SCALE_PACKED = 1, 2
-ROUND_RTN, ROUND_SR_BITS, ROUND_SR_PHILOX = 0, 1, 2
+ROUND_RTN, ROUND_SR_BITS, ROUND_SR_PHILOX, ROUND_SR_SLOTS = 0, 1, 2, 3
 AMAX_SCRATCH_BYTES = 16
 
 E_SHAPE, E_ALIGN, E_TIMEOUT, E_CUDA, E_UNSUPPORTED, E_LIMIT = -1, -2, -3, -4, -5, -6
@@ -43,6 +43,7 @@ EXPORTED_SYMBOLS = (
     "altob200_quantize_2d_batched",
     "altob200_dequantize",
     "altob200_philox_tile",
+    "altob200_philox_slots",
     "altob200_rht",
     "altob200_rht_dense",
     "altob200_macro_block_scaling",
@@ -82,6 +83,7 @@ class QuantParams(C.Structure):
         ("use_uos", C.c_int32),
         ("rand_tile_rows", C.c_int64),
         ("rand_tile_pairs", C.c_int64),
+        ("macro_codes", C.c_void_p),
     ]
 
 
@@ -188,6 +190,8 @@ def _declare_more(lib):
     lib.altob200_swiglu_backward.argtypes = [vp, vp, i64, i64, i64, vp, vp]
     lib.altob200_philox_tile.restype = C.c_int
     lib.altob200_philox_tile.argtypes = [C.c_uint64, C.c_uint64, i64, i64, vp, vp]
+    lib.altob200_philox_slots.restype = C.c_int
+    lib.altob200_philox_slots.argtypes = [C.c_uint64, C.c_uint64, i32, C.POINTER(i32), vp, vp]
     lib.altob200_deosc_accumulate.restype = C.c_int
     lib.altob200_deosc_accumulate.argtypes = [vp, vp, vp, vp, vp, vp, i64, i32, vp]
     lib.altob200_dge_scale.restype = C.c_int
@@ -286,8 +290,9 @@ CLIP_MODES = {"none": 0, "static": 1, "dynamic": 2}
 
 
 def _params(fmt, x, rounding, outer_scale, rand_bits, rht: Optional[Rht], flags, philox=(0, 0),
-            clip_mode: str = "none", use_uos: bool = False, rand_tile=(0, 0)) -> QuantParams:
+            clip_mode: str = "none", use_uos: bool = False, rand_tile=(0, 0), macro_codes=None) -> QuantParams:
     p = QuantParams()
+    p.macro_codes = _ptr(macro_codes)
     p.clip_mode = CLIP_MODES[clip_mode]
     p.use_uos = 1 if use_uos else 0
     p.rand_tile_rows, p.rand_tile_pairs = int(rand_tile[0]), int(rand_tile[1])
@@ -314,6 +319,20 @@ def philox_tile(seed: int, offset: int, tile_rows: int, tile_pairs: int, device)
     _require_cuda(out)
     _check(lib().altob200_philox_tile(int(seed) & 0xFFFFFFFFFFFFFFFF, int(offset) & 0xFFFFFFFFFFFFFFFF, tile_rows,
                                       tile_pairs, out.data_ptr(), _stream()), "altob200_philox_tile")
+    return out
+
+
+SLOTS_TILE = (64, 32)   # the table shape philox_slots serves
+
+
+def philox_slots(seed: int, offset: int, rht: Optional[Rht], device) -> torch.Tensor:
+    """The words of ``philox_tile(seed, offset, 64, 32)`` laid out for ``quantize_colwise`` with
+    ``ROUND_SR_SLOTS`` and the transform ``rht``: [64 positions in slot order, 64 rows]."""
+    out = torch.empty(64, 64, dtype=torch.int32, device=device)
+    _require_cuda(out)
+    _check(lib().altob200_philox_slots(int(seed) & 0xFFFFFFFFFFFFFFFF, int(offset) & 0xFFFFFFFFFFFFFFFF,
+                                       rht.n if rht else 0, rht._perm_c if rht else None, out.data_ptr(), _stream()),
+           "altob200_philox_slots")
     return out
 
 
@@ -357,11 +376,12 @@ def amax_noalloc(x: torch.Tensor, amax_bits: torch.Tensor, outer_scale: Optional
 
 def quantize_rowwise(x, fmt, codes, scale_plain=None, scale_packed=None, *, rounding=ROUND_RTN,
                      outer_scale=None, rand_bits=None, philox=(0, 0), clip_mode="none", use_uos=False,
-                     rand_tile=(0, 0)) -> None:
-    _require_cuda(x, codes, scale_plain, scale_packed, outer_scale, rand_bits)
+                     rand_tile=(0, 0), macro_codes=None) -> None:
+    _require_cuda(x, codes, scale_plain, scale_packed, outer_scale, rand_bits, macro_codes)
     assert x.dim() == 2 and x.stride(1) == 1
     flags = (SCALE_PLAIN if scale_plain is not None else 0) | (SCALE_PACKED if scale_packed is not None else 0)
-    p = _params(fmt, x, rounding, outer_scale, rand_bits, None, flags, philox, clip_mode, use_uos, rand_tile)
+    p = _params(fmt, x, rounding, outer_scale, rand_bits, None, flags, philox, clip_mode, use_uos, rand_tile,
+                macro_codes)
     _check(lib().altob200_quantize_rowwise(x.data_ptr(), x.shape[0], x.shape[1], x.stride(0), C.byref(p),
                                            codes.data_ptr(), _ptr(scale_plain), _ptr(scale_packed), _stream()),
            "altob200_quantize_rowwise")
@@ -369,11 +389,12 @@ def quantize_rowwise(x, fmt, codes, scale_plain=None, scale_packed=None, *, roun
 
 def quantize_colwise(x, fmt, codes, scale_plain=None, scale_packed=None, *, rounding=ROUND_RTN,
                      outer_scale=None, rand_bits=None, rht: Optional[Rht] = None, philox=(0, 0),
-                     clip_mode="none", use_uos=False, rand_tile=(0, 0)) -> None:
-    _require_cuda(x, codes, scale_plain, scale_packed, outer_scale, rand_bits)
+                     clip_mode="none", use_uos=False, rand_tile=(0, 0), macro_codes=None) -> None:
+    _require_cuda(x, codes, scale_plain, scale_packed, outer_scale, rand_bits, macro_codes)
     assert x.dim() == 2 and x.stride(1) == 1
     flags = (SCALE_PLAIN if scale_plain is not None else 0) | (SCALE_PACKED if scale_packed is not None else 0)
-    p = _params(fmt, x, rounding, outer_scale, rand_bits, rht, flags, philox, clip_mode, use_uos, rand_tile)
+    p = _params(fmt, x, rounding, outer_scale, rand_bits, rht, flags, philox, clip_mode, use_uos, rand_tile,
+                macro_codes)
     _check(lib().altob200_quantize_colwise(x.data_ptr(), x.shape[0], x.shape[1], x.stride(0), C.byref(p),
                                            codes.data_ptr(), _ptr(scale_plain), _ptr(scale_packed), _stream()),
            "altob200_quantize_colwise")
@@ -381,12 +402,13 @@ def quantize_colwise(x, fmt, codes, scale_plain=None, scale_packed=None, *, roun
 
 def quantize_2d(w, fmt, codes_k, codes_t=None, scale_plain=None, scale_packed_k=None, scale_packed_t=None, *,
                 outer_scale=None, clip_mode="none", use_uos=False, rounding=ROUND_RTN, rand_bits=None,
-                rand_tile=(0, 0)) -> None:
+                rand_tile=(0, 0), macro_codes=None) -> None:
     """``rounding``: ROUND_RTN, or ROUND_SR_BITS (FP4) with ``rand_bits`` = words by (row, column pair) as in
     ``quantize_rowwise``: [2, rows, cols/2], or the periodic table [2, tile_rows, tile_pairs] with ``rand_tile``."""
-    _require_cuda(w, codes_k, codes_t, scale_plain, scale_packed_k, scale_packed_t, outer_scale, rand_bits)
+    _require_cuda(w, codes_k, codes_t, scale_plain, scale_packed_k, scale_packed_t, outer_scale, rand_bits, macro_codes)
     assert w.dim() == 2 and w.stride(1) == 1
-    p = _params(fmt, w, rounding, outer_scale, rand_bits, None, 0, (0, 0), clip_mode, use_uos, rand_tile)
+    p = _params(fmt, w, rounding, outer_scale, rand_bits, None, 0, (0, 0), clip_mode, use_uos, rand_tile,
+                macro_codes)
     _check(lib().altob200_quantize_2d(w.data_ptr(), w.shape[0], w.shape[1], w.stride(0), C.byref(p),
                                       codes_k.data_ptr(), _ptr(codes_t), _ptr(scale_plain), _ptr(scale_packed_k),
                                       _ptr(scale_packed_t), _stream()),
@@ -395,13 +417,14 @@ def quantize_2d(w, fmt, codes_k, codes_t=None, scale_plain=None, scale_packed_k=
 
 def quantize_2d_batched(w3, fmt, codes_k, codes_t=None, scale_plain=None, scale_packed_k=None, scale_packed_t=None,
                         *, outer_scale=None, clip_mode="none", use_uos=False, rounding=ROUND_RTN, rand_bits=None,
-                        rand_tile=(0, 0)) -> None:
+                        rand_tile=(0, 0), macro_codes=None) -> None:
     """``w3`` [batch, rows, cols] (last dim contiguous, equal batch stride): every matrix quantised in 2-D
     blocks by one launch; outputs are the per-matrix outputs of ``quantize_2d`` stacked along a leading
     batch dimension.  Random words, if any, are indexed by the rows of the flattened [batch * rows, cols] view."""
-    _require_cuda(w3, codes_k, codes_t, scale_plain, scale_packed_k, scale_packed_t, outer_scale, rand_bits)
+    _require_cuda(w3, codes_k, codes_t, scale_plain, scale_packed_k, scale_packed_t, outer_scale, rand_bits, macro_codes)
     assert w3.dim() == 3 and w3.stride(2) == 1
-    p = _params(fmt, w3, rounding, outer_scale, rand_bits, None, 0, (0, 0), clip_mode, use_uos, rand_tile)
+    p = _params(fmt, w3, rounding, outer_scale, rand_bits, None, 0, (0, 0), clip_mode, use_uos, rand_tile,
+                macro_codes)
     _check(lib().altob200_quantize_2d_batched(w3.data_ptr(), w3.shape[0], w3.stride(0), w3.shape[1], w3.shape[2],
                                               w3.stride(1), C.byref(p), codes_k.data_ptr(), _ptr(codes_t),
                                               _ptr(scale_plain), _ptr(scale_packed_k), _ptr(scale_packed_t), _stream()),

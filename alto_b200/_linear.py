@@ -83,6 +83,15 @@ def sr_args(use_sr: bool, name: str, rows: int, cols: int, device) -> dict:
                 rand_tile=tile)
 
 
+def sr_args_cols(use_sr: bool, name: str, rows: int, cols: int, device, rht: Optional[L.Rht] = None) -> dict:
+    """``sr_args`` for the column-wise quantizer with the fused transform ``rht``: the same words, from a table
+    laid out for that kernel where the view fills the whole 64 x 64 tile."""
+    if not use_sr or _sr_bits_provider is not None or L.sr_tile_dims(rows, cols) != L.SLOTS_TILE:
+        return sr_args(use_sr, name, rows, cols, device)
+    seed, offset = draw_philox()
+    return dict(rounding=L.ROUND_SR_SLOTS, rand_bits=L.philox_slots(seed, offset, rht, device), rand_tile=L.SLOTS_TILE)
+
+
 RTN = dict(rounding=L.ROUND_RTN)
 
 # ---------------------------------------------------------------------------------------
@@ -262,8 +271,8 @@ def backward_operands(g2, fmt, *, use_2dblock_x, use_sr_grad, use_outer_scale, r
                         sr_args(use_sr_grad, "dy_n", M, N, g2.device))
     g_n = quant_rows(g2, fmt, None if og is None else og[0:1], sr_args(use_sr_grad, "dy_n", M, N, g2.device),
                      use_uos)
-    g_m = cols_operand(g2, fmt, use_outer_scale, og, rht, dense, sr_args(use_sr_grad, "dy_m", N, M, g2.device),
-                       use_uos, clip_mode)
+    g_m = cols_operand(g2, fmt, use_outer_scale, og, rht, dense,
+                       sr_args_cols(use_sr_grad, "dy_m", N, M, g2.device, rht), use_uos, clip_mode)
     return g_n, g_m
 
 
@@ -392,7 +401,7 @@ def linear_backward(ctx, grad_output):
         side = _side_stream(g2.device)
         og = outer_scales(g2, ctx.use_outer_scale, rht)
         sr_n = sr_args(ctx.use_sr_grad, "dy_n", M, N, g2.device)  # drawn in the same order as without overlap
-        sr_m = sr_args(ctx.use_sr_grad, "dy_m", N, M, g2.device)
+        sr_m = sr_args_cols(ctx.use_sr_grad, "dy_m", N, M, g2.device, rht)
         o_m = None if og is None else (og[1:2] if rht is not None else og[0:1])
         g_m = quant_cols(g2, fmt, o_m, rht, sr_m)
         ready = torch.cuda.Event()
@@ -415,7 +424,7 @@ def linear_backward(ctx, grad_output):
         # beside the second quantizer of dY and the wgrad GEMM.  Random words are drawn in the usual order.
         og = outer_scales(g2, ctx.use_outer_scale, ctx.rht)
         sr_n = sr_args(ctx.use_sr_grad, "dy_n", M, N, g2.device)
-        sr_m = sr_args(ctx.use_sr_grad, "dy_m", N, M, g2.device)
+        sr_m = sr_args_cols(ctx.use_sr_grad, "dy_m", N, M, g2.device, ctx.rht)
         g_n = quant_rows(g2, ctx.fmt, None if og is None else og[0:1], sr_n, ctx.use_uos)
         dx2 = gemm(g_n, w_t, grad_output.dtype)
         dx_hook(dx2)

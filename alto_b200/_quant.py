@@ -121,13 +121,16 @@ def quantize(x: torch.Tensor, fmt: int, axis: int, is_2d: bool, *, outer_scale: 
         if nb > 1 and N % tile[0] != 0:
             raise NotImplementedError("stochastic rounding of a batched tensor whose rows do not fill whole "
                                       "64-row tiles per batch entry is not implemented")
-        table = L.philox_tile(philox[0], philox[1], tile[0], tile[1], dev)
+        slots = tile == L.SLOTS_TILE
+        table = (L.philox_slots(philox[0], philox[1], rht, dev) if slots
+                 else L.philox_tile(philox[0], philox[1], tile[0], tile[1], dev))
     for b in range(nb):
         xb = x3[b]
         if xb.stride(-1) != 1 or (xb.stride(0) * xb.element_size()) % 16 != 0:
             xb = xb.contiguous()
         if table is not None:
-            L.quantize_colwise(xb, fmt, codes[b], scales[b], None, rounding=L.ROUND_SR_BITS, outer_scale=outer_scale,
+            L.quantize_colwise(xb, fmt, codes[b], scales[b], None,
+                               rounding=L.ROUND_SR_SLOTS if slots else L.ROUND_SR_BITS, outer_scale=outer_scale,
                                rand_bits=table, rand_tile=tile, rht=rht, **opts)
             continue
         L.quantize_colwise(xb, fmt, codes[b], scales[b], None, rounding=rounding, outer_scale=outer_scale,

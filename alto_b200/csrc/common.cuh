@@ -134,6 +134,18 @@ __device__ __forceinline__ void nvfp4_block_scale(float amax, bool use_outer, fl
 }
 
 // ---------------------------------------------------------------------------------------
+// Factor of a macro block (two-level scaling) from its maximum, and from its stored code:
+//   alto/kernels/fp4/mxfp4/macro_block_scaling.py:70-85
+// ---------------------------------------------------------------------------------------
+__device__ __forceinline__ float macro_factor_from_amax(float amax, uint32_t* code) {
+  amax = fmaxf(amax, 1e-12f);
+  const uint32_t bits = f2u(__fdiv_rn(6.0f, amax)) & 0x007F8000u;
+  *code = bits >> 15;
+  return u2f(bits + (127u << 23));
+}
+__device__ __forceinline__ float macro_factor_from_code(uint32_t code) { return u2f((code << 15) + (127u << 23)); }
+
+// ---------------------------------------------------------------------------------------
 // Exact fp32 division x / q.
 //
 // For a bf16-valued numerator the sequence  y = x*r; e = fma(-y, q, x); y' = fma(e, r, y)

@@ -28,14 +28,6 @@ struct MacroArgs {
   int wide;            // rows are a multiple of 8 elements and 32-byte (fp32) / 16-byte (bf16) aligned
 };
 
-__device__ __forceinline__ float macro_factor_from_amax(float amax, uint32_t* code) {
-  amax = fmaxf(amax, 1e-12f);
-  const uint32_t bits = f2u(__fdiv_rn(6.0f, amax)) & 0x007F8000u;
-  *code = bits >> 15;
-  return u2f(bits + (127u << 23));
-}
-__device__ __forceinline__ float macro_factor_from_code(uint32_t code) { return u2f((code << 15) + (127u << 23)); }
-
 template <bool IN_BF16>
 __device__ __forceinline__ void load4(const void* base, int64_t off, int valid, bool vec, float v[4]) {
   // `valid` elements (0..4) starting at element offset `off` exist; the rest read as zero

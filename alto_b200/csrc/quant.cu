@@ -183,21 +183,6 @@ __device__ __forceinline__ uint32_t merge_shifted(uint32_t x, int sh, uint32_t a
   return r;
 }
 
-// The scaled element up to the sign of a zero (the stochastic-rounding encoder takes the sign from x).
-template <int FMT, bool IN_BF16, bool FAST>
-__device__ __forceinline__ float scale_elem_mag(float x, const BlockScale& s) {
-  return scale_elem<FMT, IN_BF16, FAST>(x, s);
-}
-
-template <int FMT>
-__device__ __forceinline__ float2 scale_pair_mag(float2 x, const BlockScale& s0, const BlockScale& s1) {
-  const float2 r = make_float2(s0.r, s1.r);
-  const float2 y = __fmul2_rn(x, r);
-  if (Fmt<FMT>::MX) return y;
-  const float2 e = __ffma2_rn(y, make_float2(-s0.q, -s1.q), x);
-  return __ffma2_rn(e, r, y);
-}
-
 // Eight elements of one block scaled and quantised into four FP4 bytes (element 0 in the lowest nibble).
 // SR words: r0[j] for element 2j, r1[j] for element 2j + 1; FAST also means that the elements are finite.
 template <int FMT, bool IN_BF16, int ROUND, bool FAST>
@@ -474,7 +459,7 @@ struct RhtParams {
   float sign[16];  // sign applied to slot k after the butterfly
   int64_t row_off[16];  // byte offset of row pinv[k] from the first row of a 16-row group (column passes)
   float qsign[16];      // sign[k] / sqrt(16): the factor applied to slot k
-  int perm_off[16];     // pinv[k] * 8: byte offset of slot k's row in the shared-memory position table, per thread of the CTA
+  uint32_t psel[4], pmask[4];  // output word w of four positions: byte selectors within each half of the slots, half mask
 };
 
 __device__ __forceinline__ void hadamard16(float* z) {
@@ -533,30 +518,42 @@ struct ColwiseArgs {
   PhiloxKeys pk;
   RhtParams rht;
   MxOpts mx;
+  uint8_t* macro_codes;  // MACRO: [cols, ceil(rows / 128)] factor codes, written
 };
 
-// Threads per CTA = rows per CTA tile.  128 rather than 256: more, smaller CTAs per SM (four of the
-// 128-register stochastic-rounding variant instead of two), so that the start-up loads and the
-// barrier of one overlap the arithmetic of the others (measured 5-6 % on the bench's launches).
+// Threads per CTA = rows per CTA tile.  128 rather than 256: more, smaller CTAs per SM, so that the start-up
+// loads and the barrier of one overlap the arithmetic of the others.
 constexpr int COL_NT = 128;
 constexpr int COL_TN = 64;   // columns per CTA tile
 
-template <int FMT, bool IN_BF16, int ROUND, bool RHT>
+// What bounds the kernel is the integer pipe, so codes are never handled one by one: the converter packs the
+// codes of a lane's two columns into one byte, four slots into one word; the output permutation of the
+// Hadamard transform moves those bytes (three instructions for four positions of both columns), and the two
+// columns are separated eight codes at a time.  The random words of stochastic rounding belong to output
+// positions: with ROUND_SR_SLOTS the table is laid out by slot (altob200_philox_slots), so that the codes can
+// be made in slot order and neighbouring lanes read neighbouring words.
+// MACRO (MXFP4 from bf16): the two-level recipe's scaling runs in front of the quantisation - a CTA tile is one
+// macro block of 128 rows per column, so its maxima only have to cross the four warps.
+template <int FMT, bool IN_BF16, int ROUND, bool RHT, bool MACRO>
 __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a) {
   grid_dependency_wait();
   using F = Fmt<FMT>;
   constexpr int B = F::B;
   constexpr int NT = COL_NT;   // threads per CTA
+  constexpr int WARPS = NT / 32;
   constexpr int COL_TM = NT;               // rows per CTA tile
-  constexpr int NBLK = COL_TM / B;          // row blocks per tile (16 or 8)
-  constexpr int ITERS = NBLK / (NT / 32);   // per warp
+  constexpr int NBLK = COL_TM / B;          // row blocks per tile (8 or 4)
+  constexpr int ITERS = NBLK / WARPS;       // per warp
   constexpr int ROW_BYTES = F::FP4 ? COL_TM / 2 : COL_TM;  // bytes per output row per tile
   constexpr int BLK_BYTES = F::FP4 ? B / 2 : B;            // bytes per block per column
+  static_assert(!MACRO || (FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && COL_TM == 128 && ITERS == 1), "macro blocks");
   // codes staged as [block][column][BLK_BYTES]; scales as [column][NBLK]
   __shared__ __align__(16) uint8_t s_codes[COL_TN * ROW_BYTES];
   __shared__ __align__(16) uint8_t s_sf[COL_TN * NBLK];
   __shared__ float s_sf_plain[Fmt<FMT>::MX ? 1 : COL_TN * NBLK];
-  __shared__ float2 s_perm[(RHT && ROUND != ALTOB200_ROUND_RTN) ? 16 : 1][NT];   // (column c, column c + 1) per thread
+  constexpr bool WORDS_TO_SLOTS = RHT && ROUND == ALTOB200_ROUND_SR_PHILOX;
+  __shared__ uint2 s_words[WORDS_TO_SLOTS ? 16 : 1][NT];   // (column c, column c + 1) per thread
+  __shared__ uint32_t s_macro[MACRO ? WARPS : 1][32];
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t m0 = (int64_t)blockIdx.y * COL_TM;
@@ -580,7 +577,7 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
   if (IN_BF16) {
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
-      const int64_t mb = m0 + (int64_t)(warp * ITERS + it) * B;
+      const int64_t mb = m0 + (int64_t)(warp + WARPS * it) * B;
       const bool ok = col_ok && mb < a.rows;
       const uint8_t* base = reinterpret_cast<const uint8_t*>(a.x) + (mb * a.ld + c) * ESZ;
 #pragma unroll
@@ -592,231 +589,222 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
 
 #pragma unroll
   for (int it = 0; it < ITERS; ++it) {
-    const int blk = warp * ITERS + it;
+    const int blk = warp + WARPS * it;
     const int64_t mb = m0 + (int64_t)blk * B;
     const bool ok = col_ok && mb < a.rows;  // rows % B == 0
-    float v0[B], v1[B];
+    // bf16: both columns of a slot travel as one packed pair (pw); fp32: as two floats (v0, v1)
+    uint32_t pw[IN_BF16 ? B : 1];
+    float v0[IN_BF16 ? 16 : B], v1[IN_BF16 ? 16 : B];
+    uint32_t am0 = 0, am1 = 0;   // block maxima of |x|, bits of the input type
     if (IN_BF16) {
+      uint32_t acc = 0;
 #pragma unroll
-      for (int k = 0; k < B; ++k) {
-        const uint32_t w = pre[it % (IN_BF16 ? ITERS : 1)][k % (IN_BF16 ? B : 1)];
-        v0[k] = bf16lo_to_f32(w);
-        v1[k] = bf16hi_to_f32(w);
+      for (int g = 0; g < B; g += 16) {
+        uint32_t* w = pw + (IN_BF16 ? g : 0);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) w[k % (IN_BF16 ? 16 : 1)] = pre[it % (IN_BF16 ? ITERS : 1)][(g + k) % (IN_BF16 ? B : 1)];
+        if (RHT) {
+          // y = (H z) / sqrt(16), rounded to bf16: one conversion per pair
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            v0[k] = bf16lo_to_f32(w[k % (IN_BF16 ? 16 : 1)]);
+            v1[k] = bf16hi_to_f32(w[k % (IN_BF16 ? 16 : 1)]);
+          }
+          hadamard16_pair(v0, v1);
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            // the fused +0 turns a -0 product into the +0 that a dot product yields
+            const float sg = a.rht.qsign[k];
+            const float2 sc = __ffma2_rn(make_float2(v0[k], v1[k]), make_float2(sg, sg), make_float2(0.0f, 0.0f));
+            const __nv_bfloat162 p2 = __floats2bfloat162_rn(sc.x, sc.y);
+            w[k % (IN_BF16 ? 16 : 1)] = *reinterpret_cast<const uint32_t*>(&p2);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 16; k += 2)
+          acc = absmax2_bf16x2(acc, w[k % (IN_BF16 ? 16 : 1)], w[(k + 1) % (IN_BF16 ? 16 : 1)]);
       }
+      if (MACRO) {
+        // factor of the column's 128 rows (csrc/macro_scale.cu), then y = bf16(x * factor); rounding is
+        // monotone, so the block maximum is scaled instead of searched again
+        s_macro[MACRO ? warp : 0][lane] = acc;
+        __syncthreads();
+        uint32_t m = s_macro[0][lane];
+#pragma unroll
+        for (int w = 1; w < (MACRO ? WARPS : 1); ++w) m = __vmaxu2(m, s_macro[w][lane]);
+        uint32_t code0, code1;
+        const float f0 = macro_factor_from_amax(bf16lo_to_f32(m), &code0);
+        const float f1 = macro_factor_from_amax(bf16hi_to_f32(m), &code1);
+        if (warp == 0 && col_ok) {
+          uint8_t* dst = a.macro_codes + c * gridDim.y + blockIdx.y;
+          dst[0] = (uint8_t)code0;
+          dst[gridDim.y] = (uint8_t)code1;
+        }
+        auto scaled = [&](uint32_t w) {
+          const __nv_bfloat162 p2 = __floats2bfloat162_rn(__fmul_rn(bf16lo_to_f32(w), f0), __fmul_rn(bf16hi_to_f32(w), f1));
+          return *reinterpret_cast<const uint32_t*>(&p2);
+        };
+        acc = scaled(acc) & 0x7FFF7FFFu;
+#pragma unroll
+        for (int k = 0; k < B; ++k) pw[k % (IN_BF16 ? B : 1)] = scaled(pw[k % (IN_BF16 ? B : 1)]);
+      }
+      am0 = acc & 0xFFFFu;
+      am1 = acc >> 16;
     } else {
       const uint8_t* base = reinterpret_cast<const uint8_t*>(a.x) + (mb * a.ld + c) * ESZ;
 #pragma unroll
       for (int k = 0; k < B; ++k) {
         float2 f = make_float2(0.f, 0.f);
         if (ok) f = __ldg(reinterpret_cast<const float2*>(base + a.rht.row_off[k & 15] + (k >= 16 ? half_blk : 0)));
-        v0[k] = f.x;
-        v1[k] = f.y;
+        v0[k % (IN_BF16 ? 16 : B)] = f.x;
+        v1[k % (IN_BF16 ? 16 : B)] = f.y;
       }
-    }
-    // ---- transform: y = (H z) / sqrt(16), rounded to the input dtype ----
-    if (RHT) {
-#pragma unroll
-      for (int g = 0; g < B; g += 16) {
-        hadamard16_pair(v0 + g, v1 + g);
-      }
-    }
-    // ---- scale by +-1/sqrt(16) (exact), round to the input dtype, block amax on the rounded bits ----
-    uint32_t am0 = 0, am1 = 0;
-    if (RHT && IN_BF16) {
-      // both columns of a lane travel as one packed bf16 pair: one conversion and one packed maximum
-      uint32_t acc = 0;
-#pragma unroll
-      for (int k = 0; k < B; ++k) {
-        // the fused +0 turns a -0 product into the +0 that a dot product yields
-        const float sg = a.rht.qsign[k & 15];
-        const float2 sc = __ffma2_rn(make_float2(v0[k], v1[k]), make_float2(sg, sg), make_float2(0.0f, 0.0f));
-        const __nv_bfloat162 p2 = __floats2bfloat162_rn(sc.x, sc.y);
-        const uint32_t pw = *reinterpret_cast<const uint32_t*>(&p2);
-        acc = absmax_bf16x2(acc, pw);
-        v0[k] = bf16lo_to_f32(pw);
-        v1[k] = bf16hi_to_f32(pw);
-      }
-      am0 = acc & 0xFFFFu;
-      am1 = acc >> 16;
-    } else {
       if (RHT) {
 #pragma unroll
-        for (int k = 0; k < B; ++k) {
+        for (int g = 0; g < (IN_BF16 ? 16 : B); g += 16) hadamard16_pair(v0 + g, v1 + g);
+#pragma unroll
+        for (int k = 0; k < (IN_BF16 ? 16 : B); ++k) {
           const float sg = a.rht.qsign[k & 15];
           v0[k] = __fmaf_rn(v0[k], sg, 0.0f);
           v1[k] = __fmaf_rn(v1[k], sg, 0.0f);
         }
       }
 #pragma unroll
-      for (int k = 0; k < B; ++k) {
+      for (int k = 0; k < (IN_BF16 ? 16 : B); ++k) {
         const uint32_t b0 = f2u(v0[k]) & 0x7FFFFFFFu, b1 = f2u(v1[k]) & 0x7FFFFFFFu;
         am0 = b0 > am0 ? b0 : am0;
         am1 = b1 > am1 ? b1 : am1;
       }
-      if (IN_BF16) {
-        am0 >>= 16;
-        am1 >>= 16;
-      }
     }
+    const bool clip = F::MX && a.mx.clip == 1;
+    // the two elements of slot k
+    auto slot = [&](int k) -> float2 {
+      float2 x = IN_BF16 ? make_float2(bf16lo_to_f32(pw[k % (IN_BF16 ? B : 1)]), bf16hi_to_f32(pw[k % (IN_BF16 ? B : 1)]))
+                         : make_float2(v0[k % (IN_BF16 ? 16 : B)], v1[k % (IN_BF16 ? 16 : B)]);
+      if (clip) x = make_float2(round_in<IN_BF16>(__fmul_rn(x.x, 0.75f)), round_in<IN_BF16>(__fmul_rn(x.y, 0.75f)));
+      return x;
+    };
     BlockScale s0, s1;
     if (F::MX && (a.mx.clip | a.mx.uos)) {
       float sum0 = 0.0f, sq0 = 0.0f, sum1 = 0.0f, sq1 = 0.0f;
       if (a.mx.clip == 2) {
 #pragma unroll
         for (int k = 0; k < B; ++k) {
-          sum0 = __fadd_rn(sum0, v0[k]);
-          sq0 = __fadd_rn(sq0, round_in<IN_BF16>(__fmul_rn(v0[k], v0[k])));
-          sum1 = __fadd_rn(sum1, v1[k]);
-          sq1 = __fadd_rn(sq1, round_in<IN_BF16>(__fmul_rn(v1[k], v1[k])));
+          const float2 x = slot(k);
+          sum0 = __fadd_rn(sum0, x.x);
+          sq0 = __fadd_rn(sq0, round_in<IN_BF16>(__fmul_rn(x.x, x.x)));
+          sum1 = __fadd_rn(sum1, x.y);
+          sq1 = __fadd_rn(sq1, round_in<IN_BF16>(__fmul_rn(x.y, x.y)));
         }
       }
       s0 = make_block_scale_opts<FMT, IN_BF16>(am0, sum0, sq0, B, a.mx);
       s1 = make_block_scale_opts<FMT, IN_BF16>(am1, sum1, sq1, B, a.mx);
-      if (a.mx.clip == 1) {
-#pragma unroll
-        for (int k = 0; k < B; ++k) {
-          v0[k] = round_in<IN_BF16>(__fmul_rn(v0[k], 0.75f));
-          v1[k] = round_in<IN_BF16>(__fmul_rn(v1[k], 0.75f));
-        }
-      }
     } else {
       s0 = make_block_scale<FMT, IN_BF16>(am0, os);
       s1 = make_block_scale<FMT, IN_BF16>(am1, os);
     }
+    const bool fast = block_fast<IN_BF16, ROUND>(s0, am0) && block_fast<IN_BF16, ROUND>(s1, am1);
 
     // ---- quantise in slot order ----
     if (F::FP4) {
 #pragma unroll
       for (int h = 0; h < B / 16; ++h) {
-        // With stochastic rounding the random word belongs to the OUTPUT position, so the
-        // transformed values are first moved from slot order to position order through a
-        // private shared-memory column (static register index, dynamic address).
-        constexpr bool TO_POS = RHT && ROUND != ALTOB200_ROUND_RTN;
-        float y0[16], y1[16];
+        // random words by slot: r[k] for columns c and c + 1
+        uint2 r[ROUND == ALTOB200_ROUND_RTN ? 1 : 16];
+        if (ROUND == ALTOB200_ROUND_SR_SLOTS) {
+          // [64 positions, slot order within groups of 16][64 columns]
+          const uint2* t = reinterpret_cast<const uint2*>(a.rand_bits + ((uint32_t)(mb + 16 * h) & 63u) * 64u + tile_row0);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          y0[j] = v0[16 * h + j];
-          y1[j] = v1[16 * h + j];
-        }
-        if (TO_POS) {
+          for (int k = 0; k < 16; ++k) r[k % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = __ldg(t + 32 * k);
+        } else if (ROUND == ALTOB200_ROUND_SR_BITS) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            // row pinv[j] of the table (NT pairs of 8 bytes per row): both columns in one 8-byte access
-            float2* dst = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(&s_perm[0][threadIdx.x]) +
-                                                    a.rht.perm_off[j] * NT);
-            *dst = make_float2(y0[j], y1[j]);
-          }
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float2 t = s_perm[j][threadIdx.x];
-            y0[j] = t.x;
-            y1[j] = t.y;
-          }
-        }
-        // random words by position: r0[i]/r1[i] for column c / c+1
-        uint32_t r0[16], r1[16];
-        if (ROUND == ALTOB200_ROUND_SR_BITS) {
-          if (a.tile_rows != 0 && (a.tile_pairs & 7) == 0) {
-            // periodic table: the 8 pairs of these 16 rows are 8 consecutive, 32-byte aligned words of
-            // one table row in each plane (tile_pairs is a multiple of 8) -> four 16-byte loads per column
-            const uint32_t tp = (uint32_t)a.tile_pairs;
-            const uint32_t base = (uint32_t)((mb + 16 * h) >> 1) % tp;
-            const uint32_t plane = (uint32_t)a.tile_rows * tp;
-            const uint32_t* t0 = a.rand_bits + tile_row0 * tp + base;
-            const uint32_t* t1 = a.rand_bits + tile_row1 * tp + base;
-            uint4 e0[2], o0[2], e1[2], o1[2];  // even / odd planes of column c and c + 1
-#pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              e0[q] = o0[q] = e1[q] = o1[q] = make_uint4(0u, 0u, 0u, 0u);
-              if (ok) {
-                e0[q] = __ldg(reinterpret_cast<const uint4*>(t0) + q);
-                o0[q] = __ldg(reinterpret_cast<const uint4*>(t0 + plane) + q);
-                e1[q] = __ldg(reinterpret_cast<const uint4*>(t1) + q);
-                o1[q] = __ldg(reinterpret_cast<const uint4*>(t1 + plane) + q);
+          for (int k = 0; k < 16; ++k) {
+            uint2 w = make_uint2(0u, 0u);
+            if (ok) {
+              const int64_t pos = mb + 16 * h + a.rht.pinv[k], idx = pos >> 1;
+              if (a.tile_rows != 0) {
+                const uint32_t* t = a.rand_bits + (pos & 1) * a.tile_rows * a.tile_pairs + (uint32_t)idx % (uint32_t)a.tile_pairs;
+                w = make_uint2(__ldg(t + (int64_t)tile_row0 * a.tile_pairs), __ldg(t + (int64_t)tile_row1 * a.tile_pairs));
+              } else {
+                const uint32_t* t = a.rand_bits + (pos & 1) * a.cols * half_rows + c * half_rows + idx;
+                w = make_uint2(__ldg(t), __ldg(t + half_rows));
               }
             }
-            const uint32_t ev0[8] = {e0[0].x, e0[0].y, e0[0].z, e0[0].w, e0[1].x, e0[1].y, e0[1].z, e0[1].w};
-            const uint32_t od0[8] = {o0[0].x, o0[0].y, o0[0].z, o0[0].w, o0[1].x, o0[1].y, o0[1].z, o0[1].w};
-            const uint32_t ev1[8] = {e1[0].x, e1[0].y, e1[0].z, e1[0].w, e1[1].x, e1[1].y, e1[1].z, e1[1].w};
-            const uint32_t od1[8] = {o1[0].x, o1[0].y, o1[0].z, o1[0].w, o1[1].x, o1[1].y, o1[1].z, o1[1].w};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              r0[2 * j] = ev0[j]; r0[2 * j + 1] = od0[j];
-              r1[2 * j] = ev1[j]; r1[2 * j + 1] = od1[j];
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              r0[i] = r1[i] = 0;
-              if (ok) {
-                const int64_t idx = (mb + 16 * h + i) >> 1;
-                if (a.tile_rows != 0) {
-                  const int64_t plane = (int64_t)(i & 1) * a.tile_rows * a.tile_pairs;
-                  const int64_t pi = idx % a.tile_pairs;
-                  r0[i] = __ldg(a.rand_bits + plane + (int64_t)tile_row0 * a.tile_pairs + pi);
-                  r1[i] = __ldg(a.rand_bits + plane + (int64_t)tile_row1 * a.tile_pairs + pi);
-                } else {
-                  const int64_t plane = (int64_t)(i & 1) * a.cols * half_rows;
-                  r0[i] = __ldg(a.rand_bits + plane + c * half_rows + idx);
-                  r1[i] = __ldg(a.rand_bits + plane + (c + 1) * half_rows + idx);
-                }
-              }
-            }
+            r[k % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = w;
           }
         } else if (ROUND == ALTOB200_ROUND_SR_PHILOX) {
           const uint64_t p0 = (uint64_t)(c * half_rows + ((mb + 16 * h) >> 1));        // pair index, column c
           const uint64_t p1 = (uint64_t)((c + 1) * half_rows + ((mb + 16 * h) >> 1));  // column c + 1
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            uint32_t o[4];
+            uint32_t o0[4], o1[4];
             uint64_t ctr = a.philox_offset + (p0 >> 1) + i;
-            philox4x32_10_keys((uint32_t)ctr, (uint32_t)(ctr >> 32), a.pk, o);
-            r0[4 * i] = o[0]; r0[4 * i + 1] = o[1]; r0[4 * i + 2] = o[2]; r0[4 * i + 3] = o[3];
+            philox4x32_10_keys((uint32_t)ctr, (uint32_t)(ctr >> 32), a.pk, o0);
             ctr = a.philox_offset + (p1 >> 1) + i;
-            philox4x32_10_keys((uint32_t)ctr, (uint32_t)(ctr >> 32), a.pk, o);
-            r1[4 * i] = o[0]; r1[4 * i + 1] = o[1]; r1[4 * i + 2] = o[2]; r1[4 * i + 3] = o[3];
+            philox4x32_10_keys((uint32_t)ctr, (uint32_t)(ctr >> 32), a.pk, o1);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) r[(4 * i + q) % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = make_uint2(o0[q], o1[q]);
+          }
+          if (WORDS_TO_SLOTS) {   // position order -> slot order through a private shared-memory column
+#pragma unroll
+            for (int k = 0; k < 16; ++k) s_words[k % (WORDS_TO_SLOTS ? 16 : 1)][threadIdx.x] = r[k % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)];
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+              r[k % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = s_words[WORDS_TO_SLOTS ? a.rht.pinv[k] : 0][threadIdx.x];
           }
         }
-        // nibble j = code of entry j (slot order, or position order if TO_POS), in two 32-bit halves
-        uint32_t w0h[2] = {0u, 0u}, w1h[2] = {0u, 0u};
-        with_uniform_fast(s0.fast && s1.fast, [&](auto fast_tag) {
+        // byte k % 4 of word k / 4: code of slot k, column c in the low nibble and c + 1 in the high one
+        uint32_t by_slot[4];
+        with_uniform_fast(fast, [&](auto fast_tag) {
           constexpr bool FAST = decltype(fast_tag)::value;
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            uint32_t c0, c1;
-            if (ROUND == ALTOB200_ROUND_RTN) {
-              // the hardware converter takes one value of each column per call
-              const uint32_t b = e2m1x2_rtn_hw(scale_elem<FMT, IN_BF16, FAST>(y0[j], s0),
-                                               scale_elem<FMT, IN_BF16, FAST>(y1[j], s1));
-              c0 = b & 0xFu;
-              c1 = b >> 4;
-            } else if (FAST) {
-              // both columns' quotients with packed operations (the same three roundings per element)
-              const float2 q = scale_pair_mag<FMT>(make_float2(y0[j], y1[j]), s0, s1);
-              c0 = e2m1_sr_code(q.x, f2u(y0[j]), r0[j]);
-              c1 = e2m1_sr_code(q.y, f2u(y1[j]), r1[j]);
-            } else {
-              c0 = e2m1_sr_code(scale_elem_mag<FMT, IN_BF16, FAST>(y0[j], s0), f2u(y0[j]), r0[j]);
-              c1 = e2m1_sr_code(scale_elem_mag<FMT, IN_BF16, FAST>(y1[j], s1), f2u(y1[j]), r1[j]);
+          for (int w = 0; w < 4; ++w) {
+            float q[8], sgn[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 x = slot(16 * h + 4 * w + j);
+              q[2 * j] = scale_elem<FMT, IN_BF16, FAST>(x.x, s0);
+              q[2 * j + 1] = scale_elem<FMT, IN_BF16, FAST>(x.y, s1);
+              sgn[2 * j] = x.x;
+              sgn[2 * j + 1] = x.y;
             }
-            // disjoint bits: adding is or-ing, and the multiply-add pipe has room where the ALU pipe has not
-            w0h[j >> 3] = merge_shifted(c0, 4 * (j & 7), w0h[j >> 3]);
-            w1h[j >> 3] = merge_shifted(c1, 4 * (j & 7), w1h[j >> 3]);
+            if (ROUND == ALTOB200_ROUND_RTN) {
+              by_slot[w] = e2m1x8_rtn_hw(q);
+            } else if (FAST) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint2 rw = r[(4 * w + j) % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)];
+                q[2 * j] = e2m1_sr_value(q[2 * j], rw.x);
+                q[2 * j + 1] = e2m1_sr_value(q[2 * j + 1], rw.y);
+              }
+              by_slot[w] = e2m1x8_rtn_hw(q);
+            } else {
+              by_slot[w] = 0u;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint2 rw = r[(4 * w + j) % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)];
+                by_slot[w] = merge_shifted(e2m1_sr_code(q[2 * j], f2u(sgn[2 * j]), rw.x), 8 * j, by_slot[w]);
+                by_slot[w] = merge_shifted(e2m1_sr_code(q[2 * j + 1], f2u(sgn[2 * j + 1]), rw.y), 8 * j + 4, by_slot[w]);
+              }
+            }
           }
         });
-        const uint64_t w0 = ((uint64_t)w0h[1] << 32) | w0h[0], w1 = ((uint64_t)w1h[1] << 32) | w1h[0];
-        uint64_t o0 = w0, o1 = w1;
-        if (RHT && !TO_POS) {  // output position i takes slot perm[i]
-          o0 = o1 = 0;
+        uint32_t u0[4], u1[4];   // bytes 0 and 2: two positions of column c / c + 1
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            o0 |= ((w0 >> (4 * a.rht.perm[i])) & 0xFull) << (4 * i);
-            o1 |= ((w1 >> (4 * a.rht.perm[i])) & 0xFull) << (4 * i);
+        for (int w = 0; w < 4; ++w) {
+          uint32_t o = by_slot[w];
+          if (RHT) {   // output position i takes slot perm[i]
+            const uint32_t lo = __byte_perm(by_slot[0], by_slot[1], a.rht.psel[w]);
+            const uint32_t hi = __byte_perm(by_slot[2], by_slot[3], a.rht.psel[w]);
+            o = (lo & ~a.rht.pmask[w]) | (hi & a.rht.pmask[w]);
           }
+          const uint32_t o4 = o >> 4, o8 = o >> 8;
+          u0[w] = (o & 0x0F0F0F0Fu) | (o4 & 0xF0F0F0F0u);
+          u1[w] = (o4 & 0x0F0F0F0Fu) | (o8 & 0xF0F0F0F0u);
         }
         uint8_t* d = s_codes + ((size_t)blk * COL_TN + 2 * lane) * BLK_BYTES + 8 * h;
-        *reinterpret_cast<uint2*>(d) = make_uint2((uint32_t)o0, (uint32_t)(o0 >> 32));
-        *reinterpret_cast<uint2*>(d + BLK_BYTES) = make_uint2((uint32_t)o1, (uint32_t)(o1 >> 32));
+        *reinterpret_cast<uint2*>(d) = make_uint2(__byte_perm(u0[0], u0[1], 0x6420), __byte_perm(u0[2], u0[3], 0x6420));
+        *reinterpret_cast<uint2*>(d + BLK_BYTES) = make_uint2(__byte_perm(u1[0], u1[1], 0x6420), __byte_perm(u1[2], u1[3], 0x6420));
       }
     } else {
       // FP8: one byte per element, no transform (the reference asserts that MXFP8 runs
@@ -829,8 +817,9 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
           float q0[4], q1[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            q0[j] = scale_elem<FMT, IN_BF16, FAST>(v0[k + j], s0);
-            q1[j] = scale_elem<FMT, IN_BF16, FAST>(v1[k + j], s1);
+            const float2 x = slot(k + j);
+            q0[j] = scale_elem<FMT, IN_BF16, FAST>(x.x, s0);
+            q1[j] = scale_elem<FMT, IN_BF16, FAST>(x.y, s1);
           }
           *reinterpret_cast<uint32_t*>(d + k) = fp8x2_rtn_hw<F::E5M2>(q0[0], q0[1]) |
                                                 (fp8x2_rtn_hw<F::E5M2>(q0[2], q0[3]) << 16);
@@ -1596,7 +1585,7 @@ static int fill_rht(RhtParams* r, int n, const int32_t* perm, const int32_t* sig
   if (n == 0) {
     for (int i = 0; i < 16; ++i) {
       r->pinv[i] = (int8_t)i; r->perm[i] = (int8_t)i; r->sign[i] = 1.0f;
-      r->qsign[i] = 0.25f; r->perm_off[i] = i * 8;
+      r->qsign[i] = 0.25f;
     }
     return ALTOB200_OK;
   }
@@ -1616,7 +1605,9 @@ static int fill_rht(RhtParams* r, int n, const int32_t* perm, const int32_t* sig
   }
   for (int k = 0; k < 16; ++k) {
     r->qsign[k] = 0.25f * r->sign[k];
-    r->perm_off[k] = (int)r->pinv[k] * 8;
+    if ((k & 3) == 0) r->psel[k >> 2] = r->pmask[k >> 2] = 0u;
+    r->psel[k >> 2] |= (uint32_t)(perm[k] & 7) << (4 * (k & 3));
+    r->pmask[k >> 2] |= (perm[k] & 8) != 0 ? 0xFFu << (8 * (k & 3)) : 0u;
   }
   return ALTOB200_OK;
 }
@@ -1644,30 +1635,43 @@ static int launch_rowwise(const RowwiseArgs& a, int rounding, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }
 
+template <int FMT, bool IN_BF16, int ROUND, bool RHT>
+static void launch_colwise_kernel(const ColwiseArgs& a, cudaStream_t st) {
+  const dim3 grid((unsigned)ceil_div(a.cols, COL_TN), (unsigned)ceil_div(a.rows, COL_NT)), block(COL_NT);
+  constexpr bool CAN_MACRO = FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && (ROUND == ALTOB200_ROUND_RTN || ROUND == ALTOB200_ROUND_SR_SLOTS);
+  if (CAN_MACRO && a.macro_codes != nullptr)
+    (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, ROUND, RHT, CAN_MACRO>, grid, block, 0, st, a);
+  else
+    (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, ROUND, RHT, false>, grid, block, 0, st, a);
+}
+
 template <int FMT, bool IN_BF16>
 static int launch_colwise(const ColwiseArgs& a, int rounding, cudaStream_t st) {
+  constexpr bool FP4 = Fmt<FMT>::FP4;
   const bool rht = a.rht.n != 0;
-  if (!Fmt<FMT>::FP4 && (rht || rounding != ALTOB200_ROUND_RTN)) return ALTOB200_EUNSUPPORTED;
-  const unsigned gx = (unsigned)ceil_div(a.cols, COL_TN);
-  if (rounding == ALTOB200_ROUND_RTN) {
-    constexpr int NT = COL_NT;
-    const dim3 grid(gx, (unsigned)ceil_div(a.rows, NT));
-    if (rht) (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, Fmt<FMT>::FP4>, dim3(grid), dim3(NT), 0, st, a);
-    else (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, false>, dim3(grid), dim3(NT), 0, st, a);
-  } else if (rounding == ALTOB200_ROUND_SR_BITS) {
-    constexpr int R = Fmt<FMT>::FP4 ? ALTOB200_ROUND_SR_BITS : ALTOB200_ROUND_RTN;
-    constexpr int NT = COL_NT;
-    const dim3 grid(gx, (unsigned)ceil_div(a.rows, NT));
-    if (rht) (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, R, Fmt<FMT>::FP4>, dim3(grid), dim3(NT), 0, st, a);
-    else (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, R, false>, dim3(grid), dim3(NT), 0, st, a);
-  } else if (rounding == ALTOB200_ROUND_SR_PHILOX) {
-    constexpr int R = Fmt<FMT>::FP4 ? ALTOB200_ROUND_SR_PHILOX : ALTOB200_ROUND_RTN;
-    constexpr int NT = COL_NT;
-    const dim3 grid(gx, (unsigned)ceil_div(a.rows, NT));
-    if (rht) (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, R, Fmt<FMT>::FP4>, dim3(grid), dim3(NT), 0, st, a);
-    else (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, R, false>, dim3(grid), dim3(NT), 0, st, a);
-  } else {
-    return ALTOB200_EUNSUPPORTED;
+  if (!FP4 && (rht || rounding != ALTOB200_ROUND_RTN)) return ALTOB200_EUNSUPPORTED;
+  constexpr int BITS = FP4 ? ALTOB200_ROUND_SR_BITS : ALTOB200_ROUND_RTN;
+  constexpr int PHILOX = FP4 ? ALTOB200_ROUND_SR_PHILOX : ALTOB200_ROUND_RTN;
+  constexpr int SLOTS = FP4 ? ALTOB200_ROUND_SR_SLOTS : ALTOB200_ROUND_RTN;
+  switch (rounding) {
+    case ALTOB200_ROUND_RTN:
+      if (rht) launch_colwise_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, FP4>(a, st);
+      else launch_colwise_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, false>(a, st);
+      break;
+    case ALTOB200_ROUND_SR_BITS:
+      if (rht) launch_colwise_kernel<FMT, IN_BF16, BITS, FP4>(a, st);
+      else launch_colwise_kernel<FMT, IN_BF16, BITS, false>(a, st);
+      break;
+    case ALTOB200_ROUND_SR_PHILOX:
+      if (rht) launch_colwise_kernel<FMT, IN_BF16, PHILOX, FP4>(a, st);
+      else launch_colwise_kernel<FMT, IN_BF16, PHILOX, false>(a, st);
+      break;
+    case ALTOB200_ROUND_SR_SLOTS:
+      if (rht) launch_colwise_kernel<FMT, IN_BF16, SLOTS, FP4>(a, st);
+      else launch_colwise_kernel<FMT, IN_BF16, SLOTS, false>(a, st);
+      break;
+    default:
+      return ALTOB200_EUNSUPPORTED;
   }
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }
@@ -1740,6 +1744,22 @@ __global__ void __launch_bounds__(256) philox_tile_kernel(uint32_t* out, int64_t
   }
 }
 
+// The same words of a 64 x 32 table as the column-wise quantizer reads them: [position][row], where the
+// positions (two per pair) of every group of 16 are in the order of the transform's slots (position pinv[k]
+// is slot k; the identity without a transform).
+struct SlotOrder {
+  int8_t pinv[16];
+};
+__global__ void __launch_bounds__(256) philox_slots_kernel(uint32_t* out, uint32_t offset, PhiloxKeys pk, SlotOrder order) {
+  grid_dependency_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;   // row fastest: neighbouring threads write neighbours
+  const int row = i & 63, slot = i >> 6;                 // slot of the 64 positions
+  const int pos = (slot & ~15) + order.pinv[slot & 15];
+  uint32_t o[4];
+  philox4x32_10_keys(offset + (uint32_t)(row * 32 + (pos >> 1)), 0u, pk, o);
+  out[slot * 64 + row] = (pos & 1) != 0 ? o[1] : o[0];
+}
+
 // clip_mode / use_uos exist for MXFP4 only, as in the reference
 static int fill_mx_opts(MxOpts* o, const altob200_quant_params* p, bool allow_dynamic) {
   o->clip = p->clip_mode;
@@ -1790,6 +1810,24 @@ int altob200_philox_tile(uint64_t seed, uint64_t offset, int64_t tile_rows, int6
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }
 
+int altob200_philox_slots(uint64_t seed, uint64_t offset, int32_t rht_n, const int32_t* rht_perm, uint32_t* out,
+                          void* stream) {
+  if (out == nullptr || (rht_n != 0 && (rht_n != 16 || rht_perm == nullptr))) return ALTOB200_EINVAL_SHAPE;
+  if (!aligned16(out)) return ALTOB200_EINVAL_ALIGN;
+  SlotOrder order;
+  bool seen[16] = {false};
+  for (int i = 0; i < 16; ++i) {
+    const int k = rht_n != 0 ? rht_perm[i] : i;
+    if (k < 0 || k > 15 || seen[k]) return ALTOB200_EINVAL_SHAPE;
+    seen[k] = true;
+    order.pinv[k] = (int8_t)i;
+  }
+  PhiloxKeys pk;
+  philox_make_keys(seed, &pk);
+  (void)launch_after(philox_slots_kernel, dim3(16), dim3(256), 0, (cudaStream_t)stream, out, (uint32_t)offset, pk, order);
+  return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
+}
+
 int altob200_quantize_rowwise(const void* x, int64_t rows, int64_t cols, int64_t ld,
                               const altob200_quant_params* p, void* codes, void* scale_plain,
                               void* scale_packed, void* stream) {
@@ -1837,8 +1875,18 @@ int altob200_quantize_colwise(const void* x, int64_t rows, int64_t cols, int64_t
   if (!aligned16(x) || (ld * esz) % 16 != 0 || !aligned16(codes) || out_row_bytes % 16 != 0)
     return ALTOB200_EINVAL_ALIGN;
   if (p->rounding == ALTOB200_ROUND_SR_BITS && p->rand_bits == nullptr) return ALTOB200_EINVAL_SHAPE;
+  if (p->rounding == ALTOB200_ROUND_SR_SLOTS) {
+    // one word pair per lane and slot: the table has 64 rows, and column c of an 8-byte load is even
+    if (p->rand_bits == nullptr || p->rand_tile_rows != 64 || p->rand_tile_pairs != 32) return ALTOB200_EINVAL_SHAPE;
+    if (!aligned16(p->rand_bits)) return ALTOB200_EINVAL_ALIGN;
+  }
   cudaStream_t st = (cudaStream_t)stream;
   ColwiseArgs a;
+  a.macro_codes = (uint8_t*)p->macro_codes;
+  if (a.macro_codes != nullptr &&
+      (p->format != ALTOB200_FMT_MXFP4 || p->in_dtype != ALTOB200_DT_BF16 ||
+       (p->rounding != ALTOB200_ROUND_RTN && p->rounding != ALTOB200_ROUND_SR_SLOTS)))
+    return ALTOB200_EUNSUPPORTED;
   a.x = x; a.rows = rows; a.cols = cols; a.ld = ld;
   a.codes = (uint8_t*)codes; a.scale_plain = scale_plain; a.scale_packed = (uint8_t*)scale_packed;
   a.ncol_tiles = ceil_div(rows / B, 4);

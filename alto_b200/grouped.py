@@ -154,7 +154,8 @@ class GroupedLinearFunction(torch.autograd.Function):
             g_n = E.quant_rows(g2, ctx.fmt_grad, None if og is None else og[0:1],
                                E.sr_args(ctx.use_sr_grad, "dy_n", M, N, g2.device), ctx.use_uos)
             g_m = E.cols_operand(g2, ctx.fmt_grad, ctx.use_outer_scale, og, ctx.rht, ctx.dense_transform,
-                                 E.sr_args(ctx.use_sr_grad, "dy_m", N, M, g2.device), ctx.use_uos, ctx.clip_mode)
+                                 E.sr_args_cols(ctx.use_sr_grad, "dy_m", N, M, g2.device, ctx.rht), ctx.use_uos,
+                                 ctx.clip_mode)
         grad_inputs = grad_weights = None
         if ctx.needs_input_grad[0]:
             grad_inputs = _grouped_gemm(g_n, w_t, K, n_exp, group_expert, grad_output.dtype)

@@ -61,6 +61,7 @@ extern "C" {
 #define ALTOB200_ROUND_RTN 0
 #define ALTOB200_ROUND_SR_BITS 1   /* stochastic rounding, caller supplies 32 random bits per element */
 #define ALTOB200_ROUND_SR_PHILOX 2 /* stochastic rounding, Philox-4x32-10 generated in the kernel     */
+#define ALTOB200_ROUND_SR_SLOTS 3  /* column-wise quantizer: words from a table of altob200_philox_slots */
 
 int altob200_version(void);
 const char* altob200_status_string(int status);
@@ -125,6 +126,13 @@ typedef struct altob200_quant_params {
    * row-wise quantizer.                                                                  */
   int64_t rand_tile_rows;
   int64_t rand_tile_pairs;
+  /* Two-level ("blockwise") MXFP4 from bf16, or NULL: every macro block of 128 elements along the
+   * quantisation axis (128 x 128 tiles for the 2-D quantizer) is first multiplied by its factor and rounded
+   * to bf16, exactly what altob200_macro_block_scaling writes, and the factor codes go to macro_codes in
+   * that function's layout (row-wise: [rows, ceil(cols/128)], column-wise: [cols, ceil(rows/128)], 2-D:
+   * [batch, ceil(rows/128), ceil(cols/128)]).  Rounding RTN, or SR_BITS with a periodic table (row-wise,
+   * 2-D) / SR_SLOTS (column-wise).  The column-wise quantizer applies the Hadamard transform before it. */
+  uint8_t* macro_codes;
 } altob200_quant_params;
 
 /*
@@ -240,6 +248,15 @@ int altob200_quantize_2d(const void* w, int64_t rows, int64_t cols, int64_t ld,
 int altob200_quantize_2d_batched(const void* w, int64_t batch, int64_t batch_stride, int64_t rows, int64_t cols,
                                  int64_t ld, const altob200_quant_params* p, void* codes_k, void* codes_t,
                                  void* scale_plain, void* scale_packed_k, void* scale_packed_t, void* stream);
+
+/*
+ * The words altob200_philox_tile draws for a 64 x 32 table, laid out for the column-wise quantizer with
+ * ALTOB200_ROUND_SR_SLOTS (rand_tile_rows = 64, rand_tile_pairs = 32): out[64][64], first index the position
+ * along the quantisation axis - within every group of 16 in slot order of the Hadamard transform given by
+ * `rht_perm` (HOST array of 16; rht_n = 0: none) - second index the row of the axis-last view.
+ */
+int altob200_philox_slots(uint64_t seed, uint64_t offset, int32_t rht_n, const int32_t* rht_perm, uint32_t* out,
+                          void* stream);
 
 /*
  * The reference's table of stochastic-rounding words: out[0][m][n], out[1][m][n] = first and second
