@@ -135,31 +135,35 @@ def _code_cols(fmt: int, n: int) -> int:
     return n // 2 if L.is_fp4(fmt) else n
 
 
-def quant_rows(x2, fmt, outer, sr: dict, use_uos: bool = False) -> Operand:
+def quant_rows(x2, fmt, outer, sr: dict, use_uos: bool = False, macro_codes=None) -> Operand:
     R, Cc = x2.shape
     codes = torch.empty(R, _code_cols(fmt, Cc), dtype=torch.uint8, device=x2.device)
     sf = _packed(R, Cc // L.block_of(fmt), x2.device)
-    L.quantize_rowwise(x2, fmt, codes, None, sf, outer_scale=outer, use_uos=use_uos, **sr)
+    L.quantize_rowwise(x2, fmt, codes, None, sf, outer_scale=outer, use_uos=use_uos, macro_codes=macro_codes,
+                       **sr)
     return Operand(codes, sf, outer, R, Cc, fmt)
 
 
-def quant_cols(x2, fmt, outer, rht, sr: dict, use_uos: bool = False, clip_mode: str = "none") -> Operand:
+def quant_cols(x2, fmt, outer, rht, sr: dict, use_uos: bool = False, clip_mode: str = "none",
+               macro_codes=None) -> Operand:
     R, Cc = x2.shape
     codes = torch.empty(Cc, _code_cols(fmt, R), dtype=torch.uint8, device=x2.device)
     sf = _packed(Cc, R // L.block_of(fmt), x2.device)
     L.quantize_colwise(x2, fmt, codes, None, sf, outer_scale=outer, rht=rht, use_uos=use_uos, clip_mode=clip_mode,
-                       **sr)
+                       macro_codes=macro_codes, **sr)
     return Operand(codes, sf, outer, Cc, R, fmt)
 
 
-def quant_2d(x2, fmt, outer, want_t: bool, use_uos: bool = False, sr: Optional[dict] = None) -> Tuple[Operand, Optional[Operand]]:
+def quant_2d(x2, fmt, outer, want_t: bool, use_uos: bool = False, sr: Optional[dict] = None,
+             macro_codes=None) -> Tuple[Operand, Optional[Operand]]:
     R, Cc = x2.shape
     b = L.block_of(fmt)
     ck = torch.empty(R, _code_cols(fmt, Cc), dtype=torch.uint8, device=x2.device)
     sk = _packed(R, Cc // b, x2.device)
     ct = torch.empty(Cc, _code_cols(fmt, R), dtype=torch.uint8, device=x2.device) if want_t else None
     stt = _packed(Cc, R // b, x2.device) if want_t else None
-    L.quantize_2d(x2, fmt, ck, ct, None, sk, stt, outer_scale=outer, use_uos=use_uos, **(sr or {}))
+    L.quantize_2d(x2, fmt, ck, ct, None, sk, stt, outer_scale=outer, use_uos=use_uos,
+                  macro_codes=macro_codes, **(sr or {}))
     return Operand(ck, sk, outer, R, Cc, fmt), (Operand(ct, stt, outer, Cc, R, fmt) if want_t else None)
 
 

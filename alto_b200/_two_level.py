@@ -17,6 +17,7 @@ they are for every axis and block shape.
 """
 from __future__ import annotations
 
+import functools
 from typing import Optional, Tuple
 
 import torch
@@ -30,18 +31,47 @@ MX = L.FMT_MXFP4
 STATIC_CLIP_WGRAD = 16.0 / 9.0
 
 
+def _fusable(t: torch.Tensor) -> bool:
+    """The quantizers apply the macro factors themselves to bf16 tensors whose rows they can read as they are
+    (16-byte alignment); for the rest ``macro_block_scaling`` runs first.  Same codes, scales and factors."""
+    return (t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.data_ptr() % 16 == 0
+            and all(st * t.element_size() % 16 == 0 for st in t.stride()[:-1]))
+
+
+def _chunks(n: int) -> int:
+    return (n + 127) // 128
+
+
 def rows_operand(t2: torch.Tensor, use_uos: bool, sr: Optional[dict] = None) -> E.Operand:
     """t2 [R, C] -> operand [R, C] reduced along C: 1-D macro blocks and MXFP4 blocks along the last axis."""
-    ts, mbs = macro_block_scaling(t2, axis=-1, use_2d_block=False)            # mbs [R, ceil(C/128)]
-    op = E.quant_rows(ts, MX, None, sr or E.RTN, use_uos)
+    if _fusable(t2):
+        R, Cc = t2.shape
+        mbs = torch.empty(R, _chunks(Cc), dtype=torch.uint8, device=t2.device)
+        op = E.quant_rows(t2, MX, None, sr or E.RTN, use_uos, macro_codes=mbs)
+    else:
+        ts, mbs = macro_block_scaling(t2, axis=-1, use_2d_block=False)        # mbs [R, ceil(C/128)]
+        op = E.quant_rows(ts, MX, None, sr or E.RTN, use_uos)
     op.macro = L.MacroScale(mbs, mbs.shape[-1], 1, 0)
     return op
 
 
-def cols_operand(t2: torch.Tensor, use_uos: bool, clip_mode: str = "none", sr: Optional[dict] = None) -> E.Operand:
-    """t2 [R, C] -> operand [C, R] reduced along R (the token axis): blocks run down the rows of t2."""
-    ts, mbs = macro_block_scaling(t2, axis=0, use_2d_block=False)             # mbs [C, ceil(R/128)]
-    op = E.quant_cols(ts, MX, None, None, sr or E.RTN, use_uos, clip_mode)
+def cols_operand(t2: torch.Tensor, use_uos: bool, clip_mode: str = "none", sr: Optional[dict] = None,
+                 hadamard_transform=None) -> E.Operand:
+    """t2 [R, C] -> operand [C, R] reduced along R (the token axis) after the optional rotation: blocks run
+    down the rows of t2.  ``sr`` from ``E.sr_args_cols`` with the transform's ``rht_of``."""
+    rht = rht_of(hadamard_transform)
+    sr = sr or E.RTN
+    if rht is None:
+        t2 = _rotate(t2, hadamard_transform)
+    if _fusable(t2) and sr["rounding"] in (L.ROUND_RTN, L.ROUND_SR_SLOTS):
+        R, Cc = t2.shape
+        mbs = torch.empty(Cc, _chunks(R), dtype=torch.uint8, device=t2.device)
+        op = E.quant_cols(t2, MX, None, rht, sr, use_uos, clip_mode, macro_codes=mbs)
+    else:
+        if rht is not None:
+            t2 = _rotate(t2, hadamard_transform)
+        ts, mbs = macro_block_scaling(t2, axis=0, use_2d_block=False)         # mbs [C, ceil(R/128)]
+        op = E.quant_cols(ts, MX, None, None, sr, use_uos, clip_mode)
     op.macro = L.MacroScale(mbs, mbs.shape[-1], 1, 0)
     return op
 
@@ -49,8 +79,13 @@ def cols_operand(t2: torch.Tensor, use_uos: bool, clip_mode: str = "none", sr: O
 def tiles_operands(t2: torch.Tensor, use_uos: bool, sr: Optional[dict] = None) -> Tuple[E.Operand, E.Operand]:
     """t2 [R, C] in 128 x 128 macro tiles and 32 x 32 MXFP4 blocks, quantised once:
     -> (operand [R, C] reduced along C, operand [C, R] reduced along R)."""
-    ts, mbs = macro_block_scaling(t2, axis=-1, use_2d_block=True)             # mbs [ceil(R/128), ceil(C/128)]
-    op_k, op_t = E.quant_2d(ts, MX, None, True, use_uos, sr)
+    if _fusable(t2):
+        R, Cc = t2.shape
+        mbs = torch.empty(_chunks(R), _chunks(Cc), dtype=torch.uint8, device=t2.device)
+        op_k, op_t = E.quant_2d(t2, MX, None, True, use_uos, sr, macro_codes=mbs)
+    else:
+        ts, mbs = macro_block_scaling(t2, axis=-1, use_2d_block=True)         # mbs [ceil(R/128), ceil(C/128)]
+        op_k, op_t = E.quant_2d(ts, MX, None, True, use_uos, sr)
     nc = mbs.shape[-1]
     op_k.macro = L.MacroScale(mbs, nc, 1, 7)
     op_t.macro = L.MacroScale(mbs, 1, nc, 7)
@@ -62,6 +97,13 @@ def gemm(a: E.Operand, b: E.Operand, out_dtype: torch.dtype, out_scale: float = 
     out = torch.empty(a.rows, b.rows, dtype=out_dtype, device=a.codes.device)
     L.gemm_mxfp4_two_level(a.rows, b.rows, a.k, a.codes, a.scales, a.macro, b.codes, b.scales, b.macro, out, out_scale)
     return out
+
+
+def rht_of(hadamard_transform) -> Optional[L.Rht]:
+    """The transform as launch parameters where the column-wise quantizer can apply it, else None."""
+    if hadamard_transform is None or not hadamard_transform.is_fused:
+        return None
+    return hadamard_transform.device_params()
 
 
 def _rotate(t2: torch.Tensor, hadamard_transform) -> torch.Tensor:
@@ -89,8 +131,11 @@ def _grad_operands(ctx, g2: torch.Tensor, M: int, N: int) -> Tuple[E.Operand, E.
     if ctx.use_2dblock_x:
         return tiles_operands(g2, ctx.use_uos, E.sr_args(ctx.use_sr_grad, "dy_n", M, N, g2.device))
     g_n = rows_operand(g2, ctx.use_uos, E.sr_args(ctx.use_sr_grad, "dy_n", M, N, g2.device))
-    g_m = cols_operand(_rotate(g2, ctx.hadamard_transform), ctx.use_uos, ctx.clip_mode,
-                       E.sr_args(ctx.use_sr_grad, "dy_m", N, M, g2.device))
+    # (words in slot order only fit the fused kernel, so an input it cannot read takes the plain table)
+    rht = rht_of(ctx.hadamard_transform)
+    draw = E.sr_args if not _fusable(g2) else functools.partial(E.sr_args_cols, rht=rht)
+    g_m = cols_operand(g2, ctx.use_uos, ctx.clip_mode, draw(ctx.use_sr_grad, "dy_m", N, M, g2.device),
+                       ctx.hadamard_transform)
     return g_n, g_m
 
 
@@ -125,7 +170,7 @@ def linear_forward(ctx, x, weight, use_2dblock_x: bool, use_2dblock_w: bool, use
     if not use_2dblock_w:
         w_t = cols_operand(w2, use_uos)
     if not use_2dblock_x:
-        x_m = cols_operand(_rotate(x2, hadamard_transform), use_uos, clip_mode)
+        x_m = cols_operand(x2, use_uos, clip_mode, None, hadamard_transform)
     _save_macro(ctx, x_m, w_t)
     ctx.dims = (M, K, N)
     ctx.use_2dblock_x, ctx.use_sr_grad, ctx.hadamard_transform = use_2dblock_x, use_sr_grad, hadamard_transform
@@ -157,13 +202,19 @@ def _weight_stack(w3: torch.Tensor, use_2dblock_w: bool, use_uos: bool) -> Tuple
     """[E, N, K] -> (W along K stacked [E*N, K], W along N stacked [E*K, N]) with per-expert factor codes."""
     n_exp, N, K = w3.shape
     if use_2dblock_w:
-        ws, mbs = macro_block_scaling(w3, axis=-1, use_2d_block=True)        # mbs [E, ceil(N/128), ceil(K/128)]
+        # mbs [E, ceil(N/128), ceil(K/128)]
+        if _fusable(w3):
+            ws, fused = w3, dict(macro_codes=torch.empty(n_exp, _chunks(N), _chunks(K), dtype=torch.uint8,
+                                                         device=w3.device))
+            mbs = fused["macro_codes"]
+        else:
+            (ws, mbs), fused = macro_block_scaling(w3, axis=-1, use_2d_block=True), {}
         cc = E._code_cols(MX, K)
         ck = torch.empty(n_exp, N, cc, dtype=torch.uint8, device=w3.device)
         ct = torch.empty(n_exp, K, E._code_cols(MX, N), dtype=torch.uint8, device=w3.device)
         sk = torch.empty(n_exp * L.packed_scale_bytes(N, K // 32), dtype=torch.uint8, device=w3.device)
         st = torch.empty(n_exp * L.packed_scale_bytes(K, N // 32), dtype=torch.uint8, device=w3.device)
-        L.quantize_2d_batched(ws, MX, ck, ct, None, sk, st, use_uos=use_uos)
+        L.quantize_2d_batched(ws, MX, ck, ct, None, sk, st, use_uos=use_uos, **fused)
         w_k = E.Operand(ck.view(n_exp * N, cc), sk, None, n_exp * N, K, MX)
         w_t = E.Operand(ct.view(n_exp * K, -1), st, None, n_exp * K, N, MX)
         nr, nc = mbs.shape[-2], mbs.shape[-1]
@@ -210,7 +261,7 @@ class GroupedTwoLevelFunction(torch.autograd.Function):
             x_k, x_m = tiles_operands(x2, use_uos)
         else:
             x_k = rows_operand(x2, use_uos)
-            x_m = cols_operand(_rotate(x2, hadamard_transform), use_uos, clip_mode)
+            x_m = cols_operand(x2, use_uos, clip_mode, None, hadamard_transform)
         w_k, w_t = _weight_stack(w3, use_2dblock_w, use_uos)
         y = torch.empty(M, N, dtype=inputs.dtype, device=inputs.device)
         L.gemm_mxfp4_two_level(M, N, K, x_k.codes, x_k.scales, x_k.macro, w_k.codes, w_k.scales, w_k.macro, y,

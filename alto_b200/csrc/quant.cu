@@ -242,6 +242,15 @@ __device__ __forceinline__ uint32_t fold_bf16x2(uint32_t acc) {
   return lo > hi ? lo : hi;
 }
 
+__device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const uint32_t t = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    v = t > v ? t : v;
+  }
+  return v;
+}
+
 // =======================================================================================
 // Row-wise quantizer
 // =======================================================================================
@@ -259,6 +268,7 @@ struct RowwiseArgs {
   uint64_t philox_seed, philox_offset;
   PhiloxKeys pk;
   MxOpts mx;
+  uint8_t* macro_codes;  // MACRO: [rows, ceil(cols / 128)] factor codes, written
 };
 
 // A warp task is 4 consecutive rows x 512 contiguous columns (a lane: 16 columns of each row).  The
@@ -269,10 +279,14 @@ struct RowwiseArgs {
 // spill, more leave too few warps to cover the issue slots.
 constexpr int ROW_R = 4;
 
-template <int FMT, bool IN_BF16, int ROUND>
+// MACRO (MXFP4 from bf16): the two-level recipe's scaling runs in front of the quantisation; a macro block of
+// 128 columns is eight neighbouring lanes.
+template <int FMT, bool IN_BF16, int ROUND, bool MACRO>
 __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a) {
   grid_dependency_wait();
   using F = Fmt<FMT>;
+  static_assert(!MACRO || (FMT == ALTOB200_FMT_MXFP4 && IN_BF16), "macro blocks");
+  const int64_t macro_chunks = (a.cols + 127) >> 7;
   constexpr int LPB = F::B / 16;  // lanes per block
   constexpr int ESZ = IN_BF16 ? 2 : 4;
   constexpr int NV = IN_BF16 ? 2 : 4;  // 16-byte vectors per lane and row
@@ -378,6 +392,29 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
         for (int j = 0; j < 16; ++j) {
           const uint32_t b = f2u(v[j]) & 0x7FFFFFFFu;
           amax_bits = b > amax_bits ? b : amax_bits;
+        }
+      }
+      if (MACRO) {
+        // factor of the row's 128 columns (NaNs do not take part in the maximum, csrc/macro_scale.cu), then
+        // y = bf16(x * factor); rounding is monotone, so the lane's maximum is scaled instead of searched again
+        float m = u2f(amax_bits << 16);
+        if (__any_sync(0xFFFFFFFFu, amax_bits > 0x7F80u)) {
+          m = 0.0f;
+#pragma unroll
+          for (int j = 0; j < 16; ++j) m = fmaxf(m, fabsf(v[j]));
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+        uint32_t code;
+        const float f = macro_factor_from_amax(m, &code);
+        if (active && (lane & 7) == 0) a.macro_codes[row * macro_chunks + (col >> 7)] = (uint8_t)code;
+        amax_bits = f32_to_bf16_bits(__fmul_rn(u2f(amax_bits << 16), f)) & 0x7FFFu;
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+          const __nv_bfloat162 p2 = __floats2bfloat162_rn(__fmul_rn(v[j], f), __fmul_rn(v[j + 1], f));
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(&p2);
+          v[j] = bf16lo_to_f32(w);
+          v[j + 1] = bf16hi_to_f32(w);
         }
       }
       if (LPB == 2) {
@@ -910,6 +947,7 @@ struct Quant2dArgs {
   // batch of equally shaped matrices: input stride in elements, outputs stacked contiguously; the
   // rows of the stochastic-rounding view are the rows of all matrices, one after the other
   int64_t batch, batch_stride, packed_k_bytes, packed_t_bytes;
+  uint8_t* macro_codes;  // MACRO: [batch, ceil(rows / 128), ceil(cols / 128)] factor codes, written
 };
 
 // 4 x 4 byte transpose: out[b] = (in[0].byte b, in[1].byte b, in[2].byte b, in[3].byte b)
@@ -930,7 +968,9 @@ __device__ __forceinline__ void transpose4x4_bytes(const uint32_t* in, uint32_t*
 // contiguous bytes per row per warp); for the transposed packing the thread's 16 x 8 codes are
 // transposed in registers (nibble merge of row pairs, then 4 x 4 byte transposes) and every column
 // receives 8 (FP4) or 16 (FP8) contiguous bytes per lane, 32 contiguous bytes per warp and column.
-template <int FMT, bool IN_BF16, int ROUND, bool BATCHED>
+// MACRO (MXFP4 from bf16): the two-level recipe's scaling of 128 x 128 tiles runs in front of the quantisation;
+// a tile is four warps of 32 rows x 128 columns, whose maxima meet in shared memory.
+template <int FMT, bool IN_BF16, int ROUND, bool BATCHED, bool MACRO>
 __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
   grid_dependency_wait();
   using F = Fmt<FMT>;
@@ -940,9 +980,14 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
   constexpr int TR = 16 * LR, TC = 8 * LC;  // warp tile: 64 x 64 or 32 x 128
   constexpr int ESZ = IN_BF16 ? 2 : 4;
   const int lane = threadIdx.x & 31;
-  const int64_t tiles_c = (a.cols + TC - 1) / TC, tiles_r = (a.rows + TR - 1) / TR;
+  static_assert(!MACRO || (FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && TR == 32 && TC == 128), "macro tiles");
+  // MACRO: row tiles are counted in whole macro tiles, and four consecutive warps take one of them
+  const int64_t tiles_c = (a.cols + TC - 1) / TC;
+  const int64_t tiles_r = MACRO ? ((a.rows + 127) >> 7) * 4 : (a.rows + TR - 1) / TR;
   const int64_t tile_all = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (tile_all >= tiles_c * tiles_r * a.batch) return;  // whole warps leave; nothing below synchronises the block
+  // (without MACRO whole warps leave: nothing below synchronises the block)
+  const bool live = tile_all < tiles_c * tiles_r * a.batch;
+  if (!MACRO && !live) return;
   // matrix `bi` of the batch: its outputs follow those of matrix bi - 1, so the batch index enters the
   // addresses as extra rows (bi * rows for the K packing, bi * cols for the transposed one)
   // (BATCHED is a template parameter so that the single-matrix kernel carries none of this arithmetic)
@@ -950,7 +995,13 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
   if (BATCHED) divmod_fast(tile_all, tiles_c * tiles_r, &bi, &tile);
   const int64_t rows_before = BATCHED ? bi * a.rows : 0, cols_before = BATCHED ? bi * a.cols : 0;
   int64_t tr, tc;
-  divmod_fast(tile, tiles_c, &tr, &tc);
+  if (MACRO) {
+    int64_t mr;
+    divmod_fast(tile >> 2, tiles_c, &mr, &tc);
+    tr = live ? mr * 4 + (tile & 3) : tiles_r;   // a warp without a tile lies below the matrix
+  } else {
+    divmod_fast(tile, tiles_c, &tr, &tc);
+  }
   const int lc = lane % LC, lr = lane / LC;
   const int64_t row0 = tr * TR + lr * 16, col0 = tc * TC + lc * 8;
   const bool ok = row0 < a.rows && col0 < a.cols;  // rows % B == 0 and cols % B == 0
@@ -972,6 +1023,30 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
       acc = absmax2_bf16x2(absmax2_bf16x2(acc, raw[i].x, raw[i].y), raw[i].z, raw[i].w);
     }
     amax_bits = fold_bf16x2(acc);
+    if (MACRO) {
+      __shared__ uint32_t s_macro[8];
+      const uint32_t wm = warp_max_u32(amax_bits);
+      const int warp = threadIdx.x >> 5;
+      if (lane == 0) s_macro[warp] = wm;
+      __syncthreads();
+      uint32_t m = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m = s_macro[(warp & 4) + i] > m ? s_macro[(warp & 4) + i] : m;
+      uint32_t code;
+      const float f = macro_factor_from_amax(u2f(m << 16), &code);
+      if (live && (warp & 3) == 0 && lane == 0)
+        a.macro_codes[(bi * (tiles_r >> 2) + (tr >> 2)) * tiles_c + tc] = (uint8_t)code;
+      // y = bf16(x * factor); rounding is monotone, so the maximum is scaled instead of searched again
+      auto scaled = [&](uint32_t w) {
+        const __nv_bfloat162 p2 = __floats2bfloat162_rn(__fmul_rn(bf16lo_to_f32(w), f), __fmul_rn(bf16hi_to_f32(w), f));
+        return *reinterpret_cast<const uint32_t*>(&p2);
+      };
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        raw[i % (IN_BF16 ? 16 : 1)] = make_uint4(scaled(raw[i % (IN_BF16 ? 16 : 1)].x), scaled(raw[i % (IN_BF16 ? 16 : 1)].y),
+                                                 scaled(raw[i % (IN_BF16 ? 16 : 1)].z), scaled(raw[i % (IN_BF16 ? 16 : 1)].w));
+      amax_bits = scaled(amax_bits) & 0x7FFFu;
+    }
     if (stats) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -1190,15 +1265,6 @@ struct AmaxArgs {
   uint32_t* counter;     // scratch [4]: ticket counter, running maxima; zero on entry, zero on exit
   RhtParams rht;
 };
-
-__device__ __forceinline__ uint32_t warp_max_u32(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const uint32_t t = __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    v = t > v ? t : v;
-  }
-  return v;
-}
 
 // outer = max(nan_to_num(amax) / (448 * 6), 1e-30)
 //   alto/kernels/fp4/nvfp4/nvfp_quantization.py:484-487
@@ -1617,19 +1683,29 @@ static void fill_rht_row_offsets(RhtParams* r, int64_t ld, int esz) {
   for (int k = 0; k < 16; ++k) r->row_off[k] = (int64_t)r->pinv[k] * ld * esz;
 }
 
-template <int FMT, bool IN_BF16>
-static int launch_rowwise(const RowwiseArgs& a, int rounding, cudaStream_t st) {
+template <int FMT, bool IN_BF16, int ROUND>
+static void launch_rowwise_kernel(const RowwiseArgs& a, cudaStream_t st) {
   const int64_t tasks = ceil_div(a.rows, ROW_R) * ((a.cols + 511) >> 9);
   int64_t blocks = ceil_div(tasks, 8);
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
+  constexpr bool CAN_MACRO = FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && ROUND != ALTOB200_ROUND_SR_PHILOX;
+  if (CAN_MACRO && a.macro_codes != nullptr)
+    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, CAN_MACRO>, dim3((unsigned)blocks), dim3(256), 0, st, a);
+  else
+    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, false>, dim3((unsigned)blocks), dim3(256), 0, st, a);
+}
+
+template <int FMT, bool IN_BF16>
+static int launch_rowwise(const RowwiseArgs& a, int rounding, cudaStream_t st) {
+  constexpr bool FP4 = Fmt<FMT>::FP4;
   if (rounding == ALTOB200_ROUND_RTN)
-    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN>, dim3((unsigned)blocks), dim3(256), 0, st, a);
-  else if (rounding == ALTOB200_ROUND_SR_BITS && Fmt<FMT>::FP4)
-    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, Fmt<FMT>::FP4 ? ALTOB200_ROUND_SR_BITS : ALTOB200_ROUND_RTN>, dim3((unsigned)blocks), dim3(256), 0, st, a);
-  else if (rounding == ALTOB200_ROUND_SR_PHILOX && Fmt<FMT>::FP4)
-    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, Fmt<FMT>::FP4 ? ALTOB200_ROUND_SR_PHILOX : ALTOB200_ROUND_RTN>, dim3((unsigned)blocks), dim3(256), 0, st, a);
+    launch_rowwise_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN>(a, st);
+  else if (rounding == ALTOB200_ROUND_SR_BITS && FP4)
+    launch_rowwise_kernel<FMT, IN_BF16, FP4 ? ALTOB200_ROUND_SR_BITS : ALTOB200_ROUND_RTN>(a, st);
+  else if (rounding == ALTOB200_ROUND_SR_PHILOX && FP4)
+    launch_rowwise_kernel<FMT, IN_BF16, FP4 ? ALTOB200_ROUND_SR_PHILOX : ALTOB200_ROUND_RTN>(a, st);
   else
     return ALTOB200_EUNSUPPORTED;
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
@@ -1676,20 +1752,28 @@ static int launch_colwise(const ColwiseArgs& a, int rounding, cudaStream_t st) {
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }
 
-template <int FMT, bool IN_BF16>
-static int launch_2d(const Quant2dArgs& a, int rounding, cudaStream_t st) {
+template <int FMT, bool IN_BF16, int ROUND, bool BATCHED>
+static void launch_2d_kernel(const Quant2dArgs& a, cudaStream_t st) {
   // one warp per tile of 4 block columns x (64 rows for 16-blocks, 32 rows for 32-blocks)
   constexpr int TC = 4 * Fmt<FMT>::B, TR = 1024 / Fmt<FMT>::B;
-  const int64_t tiles = ceil_div(a.cols, TC) * ceil_div(a.rows, TR) * a.batch;
-  const unsigned blocks = (unsigned)ceil_div(tiles, 8);
+  constexpr bool CAN_MACRO = FMT == ALTOB200_FMT_MXFP4 && IN_BF16;
+  const bool macro = CAN_MACRO && a.macro_codes != nullptr;
+  const int64_t tiles = ceil_div(a.cols, TC) * (macro ? ceil_div(a.rows, 128) * 4 : ceil_div(a.rows, TR)) * a.batch;
+  const dim3 blocks((unsigned)ceil_div(tiles, 8));
+  if (macro) (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, ROUND, BATCHED, CAN_MACRO>, blocks, dim3(256), 0, st, a);
+  else (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, ROUND, BATCHED, false>, blocks, dim3(256), 0, st, a);
+}
+
+template <int FMT, bool IN_BF16>
+static int launch_2d(const Quant2dArgs& a, int rounding, cudaStream_t st) {
   constexpr int SR = Fmt<FMT>::FP4 ? ALTOB200_ROUND_SR_BITS : ALTOB200_ROUND_RTN;
   const bool batched = a.batch > 1;
   if (rounding == ALTOB200_ROUND_RTN) {
-    if (batched) (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, true>, dim3(blocks), dim3(256), 0, st, a);
-    else (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, false>, dim3(blocks), dim3(256), 0, st, a);
+    if (batched) launch_2d_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, true>(a, st);
+    else launch_2d_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, false>(a, st);
   } else if (rounding == ALTOB200_ROUND_SR_BITS && Fmt<FMT>::FP4) {
-    if (batched) (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, SR, true>, dim3(blocks), dim3(256), 0, st, a);
-    else (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, SR, false>, dim3(blocks), dim3(256), 0, st, a);
+    if (batched) launch_2d_kernel<FMT, IN_BF16, SR, true>(a, st);
+    else launch_2d_kernel<FMT, IN_BF16, SR, false>(a, st);
   } else {
     return ALTOB200_EUNSUPPORTED;
   }
@@ -1841,6 +1925,10 @@ int altob200_quantize_rowwise(const void* x, int64_t rows, int64_t cols, int64_t
   if (p->rht_n != 0) return ALTOB200_EUNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   RowwiseArgs a;
+  a.macro_codes = (uint8_t*)p->macro_codes;
+  if (a.macro_codes != nullptr && (p->format != ALTOB200_FMT_MXFP4 || p->in_dtype != ALTOB200_DT_BF16 ||
+                                   p->rounding == ALTOB200_ROUND_SR_PHILOX))
+    return ALTOB200_EUNSUPPORTED;
   a.x = x; a.rows = rows; a.cols = cols; a.ld = ld;
   a.codes = (uint8_t*)codes; a.scale_plain = scale_plain; a.scale_packed = (uint8_t*)scale_packed;
   a.ncol_tiles = ceil_div(cols / B, 4);
@@ -1934,6 +2022,9 @@ int altob200_quantize_2d_batched(const void* w, int64_t batch, int64_t batch_str
   if (codes_t != nullptr && !aligned16(codes_t)) return ALTOB200_EINVAL_ALIGN;
   cudaStream_t st = (cudaStream_t)stream;
   Quant2dArgs a;
+  a.macro_codes = (uint8_t*)p->macro_codes;
+  if (a.macro_codes != nullptr && (p->format != ALTOB200_FMT_MXFP4 || p->in_dtype != ALTOB200_DT_BF16))
+    return ALTOB200_EUNSUPPORTED;
   a.w = w; a.rows = rows; a.cols = cols; a.ld = ld;
   a.codes_k = (uint8_t*)codes_k; a.codes_t = (uint8_t*)codes_t; a.scale_plain = scale_plain;
   a.packed_k = (uint8_t*)scale_packed_k; a.packed_t = (uint8_t*)scale_packed_t;

@@ -1,0 +1,131 @@
+"""The quantizers' fused forms against the passes they stand for, bit for bit: the two-level macro scaling inside
+the quantizers, and stochastic rounding from a slot-ordered table."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from alto_b200 import _lib as L
+from alto_b200 import _linear as E
+from alto_b200.hadamard import HadamardFactory
+from alto_b200.macro_block_scaling import macro_block_scaling
+
+MX = L.FMT_MXFP4
+
+
+def _transform():
+    HadamardFactory.configure(block_size=16, randomized=True, dtype=torch.float32, seed=11)
+    return HadamardFactory.create_transform(device="cuda")
+
+
+def _matrix(rows, cols, kind, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(rows, cols, generator=g) * torch.exp2(torch.randint(-12, 12, (rows, 1), generator=g).float())
+    if kind == "special":
+        r = torch.rand(rows, cols, generator=g)
+        x = torch.where(r < 0.2, torch.zeros(()), x)
+        x = torch.where((r >= 0.2) & (r < 0.3), -torch.zeros(()), x)
+        x[: rows // 3] = 0.0
+        x[rows // 2, cols // 2] = float("inf")
+        x[rows - 1, 0] = float("-inf")
+        x[0, cols - 1] = float("nan")
+    return x.bfloat16().cuda()
+
+
+def _sr(rounding, rows, cols, rht=None, slots=False):
+    if rounding == "rtn":
+        return E.RTN
+    if slots:
+        return dict(rounding=L.ROUND_SR_SLOTS, rand_bits=L.philox_slots(7, 1 << 31, rht, torch.device("cuda")),
+                    rand_tile=L.SLOTS_TILE)
+    tile = L.sr_tile_dims(rows, cols)
+    return dict(rounding=L.ROUND_SR_BITS, rand_bits=L.philox_tile(7, 1 << 31, *tile, torch.device("cuda")), rand_tile=tile)
+
+
+def _same(a, b):
+    assert torch.equal(a.codes, b.codes) and torch.equal(a.scales, b.scales)
+
+
+# one tile, ragged last tiles in either direction, several tiles
+SHAPES = [(64, 64), (128, 128), (96, 160), (160, 416), (416, 1056)]
+
+
+@pytest.mark.parametrize("kind", ["normal", "special"])
+@pytest.mark.parametrize("rounding", ["rtn", "sr"])
+@pytest.mark.parametrize("shape", SHAPES + [(130, 96)])
+def test_rowwise_macro_scaling(shape, rounding, kind):
+    x = _matrix(*shape, kind)
+    codes = torch.empty(shape[0], -(-shape[1] // 128), dtype=torch.uint8, device="cuda")
+    got = E.quant_rows(x, MX, None, _sr(rounding, *shape), macro_codes=codes)
+    scaled, factors = macro_block_scaling(x, axis=-1)
+    _same(got, E.quant_rows(scaled, MX, None, _sr(rounding, *shape)))
+    assert torch.equal(codes, factors)
+
+
+@pytest.mark.parametrize("kind", ["normal", "special"])
+@pytest.mark.parametrize("clip_mode", ["none", "static", "dynamic"])
+@pytest.mark.parametrize("rotate", [False, True])
+@pytest.mark.parametrize("rounding", ["rtn", "sr"])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_colwise_macro_scaling(shape, rounding, rotate, clip_mode, kind):
+    x = _matrix(*shape, kind)
+    had = _transform() if rotate else None
+    rht = had.device_params() if rotate else None
+    codes = torch.empty(shape[1], -(-shape[0] // 128), dtype=torch.uint8, device="cuda")
+    got = E.quant_cols(x, MX, None, rht, _sr(rounding, shape[1], shape[0], rht, slots=True), clip_mode=clip_mode,
+                       macro_codes=codes)
+    scaled, factors = macro_block_scaling(had(x, left_mul=True) if rotate else x, axis=0)
+    _same(got, E.quant_cols(scaled, MX, None, None, _sr(rounding, shape[1], shape[0]), clip_mode=clip_mode))
+    assert torch.equal(codes, factors)
+
+
+@pytest.mark.parametrize("kind", ["normal", "special"])
+@pytest.mark.parametrize("rounding", ["rtn", "sr"])
+@pytest.mark.parametrize("batch", [1, 3])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_2d_macro_scaling(shape, batch, rounding, kind):
+    rows, cols = shape
+    x = torch.stack([_matrix(rows, cols, kind, seed=i) for i in range(batch)])
+    sr = _sr(rounding, batch * rows, cols)
+
+    def quantised(t, **macro):
+        out = [torch.empty(batch, rows, cols // 2, dtype=torch.uint8, device="cuda"),
+               torch.empty(batch, cols, rows // 2, dtype=torch.uint8, device="cuda"),
+               torch.empty(batch * L.packed_scale_bytes(rows, cols // 32), dtype=torch.uint8, device="cuda"),
+               torch.empty(batch * L.packed_scale_bytes(cols, rows // 32), dtype=torch.uint8, device="cuda")]
+        L.quantize_2d_batched(t, MX, out[0], out[1], None, out[2], out[3], **macro, **sr)
+        return out
+
+    codes = torch.empty(batch, -(-rows // 128), -(-cols // 128), dtype=torch.uint8, device="cuda")
+    got = quantised(x, macro_codes=codes)
+    scaled, factors = macro_block_scaling(x, axis=-1, use_2d_block=True)
+    assert all(torch.equal(g, e) for g, e in zip(got, quantised(scaled)))
+    assert torch.equal(codes, factors)
+
+
+@pytest.mark.parametrize("kind", ["normal", "special"])
+@pytest.mark.parametrize("rotate", [False, True])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("fmt", [L.FMT_NVFP4, L.FMT_MXFP4])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_stochastic_rounding_from_the_slot_ordered_table(shape, fmt, dtype, rotate, kind):
+    x = _matrix(*shape, kind).to(dtype)
+    rht = _transform().device_params() if rotate else None
+    rows, cols = shape[1], shape[0]
+    tile = _sr("sr", rows, cols)
+    # the plain table spelled out as one word per element
+    planes = tile["rand_bits"].repeat(1, -(-rows // 64), -(-cols // 64))[:, :rows, :cols // 2].contiguous()
+    got = E.quant_cols(x, fmt, None, rht, _sr("sr", rows, cols, rht, slots=True))
+    _same(got, E.quant_cols(x, fmt, None, rht, tile))
+    _same(got, E.quant_cols(x, fmt, None, rht, dict(rounding=L.ROUND_SR_BITS, rand_bits=planes)))
+
+
+def test_macro_scaling_is_refused_where_it_is_not_built():
+    x = _matrix(64, 64, "normal")
+    codes = torch.empty(64, 1, dtype=torch.uint8, device="cuda")
+    with pytest.raises(L.Altob200Error):
+        E.quant_rows(x.float(), MX, None, E.RTN, macro_codes=codes)
+    with pytest.raises(L.Altob200Error):
+        E.quant_cols(x, MX, None, None, _sr("sr", 64, 64), macro_codes=codes)
+    with pytest.raises(L.Altob200Error):
+        E.quant_2d(x, L.FMT_NVFP4, None, True, macro_codes=codes)
