@@ -44,6 +44,8 @@ EXPORTED_SYMBOLS = (
     "altob200_dequantize",
     "altob200_philox_tile",
     "altob200_philox_slots",
+    "altob200_group_experts",
+    "altob200_pack_scales",
     "altob200_rht",
     "altob200_rht_dense",
     "altob200_macro_block_scaling",
@@ -180,6 +182,10 @@ def _declare_more(lib):
     lib.altob200_rht_dense.argtypes = [vp, i32, i64, i64, i64, i32, vp, vp, i64, vp]
     lib.altob200_gather_rows.restype = C.c_int
     lib.altob200_gather_rows.argtypes = [vp, i64, i64, vp, i64, vp, vp]
+    lib.altob200_group_experts.restype = C.c_int
+    lib.altob200_group_experts.argtypes = [vp, i32, i64, vp, vp]
+    lib.altob200_pack_scales.restype = C.c_int
+    lib.altob200_pack_scales.argtypes = [vp, i64, i64, i64, i64, i32, vp, vp]
     lib.altob200_combine_rows.restype = C.c_int
     lib.altob200_combine_rows.argtypes = [vp, i64, i64, vp, vp, i64, i32, vp, vp]
     lib.altob200_spread_rows.restype = C.c_int
@@ -498,6 +504,26 @@ def deosc_accumulate(w, prev, w_qdq, prev_qdq, dist_w, dist_qdq) -> None:
     _check(lib().altob200_deosc_accumulate(w.data_ptr(), prev.data_ptr(), w_qdq.data_ptr(), prev_qdq.data_ptr(),
                                            dist_w.data_ptr(), dist_qdq.data_ptr(), w.numel(), _dt(w.dtype), _stream()),
            "altob200_deosc_accumulate")
+
+
+def group_experts(offs: torch.Tensor, n_groups: int) -> torch.Tensor:
+    """int32 [n_groups]: expert of each 128-row group from the cumulative row counts ``offs``, -1 past the last run."""
+    _require_cuda(offs)
+    assert offs.dtype == torch.int32 and offs.is_contiguous()
+    out = torch.empty(n_groups, dtype=torch.int32, device=offs.device)
+    _check(lib().altob200_group_experts(offs.data_ptr(), offs.numel(), n_groups, out.data_ptr(), _stream()),
+           "altob200_group_experts")
+    return out
+
+
+def pack_scales(scales: torch.Tensor, rows: int, block: int) -> torch.Tensor:
+    """uint8 [rows / block, ncols] (any strides) -> packed scales of [rows, ncols]."""
+    _require_cuda(scales)
+    assert scales.dtype == torch.uint8 and scales.dim() == 2 and scales.shape[0] * block == rows
+    out = torch.empty(packed_scale_bytes(rows, scales.shape[1]), dtype=torch.uint8, device=scales.device)
+    _check(lib().altob200_pack_scales(scales.data_ptr(), scales.stride(0), scales.stride(1), rows, scales.shape[1],
+                                      block, out.data_ptr(), _stream()), "altob200_pack_scales")
+    return out
 
 
 def gather_rows(src: torch.Tensor, index: torch.Tensor, out_rows: Optional[int] = None) -> torch.Tensor:

@@ -455,17 +455,11 @@ def linear_backward(ctx, grad_output):
 
 def pack_plain_scales(scales: torch.Tensor, rows: int, is_2d: bool, block: int) -> torch.Tensor:
     """Plain scales ([rows, K/block], or [rows/block, K/block] when ``is_2d``; uint8 exponents or
-    fp32 values on the E4M3 grid) -> the packed layout of the GEMM.  Pure data movement on a
-    tensor that is 1/16 or 1/32 of the operand; done with tensor ops."""
+    fp32 values on the E4M3 grid) -> the packed layout of the GEMM."""
     s = scales
     if s.dtype == torch.float32:
         s = s.to(torch.float8_e4m3fn).view(torch.uint8)
     assert s.dtype == torch.uint8
-    if is_2d:
-        s = s.repeat_interleave(block, dim=0)
-    assert s.shape[0] == rows, f"scale rows {s.shape[0]} != operand rows {rows}"
-    ncols = s.shape[1]
-    rt, ct = (rows + 127) // 128, (ncols + 3) // 4
-    buf = torch.zeros(rt * 128, ct * 4, dtype=torch.uint8, device=s.device)
-    buf[:rows, :ncols] = s
-    return buf.view(rt, 4, 32, ct, 4).permute(0, 3, 2, 1, 4).contiguous().view(-1)
+    per_row = block if is_2d else 1
+    assert s.shape[0] * per_row == rows, f"scale rows {s.shape[0] * per_row} != operand rows {rows}"
+    return L.pack_scales(s, rows, per_row)

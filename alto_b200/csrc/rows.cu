@@ -31,6 +31,45 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restric
   }
 }
 
+// Expert of every 128-row group: the number of run ends at or before the group's first row, -1 past the last run.
+// One launch where the tensor-op form (arange, multiply, bucketize, compare, fill, where) takes six.
+__global__ void __launch_bounds__(256) group_experts_kernel(const int32_t* __restrict__ offs, int num_experts,
+                                                            int64_t n_groups, int32_t* __restrict__ out) {
+  grid_dependency_wait();
+  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= n_groups) return;
+  const int64_t start = g * 128;
+  int lo = 0, hi = num_experts;   // first run end beyond `start`
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if ((int64_t)__ldg(offs + mid) <= start) lo = mid + 1;
+    else hi = mid;
+  }
+  out[g] = lo < num_experts ? lo : -1;
+}
+
+// Plain block scales (any strides; one row of scales per `block` operand rows) -> the packed layout of the GEMM,
+// padding zero.  A thread writes one word (four scale columns of a row); the tensor-op form is a fill, a strided
+// copy and a permuted copy.
+__global__ void __launch_bounds__(256) pack_scales_kernel(const uint8_t* __restrict__ src, int64_t row_stride,
+                                                          int64_t col_stride, int64_t rows, int64_t ncols, int64_t block,
+                                                          int64_t col_tiles, int64_t words, uint32_t* __restrict__ out) {
+  grid_dependency_wait();
+  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= words) return;
+  // word w of the packed buffer: tile w / 128 (row block, column tile), inside it rows r % 32 by r / 32
+  const int64_t tile = w >> 7, rb = tile / col_tiles, c0 = (tile - rb * col_tiles) * 4;
+  const int64_t r = rb * 128 + ((w & 3) << 5) + ((w >> 2) & 31);
+  uint32_t word = 0;
+  if (r < rows) {
+    const uint8_t* p = src + (r / block) * row_stride;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c0 + j < ncols) word |= (uint32_t)__ldg(p + (c0 + j) * col_stride) << (8 * j);
+  }
+  out[w] = word;
+}
+
 // Weighted combine of a token's k routed rows:  out[t] = bf16( sum_j f32( bf16( rows[index[t k + j]] * score[t k + j] ) ) ),
 // the roundings of the tensor-op form (gather, multiply in bf16, sum over k with fp32 accumulation).
 // index -1 contributes nothing; scores == NULL means weights of one.  One warp per token, 8 columns
@@ -100,6 +139,27 @@ __global__ void __launch_bounds__(256) spread_rows_kernel(const uint4* __restric
 }
 
 }  // namespace altob200
+
+extern "C" int altob200_group_experts(const int32_t* offs, int32_t num_experts, int64_t n_groups, int32_t* out,
+                                      void* stream) {
+  using namespace altob200;
+  if (offs == nullptr || out == nullptr || num_experts <= 0 || n_groups <= 0) return ALTOB200_EINVAL_SHAPE;
+  (void)launch_after(group_experts_kernel, dim3((unsigned)ceil_div(n_groups, 256)), dim3(256), 0, (cudaStream_t)stream,
+                     offs, num_experts, n_groups, out);
+  return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
+}
+
+extern "C" int altob200_pack_scales(const uint8_t* scales, int64_t row_stride, int64_t col_stride, int64_t rows,
+                                    int64_t ncols, int32_t block, uint8_t* packed, void* stream) {
+  using namespace altob200;
+  if (scales == nullptr || packed == nullptr || rows <= 0 || ncols <= 0 || block <= 0) return ALTOB200_EINVAL_SHAPE;
+  if ((reinterpret_cast<uintptr_t>(packed) & 3) != 0) return ALTOB200_EINVAL_ALIGN;
+  const int64_t col_tiles = ceil_div(ncols, 4), words = ceil_div(rows, 128) * col_tiles * 128;
+  if (ceil_div(words, 256) >= (1ll << 31)) return ALTOB200_ELIMIT;
+  (void)launch_after(pack_scales_kernel, dim3((unsigned)ceil_div(words, 256)), dim3(256), 0, (cudaStream_t)stream, scales,
+                     row_stride, col_stride, rows, ncols, (int64_t)block, col_tiles, words, (uint32_t*)packed);
+  return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
+}
 
 extern "C" int altob200_gather_rows(const void* src, int64_t src_rows, int64_t row_bytes, const int32_t* index,
                                     int64_t out_rows, void* dst, void* stream) {

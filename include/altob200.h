@@ -349,6 +349,20 @@ int altob200_deosc_accumulate(const void* w, void* prev, const void* w_qdq, cons
                               void* dist_qdq, int64_t n, int32_t dtype, void* stream);
 
 /*
+ * Expert of every group of 128 routed rows: out[g] = number of entries of offs (int32 cumulative row counts, ascending)
+ * that are <= 128 g, or -1 where that is num_experts (alto/kernels/blockwise_fp8/grouped_gemm/dsgemm_utils.py:97-112).
+ */
+int altob200_group_experts(const int32_t* offs, int32_t num_experts, int64_t n_groups, int32_t* out, void* stream);
+
+/*
+ * Plain uint8 block scales -> the packed layout of the GEMMs (altob200_packed_scale_bytes(rows, ncols) bytes, padding
+ * zero).  `scales` is [rows / block, ncols] with strides in bytes; block > 1 repeats a row of scales for that many
+ * operand rows (2-D blocks).
+ */
+int altob200_pack_scales(const uint8_t* scales, int64_t row_stride, int64_t col_stride, int64_t rows, int64_t ncols,
+                         int32_t block, uint8_t* packed, void* stream);
+
+/*
  * Row gather with zero fill: dst[i] = index[i] >= 0 ? src[index[i]] : zeros, rows of row_bytes
  * (a multiple of 16; both pointers 16-byte aligned).  The MoE token path around the grouped
  * GEMMs: sort routed rows by expert and pad each expert's run to a multiple of 128 rows (index

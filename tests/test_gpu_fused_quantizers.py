@@ -129,3 +129,26 @@ def test_macro_scaling_is_refused_where_it_is_not_built():
         E.quant_cols(x, MX, None, None, _sr("sr", 64, 64), macro_codes=codes)
     with pytest.raises(L.Altob200Error):
         E.quant_2d(x, L.FMT_NVFP4, None, True, macro_codes=codes)
+
+
+@pytest.mark.parametrize("block", [1, 32])
+@pytest.mark.parametrize("transposed", [False, True])
+@pytest.mark.parametrize("rows,ncols", [(32, 1), (128, 4), (160, 7), (4096, 45)])
+def test_packed_scales(rows, ncols, transposed, block):
+    shape = (rows // block, ncols)
+    s = torch.randint(0, 256, shape[::-1] if transposed else shape, generator=torch.Generator().manual_seed(1), dtype=torch.uint8)
+    s = s.t() if transposed else s
+    full = torch.zeros(-(-rows // 128) * 128, -(-ncols // 4) * 4, dtype=torch.uint8)
+    full[:rows, :ncols] = s.repeat_interleave(block, 0)
+    # tiles of 128 rows x 4 columns; in a tile 32 x 16 bytes: row % 32, then row / 32, then the column
+    packed = full.view(-1, 4, 32, full.shape[1] // 4, 4).permute(0, 3, 2, 1, 4).reshape(-1)
+    assert torch.equal(E.pack_plain_scales(s.cuda() if not transposed else s.t().cuda().t(), rows, block > 1, block).cpu(), packed)
+
+
+@pytest.mark.parametrize("counts", [[128], [0, 256, 0, 0, 128, 0], [128] * 300, [0, 0]])
+def test_expert_of_every_row_group(counts):
+    from alto_b200.grouped import group_experts_from_offsets
+    offs = torch.tensor(counts, dtype=torch.int64).cumsum(0).to(torch.int32)
+    rows = int(offs[-1]) + 200
+    expect = [next((e for e, end in enumerate(offs.tolist()) if end > start), -1) for start in range(0, rows, 128)]
+    assert group_experts_from_offsets(offs.cuda(), rows).tolist() == expect
