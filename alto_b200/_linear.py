@@ -34,7 +34,7 @@ _scratch = {}
 
 def amax_scratch(device: torch.device) -> torch.Tensor:
     """Zeroed per-(device, stream) scratch of the amax kernel (the kernel leaves it zeroed)."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, torch._C._cuda_getCurrentRawStream(device.index))
     buf = _scratch.get(key)
     if buf is None:
         buf = torch.zeros(L.AMAX_SCRATCH_BYTES // 4, dtype=torch.int32, device=device)
@@ -63,8 +63,7 @@ def explicit_sr_bits(provider: Callable[[str, Tuple[int, ...], torch.device], to
 def draw_philox() -> Tuple[int, int]:
     """Seed and offset from the global CPU generator, as the reference draws them when none is
     given (alto/kernels/fp4/nvfp4/nvfp_quantization.py:587-590)."""
-    v = torch.randint(0, 2 ** 31 - 1, (2,))
-    return int(v[0]), int(v[1])
+    return tuple(torch.randint(0, 2 ** 31 - 1, (2,)).tolist())
 
 
 def sr_args(use_sr: bool, name: str, rows: int, cols: int, device) -> dict:
@@ -227,40 +226,45 @@ class PrequantizedWeight:
         return len(self.shape)
 
 
-def activation_operands(x2, fmt, *, use_2dblock_x, use_outer_scale, rht, dense=None, use_uos=False, clip_mode="none"):
-    """(x_k, x_m): X along K (fprop) and X along M after the optional Hadamard rotation (wgrad)."""
-    ox = outer_scales(x2, use_outer_scale, None if use_2dblock_x else rht)
+def activation_operands(x2, fmt, *, use_2dblock_x, use_outer_scale, rht, dense=None, use_uos=False, clip_mode="none",
+                        want_m=True):
+    """(x_k, x_m): X along K (fprop) and X along M after the optional Hadamard rotation (wgrad; None when
+    ``want_m`` is off)."""
+    ox = outer_scales(x2, use_outer_scale, rht if want_m and not use_2dblock_x else None)
     if use_2dblock_x:
-        return quant_2d(x2, fmt, None if ox is None else ox[0:1], True, use_uos)
+        return quant_2d(x2, fmt, None if ox is None else ox[0:1], want_m, use_uos)
     x_k = quant_rows(x2, fmt, None if ox is None else ox[0:1], RTN, use_uos)
+    if not want_m:
+        return x_k, None
     x_m = cols_operand(x2, fmt, use_outer_scale, ox, rht, dense, RTN, use_uos, clip_mode)
     return x_k, x_m
 
 
-def weight_operands(w2, fmt, *, use_2dblock_w, use_outer_scale, use_uos=False):
-    """(w_k, w_t): W along K (fprop) and W along N (dgrad)."""
+def weight_operands(w2, fmt, *, use_2dblock_w, use_outer_scale, use_uos=False, want_t=True):
+    """(w_k, w_t): W along K (fprop) and W along N (dgrad; None when ``want_t`` is off)."""
     if isinstance(w2, PrequantizedWeight):
         torch._check(w2.fmt == fmt and w2.is_2d == bool(use_2dblock_w), lambda: (
             "the pre-quantised weight was built for another recipe than the one this linear runs"))
         return w2.w_k, w2.w_t
     ow = outer_scales(w2, use_outer_scale, None)
     if use_2dblock_w:
-        return quant_2d(w2, fmt, None if ow is None else ow[0:1], True, use_uos)
+        return quant_2d(w2, fmt, None if ow is None else ow[0:1], want_t, use_uos)
     w_k = quant_rows(w2, fmt, None if ow is None else ow[0:1], RTN, use_uos)
-    w_t = quant_cols(w2, fmt, None if ow is None else ow[0:1], None, RTN, use_uos)
+    w_t = quant_cols(w2, fmt, None if ow is None else ow[0:1], None, RTN, use_uos) if want_t else None
     return w_k, w_t
 
 
 def forward_operands(x2, w2, fmt, *, use_2dblock_x, use_2dblock_w, use_outer_scale, rht, dense=None,
-                     use_uos=False, clip_mode="none"):
+                     use_uos=False, clip_mode="none", want_m=True, want_t=True):
     """Returns (x_k, x_m, w_k, w_t): X along K (fprop), X along M after the optional Hadamard
-    rotation (wgrad), W along K (fprop), W along N (dgrad)."""
+    rotation (wgrad), W along K (fprop), W along N (dgrad); the backward operands only when wanted."""
     # Every pass over one tensor is launched before the first pass over the other: X at the benchmark
     # shapes (64 MiB) stays in the 126 MB L2 between its amax pass and its two quantizers, and W's
     # quantizer finds the tail of W that its amax pass left there.
     x_k, x_m = activation_operands(x2, fmt, use_2dblock_x=use_2dblock_x, use_outer_scale=use_outer_scale, rht=rht,
-                                   dense=dense, use_uos=use_uos, clip_mode=clip_mode)
-    w_k, w_t = weight_operands(w2, fmt, use_2dblock_w=use_2dblock_w, use_outer_scale=use_outer_scale, use_uos=use_uos)
+                                   dense=dense, use_uos=use_uos, clip_mode=clip_mode, want_m=want_m)
+    w_k, w_t = weight_operands(w2, fmt, use_2dblock_w=use_2dblock_w, use_outer_scale=use_outer_scale, use_uos=use_uos,
+                               want_t=want_t)
     return x_k, x_m, w_k, w_t
 
 
@@ -340,7 +344,11 @@ def linear_forward(ctx, name: str, x, weight, fmt, *, use_2dblock_x, use_2dblock
     rht, dense = split_transform(hadamard_transform, use_2dblock_x)
     ctx.xm_ready = None
     plain = not use_uos and clip_mode == "none"
-    if OVERLAP and not use_2dblock_x and dense is None and plain and not pre:
+    # an operand that only a gradient needs is not made when that gradient is not asked for (evaluation, frozen
+    # weights, a first layer); the DGE factor of dW reads the codes of the weight's dgrad operand
+    need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
+    want_m, want_t = need_dw, need_dx or (need_dw and use_dge)
+    if OVERLAP and want_m and want_t and not use_2dblock_x and dense is None and plain and not pre:
         main = torch.cuda.current_stream(x2.device)
         side = _side_stream(x2.device)
         ox = outer_scales(x2, use_outer_scale, rht)
@@ -365,11 +373,14 @@ def linear_forward(ctx, name: str, x, weight, fmt, *, use_2dblock_x, use_2dblock
     else:
         x_k, x_m, w_k, w_t = forward_operands(x2, w2, fmt, use_2dblock_x=use_2dblock_x, use_2dblock_w=use_2dblock_w,
                                               use_outer_scale=use_outer_scale, rht=rht, dense=dense,
-                                              use_uos=use_uos, clip_mode=clip_mode)
+                                              use_uos=use_uos, clip_mode=clip_mode, want_m=want_m, want_t=want_t)
         y = gemm(x_k, w_k, x.dtype)
-    extra_x = [x_m.outer] if x_m.outer is not None else []
-    extra_w = [w_t.outer] if w_t.outer is not None else []
-    ctx.save_for_backward(x_m.codes, x_m.scales, *extra_x, w_t.codes, w_t.scales, *extra_w)
+    saved = []
+    for op in (x_m, w_t):
+        saved += [None, None] if op is None else [op.codes, op.scales]
+        if use_outer_scale:
+            saved.append(None if op is None else op.outer)
+    ctx.save_for_backward(*saved)
     ctx.dims = (M, K, N)
     ctx.fmt = fmt
     ctx.use_2dblock_x = use_2dblock_x
@@ -393,7 +404,7 @@ def linear_backward(ctx, grad_output):
     w_t = Operand(wc, ws, wo, K, N, ctx.fmt)
     original_shape = grad_output.shape
     g2 = as_2d_rows(grad_output)
-    main = torch.cuda.current_stream(g2.device)
+    main = torch.cuda.current_stream(g2.device) if OVERLAP or ctx.xm_ready is not None else None
     if ctx.xm_ready is not None:
         main.wait_event(ctx.xm_ready)
     need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]

@@ -33,6 +33,9 @@ def _sylvester(n: int) -> Tensor:
     return H
 
 
+_SYLVESTER_16 = _sylvester(16)
+
+
 def _is_pow2(n: int) -> bool:
     return n > 0 and (n & (n - 1)) == 0
 
@@ -78,7 +81,7 @@ def random_hadamard_matrix(size: int, dtype=torch.float32, device="cpu", gen: Op
     H = _base_matrix(size).to(dtype)
     # The matrix stays on the host: the kernels take it as (perm, sign) launch parameters, and a
     # per-call host-to-device copy would stall the stream on every forward.
-    return torch.diag(Q) @ H.t()
+    return Q.unsqueeze(1) * H.t()
 
 
 class HadamardFactory:
@@ -126,7 +129,6 @@ class HadamardTransform:
     def __init__(self, weight: Tensor, perm: Optional[Tensor]):
         self.weight = weight
         self.perm = perm
-        self._scale = torch.tensor(weight.size(0), dtype=torch.float64).sqrt()
         self._rht: Optional[L.Rht] = None
         self._fusable: Optional[bool] = None
         self._dev = {}
@@ -150,7 +152,7 @@ class HadamardTransform:
             ok = self.n == 16
             if ok:
                 w = self.weight.detach().float().cpu()
-                ok = bool(torch.equal(torch.diag(w[:, 0]) @ w, _sylvester(16)))
+                ok = bool(torch.equal(w[:, :1] * w, _SYLVESTER_16))
             self._fusable = ok
         return self._fusable
 
@@ -161,7 +163,7 @@ class HadamardTransform:
                 raise NotImplementedError("this Hadamard matrix is not a row-signed Sylvester matrix of size 16; "
                                           "use the transform itself (dense kernel)")
             n = self.n
-            sign = self.weight.detach().float().cpu()[:, 0].clone()
+            sign = self.weight.detach().float().cpu()[:, 0]
             perm = self.perm.cpu().tolist() if self.perm is not None else list(range(n))
             self._rht = L.Rht(n, perm, [int(v) for v in sign.tolist()])
         return self._rht
