@@ -270,6 +270,14 @@ __device__ __forceinline__ float e2m1_decode(uint32_t c) {
   return u2f(bits | s);
 }
 
+// The two codes of a byte (low nibble first) -> two floats with the hardware converter; exact, sign of zero kept.
+__device__ __forceinline__ float2 e2m1x2_decode(uint32_t byte) {
+  uint32_t h2;
+  asm("{ .reg .b8 lo, hi; mov.b16 {lo, hi}, %1; cvt.rn.f16x2.e2m1x2 %0, lo; }" : "=r"(h2) : "h"((uint16_t)byte));
+  const __half2 h = *reinterpret_cast<const __half2*>(&h2);
+  return __half22float2(h);
+}
+
 // ---------------------------------------------------------------------------------------
 // FP8 encode: saturating round-to-nearest-even (the emulation clamps to +-max and then
 // casts, tests/unittest/mxfp8/utils.py:126-132; the Triton cast saturates natively,
