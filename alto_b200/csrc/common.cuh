@@ -63,6 +63,12 @@ __device__ __forceinline__ float u2f(uint32_t u) { return __uint_as_float(u); }
 
 // bf16 pair (little endian: element 0 in the low half) -> two floats, exact.
 __device__ __forceinline__ float bf16lo_to_f32(uint32_t w) { return u2f(w << 16); }
+// max(m, |a|, |b|), NaN if any is one
+__device__ __forceinline__ float absmax3_nan(float m, float a, float b) {
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+  return r;
+}
 __device__ __forceinline__ float bf16hi_to_f32(uint32_t w) { return u2f(w & 0xFFFF0000u); }
 
 // float -> bf16 bits, round to nearest even (what Tensor.to(torch.bfloat16) does).
@@ -164,6 +170,16 @@ __device__ __forceinline__ float div_bf16_num(float x, float q, float r) {
   const float y = __fmul_rn(x, r);
   const float e = __fmaf_rn(y, q, -x);
   return __fmaf_rn(-r, e, y);
+}
+
+// The same for an fp32 numerator, whose first product can be more than an ulp off: one correction makes it
+// faithful, and correcting a faithful quotient with r = RN(1/q) rounds it correctly (Markstein's theorem).  It needs
+// the quotient to stay finite (callers bound it per block); a residual that underflows belongs to a quotient below
+// 2^-34, which every encoder treats alike.
+__device__ __forceinline__ float div_f32_num(float x, float q, float r) {
+  float y = __fmul_rn(x, r);
+  y = __fmaf_rn(-r, __fmaf_rn(y, q, -x), y);
+  return __fmaf_rn(-r, __fmaf_rn(y, q, -x), y);
 }
 
 // x / 6 for a normal x whose quotient and residual stay normal (callers keep |x| in [2^-91, 2^120) or

@@ -102,8 +102,8 @@ __device__ __forceinline__ BlockScale make_block_scale(uint32_t amax_abs_bits, c
     } else {
       nvfp4_block_scale(amax, os.use, os.v, &s.plain, &s.q, &s.byte);
     }
-    s.fast = IN_BF16 && div_fast_ok(s.q);
     s.r = __frcp_rn(s.q);
+    s.fast = div_fast_ok(s.q) && (IN_BF16 || __fmul_rn(amax, s.r) < 1.2676506e30f);
   }
   return s;
 }
@@ -173,7 +173,7 @@ template <int FMT, bool IN_BF16, bool FAST>
 __device__ __forceinline__ float scale_elem(float x, const BlockScale& s) {
   if (!FAST) return __fdiv_rn(x, s.q);
   if (Fmt<FMT>::MX) return __fmul_rn(x, s.r);
-  return div_bf16_num(x, s.q, s.r);
+  return IN_BF16 ? div_bf16_num(x, s.q, s.r) : div_f32_num(x, s.q, s.r);
 }
 
 // acc | (x << sh) for disjoint bits, as one integer multiply-add.
@@ -1311,10 +1311,7 @@ __global__ void __launch_bounds__(256) amax_kernel(AmaxArgs a) {
       for (int u = 0; u < 4; ++u) {
       const uint4 w = wv[u];
       if (IN_BF16) {
-        uint32_t acc = absmax_bf16x2(0, w.x);
-        acc = absmax_bf16x2(acc, w.y);
-        acc = absmax_bf16x2(acc, w.z);
-        acc = absmax_bf16x2(acc, w.w);
+        const uint32_t acc = absmax2_bf16x2(absmax2_bf16x2(0, w.x, w.y), w.z, w.w);
         const uint32_t m = fold_bf16x2(acc) << 16;
         am_plain = m > am_plain ? m : am_plain;
       } else {
@@ -1335,7 +1332,8 @@ __global__ void __launch_bounds__(256) amax_kernel(AmaxArgs a) {
     const int64_t col_tiles = (a.cols + 63) >> 6;
     const int64_t n_tasks = groups * col_tiles;
     const int64_t warp0 = (int64_t)blockIdx.x * 8 + warp, n_warps = (int64_t)gridDim.x * 8;
-    uint32_t raw_rht = 0, plain16 = 0;
+    uint32_t plain16 = 0;
+    float raw_rht = 0.0f;
     for (int64_t task = warp0; task < n_tasks; task += n_warps) {
       int64_t g, ct;
       divmod_fast(task, col_tiles, &g, &ct);
@@ -1343,11 +1341,13 @@ __global__ void __launch_bounds__(256) amax_kernel(AmaxArgs a) {
       if (c >= a.cols) continue;
       const uint8_t* base = reinterpret_cast<const uint8_t*>(a.x) + ((g << 4) * a.ld + c) * (IN_BF16 ? 2 : 4);
       float v0[16], v1[16];
+      uint32_t before = 0;
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
         if (IN_BF16) {
           const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(base + a.rht.row_off[k]));
-          plain16 = absmax_bf16x2(plain16, w);
+          if (k & 1) plain16 = absmax2_bf16x2(plain16, before, w);
+          before = w;
           v0[k] = bf16lo_to_f32(w);
           v1[k] = bf16hi_to_f32(w);
         } else {
@@ -1362,15 +1362,13 @@ __global__ void __launch_bounds__(256) amax_kernel(AmaxArgs a) {
       hadamard16_pair(v0, v1);
 #pragma unroll
       for (int k = 0; k < 16; ++k) {
-        // integer maximum of the magnitudes' bits: a NaN is larger than every number, as in torch.amax
-        const uint32_t b0 = f2u(v0[k]) & 0x7FFFFFFFu, b1 = f2u(v1[k]) & 0x7FFFFFFFu;
-        raw_rht = b0 > raw_rht ? b0 : raw_rht;
-        raw_rht = b1 > raw_rht ? b1 : raw_rht;
+        // one three-input instruction for both columns; a NaN wins, as in torch.amax
+        raw_rht = absmax3_nan(raw_rht, v0[k], v1[k]);
       }
     }
     if (IN_BF16) am_plain = fold_bf16x2(plain16) << 16;
     // the row signs of the transform do not change magnitudes
-    const float y = __fmul_rn(u2f(raw_rht), 0.25f);
+    const float y = __fmul_rn(raw_rht, 0.25f);
     am_rht = IN_BF16 ? ((f32_to_bf16_bits(y) & 0x7FFFu) << 16) : (f2u(y) & 0x7FFFFFFFu);
   }
   am_plain = warp_max_u32(am_plain);
