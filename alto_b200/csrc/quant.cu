@@ -12,7 +12,7 @@
 //               block of rows, so the Hadamard butterfly and the block amax need no shuffles.
 //               Codes are transposed through shared memory so that every output row receives 64
 //               (FP4) or 128 (FP8) contiguous bytes.
-//   2D        : a warp owns 4 block columns x 64 (or 32) rows, a thread 16 rows x 8 columns in
+//   2D        : a warp owns 64 rows x 64 columns (FP8: 32 x 128), a thread 16 rows x 8 columns in
 //               registers; block maxima by shuffles, the second packing by an in-register
 //               transpose; no shared memory.
 #include <type_traits>
@@ -962,32 +962,37 @@ __device__ __forceinline__ void transpose4x4_bytes(const uint32_t* in, uint32_t*
   out[3] = __byte_perm(t2, t3, 0x7632);
 }
 
-// A thread owns 16 rows x 8 columns, kept in registers from the load to both stores; a warp owns
-// 4 block columns (LC lanes) x 16 * LR rows, so block maxima need shuffles only and the kernel uses
-// no shared memory.  The K packing is written row by row (4 or 8 bytes per row per lane, 32 or 128
-// contiguous bytes per row per warp); for the transposed packing the thread's 16 x 8 codes are
+// A thread owns 16 rows x 8 columns, kept in registers from the load to both stores; a warp owns LC x LR
+// threads, whole blocks either way, so block maxima need shuffles only and the kernel uses no shared memory.
+// The K packing is written row by row (4 or 8 bytes per row per lane, 32 or 128 contiguous bytes per row
+// per warp); for the transposed packing the thread's 16 x 8 codes are
 // transposed in registers (nibble merge of row pairs, then 4 x 4 byte transposes) and every column
-// receives 8 (FP4) or 16 (FP8) contiguous bytes per lane, 32 contiguous bytes per warp and column.
+// receives 8 (FP4) or 16 (FP8) contiguous bytes per lane, 32 contiguous bytes per warp and column (MXFP4 with
+// warps of 32 x 128, 16 bytes a column, half sectors: 78 us for 8192 x 14336 against 56).
 // MACRO (MXFP4 from bf16): the two-level recipe's scaling of 128 x 128 tiles runs in front of the quantisation;
-// a tile is four warps of 32 rows x 128 columns, whose maxima meet in shared memory.
+// a tile is the four warps of a CTA, whose maxima meet in shared memory.
+// CTAs of 128 threads, five of them an SM (four with the words of stochastic rounding): with 256 threads and 105
+// registers two were resident and waited for their slowest warp.  8192 x 14336: NVFP4 73 -> 60 us, fp32
+// (x 4096) 46 -> 39; two-level MXFP4, with the warp tile above, 90 -> 67.
+constexpr int WARPS_2D = 4;
 template <int FMT, bool IN_BF16, int ROUND, bool BATCHED, bool MACRO>
-__global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
+__global__ void __launch_bounds__(WARPS_2D * 32, ROUND == ALTOB200_ROUND_RTN ? 5 : 4) quantize_2d_kernel(Quant2dArgs a) {
   grid_dependency_wait();
   using F = Fmt<FMT>;
   constexpr int B = F::B;
-  constexpr int LC = B / 2;          // lanes across columns: 8 columns each, 4 block columns per warp
-  constexpr int LR = 32 / LC;        // 16-row groups per warp: 4 (B = 16) or 2 (B = 32)
-  constexpr int TR = 16 * LR, TC = 8 * LC;  // warp tile: 64 x 64 or 32 x 128
+  constexpr int LC = F::FP4 ? 8 : 16;  // lanes across columns, 8 columns each
+  constexpr int LR = 32 / LC;          // 16-row groups per warp
+  constexpr int TR = 16 * LR, TC = 8 * LC;  // warp tile: 64 x 64 (FP4) or 32 x 128: 32-byte sectors in both packings
   constexpr int ESZ = IN_BF16 ? 2 : 4;
   const int lane = threadIdx.x & 31;
-  static_assert(!MACRO || (FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && TR == 32 && TC == 128), "macro tiles");
-  // MACRO: row tiles are counted in whole macro tiles, and four consecutive warps take one of them
-  const int64_t tiles_c = (a.cols + TC - 1) / TC;
-  const int64_t tiles_r = MACRO ? ((a.rows + 127) >> 7) * 4 : (a.rows + TR - 1) / TR;
-  const int64_t tile_all = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
-  // (without MACRO whole warps leave: nothing below synchronises the block)
-  const bool live = tile_all < tiles_c * tiles_r * a.batch;
-  if (!MACRO && !live) return;
+  static_assert(!MACRO || (FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && TR == 64 && TC == 64), "macro tiles");
+  // MACRO: the four warps of a CTA take one macro tile, 2 x 2; tiles_r x tiles_c counts macro tiles then
+  constexpr int PER = MACRO ? 2 : 1;   // warp tiles per counted tile in either direction
+  const int64_t tiles_c = (a.cols + TC * PER - 1) / (TC * PER), tiles_r = (a.rows + TR * PER - 1) / (TR * PER);
+  const int64_t warp_all = (int64_t)blockIdx.x * WARPS_2D + (threadIdx.x >> 5);
+  const int64_t tile_all = MACRO ? warp_all >> 2 : warp_all;
+  // (whole warps leave, with MACRO whole CTAs)
+  if (tile_all >= tiles_c * tiles_r * a.batch) return;
   // matrix `bi` of the batch: its outputs follow those of matrix bi - 1, so the batch index enters the
   // addresses as extra rows (bi * rows for the K packing, bi * cols for the transposed one)
   // (BATCHED is a template parameter so that the single-matrix kernel carries none of this arithmetic)
@@ -995,12 +1000,11 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
   if (BATCHED) divmod_fast(tile_all, tiles_c * tiles_r, &bi, &tile);
   const int64_t rows_before = BATCHED ? bi * a.rows : 0, cols_before = BATCHED ? bi * a.cols : 0;
   int64_t tr, tc;
+  divmod_fast(tile, tiles_c, &tr, &tc);
+  const int64_t macro_tile = (bi * tiles_r + tr) * tiles_c + tc;
   if (MACRO) {
-    int64_t mr;
-    divmod_fast(tile >> 2, tiles_c, &mr, &tc);
-    tr = live ? mr * 4 + (tile & 3) : tiles_r;   // a warp without a tile lies below the matrix
-  } else {
-    divmod_fast(tile, tiles_c, &tr, &tc);
+    tr = tr * 2 + ((threadIdx.x >> 6) & 1);
+    tc = tc * 2 + ((threadIdx.x >> 5) & 1);
   }
   const int lc = lane % LC, lr = lane / LC;
   const int64_t row0 = tr * TR + lr * 16, col0 = tc * TC + lc * 8;
@@ -1024,18 +1028,17 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
     }
     amax_bits = fold_bf16x2(acc);
     if (MACRO) {
-      __shared__ uint32_t s_macro[8];
+      __shared__ uint32_t s_macro[WARPS_2D];
       const uint32_t wm = warp_max_u32(amax_bits);
       const int warp = threadIdx.x >> 5;
       if (lane == 0) s_macro[warp] = wm;
       __syncthreads();
       uint32_t m = 0;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) m = s_macro[(warp & 4) + i] > m ? s_macro[(warp & 4) + i] : m;
+      for (int i = 0; i < WARPS_2D; ++i) m = s_macro[i] > m ? s_macro[i] : m;
       uint32_t code;
       const float f = macro_factor_from_amax(u2f(m << 16), &code);
-      if (live && (warp & 3) == 0 && lane == 0)
-        a.macro_codes[(bi * (tiles_r >> 2) + (tr >> 2)) * tiles_c + tc] = (uint8_t)code;
+      if (threadIdx.x == 0) a.macro_codes[macro_tile] = (uint8_t)code;
       // y = bf16(x * factor); rounding is monotone, so the maximum is scaled instead of searched again
       auto scaled = [&](uint32_t w) {
         const __nv_bfloat162 p2 = __floats2bfloat162_rn(__fmul_rn(bf16lo_to_f32(w), f), __fmul_rn(bf16hi_to_f32(w), f));
@@ -1214,37 +1217,43 @@ __global__ void __launch_bounds__(256) quantize_2d_kernel(Quant2dArgs a) {
     else reinterpret_cast<float*>(a.scale_plain)[idx] = s.plain;
   }
   const uint32_t my_byte = ok ? s.byte : 0u;  // blocks outside the matrix contribute zero bytes
+  constexpr int BC = TC / B, BR = TR / B;   // the warp's blocks: 4 x 4 (NVFP4), 2 x 2 (MXFP4), 4 columns x 1 row (FP8)
   if (a.packed_k != nullptr) {
-    // one word per row: the scale bytes of the warp's 4 block columns; the rows of a group are
-    // shared out over its LC lanes
+    // per row the scale bytes of the warp's BC block columns: a word, or half of one; the rows of a group
+    // are shared out over its LC lanes
     uint32_t word = 0;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) word |= __shfl_sync(0xFFFFFFFFu, my_byte, lr * LC + j * (B / 8)) << (8 * j);
-    const int64_t kb = tc * 4;
-    if (row_ok) {
+    for (int j = 0; j < BC; ++j) word |= __shfl_sync(0xFFFFFFFFu, my_byte, lr * LC + j * (B / 8)) << (8 * j);
+    const int64_t kb = tc * BC;
+    if (row_ok && (BC == 4 || kb < a.nct_k * 4)) {
 #pragma unroll
       for (int i = 0; i < 16 / LC; ++i) {
         const int64_t row = row0 + lc * (16 / LC) + i;
-        *reinterpret_cast<uint32_t*>(a.packed_k + bi * a.packed_k_bytes + packed_scale_offset(row, kb, a.nct_k)) = word;
+        uint8_t* dst = a.packed_k + bi * a.packed_k_bytes + packed_scale_offset(row, kb, a.nct_k);
+        if (BC == 4) *reinterpret_cast<uint32_t*>(dst) = word;
+        else *reinterpret_cast<uint16_t*>(dst) = (uint16_t)word;
       }
     }
   }
   if (a.packed_t != nullptr) {
     // rows of this layout are the matrix columns, scale columns the row blocks
-    if (LR == 4) {
-      // B = 16: the warp's 4 row groups are the 4 bytes of one word; the 8 columns of a lane are
-      // shared out over the 4 row groups
+    if (BR > 1) {
+      // the BR row blocks are the bytes of one word or half-word; the 8 columns of a lane are shared out over
+      // the 4 row groups
       uint32_t word = 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) word |= __shfl_sync(0xFFFFFFFFu, my_byte, j * LC + lc) << (8 * j);
-      if (col_ok) {
+      for (int j = 0; j < BR; ++j) word |= __shfl_sync(0xFFFFFFFFu, my_byte, j * (B / 16) * LC + lc) << (8 * j);
+      const int64_t kb = tr * BR;
+      if (col_ok && (BR == 4 || kb < a.nct_t * 4)) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-          *reinterpret_cast<uint32_t*>(a.packed_t + bi * a.packed_t_bytes +
-                                       packed_scale_offset(col0 + 2 * lr + e, tr * 4, a.nct_t)) = word;
+        for (int e = 0; e < 2; ++e) {
+          uint8_t* dst = a.packed_t + bi * a.packed_t_bytes + packed_scale_offset(col0 + 2 * lr + e, kb, a.nct_t);
+          if (BR == 4) *reinterpret_cast<uint32_t*>(dst) = word;
+          else *reinterpret_cast<uint16_t*>(dst) = (uint16_t)word;
+        }
       }
     } else {
-      // B = 32: the warp holds one row block, one byte per column
+      // one row block, one byte per column
       if (ok) {
 #pragma unroll
         for (int e = 0; e < 4; ++e)
@@ -1767,14 +1776,14 @@ static int launch_colwise(const ColwiseArgs& a, int rounding, cudaStream_t st) {
 
 template <int FMT, bool IN_BF16, int ROUND, bool BATCHED>
 static void launch_2d_kernel(const Quant2dArgs& a, cudaStream_t st) {
-  // one warp per tile of 4 block columns x (64 rows for 16-blocks, 32 rows for 32-blocks)
-  constexpr int TC = 4 * Fmt<FMT>::B, TR = 1024 / Fmt<FMT>::B;
+  constexpr int TC = Fmt<FMT>::FP4 ? 64 : 128, TR = Fmt<FMT>::FP4 ? 64 : 32;   // a warp's tile
   constexpr bool CAN_MACRO = FMT == ALTOB200_FMT_MXFP4 && IN_BF16;
   const bool macro = CAN_MACRO && a.macro_codes != nullptr;
-  const int64_t tiles = ceil_div(a.cols, TC) * (macro ? ceil_div(a.rows, 128) * 4 : ceil_div(a.rows, TR)) * a.batch;
-  const dim3 blocks((unsigned)ceil_div(tiles, 8));
-  if (macro) (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, ROUND, BATCHED, CAN_MACRO>, blocks, dim3(256), 0, st, a);
-  else (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, ROUND, BATCHED, false>, blocks, dim3(256), 0, st, a);
+  const int64_t tiles = (macro ? ceil_div(a.cols, 128) * ceil_div(a.rows, 128) * 4
+                               : ceil_div(a.cols, TC) * ceil_div(a.rows, TR)) * a.batch;
+  const dim3 blocks((unsigned)ceil_div(tiles, WARPS_2D)), block(WARPS_2D * 32);
+  if (macro) (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, ROUND, BATCHED, CAN_MACRO>, blocks, block, 0, st, a);
+  else (void)launch_after(quantize_2d_kernel<FMT, IN_BF16, ROUND, BATCHED, false>, blocks, block, 0, st, a);
 }
 
 template <int FMT, bool IN_BF16>
