@@ -397,8 +397,8 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                           (m0 >> margs.ma.shift) * margs.ma.row_stride;
       const uint8_t* pb = margs.mb.codes + (int64_t)mt.expert * margs.mb.expert_stride +
                           (mt.chunk0 + fc) * margs.mb.chunk_stride + (n0 >> margs.mb.shift) * margs.mb.row_stride;
-      // offsets of the lane's rows from the tile's first (a row beyond the matrix reads the last one): they
-      // stay below 256 * 2^24, the chunks of the longest K the host accepts
+      // offsets of the lane's rows from the tile's first (a row beyond the matrix reads the last one); the host
+      // refuses strides that would not fit
       constexpr int NB = B_UNIFORM ? 2 : 4;
       uint32_t off_a[2], off_b[NB];
       const uint32_t m_last = (uint32_t)(args.M - m0 < BM ? args.M - m0 : BM) - 1u;

@@ -152,3 +152,29 @@ def test_expert_of_every_row_group(counts):
     rows = int(offs[-1]) + 200
     expect = [next((e for e, end in enumerate(offs.tolist()) if end > start), -1) for start in range(0, rows, 128)]
     assert group_experts_from_offsets(offs.cuda(), rows).tolist() == expect
+
+
+@pytest.mark.parametrize("needs", [(True, False), (False, True), (False, False)])
+@pytest.mark.parametrize("weight_2d", [False, True])
+@pytest.mark.parametrize("recipe", ["nvfp4", "mxfp4", "mxfp8"])
+def test_operands_of_gradients_that_are_not_asked_for(recipe, weight_2d, needs):
+    from alto_b200 import mxfp4, mxfp8, nvfp4
+    calls = {"nvfp4": lambda x, w: nvfp4._to_nvfp4_then_scaled_mm(x, w, False, weight_2d, True, use_outer_scale=True,
+                                                                 use_hadamard=True),
+             "mxfp4": lambda x, w: mxfp4._to_mxfp4_then_scaled_mm(x, w, False, weight_2d, True, True, "none", True),
+             "mxfp8": lambda x, w: mxfp8._to_mxfp8_then_scaled_mm(x, w, "e4m3", False, False, weight_2d)}
+    x0, w0, dy = _matrix(128, 192, "normal"), _matrix(160, 192, "normal", 1), _matrix(128, 160, "normal", 2)
+
+    def step(need_x, need_w):
+        _transform()
+        torch.manual_seed(5)
+        x, w = x0.clone().requires_grad_(need_x), w0.clone().requires_grad_(need_w)
+        y = calls[recipe](x, w)
+        if need_x or need_w:
+            y.backward(dy)
+        return y.detach(), x.grad, w.grad
+
+    full, got = step(True, True), step(*needs)
+    assert torch.equal(got[0], full[0])
+    for need, g, f in zip(needs, got[1:], full[1:]):
+        assert torch.equal(g, f) if need else g is None
