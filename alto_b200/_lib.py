@@ -23,7 +23,7 @@ LIB_PATH = _PKG / "libaltob200.so"
 # enums of include/altob200.h
 FMT_NVFP4, FMT_MXFP4, FMT_MXFP8_E4M3, FMT_MXFP8_E5M2 = 0, 1, 2, 3
 DT_BF16, DT_F32 = 0, 1
-SCALE_PLAIN, SCALE_PACKED = 1, 2
+SCALE_PLAIN, SCALE_PACKED, SCALE_MACRO = 1, 2, 4
 ROUND_RTN, ROUND_SR_BITS, ROUND_SR_PHILOX, ROUND_SR_SLOTS = 0, 1, 2, 3
 AMAX_SCRATCH_BYTES = 16
 
@@ -301,6 +301,8 @@ def _params(fmt, x, rounding, outer_scale, rand_bits, rht: Optional[Rht], flags,
             clip_mode: str = "none", use_uos: bool = False, rand_tile=(0, 0), macro_codes=None) -> QuantParams:
     p = QuantParams()
     p.macro_codes = _ptr(macro_codes)
+    if macro_codes is not None:
+        flags |= SCALE_MACRO
     p.clip_mode = CLIP_MODES[clip_mode]
     p.use_uos = 1 if use_uos else 0
     p.rand_tile_rows, p.rand_tile_pairs = int(rand_tile[0]), int(rand_tile[1])

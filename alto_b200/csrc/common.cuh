@@ -200,13 +200,6 @@ __device__ __forceinline__ float div_by_6(float x) {
 // even on the E2M1 grid including its subnormal 0.5, saturation to 6, sign of zero kept (checked
 // against the oracle on the golden vectors and on random data in the GPU tests).
 // ---------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t e2m1x2_rtn_hw(float v0, float v1) {
-  uint16_t r;
-  asm("{ .reg .b8 t; cvt.rn.satfinite.e2m1x2.f32 t, %1, %2; cvt.u16.u8 %0, t; }"
-      : "=h"(r)
-      : "f"(v1), "f"(v0));
-  return (uint32_t)r;
-}
 // Eight floats -> four bytes, element 0 in the lowest nibble: the converters write into the bytes of one
 // register, nothing is shifted or merged.
 __device__ __forceinline__ uint32_t e2m1x8_rtn_hw(const float* v) {
@@ -275,17 +268,7 @@ __device__ __forceinline__ float e2m1_sr_value(float v, uint32_t rnd) {
   return u2f(f2u(w) | (f2u(v) & 0x80000000u));
 }
 
-// E2M1 decode to fp32 (alto/kernels/fp4/fp4_common/triton_fp4_ops.py:100-132).
-__device__ __forceinline__ float e2m1_decode(uint32_t c) {
-  const uint32_t s = (c & 8u) << 28;
-  const uint32_t m = c & 7u;
-  uint32_t bits;
-  if (m == 0u) bits = 0u;
-  else if (m == 1u) bits = 0x3F000000u;
-  else bits = (((m >> 1) - 1u + 127u) << 23) | ((m & 1u) << 22);
-  return u2f(bits | s);
-}
-
+// E2M1 decode (alto/kernels/fp4/fp4_common/triton_fp4_ops.py:100-132).
 // The two codes of a byte (low nibble first) -> two floats with the hardware converter; exact, sign of zero kept.
 __device__ __forceinline__ float2 e2m1x2_decode(uint32_t byte) {
   uint32_t h2;

@@ -23,8 +23,8 @@
 //                 staging buffer and hands it to a TMA store (which also clips ragged M/N edges); two
 //                 staging buffers per warp keep stores in flight.
 //   warp 10     : waits on the stage's barriers on behalf of the MMA issuer.
-// The CTA-pair kernel (cta_group::2, 256 x 256 tiles, 512 threads) and the two-level MXFP4 kernel
-// (gemm_macro.cuh) have the same roles; their layouts are described at the kernels.
+// The CTA-pair kernel (cta_group::2, 256 x 256 tiles, 512 threads) has the same roles.  The two-level
+// MXFP4 kernel (gemm_macro.cuh) divides the work differently; both layouts are described at the kernels.
 // Every mbarrier wait is bounded by a cycle count; a wait that gives up records {kernel, block, site}
 // in a device status word, raises a CTA-wide abort flag, and all roles fall through to the common
 // teardown that frees tensor memory.  All kernels are launched with programmatic stream serialisation

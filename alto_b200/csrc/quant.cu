@@ -492,7 +492,6 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
 struct RhtParams {
   int n;           // 0 or 16
   int8_t pinv[16]; // slot k reads row pinv[k] of the block
-  int8_t perm[16]; // output position i takes slot perm[i]
   float sign[16];  // sign applied to slot k after the butterfly
   int64_t row_off[16];  // byte offset of row pinv[k] from the first row of a 16-row group (column passes)
   float qsign[16];      // sign[k] / sqrt(16): the factor applied to slot k
@@ -1672,7 +1671,7 @@ static int fill_rht(RhtParams* r, int n, const int32_t* perm, const int32_t* sig
   r->n = n;
   if (n == 0) {
     for (int i = 0; i < 16; ++i) {
-      r->pinv[i] = (int8_t)i; r->perm[i] = (int8_t)i; r->sign[i] = 1.0f;
+      r->pinv[i] = (int8_t)i; r->sign[i] = 1.0f;
       r->qsign[i] = 0.25f;
     }
     return ALTOB200_OK;
@@ -1687,7 +1686,6 @@ static int fill_rht(RhtParams* r, int n, const int32_t* perm, const int32_t* sig
   }
   // W[i][j] = sign[perm[i]] * H[perm[i]][perm[j]]:  z[k] = x[pinv[k]],  y[i] = sign[perm[i]] * (H z)[perm[i]]
   for (int i = 0; i < 16; ++i) {
-    r->perm[i] = (int8_t)perm[i];
     r->pinv[perm[i]] = (int8_t)i;
     r->sign[i] = (float)sign[i];
   }
@@ -1819,6 +1817,11 @@ static int launch_2d(const Quant2dArgs& a, int rounding, cudaStream_t st) {
     }                                                                                       \
   } while (0)
 
+// the field is younger than the struct: read only for callers that announce it
+static uint8_t* macro_codes_of(const altob200_quant_params* p) {
+  return (p->scale_flags & ALTOB200_SCALE_MACRO) != 0 ? p->macro_codes : nullptr;
+}
+
 static int block_of(int fmt) { return fmt == ALTOB200_FMT_NVFP4 ? 16 : 32; }
 static bool is_fp4(int fmt) { return fmt == ALTOB200_FMT_NVFP4 || fmt == ALTOB200_FMT_MXFP4; }
 
@@ -1947,7 +1950,7 @@ int altob200_quantize_rowwise(const void* x, int64_t rows, int64_t cols, int64_t
   if (p->rht_n != 0) return ALTOB200_EUNSUPPORTED;
   cudaStream_t st = (cudaStream_t)stream;
   RowwiseArgs a;
-  a.macro_codes = (uint8_t*)p->macro_codes;
+  a.macro_codes = macro_codes_of(p);
   if (a.macro_codes != nullptr && (p->format != ALTOB200_FMT_MXFP4 || p->in_dtype != ALTOB200_DT_BF16 ||
                                    p->rounding == ALTOB200_ROUND_SR_PHILOX))
     return ALTOB200_EUNSUPPORTED;
@@ -1992,7 +1995,7 @@ int altob200_quantize_colwise(const void* x, int64_t rows, int64_t cols, int64_t
   }
   cudaStream_t st = (cudaStream_t)stream;
   ColwiseArgs a;
-  a.macro_codes = (uint8_t*)p->macro_codes;
+  a.macro_codes = macro_codes_of(p);
   if (a.macro_codes != nullptr &&
       (p->format != ALTOB200_FMT_MXFP4 || p->in_dtype != ALTOB200_DT_BF16 ||
        (p->rounding != ALTOB200_ROUND_RTN && p->rounding != ALTOB200_ROUND_SR_SLOTS)))
@@ -2044,7 +2047,7 @@ int altob200_quantize_2d_batched(const void* w, int64_t batch, int64_t batch_str
   if (codes_t != nullptr && !aligned16(codes_t)) return ALTOB200_EINVAL_ALIGN;
   cudaStream_t st = (cudaStream_t)stream;
   Quant2dArgs a;
-  a.macro_codes = (uint8_t*)p->macro_codes;
+  a.macro_codes = macro_codes_of(p);
   if (a.macro_codes != nullptr && (p->format != ALTOB200_FMT_MXFP4 || p->in_dtype != ALTOB200_DT_BF16))
     return ALTOB200_EUNSUPPORTED;
   a.w = w; a.rows = rows; a.cols = cols; a.ld = ld;

@@ -291,6 +291,7 @@ def run_ours(args):
     timer.wrap(L, "gemm_blockscaled", "gemm", lambda fa, fb, m, n, k, *a, **kw: 2.0 * m * n * k)
     timer.wrap(L, "gemm_mxfp4_two_level", "gemm", lambda m, n, k, *a, **kw: 2.0 * m * n * k)
     timer.count(L, "philox_tile")   # the two 16 KB random-word tables of a step's stochastic-rounding quantizers
+    timer.count(L, "philox_slots")
 
     g = torch.Generator(device=dev).manual_seed(rank)
     gw = torch.Generator(device=dev).manual_seed(12345)  # identical weights on every rank

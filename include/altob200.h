@@ -57,6 +57,7 @@ extern "C" {
 /* scale output layouts */
 #define ALTOB200_SCALE_PLAIN 1
 #define ALTOB200_SCALE_PACKED 2
+#define ALTOB200_SCALE_MACRO 4  /* altob200_quant_params.macro_codes is set (the field is not read otherwise) */
 /* rounding */
 #define ALTOB200_ROUND_RTN 0
 #define ALTOB200_ROUND_SR_BITS 1   /* stochastic rounding, caller supplies 32 random bits per element */
@@ -126,7 +127,8 @@ typedef struct altob200_quant_params {
    * row-wise quantizer.                                                                  */
   int64_t rand_tile_rows;
   int64_t rand_tile_pairs;
-  /* Two-level ("blockwise") MXFP4 from bf16, or NULL: every macro block of 128 elements along the
+  /* Two-level ("blockwise") MXFP4 from bf16, only read with ALTOB200_SCALE_MACRO in scale_flags (callers built
+   * before this field existed need no change): every macro block of 128 elements along the
    * quantisation axis (128 x 128 tiles for the 2-D quantizer) is first multiplied by its factor and rounded
    * to bf16, exactly what altob200_macro_block_scaling writes, and the factor codes go to macro_codes in
    * that function's layout (row-wise: [rows, ceil(cols/128)], column-wise: [cols, ceil(rows/128)], 2-D:

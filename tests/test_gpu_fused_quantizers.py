@@ -46,6 +46,21 @@ def _same(a, b):
     assert torch.equal(a.codes, b.codes) and torch.equal(a.scales, b.scales)
 
 
+def test_macro_field_needs_its_flag():
+    """A caller built against the struct without the field passes whatever lies behind it: not read."""
+    x = _matrix(64, 128, "normal")
+    guard = torch.full((64,), 77, dtype=torch.uint8, device="cuda")
+    out = [torch.empty(64, 64, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    scales = [torch.empty(64, 4, dtype=torch.uint8, device="cuda") for _ in range(2)]
+    L.quantize_rowwise(x, MX, out[0], scales[0], None)
+    p = L._params(MX, x, L.ROUND_RTN, None, None, None, L.SCALE_PLAIN)
+    p.macro_codes = guard.data_ptr()
+    rc = L.lib().altob200_quantize_rowwise(x.data_ptr(), 64, 128, 128, L.C.byref(p), out[1].data_ptr(),
+                                           scales[1].data_ptr(), None, L._stream())
+    assert rc == 0 and (guard == 77).all()
+    assert torch.equal(out[0], out[1]) and torch.equal(scales[0], scales[1])
+
+
 # one tile, ragged last tiles in either direction, several tiles
 SHAPES = [(64, 64), (128, 128), (96, 160), (160, 416), (416, 1056)]
 
