@@ -473,4 +473,10 @@ def pack_plain_scales(scales: torch.Tensor, rows: int, is_2d: bool, block: int) 
     assert s.dtype == torch.uint8
     per_row = block if is_2d else 1
     assert s.shape[0] * per_row == rows, f"scale rows {s.shape[0] * per_row} != operand rows {rows}"
-    return L.pack_scales(s, rows, per_row)
+    if s.is_cuda and s.numel() > 0:
+        return L.pack_scales(s, rows, per_row)
+    # host tensors (weight shards are laid out before they reach a device) and empty operands
+    ncols, rt, ct = s.shape[1], (rows + 127) // 128, (s.shape[1] + 3) // 4
+    buf = torch.zeros(rt * 128, ct * 4, dtype=torch.uint8, device=s.device)
+    buf[:rows, :ncols] = s.repeat_interleave(per_row, dim=0)
+    return buf.view(rt, 4, 32, ct, 4).permute(0, 3, 2, 1, 4).contiguous().view(-1)

@@ -156,3 +156,25 @@ def test_nvtx_ranges_wrap_boundary_calls_only_when_asked(monkeypatch):
     with pytest.raises(ValueError):
         g(-1)
     assert events == [("push", "alto_b200::unit"), ("pop",), ("push", "alto_b200::unit"), ("pop",)]
+
+
+@pytest.mark.parametrize("offs,rows,expect", [([128, 384], 600, [0, 1, 1, -1, -1]), ([128], 0, []), ([], 256, [-1, -1]),
+                                              ([0, 128, 128, 256], 256, [1, 3])])
+def test_group_experts_of_host_offsets(offs, rows, expect):
+    from alto_b200.grouped import group_experts_from_offsets
+    got = group_experts_from_offsets(torch.tensor(offs, dtype=torch.int32), rows)
+    assert got.dtype == torch.int32 and got.tolist() == expect
+
+
+@pytest.mark.parametrize("rows,ncols,block", [(128, 4, 1), (96, 6, 1), (160, 5, 32), (0, 4, 1), (128, 0, 1)])
+def test_packed_scales_of_host_tensors(rows, ncols, block):
+    """Row r, column c lies at byte (r % 32) * 16 + (r / 32 % 4) * 4 + c % 4 of 512-byte tile (r / 128, c / 4)."""
+    from alto_b200._linear import pack_plain_scales
+    s = torch.randint(1, 255, (rows // block, ncols), generator=torch.Generator().manual_seed(1), dtype=torch.uint8)
+    got = pack_plain_scales(s, rows, block > 1, block)
+    ct = -(-ncols // 4)
+    want = torch.zeros(-(-rows // 128) * ct * 512, dtype=torch.uint8)
+    for r in range(rows):
+        for c in range(ncols):
+            want[(r // 128 * ct + c // 4) * 512 + r % 32 * 16 + r // 32 % 4 * 4 + c % 4] = s[r // block, c]
+    assert torch.equal(got, want)
