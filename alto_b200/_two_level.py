@@ -33,8 +33,9 @@ STATIC_CLIP_WGRAD = 16.0 / 9.0
 
 def _fusable(t: torch.Tensor) -> bool:
     """The quantizers apply the macro factors themselves to bf16 tensors whose rows they can read as they are
-    (16-byte alignment); for the rest ``macro_block_scaling`` runs first.  Same codes, scales and factors."""
-    return (t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.data_ptr() % 16 == 0
+    (16-byte alignment, rows that do not overlap); for the rest ``macro_block_scaling`` runs first.  Same codes,
+    scales and factors."""
+    return (t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.stride(-2) >= t.shape[-1] and t.data_ptr() % 16 == 0
             and all(st * t.element_size() % 16 == 0 for st in t.stride()[:-1]))
 
 

@@ -193,3 +193,23 @@ def test_operands_of_gradients_that_are_not_asked_for(recipe, weight_2d, needs):
     assert torch.equal(got[0], full[0])
     for need, g, f in zip(needs, got[1:], full[1:]):
         assert torch.equal(g, f) if need else g is None
+
+
+@pytest.mark.parametrize("form", ["expanded", "overlapping", "column slice", "odd offset"])
+def test_two_level_operands_of_views(form):
+    """Rows the fused quantizers cannot read as they are give what a contiguous copy gives."""
+    from alto_b200 import _two_level as T
+    base = _matrix(160, 512, "normal")
+    t = {"expanded": lambda: base[:1, :256].expand(96, 256),
+         "overlapping": lambda: base.flatten().as_strided((96, 256), (64, 1)),
+         "column slice": lambda: base[:96, 64:320],
+         "odd offset": lambda: base[:96, 3:259]}[form]()
+    makers = [lambda v: T.rows_operand(v, False), lambda v: T.cols_operand(v, False),
+              lambda v: T.tiles_operands(v, False)[0]]
+    if form == "column slice":   # the transform itself takes no overlapping or misaligned rows
+        rht = _transform()
+        makers.append(lambda v: T.cols_operand(v, False, "none", None, rht))
+    for make in makers:
+        got, want = make(t), make(t.contiguous())
+        _same(got, want)
+        assert torch.equal(got.macro.codes, want.macro.codes)
