@@ -550,6 +550,7 @@ struct ColwiseArgs {
   const float* outer;
   const uint32_t* rand_bits;  // [2][cols][rows/2], or a periodic tile [2][tile_rows][tile_pairs]
   int64_t tile_rows, tile_pairs;
+  bool rand_vec;              // the words of 16 rows can be read in 16-byte vectors
   uint64_t philox_seed, philox_offset;
   PhiloxKeys pk;
   RhtParams rht;
@@ -571,7 +572,10 @@ constexpr int COL_TN = 64;   // columns per CTA tile
 // MACRO (MXFP4 from bf16): the two-level recipe's scaling runs in front of the quantisation - a CTA tile is one
 // macro block of 128 rows per column, so its maxima only have to cross the four warps.
 template <int FMT, bool IN_BF16, int ROUND, bool RHT, bool MACRO>
-__global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a) {
+// (fp32 blocks of 32 with words by position are held to the 128 registers of four CTAs an SM: 63 -> 58 us for
+// 8192 x 4096; 0 leaves the others to the compiler)
+__global__ void __launch_bounds__(COL_NT, !IN_BF16 && Fmt<FMT>::B == 32 && ROUND == ALTOB200_ROUND_SR_BITS ? 4 : 0)
+quantize_colwise_kernel(ColwiseArgs a) {
   grid_dependency_wait();
   using F = Fmt<FMT>;
   constexpr int B = F::B;
@@ -587,8 +591,10 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
   __shared__ __align__(16) uint8_t s_codes[COL_TN * ROW_BYTES];
   __shared__ __align__(16) uint8_t s_sf[COL_TN * NBLK];
   __shared__ float s_sf_plain[Fmt<FMT>::MX ? 1 : COL_TN * NBLK];
-  constexpr bool WORDS_TO_SLOTS = RHT && ROUND == ALTOB200_ROUND_SR_PHILOX;
-  __shared__ uint2 s_words[WORDS_TO_SLOTS ? 16 : 1][NT];   // (column c, column c + 1) per thread
+  // words that come in position order: the values of a thread's two columns are moved there from slot order
+  constexpr bool TO_POS = RHT && (ROUND == ALTOB200_ROUND_SR_PHILOX || ROUND == ALTOB200_ROUND_SR_BITS);
+  using Pair = typename std::conditional<IN_BF16, uint32_t, float2>::type;
+  __shared__ Pair s_pos[TO_POS ? 16 : 1][NT];
   __shared__ uint32_t s_macro[MACRO ? WARPS : 1][32];
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -720,6 +726,27 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
       if (clip) x = make_float2(round_in<IN_BF16>(__fmul_rn(x.x, 0.75f)), round_in<IN_BF16>(__fmul_rn(x.y, 0.75f)));
       return x;
     };
+    // slot order -> position order through a private column of shared memory (moving the words instead, behind
+    // their loads, takes 20 % longer)
+    auto to_positions = [&]() {
+#pragma unroll
+      for (int g = 0; g < B; g += 16) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          Pair& dst = s_pos[TO_POS ? a.rht.pinv[k] : 0][threadIdx.x];
+          if constexpr (IN_BF16) dst = pw[g + k];
+          else dst = make_float2(v0[g + k], v1[g + k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const Pair src = s_pos[TO_POS ? k : 0][threadIdx.x];
+          if constexpr (IN_BF16) pw[g + k] = src;
+          else { v0[g + k] = src.x; v1[g + k] = src.y; }
+        }
+      }
+    };
+    // (the statistics of the dynamic clip are summed in slot order)
+    if (TO_POS && !F::MX) to_positions();
     BlockScale s0, s1;
     if (F::MX && (a.mx.clip | a.mx.uos)) {
       float sum0 = 0.0f, sq0 = 0.0f, sum1 = 0.0f, sq1 = 0.0f;
@@ -740,12 +767,13 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
       s1 = make_block_scale<FMT, IN_BF16>(am1, os);
     }
     const bool fast = block_fast<IN_BF16, ROUND>(s0, am0) && block_fast<IN_BF16, ROUND>(s1, am1);
+    if (TO_POS && F::MX) to_positions();
 
-    // ---- quantise in slot order ----
+    // ---- quantise in slot order (position order after the move) ----
     if (F::FP4) {
 #pragma unroll
       for (int h = 0; h < B / 16; ++h) {
-        // random words by slot: r[k] for columns c and c + 1
+        // random words in the order of the values: r[k] for columns c and c + 1
         uint2 r[ROUND == ALTOB200_ROUND_RTN ? 1 : 16];
         if (ROUND == ALTOB200_ROUND_SR_SLOTS) {
           // [64 positions, slot order within groups of 16][64 columns]
@@ -753,20 +781,39 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
 #pragma unroll
           for (int k = 0; k < 16; ++k) r[k % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = __ldg(t + 32 * k);
         } else if (ROUND == ALTOB200_ROUND_SR_BITS) {
+          // by position: the 8 pairs of these 16 rows are 8 words of either plane, consecutive and 32-byte aligned
+          // unless the caller's table says otherwise (rand_vec).  NVFP4 bf16 8192 x 4096 with the transform, periodic
+          // table / full planes: 62 / 61 us; with one 4-byte load (and one modulo) a word 144 / 166
+          const bool tiled = a.tile_rows != 0;
+          const int64_t idx = (mb + 16 * h) >> 1;
+          const int64_t pitch = tiled ? a.tile_pairs : half_rows;
+          const int64_t plane = (tiled ? a.tile_rows : a.cols) * pitch;
+          const uint32_t* t0 = a.rand_bits + (tiled ? (int64_t)tile_row0 : c) * pitch;
+          const uint32_t* t1 = a.rand_bits + (tiled ? (int64_t)tile_row1 : c + 1) * pitch;
+          if (!ok) {
 #pragma unroll
-          for (int k = 0; k < 16; ++k) {
-            uint2 w = make_uint2(0u, 0u);
-            if (ok) {
-              const int64_t pos = mb + 16 * h + a.rht.pinv[k], idx = pos >> 1;
-              if (a.tile_rows != 0) {
-                const uint32_t* t = a.rand_bits + (pos & 1) * a.tile_rows * a.tile_pairs + (uint32_t)idx % (uint32_t)a.tile_pairs;
-                w = make_uint2(__ldg(t + (int64_t)tile_row0 * a.tile_pairs), __ldg(t + (int64_t)tile_row1 * a.tile_pairs));
-              } else {
-                const uint32_t* t = a.rand_bits + (pos & 1) * a.cols * half_rows + c * half_rows + idx;
-                w = make_uint2(__ldg(t), __ldg(t + half_rows));
+            for (int i = 0; i < 16; ++i) r[i % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = make_uint2(0u, 0u);
+          } else if (a.rand_vec) {
+            const int64_t p = tiled ? (int64_t)((uint32_t)idx % (uint32_t)a.tile_pairs) : idx;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+#pragma unroll
+              for (int odd = 0; odd < 2; ++odd) {
+                const uint4 w0 = __ldg(reinterpret_cast<const uint4*>(t0 + odd * plane + p) + q);
+                const uint4 w1 = __ldg(reinterpret_cast<const uint4*>(t1 + odd * plane + p) + q);
+                const uint32_t u0[4] = {w0.x, w0.y, w0.z, w0.w}, u1[4] = {w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  r[(8 * q + 2 * j + odd) % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = make_uint2(u0[j], u1[j]);
               }
             }
-            r[k % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = w;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int64_t pair = idx + (i >> 1);
+              const int64_t p = (i & 1) * plane + (tiled ? (int64_t)((uint32_t)pair % (uint32_t)a.tile_pairs) : pair);
+              r[i % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = make_uint2(__ldg(t0 + p), __ldg(t1 + p));
+            }
           }
         } else if (ROUND == ALTOB200_ROUND_SR_PHILOX) {
           const uint64_t p0 = (uint64_t)(c * half_rows + ((mb + 16 * h) >> 1));        // pair index, column c
@@ -780,13 +827,6 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
             philox4x32_10_keys((uint32_t)ctr, (uint32_t)(ctr >> 32), a.pk, o1);
 #pragma unroll
             for (int q = 0; q < 4; ++q) r[(4 * i + q) % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = make_uint2(o0[q], o1[q]);
-          }
-          if (WORDS_TO_SLOTS) {   // position order -> slot order through a private shared-memory column
-#pragma unroll
-            for (int k = 0; k < 16; ++k) s_words[k % (WORDS_TO_SLOTS ? 16 : 1)][threadIdx.x] = r[k % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)];
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-              r[k % (ROUND == ALTOB200_ROUND_RTN ? 1 : 16)] = s_words[WORDS_TO_SLOTS ? a.rht.pinv[k] : 0][threadIdx.x];
           }
         }
         // byte k % 4 of word k / 4: code of slot k, column c in the low nibble and c + 1 in the high one
@@ -829,7 +869,7 @@ __global__ void __launch_bounds__(COL_NT) quantize_colwise_kernel(ColwiseArgs a)
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
           uint32_t o = by_slot[w];
-          if (RHT) {   // output position i takes slot perm[i]
+          if (RHT && !TO_POS) {   // output position i takes slot perm[i]
             const uint32_t lo = __byte_perm(by_slot[0], by_slot[1], a.rht.psel[w]);
             const uint32_t hi = __byte_perm(by_slot[2], by_slot[3], a.rht.psel[w]);
             o = (lo & ~a.rht.pmask[w]) | (hi & a.rht.pmask[w]);
@@ -2009,6 +2049,8 @@ int altob200_quantize_colwise(const void* x, int64_t rows, int64_t cols, int64_t
   if (a.tile_rows != 0 && (rows >= (1ll << 32) || cols >= (1ll << 32) || a.tile_rows >= (1ll << 32) ||
                            a.tile_pairs >= (1ll << 32)))
     return ALTOB200_ELIMIT;
+  // rows are a multiple of 32 here (see out_row_bytes): planes start and continue on 16-word boundaries
+  a.rand_vec = aligned16(a.rand_bits) && (a.tile_rows == 0 || a.tile_pairs % 8 == 0);
   a.philox_seed = p->philox_seed; a.philox_offset = p->philox_offset;
   philox_make_keys(p->philox_seed, &a.pk);
   int rc = fill_rht(&a.rht, p->rht_n, p->rht_perm, p->rht_sign);

@@ -213,3 +213,25 @@ def test_two_level_operands_of_views(form):
         got, want = make(t), make(t.contiguous())
         _same(got, want)
         assert torch.equal(got.macro.codes, want.macro.codes)
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("tile", [None, (64, 32), (5, 8), (3, 12), (64, 6)])
+@pytest.mark.parametrize("rotate", [False, True])
+@pytest.mark.parametrize("fmt", [L.FMT_NVFP4, L.FMT_MXFP4])
+@pytest.mark.parametrize("shape", [(32, 8), (96, 160), (160, 416)])
+def test_column_blocks_with_explicit_words(shape, fmt, rotate, tile, offset):
+    """Words in vectors (16-byte aligned, whole groups of 16 rows) or one by one: the codes that the row-wise
+    quantizer makes of the transposed matrix with the same words."""
+    x = _matrix(*shape, "normal")
+    rows, cols = shape[1], shape[0]                      # of the axis-last view
+    n_rows, n_pairs = tile or (rows, cols // 2)
+    g = torch.Generator().manual_seed(3)
+    flat = torch.randint(-2 ** 31, 2 ** 31 - 1, (2 * n_rows * n_pairs + offset,), generator=g, dtype=torch.int32).cuda()
+    table = flat[offset:].view(2, n_rows, n_pairs)
+    planes = table[:, torch.arange(rows, device="cuda") % n_rows][:, :, torch.arange(cols // 2, device="cuda") % n_pairs]
+    had = _transform() if rotate else None
+    got = E.quant_cols(x, fmt, None, had.device_params() if rotate else None,
+                       dict(rounding=L.ROUND_SR_BITS, rand_bits=table, rand_tile=tile or (0, 0)))
+    view = (had(x, left_mul=True) if rotate else x).t().contiguous()
+    _same(got, E.quant_rows(view, fmt, None, dict(rounding=L.ROUND_SR_BITS, rand_bits=planes.contiguous())))
