@@ -1541,20 +1541,37 @@ static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N,
 #undef LAUNCH
 }
 
+template <int HN, bool B_UNIFORM>
 static int launch_gemm_macro(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td,
-                             const MacroGemmArgs& margs, cudaStream_t st) {
-  using C = CfgMacro;
-  const bool b_uniform = margs.mb.shift >= 7;   // one B factor per column tile and chunk
-  auto kernel = b_uniform ? gemm_macro_kernel<true> : gemm_macro_kernel<false>;
-  static std::atomic<int> attr_set[2][MAX_DEVICES];
-  const int rc = ensure_smem_attr(kernel, C::SMEM_BYTES, attr_set[b_uniform ? 1 : 0]);
+                             const MacroGemmArgs& margs, int64_t grid, cudaStream_t st) {
+  using C = CfgMacro<HN>;
+  auto kernel = gemm_macro_kernel<HN, B_UNIFORM>;
+  static std::atomic<int> attr_set[MAX_DEVICES];
+  const int rc = ensure_smem_attr(kernel, C::SMEM_BYTES, attr_set);
   if (rc != ALTOB200_OK) return rc;
-  const GemmArgs& a = margs.g;
-  const int64_t tiles = ceil_div(a.M, BM) * ceil_div(a.N, C::BN) * (a.k_offs != nullptr ? a.num_batches : 1);
-  int64_t grid = sm_count_gemm();
-  if (grid > tiles) grid = tiles;
   (void)launch_after(kernel, dim3((unsigned)grid), dim3(NUM_THREADS_MACRO), C::SMEM_BYTES, st, ta, tb, td, margs);
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
+}
+
+// Columns of a half: 128 (tiles of 128 x 256) or 64 (128 x 128).  A wide tile takes less time per column of a
+// chunk, but there are half as many, so it loses where they leave SMs without work or a last wave nearly empty,
+// and its epilogue has nothing to overlap with, which counts where the K range is short.  The estimate is in chunk
+// times of a narrow tile (0.33 us with one B factor per tile, 0.37 with one per column), fitted to
+//                                      one B factor, us: narrow / wide     per column, us: narrow / wide
+//   320 x 288 x 14336 (9 / 6 tiles)            39.0 / 59.3                        43.9 / 83.8
+//   512 x 4096 x 4096 (one wave each)          14.7 / 21.4                        16.2 / 25.9
+//   2048^3 (two waves / one)                   15.6 / 14.3                        17.3 / 16.6
+//   4096^3 (seven / four)                      81.4 / 75.9                        91.6 / 94.2
+//   16 ranges of 128, 5760 x 2880                                                 188 / 213
+//   8 ranges of 384, 2880 x 2880                                                  70.3 / 68.8
+static int macro_half(int64_t row_tiles, int64_t N, int64_t chunks, bool b_uniform, int64_t* grid) {
+  const int64_t sms = sm_count_gemm();
+  const int64_t narrow = row_tiles * ceil_div(N, 128), wide = row_tiles * ceil_div(N, 256);
+  const double t_narrow = (double)ceil_div(narrow, sms) * (4.0 + (double)chunks);
+  const double t_wide = (double)ceil_div(wide, sms) * (9.0 + (b_uniform ? 1.56 : 1.77) * (double)chunks);
+  const int64_t tiles = t_narrow <= t_wide ? narrow : wide;
+  *grid = tiles < sms ? tiles : sms;
+  return t_narrow <= t_wide ? 64 : 128;
 }
 
 static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_experts, const void* a_codes,
@@ -1581,16 +1598,21 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   const int64_t b_rows = N * (row_groups ? num_experts : 1);
   if (M >= (1ll << 31) || b_rows >= (1ll << 31) || k_bytes >= (1ll << 31)) return ALTOB200_ELIMIT;
   // the kernel addresses the factor codes of a tile's rows by 32-bit offsets from its first row
-  const int64_t span_a = (M < BM ? M : BM) - 1, span_b = (N < CfgMacro::BN ? N : CfgMacro::BN) - 1;
+  const int64_t span_a = (M < BM ? M : BM) - 1, span_b = (N < 256 ? N : 256) - 1;
   if (a_macro->row_stride < 0 || b_macro->row_stride < 0 ||
       (span_a >> a_macro->row_shift) * a_macro->row_stride >= (1ll << 32) ||
       (span_b >> b_macro->row_shift) * b_macro->row_stride >= (1ll << 32))
     return ALTOB200_ELIMIT;
 
+  const bool b_uniform = b_macro->row_shift == 7;   // one B factor per 128 columns and chunk
+  const int64_t batches = k_offs != nullptr ? num_experts : 1;
+  int64_t grid = 0;
+  const int HN = macro_half(ceil_div(M, BM) * batches, N, ceil_div(K / batches, 128), b_uniform, &grid);
+
   CUtensorMap ta, tb, td;
   int rc = make_tmap(&ta, a_codes, M, k_bytes, BM);
   if (rc != ALTOB200_OK) return rc;
-  rc = make_tmap(&tb, b_codes, b_rows, k_bytes, CfgMacro::HN);
+  rc = make_tmap(&tb, b_codes, b_rows, k_bytes, HN);
   if (rc != ALTOB200_OK) return rc;
   rc = make_tmap_out(&td, d, k_offs != nullptr ? num_experts : 1, M, N, ldd, out_dtype == ALTOB200_DT_BF16, 128, 16);
   if (rc != ALTOB200_OK) return rc;
@@ -1604,17 +1626,22 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   g.d = d; g.ldd = ldd; g.out_bf16 = out_dtype == ALTOB200_DT_BF16;
   g.num_experts = row_groups ? num_experts : 0; g.group_expert = group_expert;
   g.sfb_expert_stride = (int64_t)altob200_packed_scale_bytes(N, K / 32);
-  g.k_offs = k_offs; g.num_batches = k_offs != nullptr ? num_experts : 1;
+  g.k_offs = k_offs; g.num_batches = (int)batches;
   {
     const int64_t tiles_m = ceil_div(M, BM);
     int64_t gm = 8;
     if (gm > tiles_m) gm = tiles_m;
     const int64_t n_groups = ceil_div(tiles_m, gm);
     g.group_m = (int)ceil_div(tiles_m, n_groups);
+    const int64_t tiles_n = ceil_div(N, 2 * HN);
+    m.per_batch = make_tile_div(tiles_m * tiles_n);
+    m.per_group = make_tile_div(g.group_m * tiles_n);
+    m.rows_full = make_tile_div(g.group_m);
+    m.rows_last = make_tile_div(tiles_m - (ceil_div(tiles_m, g.group_m) - 1) * g.group_m);
   }
   g.wait_ns = wait_limit_ns();
   for (int j = 0; j < 4; ++j)
-    g.idesc[j] = make_idesc(KIND_MXF4, ALTOB200_FMT_MXFP4, ALTOB200_FMT_MXFP4, BM, CfgMacro::HN, (j & 1) * 2);
+    g.idesc[j] = make_idesc(KIND_MXF4, ALTOB200_FMT_MXFP4, ALTOB200_FMT_MXFP4, BM, HN, (j & 1) * 2);
 #ifdef ALTOB200_GEMM_PROFILE
   {
     const char* e = getenv("ALTOB200_GEMM_DEBUG");
@@ -1626,7 +1653,10 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   m.mb.codes = b_macro->codes; m.mb.row_stride = b_macro->row_stride; m.mb.chunk_stride = b_macro->chunk_stride;
   m.mb.expert_stride = row_groups ? b_macro->expert_stride : 0; m.mb.shift = b_macro->row_shift;
   m.out_scale = out_scale;
-  return launch_gemm_macro(ta, tb, td, m, (cudaStream_t)stream);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (HN == 64)
+    return b_uniform ? launch_gemm_macro<64, true>(ta, tb, td, m, grid, st) : launch_gemm_macro<64, false>(ta, tb, td, m, grid, st);
+  return b_uniform ? launch_gemm_macro<128, true>(ta, tb, td, m, grid, st) : launch_gemm_macro<128, false>(ta, tb, td, m, grid, st);
 }
 
 }  // namespace altob200
