@@ -17,7 +17,6 @@ they are for every axis and block shape.
 """
 from __future__ import annotations
 
-import functools
 from typing import Optional, Tuple
 
 import torch
@@ -37,6 +36,12 @@ def _fusable(t: torch.Tensor) -> bool:
     scales and factors."""
     return (t.dtype == torch.bfloat16 and t.stride(-1) == 1 and t.stride(-2) >= t.shape[-1] and t.data_ptr() % 16 == 0
             and all(st * t.element_size() % 16 == 0 for st in t.stride()[:-1]))
+
+
+def _fusable_cols(t2: torch.Tensor, rht: Optional[L.Rht], clip_mode: str) -> bool:
+    """Whether the column-wise quantizer may also rotate: the statistics of the dynamic clip depend on the order
+    of their sums, which is that of the rows, and behind a rotation inside the kernel that of the butterfly."""
+    return _fusable(t2) and not (rht is not None and clip_mode == "dynamic")
 
 
 def _chunks(n: int) -> int:
@@ -59,12 +64,13 @@ def rows_operand(t2: torch.Tensor, use_uos: bool, sr: Optional[dict] = None) -> 
 def cols_operand(t2: torch.Tensor, use_uos: bool, clip_mode: str = "none", sr: Optional[dict] = None,
                  hadamard_transform=None) -> E.Operand:
     """t2 [R, C] -> operand [C, R] reduced along R (the token axis) after the optional rotation: blocks run
-    down the rows of t2.  ``sr`` from ``E.sr_args_cols`` with the transform's ``rht_of``."""
+    down the rows of t2.  ``sr`` from ``E.sr_args_cols`` with the transform's ``rht_of`` where the quantizer
+    applies it (``_fusable_cols``), else without."""
     rht = rht_of(hadamard_transform)
     sr = sr or E.RTN
     if rht is None:
         t2 = _rotate(t2, hadamard_transform)
-    if _fusable(t2) and sr["rounding"] in (L.ROUND_RTN, L.ROUND_SR_SLOTS):
+    if _fusable_cols(t2, rht, clip_mode) and sr["rounding"] in (L.ROUND_RTN, L.ROUND_SR_SLOTS):
         R, Cc = t2.shape
         mbs = torch.empty(Cc, _chunks(R), dtype=torch.uint8, device=t2.device)
         op = E.quant_cols(t2, MX, None, rht, sr, use_uos, clip_mode, macro_codes=mbs)
@@ -132,10 +138,11 @@ def _grad_operands(ctx, g2: torch.Tensor, M: int, N: int) -> Tuple[E.Operand, E.
     if ctx.use_2dblock_x:
         return tiles_operands(g2, ctx.use_uos, E.sr_args(ctx.use_sr_grad, "dy_n", M, N, g2.device))
     g_n = rows_operand(g2, ctx.use_uos, E.sr_args(ctx.use_sr_grad, "dy_n", M, N, g2.device))
-    # (words in slot order only fit the fused kernel, so an input it cannot read takes the plain table)
+    # the table's order is that of the transform inside the quantizer, if it runs there
     rht = rht_of(ctx.hadamard_transform)
-    draw = E.sr_args if not _fusable(g2) else functools.partial(E.sr_args_cols, rht=rht)
-    g_m = cols_operand(g2, ctx.use_uos, ctx.clip_mode, draw(ctx.use_sr_grad, "dy_m", N, M, g2.device),
+    if not _fusable_cols(g2, rht, ctx.clip_mode):
+        rht = None
+    g_m = cols_operand(g2, ctx.use_uos, ctx.clip_mode, E.sr_args_cols(ctx.use_sr_grad, "dy_m", N, M, g2.device, rht),
                        ctx.hadamard_transform)
     return g_n, g_m
 

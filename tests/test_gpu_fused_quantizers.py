@@ -235,3 +235,37 @@ def test_column_blocks_with_explicit_words(shape, fmt, rotate, tile, offset):
                        dict(rounding=L.ROUND_SR_BITS, rand_bits=table, rand_tile=tile or (0, 0)))
     view = (had(x, left_mul=True) if rotate else x).t().contiguous()
     _same(got, E.quant_rows(view, fmt, None, dict(rounding=L.ROUND_SR_BITS, rand_bits=planes.contiguous())))
+
+
+def test_dynamic_clip_behind_a_rotation_sums_in_row_order():
+    """Rotated columns of +-M whose running sum overflows in some orders of the rows and not in others: the block
+    statistics, hence the codes, are those of the separate passes."""
+    from alto_b200 import _two_level as T
+    had = _transform()
+    x = torch.zeros(128, 16, dtype=torch.bfloat16, device="cuda")
+    x[torch.arange(16), torch.arange(16)] = 3.3e38
+    got = T.cols_operand(x, False, "dynamic", None, had)
+    scaled, factors = macro_block_scaling(had(x, left_mul=True), axis=0)
+    _same(got, E.quant_cols(scaled, MX, None, None, E.RTN, clip_mode="dynamic"))
+    assert torch.equal(got.macro.codes, factors)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("clip_mode", ["none", "dynamic"])
+def test_two_level_gradients_draw_the_same_words_on_every_route(dtype, clip_mode, monkeypatch):
+    """Rounding words of a gradient that is rotated inside the quantizer, before it, or in fp32: those of the
+    plain table."""
+    from types import SimpleNamespace
+    from alto_b200 import _two_level as T
+    had = _transform()
+    g = (_matrix(160, 192, "normal") * 1e-3).to(dtype)
+    ctx = SimpleNamespace(use_2dblock_x=False, use_uos=False, use_sr_grad=True, hadamard_transform=had,
+                          clip_mode=clip_mode)
+    torch.manual_seed(9)
+    got = T._grad_operands(ctx, g, 160, 192)
+    monkeypatch.setattr(L, "SLOTS_TILE", None)           # no view takes the slot-ordered table
+    torch.manual_seed(9)
+    want = T._grad_operands(ctx, g, 160, 192)
+    for a, b in zip(got, want):
+        _same(a, b)
+        assert torch.equal(a.macro.codes, b.macro.codes)
