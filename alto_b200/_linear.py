@@ -344,8 +344,8 @@ def linear_forward(ctx, name: str, x, weight, fmt, *, use_2dblock_x, use_2dblock
     rht, dense = split_transform(hadamard_transform, use_2dblock_x)
     ctx.xm_ready = None
     plain = not use_uos and clip_mode == "none"
-    # an operand that only a gradient needs is not made when that gradient is not asked for (evaluation, frozen
-    # weights, a first layer); the DGE factor of dW reads the codes of the weight's dgrad operand
+    # an operand that only a gradient needs is not made when that gradient is not asked for (frozen weights, a first
+    # layer; evaluation, whose inputs come detached); the DGE factor of dW reads the codes of the weight's dgrad operand
     need_dx, need_dw = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
     want_m, want_t = need_dw, need_dx or (need_dw and use_dge)
     if OVERLAP and want_m and want_t and not use_2dblock_x and dense is None and plain and not pre:

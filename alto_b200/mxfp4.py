@@ -17,7 +17,7 @@ from . import _quant as Q
 from . import _two_level as T
 from .hadamard import HadamardFactory, HadamardTransform
 from .macro_block_scaling import macro_block_descaling, macro_block_scaling
-from .nvfp4 import unwrap_weight_wrapper
+from .nvfp4 import outside_of_grad_mode, unwrap_weight_wrapper
 
 BLOCK_SIZE_DEFAULT = 32
 
@@ -176,5 +176,6 @@ def _to_mxfp4_then_scaled_mm(
             hadamard_transform = HadamardFactory.create_transform(device=b.device)
     else:
         hadamard_transform = None
+    a, b = outside_of_grad_mode(a, b)
     return MXFP4LinearFunction.apply(a, b, use_2dblock_x, use_2dblock_w, use_sr_grad, use_dge, clip_mode,
                                      use_macro_block_scaling, hadamard_transform, use_uos)

@@ -15,7 +15,7 @@ import torch
 from . import _lib as L
 from . import _linear as E
 from . import _quant as Q
-from .nvfp4 import unwrap_weight_wrapper
+from .nvfp4 import outside_of_grad_mode, unwrap_weight_wrapper
 
 BLOCK_SIZE_DEFAULT = 32
 SUPPORTED_FORMATS = ["e4m3", "e5m2"]
@@ -152,4 +152,5 @@ def _to_mxfp8_then_scaled_mm(
     use_2dblock_x: bool = False,
     use_2dblock_w: bool = False,
 ) -> torch.Tensor:
+    a, b = outside_of_grad_mode(a, b)
     return MXFP8LinearFunction.apply(a, b, fp8_variant, use_sr_grad, use_2dblock_x, use_2dblock_w)

@@ -51,6 +51,16 @@ def unwrap_weight_wrapper(weight: torch.Tensor) -> torch.Tensor:
     return weight.as_subclass(torch.Tensor)
 
 
+def outside_of_grad_mode(x: torch.Tensor, weight: torch.Tensor):
+    """The inputs of a linear function as its forward should see them: inside an autograd ``forward`` grad mode is
+    always off and ``needs_input_grad`` only repeats ``requires_grad``, which the parameters of an evaluation pass
+    keep, so outside of grad mode they are handed over detached."""
+    if torch.is_grad_enabled():
+        return x, weight
+    plain = unwrap_weight_wrapper(weight)
+    return x.detach(), plain.detach() if isinstance(plain, torch.Tensor) else weight
+
+
 from ._linear import amax_scratch as _amax_scratch, draw_philox as _draw_philox, explicit_sr_bits  # noqa: E402,F401
 
 # ---------------------------------------------------------------------------------------
@@ -223,5 +233,6 @@ def _to_nvfp4_then_scaled_mm(
     if use_hadamard:
         with torch.no_grad():
             hadamard_transform = HadamardFactory.create_transform(device=b.device)
+    a, b = outside_of_grad_mode(a, b)
     return NVFP4LinearFunction.apply(a, b, use_2dblock_x, use_2dblock_w, use_sr_grad, use_outer_scale,
                                      hadamard_transform, use_dge, scale_format)
