@@ -34,7 +34,8 @@ _scratch = {}
 
 def amax_scratch(device: torch.device) -> torch.Tensor:
     """Zeroed per-(device, stream) scratch of the amax kernel (the kernel leaves it zeroed)."""
-    key = (device.index, torch._C._cuda_getCurrentRawStream(device.index))
+    index = torch.cuda.current_device() if device.index is None else device.index
+    key = (index, torch._C._cuda_getCurrentRawStream(index))
     buf = _scratch.get(key)
     if buf is None:
         buf = torch.zeros(L.AMAX_SCRATCH_BYTES // 4, dtype=torch.int32, device=device)
