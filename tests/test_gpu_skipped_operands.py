@@ -55,7 +55,8 @@ def test_evaluation_of_parameters(monkeypatch, recipe, weight_2d, mode):
 
 def test_evaluation_of_a_converted_module(monkeypatch):
     from alto_b200 import dispatch
-    config = dispatch.TrainingOpConfig("mxfp8_e4m3", False, True, False, False, False)
+    config = dispatch.TrainingOpConfig(precision="mxfp8_e4m3", use_2dblock_x=False, use_2dblock_w=True, use_hadamard=False,
+                                       use_sr_grad=False, use_dge=False)
     layer = torch.nn.Linear(192, 160, bias=False, dtype=torch.bfloat16, device="cuda")
     w = layer.weight.detach().clone()
     x = torch.randn(128, 192, generator=torch.Generator().manual_seed(0)).bfloat16().cuda()
