@@ -463,21 +463,20 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                           (m0 >> margs.ma.shift) * margs.ma.row_stride;
       const uint8_t* pb = margs.mb.codes + (int64_t)mt.expert * margs.mb.expert_stride +
                           (mt.chunk0 + fc) * margs.mb.chunk_stride + (n0 >> margs.mb.shift) * margs.mb.row_stride;
-      // offsets of the lane's rows from the tile's first (a row beyond the matrix reads the last one); the host
-      // refuses strides that would not fit
+      // offsets of the lane's rows from the tile's first (a row beyond the matrix reads the last one)
       constexpr int NB = B_UNIFORM ? C::SFB_BLOCKS : C::BN / 64;
-      uint32_t off_a[2], off_b[NB];
+      int64_t off_a[2], off_b[NB];
       const uint32_t m_last = (uint32_t)(args.M - m0 < BM ? args.M - m0 : BM) - 1u;
       const uint32_t n_last = (uint32_t)(args.N - n0 < C::BN ? args.N - n0 : C::BN) - 1u;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const uint32_t r = (uint32_t)(quad * 32 + 16 * i + fr);
-        off_a[i] = ((r < m_last ? r : m_last) >> margs.ma.shift) * (uint32_t)margs.ma.row_stride;
+        off_a[i] = (int64_t)((r < m_last ? r : m_last) >> margs.ma.shift) * margs.ma.row_stride;
       }
 #pragma unroll
       for (int i = 0; i < NB; ++i) {
         const uint32_t r = (uint32_t)(B_UNIFORM ? 128 * i : quad * (C::BN / 4) + 16 * i + fr);
-        off_b[i] = ((r < n_last ? r : n_last) >> (B_UNIFORM ? 7 : 0)) * (uint32_t)margs.mb.row_stride;
+        off_b[i] = (int64_t)((r < n_last ? r : n_last) >> (B_UNIFORM ? 7 : 0)) * margs.mb.row_stride;
       }
       uint32_t ca[2], cb[NB];
       auto load_codes = [&](int ks) {

@@ -1597,12 +1597,6 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   const bool row_groups = group_expert != nullptr;
   const int64_t b_rows = N * (row_groups ? num_experts : 1);
   if (M >= (1ll << 31) || b_rows >= (1ll << 31) || k_bytes >= (1ll << 31)) return ALTOB200_ELIMIT;
-  // the kernel addresses the factor codes of a tile's rows by 32-bit offsets from its first row
-  const int64_t span_a = (M < BM ? M : BM) - 1, span_b = (N < 256 ? N : 256) - 1;
-  if (a_macro->row_stride < 0 || b_macro->row_stride < 0 ||
-      (span_a >> a_macro->row_shift) * a_macro->row_stride >= (1ll << 32) ||
-      (span_b >> b_macro->row_shift) * b_macro->row_stride >= (1ll << 32))
-    return ALTOB200_ELIMIT;
 
   const bool b_uniform = b_macro->row_shift == 7;   // one B factor per 128 columns and chunk
   const int64_t batches = k_offs != nullptr ? num_experts : 1;

@@ -1,4 +1,4 @@
-"""Calls at the edge of what the host functions take."""
+"""Calls at the edge of what the host functions and the C interface take."""
 import pytest
 import torch
 
@@ -21,3 +21,40 @@ def test_run_ends_are_a_vector():
     for t in (offs, offs.cuda()):
         with pytest.raises(RuntimeError):
             group_experts_from_offsets(t, 256)
+
+
+class _Strided(L.MacroScale):
+    """Factor codes whose row r starts ``first + r * row_stride`` bytes into a buffer."""
+
+    __slots__ = ("first",)
+
+    def desc(self):
+        d = super().desc()
+        d.codes += self.first
+        return d
+
+
+@pytest.mark.parametrize("m,n,stride", [(130, 96, "reversed"), (256, 416, "reversed"), (130, 96, "beyond 32 bits")])
+def test_two_level_factors_with_any_row_stride(m, n, stride):
+    k = 384
+    g = torch.Generator().manual_seed(0)
+    a = T.rows_operand(torch.randn(m, k, generator=g).bfloat16().cuda(), False)
+    b = T.rows_operand(torch.randn(n, k, generator=g).bfloat16().cuda(), False)
+
+    def moved(op):
+        rows, nc = op.macro.codes.shape
+        if stride == "reversed":
+            scale = _Strided(op.macro.codes.flip(0).contiguous(), -nc, 1, 0)
+            scale.first = (rows - 1) * nc
+        else:
+            pitch = (1 << 32) // 96            # rows of one tile lie more than 2^32 bytes apart
+            buf = torch.empty((rows - 1) * pitch + nc, dtype=torch.uint8, device="cuda")
+            buf.as_strided((rows, nc), (pitch, 1)).copy_(op.macro.codes)
+            scale = _Strided(buf, pitch, 1, 0)
+            scale.first = 0
+        return scale
+
+    want, got = (torch.empty(m, n, dtype=torch.float32, device="cuda") for _ in range(2))
+    L.gemm_mxfp4_two_level(m, n, k, a.codes, a.scales, a.macro, b.codes, b.scales, b.macro, want)
+    L.gemm_mxfp4_two_level(m, n, k, a.codes, a.scales, moved(a), b.codes, b.scales, moved(b), got)
+    assert torch.equal(got, want)
