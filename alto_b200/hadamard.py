@@ -26,14 +26,14 @@ from torch import Tensor
 from . import _lib as L
 
 
-def _sylvester(n: int) -> Tensor:
-    H = torch.ones(1, 1)
+def _sylvester(n: int, **options) -> Tensor:
+    H = torch.ones(1, 1, **options)
     while H.shape[0] < n:
         H = torch.vstack((torch.hstack((H, H)), torch.hstack((H, -H))))
     return H
 
 
-_SYLVESTER_16 = _sylvester(16)
+_SYLVESTER_16 = _sylvester(16, dtype=torch.float32, device="cpu")   # whatever the defaults are at import
 
 
 def _is_pow2(n: int) -> bool:
@@ -43,9 +43,10 @@ def _is_pow2(n: int) -> bool:
 _BASE_CACHE = {}
 
 
-def _base_matrix(n: int) -> Tensor:
+def _base_matrix_t(n: int) -> Tensor:
+    """The transposed base matrix, contiguous like the products made of it."""
     if n not in _BASE_CACHE:
-        _BASE_CACHE[n] = _load_base_matrix(n)
+        _BASE_CACHE[n] = _load_base_matrix(n).t().contiguous()
     return _BASE_CACHE[n]
 
 
@@ -78,10 +79,10 @@ def random_hadamard_matrix(size: int, dtype=torch.float32, device="cpu", gen: Op
     """diag(Q) @ H^T with Q drawn as ``torch.randint(0, 2, (size,), dtype=dtype) * 2 - 1``."""
     Q = torch.randint(low=0, high=2, size=(size,), generator=gen, dtype=dtype)
     Q = Q * 2 - 1
-    H = _base_matrix(size).to(dtype)
+    Ht = _base_matrix_t(size).to(dtype)
     # The matrix stays on the host: the kernels take it as (perm, sign) launch parameters, and a
     # per-call host-to-device copy would stall the stream on every forward.
-    return Q.unsqueeze(1) * H.t()
+    return Q.unsqueeze(1) * Ht
 
 
 class HadamardFactory:

@@ -178,3 +178,25 @@ def test_packed_scales_of_host_tensors(rows, ncols, block):
         for c in range(ncols):
             want[(r // 128 * ct + c // 4) * 512 + r % 32 * 16 + r // 32 % 4 * 4 + c % 4] = s[r // block, c]
     assert torch.equal(got, want)
+
+
+def test_random_hadamard_matrix_is_contiguous():
+    from alto_b200.hadamard import random_hadamard_matrix
+    for size in (16, 32):
+        m = random_hadamard_matrix(size, gen=torch.Generator().manual_seed(0))
+        assert m.is_contiguous() and torch.equal(m @ m.t(), size * torch.eye(size))
+
+
+def test_transform_of_a_module_imported_under_another_device():
+    """The package may first be imported where tensors are made on the meta device, in a wider default type."""
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "torch.set_default_dtype(torch.float64)\n"
+            "with torch.device('meta'):\n"
+            "    from alto_b200.hadamard import HadamardFactory\n"
+            "torch.set_default_dtype(torch.float32)\n"
+            "HadamardFactory.configure(block_size=16, randomized=True, dtype=torch.float32, seed=3)\n"
+            "t = HadamardFactory.create_transform(device='cpu')\n"
+            "assert t.is_fused\n")
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300)
