@@ -269,3 +269,23 @@ def test_two_level_gradients_draw_the_same_words_on_every_route(dtype, clip_mode
     for a, b in zip(got, want):
         _same(a, b)
         assert torch.equal(a.macro.codes, b.macro.codes)
+
+
+@pytest.mark.parametrize("shape", [(64, 64), (160, 416)])
+def test_macro_scaling_with_a_word_for_every_element(shape):
+    """The fused row-wise and 2-D forms with full planes of words instead of a periodic table."""
+    x = _matrix(*shape, "normal")
+    g = torch.Generator().manual_seed(4)
+    words = torch.randint(-2 ** 31, 2 ** 31 - 1, (2, shape[0], shape[1] // 2), generator=g, dtype=torch.int32).cuda()
+    sr = dict(rounding=L.ROUND_SR_BITS, rand_bits=words)
+    for two_d in (False, True):
+        chunks = (-(-shape[0] // 128) if two_d else shape[0], -(-shape[1] // 128))
+        codes = torch.empty(chunks, dtype=torch.uint8, device="cuda")
+        scaled, factors = macro_block_scaling(x, axis=-1, use_2d_block=two_d)
+        if two_d:
+            got, want = E.quant_2d(x, MX, None, True, False, sr, codes), E.quant_2d(scaled, MX, None, True, False, sr)
+        else:
+            got, want = [E.quant_rows(x, MX, None, sr, macro_codes=codes)], [E.quant_rows(scaled, MX, None, sr)]
+        for a, b in zip(got, want):
+            _same(a, b)
+        assert torch.equal(codes, factors)

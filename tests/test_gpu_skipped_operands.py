@@ -67,3 +67,21 @@ def test_evaluation_of_a_converted_module(monkeypatch):
     assert layer.weight.requires_grad and evaluated == plain and torch.equal(y0, y1)
     trained, _ = _launches(monkeypatch, lambda: layer(x))
     assert trained != plain
+
+
+@pytest.mark.parametrize("weight_2d", [False, True])
+@pytest.mark.parametrize("recipe", list(CALLS))
+def test_forward_of_a_frozen_side(monkeypatch, recipe, weight_2d):
+    """Only dX asked for: X is not quantised along the tokens.  Only dW: the weight has no second packing."""
+    x, w = torch.randn(128, 192).bfloat16().cuda(), torch.randn(160, 192).bfloat16().cuda()
+
+    def seen(need_x, need_w):
+        launches, _ = _launches(monkeypatch, lambda: CALLS[recipe](x.clone().requires_grad_(need_x),
+                                                                   w.clone().requires_grad_(need_w), weight_2d))
+        return (sum(name == "quantize_colwise" for name, _, _ in launches), sum(t for _, t, _ in launches))
+
+    transposed = int(weight_2d)                       # 2-D blocks: the second packing; 1-D: a column-wise launch
+    assert seen(True, True) == (2 - transposed, transposed)
+    assert seen(True, False) == (1 - transposed, transposed)
+    assert seen(False, True) == (1, 0)
+    assert seen(False, False) == (0, 0)
