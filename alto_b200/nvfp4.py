@@ -55,7 +55,7 @@ def outside_of_grad_mode(x: torch.Tensor, weight: torch.Tensor):
     """The inputs of a linear function as its forward should see them: inside an autograd ``forward`` grad mode is
     always off and ``needs_input_grad`` only repeats ``requires_grad``, which the parameters of an evaluation pass
     keep, so outside of grad mode they are handed over detached."""
-    if torch.is_grad_enabled():
+    if torch.is_grad_enabled() or not (x.requires_grad or getattr(weight, "requires_grad", False)):
         return x, weight
     plain = unwrap_weight_wrapper(weight)
     return x.detach(), plain.detach() if isinstance(plain, torch.Tensor) else weight
