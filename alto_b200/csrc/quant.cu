@@ -275,8 +275,9 @@ struct RowwiseArgs {
 // loads of all four rows are issued before the first is consumed (128 bytes per lane in flight), and
 // the index arithmetic of a task (row and chunk, pointers, position in the periodic random table) is
 // paid once per 64 elements of a lane.
-// Three resident blocks per SM (at most 85 registers per thread) measured fastest: fewer registers
-// spill, more leave too few warps to cover the issue slots.
+// Three resident blocks per SM (at most 85 registers per thread): other block sizes and counts measured within
+// 3 %, although the stochastic-rounding variants spill (NVFP4 bf16 72 bytes, fp32 428); all of them are faster
+// than the body that spilled less (8192 x 4096 NVFP4 from a table: bf16 38 -> 33 us, fp32 70 -> 53).
 constexpr int ROW_R = 4;
 
 // MACRO (MXFP4 from bf16): the two-level recipe's scaling runs in front of the quantisation; a macro block of
@@ -573,8 +574,10 @@ constexpr int COL_TN = 64;   // columns per CTA tile
 // macro block of 128 rows per column, so its maxima only have to cross the four warps.
 template <int FMT, bool IN_BF16, int ROUND, bool RHT, bool MACRO>
 // (fp32 blocks of 32 with words by position are held to the 128 registers of four CTAs an SM: 63 -> 58 us for
-// 8192 x 4096; 0 leaves the others to the compiler)
-__global__ void __launch_bounds__(COL_NT, !IN_BF16 && Fmt<FMT>::B == 32 && ROUND == ALTOB200_ROUND_SR_BITS ? 4 : 0)
+// 8192 x 4096; drawn in the kernel, only behind the transform, 24.0 -> 22.6 us for 4096 x 2880 (without it 5.2 -> 5.4
+// for 512 x 4096); 0 leaves the others to the compiler)
+__global__ void __launch_bounds__(COL_NT, !IN_BF16 && Fmt<FMT>::B == 32 &&
+                                  (ROUND == ALTOB200_ROUND_SR_BITS || (ROUND == ALTOB200_ROUND_SR_PHILOX && RHT)) ? 4 : 0)
 quantize_colwise_kernel(ColwiseArgs a) {
   grid_dependency_wait();
   using F = Fmt<FMT>;
