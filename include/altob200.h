@@ -132,8 +132,9 @@ typedef struct altob200_quant_params {
    * quantisation axis (128 x 128 tiles for the 2-D quantizer) is first multiplied by its factor and rounded
    * to bf16, exactly what altob200_macro_block_scaling writes, and the factor codes go to macro_codes in
    * that function's layout (row-wise: [rows, ceil(cols/128)], column-wise: [cols, ceil(rows/128)], 2-D:
-   * [batch, ceil(rows/128), ceil(cols/128)]).  Rounding RTN, or SR_BITS with a periodic table (row-wise,
-   * 2-D) / SR_SLOTS (column-wise).  The column-wise quantizer applies the Hadamard transform before it. */
+   * [batch, ceil(rows/128), ceil(cols/128)]).  Rounding RTN, or SR_BITS (row-wise, 2-D; full planes or a
+   * periodic table) / SR_SLOTS (column-wise).  The column-wise quantizer applies the Hadamard transform before
+   * it; with CLIP_DYNAMIC and a transform it sums a block's statistics in the order of the transform's slots. */
   uint8_t* macro_codes;
 } altob200_quant_params;
 
