@@ -264,6 +264,11 @@ def _require_cuda(*tensors: Optional[torch.Tensor]) -> None:
             raise RuntimeError("alto_b200 kernels run on CUDA tensors only (no CPU fallback)")
 
 
+def on_current_device(t: torch.Tensor) -> bool:
+    """Whether a kernel launched here may read ``t``: launches go to the current device's stream."""
+    return t.is_cuda and t.device.index == torch.cuda.current_device()
+
+
 def packed_scale_bytes(rows: int, ncols: int) -> int:
     # altob200_packed_scale_bytes: tiles of 128 rows x 4 columns
     return (rows + 127) // 128 * ((ncols + 3) // 4) * 512

@@ -474,9 +474,9 @@ def pack_plain_scales(scales: torch.Tensor, rows: int, is_2d: bool, block: int) 
     assert s.dtype == torch.uint8
     per_row = block if is_2d else 1
     assert s.shape[0] * per_row == rows, f"scale rows {s.shape[0] * per_row} != operand rows {rows}"
-    if s.is_cuda and s.numel() > 0:
+    if s.numel() > 0 and L.on_current_device(s):
         return L.pack_scales(s, rows, per_row)
-    # host tensors (weight shards are laid out before they reach a device) and empty operands
+    # host tensors (weight shards are laid out before they reach a device), other devices and empty operands
     ncols, rt, ct = s.shape[1], (rows + 127) // 128, (s.shape[1] + 3) // 4
     buf = torch.zeros(rt * 128, ct * 4, dtype=torch.uint8, device=s.device)
     buf[:rows, :ncols] = s.repeat_interleave(per_row, dim=0)

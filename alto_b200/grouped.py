@@ -45,9 +45,9 @@ def group_experts_from_offsets(offs: torch.Tensor, m_buf: int) -> torch.Tensor:
     """int32 [ceil(m_buf / 128)]: expert of each 128-row group, -1 for groups past ``offs[-1]``.
     Computed on the device, no host synchronisation."""
     n_groups = (m_buf + ALIGN_SIZE_M - 1) // ALIGN_SIZE_M
-    if offs.is_cuda and offs.dim() == 1 and offs.numel() > 0 and n_groups > 0:
+    if offs.dim() == 1 and offs.numel() > 0 and n_groups > 0 and L.on_current_device(offs):
         return L.group_experts(offs.to(torch.int32).contiguous(), n_groups)
-    # host tensors, no expert or no row
+    # host tensors, other devices, no expert or no row
     starts = torch.arange(n_groups, device=offs.device, dtype=torch.int32) * ALIGN_SIZE_M
     e = torch.bucketize(starts, offs.to(torch.int32), right=True, out_int32=True)
     return torch.where(e >= offs.numel(), torch.full_like(e, -1), e).contiguous()

@@ -58,3 +58,21 @@ def test_two_level_factors_with_any_row_stride(m, n, stride):
     L.gemm_mxfp4_two_level(m, n, k, a.codes, a.scales, a.macro, b.codes, b.scales, b.macro, want)
     L.gemm_mxfp4_two_level(m, n, k, a.codes, a.scales, moved(a), b.codes, b.scales, moved(b), got)
     assert torch.equal(got, want)
+
+
+def test_tensors_of_another_device_are_not_handed_to_a_launch_here(monkeypatch):
+    """The two helpers also serve tensors of a device that is not current, as tensor operations do."""
+    from alto_b200.grouped import group_experts_from_offsets
+    offs = torch.tensor([128, 384], dtype=torch.int32, device="cuda")
+    scales = torch.randint(1, 255, (96, 6), dtype=torch.uint8, device="cuda")
+    experts, packed = group_experts_from_offsets(offs, 600), E.pack_plain_scales(scales, 96, False, 32)
+
+    def launched(*args, **kw):
+        raise AssertionError("a launch on the current device")
+
+    other = torch.cuda.current_device() + 1
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: other)
+    monkeypatch.setattr(L, "group_experts", launched)
+    monkeypatch.setattr(L, "pack_scales", launched)
+    assert torch.equal(group_experts_from_offsets(offs, 600), experts)
+    assert torch.equal(E.pack_plain_scales(scales, 96, False, 32), packed)
