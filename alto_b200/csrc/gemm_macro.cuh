@@ -33,7 +33,7 @@
 // and 128 x 128 x 128 block whose MMAs take 128 cycles.  HN = 64: the latency of a stage's barriers and of the fold
 // (650 cycles a chunk of 128 x 128 with a CTA to itself), and where the whole chip works the shared-memory port,
 // whose 17 KB of loads per block, against 13, took 284 cycles alone.
-// Measured at 8192 x 4096 x 14336, one factor per tile of B / one per column: 449 / 564 us (HN = 128);
+// Measured at 8192 x 4096 x 14336, one factor per tile of B / one per column: 451 / 571 us (HN = 128);
 // with 128 x 128 tiles, sixteen fold warps of 32 columns that each looked up their factors, and one issuer:
 // 572 / 924 us.  (Pieces of 32 columns: a few spilled registers more in the chunk loop of the per-column variant,
 // local memory that this kernel's small L1 does not hold: + 10 %.)
@@ -54,7 +54,7 @@ struct MacroSide {
 // Quotients of tile numbers by a divisor fixed per launch: t / d = t * m >> s for t < 2^31, with
 // s = 31 + ceil(log2 d) and m = floor(2^s / d) + 1.  A tile's coordinates are on the critical path of every role;
 // with three 64-bit divides a weight gradient of 128 rows per expert (one chunk per tile) took 26 % longer
-// (8 experts, 2880 x 2880: 64.5 us, now 51.3).
+// (8 experts, 2880 x 2880: 64.5 us, now 51.4).
 struct TileDiv {
   uint32_t d, m;
   int s;
