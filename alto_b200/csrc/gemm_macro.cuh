@@ -12,33 +12,31 @@
 // This replaces the reference's emulation of the recipe, dequantise -> descale -> bf16 matmul
 // (alto/kernels/fp4/mxfp4/mxfp_linear.py:337-356, mxfp_grouped_gemm/cg_backward.py:668-690).
 //
-// One CTA (512 threads = four warpgroups, persistent over 128 x 2 HN output tiles, each two halves of HN = 128
-// or 64 columns that share the A operand; `macro_half` in gemm_sm100.cu chooses):
-//   warpgroup 0   warp 0: producer - per stage (128 bytes of K = two chunks) three tiled TMA loads and the
-//                 bulk copies of the stage's scale tiles; warps 1 and 3: MMA issuers of the two halves - two
-//                 tcgen05.mma per chunk into one of the chunk accumulators in tensor memory (HN = 128: three for
-//                 both halves; 64: three for each), then a commit to that accumulator's "full" barrier; warp 2 idle;
+// One CTA (512 threads = four warpgroups, persistent over tiles of 128 x BN, BN = 128 or 192; `macro_tile_n` in
+// gemm_sm100.cu chooses):
+//   warpgroup 0   warp 0: producer - per stage (128 bytes of K = two chunks) two tiled TMA loads and the bulk copies
+//                 of the stage's scale tiles; warps 1 and 3: MMA issuers of alternate chunks - two tcgen05.mma into
+//                 one of the three (BN = 192: two) chunk accumulators in tensor memory, then a commit to that
+//                 accumulator's "full" barrier; warp 2: waits for these and releases the fold warps;
 //   warpgroup 1   scale transfer shared memory -> tensor memory (as in the plain kernel), and the macro
-//                 factors: the codes of the tile's rows (and columns) for the next stage's two chunks are read
-//                 a stage ahead and their reciprocals left in a shared-memory ring;
-//   warpgroups 2-3  fold + epilogue of one half each: four warps, one per tensor-memory lane quarter, 32 rows
-//                 x HN columns in HN registers per thread.  A chunk is read in pieces of 16 columns; HN = 128: one
-//                 piece is always on its way from tensor memory while another is folded; 64: the registers hold
-//                 the whole chunk, and each piece is requested for the next chunk as soon as it is folded.
-//                 acc += P * (1/fa[row]) * (1/fb[col]) in packed fp32x2 arithmetic.  After the last chunk the
-//                 registers are scaled, converted, staged and TMA-stored.
+//                 factors: their codes are read three stages ahead and the reciprocals left in a shared-memory ring;
+//   warpgroups 2-3  fold + epilogue: per tensor-memory lane quarter two warps of 32 rows x BN / 2 columns, the sums in
+//                 registers.  A warp reads its part of the chunk into registers, 64 columns at a time, gives the
+//                 accumulator back and then does acc += P * (1/fa[row]) * (1/fb[col]) in packed fp32x2 arithmetic.
+//                 After the last chunk the registers are scaled, converted, staged and TMA-stored.
 //
-// What bounds it: HN = 128: the hand-over of the chunk accumulators between the MMAs and the fold (three fit beside
-// the scales), then the fold itself, 64 (128 with per-column factors) packed operations of two cycles per scheduler
-// and 128 x 128 x 128 block whose MMAs take 128 cycles.  HN = 64: the latency of a stage's barriers and of the fold
-// (650 cycles a chunk of 128 x 128 with a CTA to itself), and where the whole chip works the shared-memory port,
-// whose 17 KB of loads per block, against 13, took 284 cycles alone.
-// Measured at 8192 x 4096 x 14336, one factor per tile of B / one per column: 451 / 571 us (HN = 128);
-// with 128 x 128 tiles, sixteen fold warps of 32 columns that each looked up their factors, and one issuer:
-// 572 / 924 us.  (Pieces of 32 columns: a few spilled registers more in the chunk loop of the per-column variant,
-// local memory that this kernel's small L1 does not hold: + 10 %.)
-// The warpgroups re-divide the register file with setmaxnreg (512 threads x 128 at launch -> 56 for the
-// small roles, 200 for the fold warps; the two must balance exactly, see CfgMacro).
+// What bounds it: the way of a chunk accumulator around the roles (MMA 128 or 192 cycles of 440 with issue and commit,
+// wait warp, read, fold, issuer; about 1300 cycles over the accumulators that fit in tensor memory).  Nothing is
+// saturated: the MMAs of a block of 128 x 128 x 128 take 128 cycles, its loads 200 to 256 at 64 bytes a cycle, reading
+// it out of tensor memory 75, its multiply-adds 140, and with one B factor per tile it takes 420.  So what counts
+// is latency: few instructions and fewer branches in the loops (a taken branch costs 25 to 40 cycles among so much
+// different code), waits of a few instructions, and issue slots left free by the fold.
+// Measured at 8192 x 4096 x 14336, one factor per tile of B / one per column: 349 / 519 us.  Before: 451 / 612 us with
+// 128 x 256 tiles of two halves, chunks read in the 16 x 256-bit layout (three times the time of the present ones)
+// in pieces of 16 columns, inlined bounded waits in every loop.  On the way, one factor per tile: the new layouts alone
+// 411, 128 x 128 tiles 410, waits as small loops and the fold released at named barriers 377, packed arithmetic 362.
+// One issuer behind a wait warp 420, two register sets for the chunks 593 (spills), one issuer that waits itself 480.
+// The warpgroups re-divide the register file with setmaxnreg (512 threads x 128 at launch, see CfgMacro).
 // Rows grouped by expert (`group_expert`) and K ranges per batch entry (`k_offs`) work as in the
 // plain kernel; every K range starts on a multiple of 128 elements, so chunks never straddle one.
 #pragma once
@@ -78,45 +76,45 @@ struct MacroGemmArgs {
 
 constexpr int NUM_THREADS_MACRO = 512;
 
-// HN: columns of a half.  128: the halves share three accumulators; 64: each half has three of its own.
-template <int HN_>
+// BN: columns of a tile.
+template <int BN_>
 struct CfgMacro {
-  static constexpr int HN = HN_;                                // columns of a half (one chunk accumulator)
-  static_assert(HN == 128 || HN == 64, "halves");
-  static constexpr int BN = 2 * HN;
+  static constexpr int BN = BN_;
+  static_assert(BN == 192 || BN == 128, "tile widths");
   static constexpr int SF_TILES = Kind<KIND_MXF4>::SF_TILES;
   static constexpr int A_BYTES = BM * STAGE_K_BYTES;
-  static constexpr int B_BYTES = HN * STAGE_K_BYTES;            // per half
+  static constexpr int B_BYTES = BN * STAGE_K_BYTES;
   static constexpr int SF_BYTES = SF_TILES * 512;               // per 128 rows of either operand
-  static constexpr int SFB_BLOCKS = BN / 128;                   // 128-row blocks of B's scales under a tile
-  static constexpr int SF_OFF = A_BYTES + 2 * B_BYTES;          // scales of A, then of B's blocks
+  static constexpr int SFB_BLOCKS = BN == 192 ? 2 : 1;          // 128-row blocks of B's scales under a tile
+  static constexpr int SF_OFF = A_BYTES + B_BYTES;              // scales of A, then of B's blocks
   static constexpr int STAGE_BYTES = SF_OFF + (1 + SFB_BLOCKS) * SF_BYTES;
   static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 128-byte swizzle atom aligned");
   static constexpr int SF_COLS = SF_TILES * 4;                  // tensor-memory columns of SF_BYTES
   static constexpr int STAGE_SF_COLS = (1 + SFB_BLOCKS) * SF_COLS;
-  static constexpr int STAGES = HN == 128 ? 3 : 4;
-  static constexpr int RING = 3;                                // chunk barriers per half, each way
-  static constexpr bool OWN_BUFS = HN == 64;
-  static constexpr int P_BUFS = OWN_BUFS ? 2 * RING : 3;        // chunk accumulators in tensor memory
-  static constexpr int PIECES = HN / 16;
-  static constexpr int FOLD_WARPS = 8;                          // four per half
-  static constexpr int EPI_UNIT = 2048;                         // 16 rows x 128 bytes
-  static constexpr int EPI_WARP_BYTES = 2 * EPI_UNIT;
+  static constexpr int STAGES = BN == 192 ? 4 : 5;
+  static constexpr int P_BUFS = BN == 192 ? 2 : 3;              // chunk accumulators in tensor memory
+  static constexpr int FOLD_WARPS = 8;                          // two per tensor-memory lane quarter
+  static constexpr int WN = BN / 2;                             // columns of a fold warp
+  static constexpr int PIECES = WN / 16;
+  static constexpr int FLIGHT = 4;                              // pieces in registers at a time
+  static constexpr int EPI_WARP_BYTES = 4096;                   // 32 rows x 32 columns: two units of bf16, one of fp32
   static constexpr int EPI_BYTES = FOLD_WARPS * EPI_WARP_BYTES;
   // Ring of reciprocal factors, per chunk 128 rows and BN columns (B_UNIFORM: the products of both, 128 rows per
   // 128 columns).  No barrier guards its reuse: a slot is rewritten FAC_STAGES stages after its last use, once
-  // that stage's operands have landed, so the MMAs of the stage STAGES earlier are done, and with them (see
-  // the issuers) both halves have read out every chunk up to two before (three with accumulators of their own) -
-  // at least one after the slot's own, which has therefore been folded.
+  // that stage's operands have landed, so the MMAs of the stage STAGES earlier are done, and with them every chunk
+  // up to P_BUFS before has been read out, in order - all but the latest of these have therefore been folded.
   static constexpr int FAC_STAGES = 8;
-  static constexpr int FAC_STRIDE = BM + BN + 4;                // floats per chunk; + 4 spreads the banks
+  static constexpr int FAC_STRIDE = BM + (BN == 192 ? 192 : 128) + 4;   // floats per chunk; + 4 spreads the banks
+  static_assert(FAC_STRIDE >= SFB_BLOCKS * BM && FAC_STRIDE >= BM + BN, "factors of a chunk");
   static constexpr int FAC_BYTES = 2 * FAC_STAGES * FAC_STRIDE * 4;
-  static_assert(FAC_STAGES >= STAGES + (OWN_BUFS ? 4 : 3), "factors are overwritten while they are in use");
+  static_assert(FAC_STAGES >= STAGES + 1 + (P_BUFS + 1) / 2, "factors are overwritten while they are in use");
   static constexpr int RCP_BYTES = 256 * 4;                     // 1 / factor for every code
-  static constexpr int TMEM_SF_BASE = P_BUFS * HN;
+  static constexpr int TMEM_SF_BASE = P_BUFS * BN;
   static constexpr int TMEM_COLS_USED = TMEM_SF_BASE + STAGES * STAGE_SF_COLS;
   static_assert(TMEM_COLS_USED <= 512, "tensor memory budget");
-  static constexpr int NUM_BARS = 3 * STAGES + 4 * RING;
+  // named barrier that hands chunk accumulator `buf` to a group of four fold warps
+  __device__ static constexpr int chunk_barrier(int group, int buf) { return 1 + 2 * buf + group; }
+  static constexpr int NUM_BARS = 3 * STAGES + 2 * P_BUFS;
   static constexpr int SMEM_BYTES =
       STAGES * STAGE_BYTES + EPI_BYTES + FAC_BYTES + RCP_BYTES + 1024 /*align*/ + 512 /*barriers*/;
   static_assert(NUM_BARS * 8 + 16 <= 512, "barrier area");
@@ -125,7 +123,7 @@ struct CfgMacro {
   // registers per thread (65536 / 512); setmaxnreg.inc can only take what setmaxnreg.dec has released
   // INSIDE the CTA and blocks for ever otherwise, so the two must balance exactly.
   static constexpr int REGS_LAUNCH = 128;
-  static constexpr int REGS_SMALL = 56, REGS_FOLD = 200;
+  static constexpr int REGS_SMALL = BN == 192 ? 72 : 96, REGS_FOLD = 256 - REGS_SMALL;
   static_assert(2 * 128 * REGS_SMALL + 2 * 128 * REGS_FOLD == NUM_THREADS_MACRO * REGS_LAUNCH,
                 "setmaxnreg budget must balance");
   static_assert(NUM_THREADS_MACRO == (8 + FOLD_WARPS) * 32, "role layout");
@@ -138,7 +136,6 @@ struct MacroTile {
   int64_t chunk0;
   int n_chunks;
   int expert;
-  int halves;       // 1 when the tile's second half lies outside the matrix
 };
 
 // (the raster of decode_tile: groups of `group_m` row tiles, each swept across all column tiles, row tile fastest)
@@ -189,93 +186,177 @@ __device__ __forceinline__ MacroTile decode_macro_tile(const MacroGemmArgs& marg
   const int64_t tail = bytes - (int64_t)(t.k_stages - 1) * STAGE_K_BYTES;
   t.last_mmas = (int)((tail + 31) / 32);
   m.n_chunks = bytes > 0 ? (int)((bytes + 63) / 64) : 0;
-  m.halves = args.N - t.nb * C::BN > C::HN ? 2 : 1;
   return m;
 }
 
-// One piece of a chunk accumulator: 16 columns of a warp's 32 rows, as two tensor-memory loads of 16 rows in
-// the 16 x 256-bit layout.  A lane gets, per group of eight columns, columns 2 (lane % 4) and + 1 of rows
-// lane / 4 and + 8 of each load: four rows and four columns of the piece, so that it needs eight factors,
-// where the layout of one row per lane needs 17 and the broadcast of the column factors out of shared memory
-// (128 bytes per register and warp) took longer than the multiply-adds.
+// One piece of a chunk accumulator: 16 columns of a warp's 32 rows.
+// One B factor per chunk: one row per lane (32 x 32-bit layout), so that a chunk needs one factor a lane.
+// Per-column factors: two loads of 16 rows in the 16 x 128-bit layout, where a lane gets columns lane % 4 + 4 g of
+// rows lane / 4 and + 8 of each load: four rows and four columns, eight factors, where a row per lane needs 17, and
+// the broadcast of the column factors out of shared memory (128 bytes per register and warp) took 550 cycles.
+// Reading a block of 128 x 128 takes 75 cycles in the 32 x 32-bit layout, 131 in the 16 x 128-bit one and 257 in the
+// 16 x 256-bit one (all warps reading, nothing else running).
 struct Piece {
-  uint32_t r[16];   // [row half 2][column group 2][row 2][column 2]
+  uint32_t r[16];   // [column 16], or [row half 2][column group 4][row 2]
 };
+template <bool B_UNIFORM>
 __device__ __forceinline__ void tc_ld_piece(uint32_t taddr, Piece& p) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t* r = p.r + 8 * h;
+  if constexpr (B_UNIFORM) {
+    uint32_t* r = p.r;
     asm volatile(
-        "tcgen05.ld.sync.aligned.16x256b.x2.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-        : "r"(taddr + ((uint32_t)(16 * h) << 16))
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
         : "memory");
+  } else {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t* r = p.r + 8 * h;
+      asm volatile(
+          "tcgen05.ld.sync.aligned.16x128b.x4.b32 "
+          "{%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+          : "r"(taddr + ((uint32_t)(16 * h) << 16))
+          : "memory");
+    }
   }
 }
-// tcgen05.wait::ld that the values in p depend on: nothing that uses them can move above it
-__device__ __forceinline__ void tc_wait_piece(Piece& p) {
+// The values in p have landed (tcgen05.wait::ld came before): nothing that uses them can move above this.
+__device__ __forceinline__ void tc_landed_piece(Piece& p) {
 #define ALTOB200_RW8(o) "+r"(p.r[o]), "+r"(p.r[o + 1]), "+r"(p.r[o + 2]), "+r"(p.r[o + 3]), "+r"(p.r[o + 4]), \
                         "+r"(p.r[o + 5]), "+r"(p.r[o + 6]), "+r"(p.r[o + 7])
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : ALTOB200_RW8(0), ALTOB200_RW8(8)
-               :
-               : "memory");
-}
-// the same for a piece whose load an earlier wait has covered
-__device__ __forceinline__ void tc_landed_piece(Piece& p) { asm volatile("" : ALTOB200_RW8(0), ALTOB200_RW8(8)); }
+  asm volatile("" : ALTOB200_RW8(0), ALTOB200_RW8(8));
 #undef ALTOB200_RW8
+}
+__device__ __forceinline__ void st_shared_u16(uint32_t addr, unsigned short v) {
+  asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
+}
 __device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ float2 ld_shared_f32x2(uint32_t addr) {
-  float2 v;
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+__device__ __forceinline__ float4 ld_shared_f32x4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ uint64_t* generic_bar(uint32_t addr) {
-  return reinterpret_cast<uint64_t*>(__cvta_shared_to_generic(addr));
-}
-
-// One look at a barrier's phase, without waiting.
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+// Bounded waits as one small loop each.  Two dozen warps' worth of different code share the instruction caches of an
+// SM, where every taken branch costs 30 to 40 cycles: a wait that is spread over inlined slow paths (mbar_wait) took
+// 200 cycles and more on a barrier that was already complete, and with it a chunk's way around the roles 1300.
+// Counted on the SM's cycle counter, as in mbar_wait; false when the limit has passed or another role has given up.
+#define ALTOB200_WAIT_LOOP(LOOK_AT)                                                                           \
+  "{\n\t.reg .pred p, q, r;\n\t.reg .u32 f, n;\n\t.reg .u64 t, t0;\n\t" LOOK_AT                                 \
+  "@p bra DONE;\n\t"                                                                                         \
+  "mov.u64 t0, %clock64;\n"                                                                                  \
+  "AGAIN:\n\t"                                                                                               \
+  "mov.u32 n, 64;\n"                                                                                         \
+  "LOOK:\n\t" LOOK_AT                                                                                        \
+  "@p bra DONE;\n\t"                                                                                         \
+  "sub.u32 n, n, 1;\n\t"                                                                                     \
+  "setp.ne.u32 q, n, 0;\n\t"                                                                                 \
+  "@q bra LOOK;\n\t"                                                                                         \
+  "ld.volatile.shared.u32 f, [%2];\n\t"                                                                      \
+  "mov.u64 t, %clock64;\n\t"                                                                                 \
+  "sub.u64 t, t, t0;\n\t"                                                                                    \
+  "setp.ne.u32 q, f, 0;\n\t"                                                                                 \
+  "setp.gt.or.u64 q, t, %1, q;\n\t"                                                                          \
+  "@!q bra AGAIN;\n"                                                                                         \
+  "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+__device__ __forceinline__ bool mbar_wait_tight(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint64_t limit_cycles) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  asm volatile(ALTOB200_WAIT_LOOP("mbarrier.try_wait.parity.shared::cta.b64 p, [%3], %4;\n\t")
+               : "=r"(ok)
+               : "l"(limit_cycles), "r"(abort_addr), "r"(bar), "r"(parity)
+               : "memory");
   return ok != 0;
 }
-
-// acc += P * ra[row] * fb[col]; B_UNIFORM: one B factor for the half and chunk, already multiplied into ra.
-// `acc` and `p` are laid out alike; fb: shared-memory address of this lane's first column factor.
+// Three barriers at once (the first two at the same parity): their answers take as long as one.
+__device__ __forceinline__ bool mbar_wait3_tight(uint32_t b0, uint32_t b1, uint32_t parity01, uint32_t b2, uint32_t parity2,
+                                                 uint32_t abort_addr, uint64_t limit_cycles) {
+  uint32_t ok;
+  asm volatile(ALTOB200_WAIT_LOOP("mbarrier.test_wait.parity.shared::cta.b64 p, [%3], %5;\n\t"
+                                  "mbarrier.test_wait.parity.shared::cta.b64 q, [%4], %5;\n\t"
+                                  "mbarrier.test_wait.parity.shared::cta.b64 r, [%6], %7;\n\t"
+                                  "and.pred p, p, q;\n\tand.pred p, p, r;\n\t")
+               : "=r"(ok)
+               : "l"(limit_cycles), "r"(abort_addr), "r"(b0), "r"(b1), "r"(parity01), "r"(b2), "r"(parity2)
+               : "memory");
+  return ok != 0;
+}
+#undef ALTOB200_WAIT_LOOP
+// A role that gave up: the others learn of it, the first one's place is kept.
+__device__ __forceinline__ void report_timeout(volatile int* abort_flag, int site) {
+  if (*abort_flag != 0) return;
+  *abort_flag = 1;
+  if (atomicCAS(&g_status[0], 0, ALTOB200_ETIMEOUT_DEVICE) == 0) {
+    g_status[1] = 1;
+    g_status[2] = (int)blockIdx.x;
+    g_status[3] = site;
+  }
+}
+// An arrival by one lane, without a branch.
+__device__ __forceinline__ void mbar_arrive_lane0(uint32_t bar, int lane) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
+      ::"r"(bar), "r"(lane)
+      : "memory");
+}
+__device__ __forceinline__ void named_barrier_sync(int id, int count) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void named_barrier_arrive(int id, int count) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+// tcgen05 instructions of one lane, without a branch around them
+__device__ __forceinline__ void tc_mma_mxf4_if(bool pred, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                               uint32_t accumulate, uint32_t sfa, uint32_t sfb) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb), "r"((uint32_t)pred)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_if(bool pred, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+      ::"r"(bar), "r"((uint32_t)pred)
+      : "memory");
+}
+// acc += P * ra[row] * fb[col]; B_UNIFORM: one B factor for the columns and chunk, already multiplied into ra[0].
+// `acc` and `p` are laid out alike; fb: shared-memory address of this lane's first column factor.  Packed arithmetic
+// takes as long as scalar but half the issue slots: beside scalar multiply-adds on every scheduler the warp that
+// issues the MMAs took 1380 cycles for a pair and the wait for it, beside packed ones 550 (alone 490).
 template <bool B_UNIFORM>
-__device__ __forceinline__ void fold_piece(float2* acc, const Piece& p, const float (&ra)[4], uint32_t fb) {
+__device__ __forceinline__ void fold_piece(float2* acc, const Piece& p, const float2 (&ra)[B_UNIFORM ? 1 : 2], uint32_t fb) {
+  if constexpr (B_UNIFORM) {
 #pragma unroll
-  for (int g = 0; g < 2; ++g) {
-    float2 f = make_float2(1.0f, 1.0f);
-    if (!B_UNIFORM) f = ld_shared_f32x2(fb + 32 * g);
+    for (int i = 0; i < 8; ++i)
+      acc[i] = __ffma2_rn(make_float2(u2f(p.r[2 * i]), u2f(p.r[2 * i + 1])), ra[0], acc[i]);
+  } else {
+    const float4 f4 = ld_shared_f32x4(fb);
+    const float f[4] = {f4.x, f4.y, f4.z, f4.w};
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {   // row half q / 2, row 8 (q % 2)
-      const int i = (q >> 1) * 4 + g * 2 + (q & 1);
-      float2 w = make_float2(ra[q], ra[q]);
-      if (!B_UNIFORM) w = __fmul2_rn(w, f);
-      acc[i] = __ffma2_rn(make_float2(u2f(p.r[2 * i]), u2f(p.r[2 * i + 1])), w, acc[i]);
-    }
+    for (int g = 0; g < 4; ++g)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {     // rows 16 h and 16 h + 8 of the lane's
+        const int i = h * 4 + g;
+        const float2 w = __fmul2_rn(ra[h], make_float2(f[g], f[g]));
+        acc[i] = __ffma2_rn(make_float2(u2f(p.r[2 * i]), u2f(p.r[2 * i + 1])), w, acc[i]);
+      }
   }
 }
 
-// B_UNIFORM: B's macro blocks are 128 x 128 tiles (one factor per half and chunk), else per column.
-template <int HN, bool B_UNIFORM>
+// B_UNIFORM: B's macro blocks are 128 x 128 tiles (one factor per 128 columns and chunk), else per column.
+template <int BN, bool B_UNIFORM>
 __global__ void __launch_bounds__(NUM_THREADS_MACRO, 1)
 gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_d, const MacroGemmArgs margs) {
-  using C = CfgMacro<HN>;
+  using C = CfgMacro<BN>;
   const GemmArgs& args = margs.g;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -286,10 +367,11 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + C::STAGES;
   uint64_t* sf_full = bars + 2 * C::STAGES;
-  uint64_t* p_full = bars + 3 * C::STAGES;        // [half][chunk % RING]
-  uint64_t* p_empty = p_full + 2 * C::RING;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_empty + 2 * C::RING);
+  uint64_t* p_full = bars + 3 * C::STAGES;        // [chunk % P_BUFS]
+  uint64_t* p_empty = p_full + C::P_BUFS;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_empty + C::P_BUFS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* never = abort_flag + 1;           // an abort flag that nothing raises
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (an output of 2^31 tiles would not fit any memory)
@@ -302,11 +384,12 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       mbar_init(&empty_bar[s], 2);
       mbar_init(&sf_full[s], 4);
     }
-    for (int p = 0; p < 2 * C::RING; ++p) {
+    for (int p = 0; p < C::P_BUFS; ++p) {
       mbar_init(&p_full[p], 1);
-      mbar_init(&p_empty[p], C::FOLD_WARPS / 2);
+      mbar_init(&p_empty[p], C::FOLD_WARPS);
     }
     *abort_flag = 0;
+    *never = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // scale staging starts from zero: a ragged last stage never feeds uninitialised scale bytes
@@ -326,6 +409,8 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
+  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see mbar_wait
   grid_dependency_wait();   // set-up done; global memory from here on (programmatic dependent launch)
 
   if (warp < 4) {
@@ -339,17 +424,18 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     if (warp == 0) {
       // ------------------------------ producer ------------------------------
       const bool elected = elect_one();
-      uint32_t it = 0;
+      const int n_row_blocks = (int)((args.N + 127) >> 7);
+      uint32_t s = 0, phase = 1;
       bool alive = true;
       for (int tile = (int)blockIdx.x; tile < n_tiles && alive; tile += (int)gridDim.x) {
         const MacroTile mt = decode_macro_tile<C>(margs, (uint32_t)tile, k_stages);
         const TileInfo& ti = mt.t;
         if (ti.skip) continue;
-        const int64_t mb = ti.mb, nb = ti.nb;
-        for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
-          const int s = it % C::STAGES;
-          alive = __all_sync(0xFFFFFFFFu,
-                             mbar_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1, abort_flag, 21, args.wait_ns));
+        const int64_t mb = ti.mb;
+        const int sfb_blk0 = (int)((ti.nb * BN) >> 7);       // first 128-row block of B's scales under this tile
+        const uint32_t n_sfb = (uint32_t)(n_row_blocks - sfb_blk0 < C::SFB_BLOCKS ? n_row_blocks - sfb_blk0 : C::SFB_BLOCKS);
+        for (int ks = 0; ks < ti.k_stages; ++ks) {
+          alive = __all_sync(0xFFFFFFFFu, mbar_wait_tight(smem_u32(&empty_bar[s]), phase, abort_addr, limit));
           if (!alive) break;
           uint8_t* st = smem + s * C::STAGE_BYTES;
           const int64_t cb0 = ti.sf_tile0 + (int64_t)ks * C::SF_TILES;
@@ -358,90 +444,107 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t sf_bytes = (uint32_t)sf_tiles * 512u;
           const int32_t kx = (int32_t)(ti.k_byte0 + (int64_t)ks * STAGE_K_BYTES);
           if (elected) {
-            const uint32_t n_b = (uint32_t)mt.halves, n_sfb = C::SFB_BLOCKS == 2 ? n_b : 1u;
-            mbar_expect_tx(&full_bar[s], C::A_BYTES + n_b * C::B_BYTES + (1u + n_sfb) * sf_bytes);
+            mbar_expect_tx(&full_bar[s], C::A_BYTES + C::B_BYTES + (1u + n_sfb) * sf_bytes);
             tma_load_2d(st, &tmap_a, kx, (int32_t)(mb * BM), &full_bar[s]);
+            tma_load_2d(st + C::A_BYTES, &tmap_b, kx, (int32_t)ti.b_row0, &full_bar[s]);
             bulk_load(st + C::SF_OFF, args.sfa + (mb * args.nct + cb0) * 512, sf_bytes, &full_bar[s]);
 #pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-              if (h < n_b)
-                tma_load_2d(st + C::A_BYTES + h * C::B_BYTES, &tmap_b, kx, (int32_t)(ti.b_row0 + h * HN), &full_bar[s]);
+            for (uint32_t h = 0; h < C::SFB_BLOCKS; ++h)
               if (h < n_sfb)
-                bulk_load(st + C::SF_OFF + (1 + h) * C::SF_BYTES, ti.sfb + ((nb * C::SFB_BLOCKS + h) * args.nct + cb0) * 512,
+                bulk_load(st + C::SF_OFF + (1 + h) * C::SF_BYTES, ti.sfb + ((int64_t)(sfb_blk0 + h) * args.nct + cb0) * 512,
                           sf_bytes, &full_bar[s]);
-            }
+          }
+          if (++s == C::STAGES) {
+            s = 0;
+            phase ^= 1u;
           }
         }
       }
+      if (!alive) report_timeout(abort_flag, 21);
     } else if (warp == 1 || warp == 3) {
       // ------------------------------ MMA issuers ------------------------------
-      // One per half: a tcgen05.mma does not run ahead of its thread's other instructions, so while one
-      // issuer waits for its barriers (~150 cycles even when they are complete) the other one's MMAs keep the
-      // tensor pipe busy.
-      // Chunk n of half h goes to accumulator (2 n + h) % 3, which held chunk n - 2 of half 1 (h = 0) or
-      // chunk n - 1 of half 0 (h = 1); with accumulators of their own to 2 (n % 3) + h, which held chunk n - 3 of
-      // the same half.  The barriers count the chunks of one half, so that whoever waits on one has waited for
-      // all its earlier phases.  A half outside the matrix runs the protocol without MMAs.
-      static_assert(C::RING == 3 && (C::OWN_BUFS ? C::P_BUFS == 6 : C::P_BUFS == 3), "order of the accumulators");
+      // Two, for alternate chunks: while one waits for its barriers the other one's MMAs keep the tensor pipe busy.
+      // Chunk m goes to accumulator m % P_BUFS, which held chunk m - P_BUFS.  Its issuer cannot mistake the phase
+      // before for the one it waits for: it has waited until chunk m - 2 - P_BUFS was drained, and chunks are drained
+      // in order, so that m - 2 P_BUFS was too (P_BUFS >= 2).
+      // A branch costs about 25 cycles here and a stage has 400, so the loop's only one is on the vote; the issuing
+      // lane's instructions are predicated.
       const bool elected = elect_one();
-      const int h = warp >> 1;
-      uint32_t it = 0, n = 0;         // stages and chunks so far
+      const uint32_t i = (uint32_t)(warp >> 1);
+      uint32_t s = 0, st_phase = 0, odd = 0;      // odd: chunks so far, modulo 2
+      uint32_t buf = i, drained = 1;              // this issuer's next accumulator and the phase it waits for
       bool alive = true;
       const uint32_t smem_base = smem_u32(smem);
-      uint64_t* const my_full = p_full + h * C::RING;
-      uint64_t* const drained = p_empty + (C::OWN_BUFS ? h : h ^ 1) * C::RING;
-      const uint32_t back = C::OWN_BUFS ? 3u : h == 0 ? 2u : 1u;
+      const uint32_t bar_full = smem_u32(full_bar), bar_sf = smem_u32(sf_full), bar_acc = smem_u32(p_empty);
       for (int tile = (int)blockIdx.x; tile < n_tiles && alive; tile += (int)gridDim.x) {
         const MacroTile mt = decode_macro_tile<C>(margs, (uint32_t)tile, k_stages);
         const TileInfo& ti = mt.t;
         if (ti.skip) continue;
-        const bool mine = h < mt.halves;
-        for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
+        // scale columns of B start at word 0 of the first block, or 64 rows (2 words) into it
+        const uint32_t sfb_off = C::SFB_BLOCKS == 2 ? (uint32_t)((ti.nb * BN) & 127) >> 5 : 0u;
+        for (int ks = 0; ks < ti.k_stages; ++ks) {
           const int n_mma = (ks == ti.k_stages - 1) ? ti.last_mmas : 4;
-          const int s = it % C::STAGES;
-          const uint32_t sfa_t = tmem_base + C::TMEM_SF_BASE + s * C::STAGE_SF_COLS;
-          // (a block of 128 rows is four columns per 128 bytes of K, 32 rows each: row 64 is two columns on)
-          const uint32_t sfb_t = sfa_t + C::SF_COLS + (HN == 128 ? h * C::SF_COLS : 2 * h);
-          const uint32_t a_lo = ((smem_base + (uint32_t)s * C::STAGE_BYTES) >> 4) | 0x10000u;
-          const uint32_t b_lo = a_lo + ((C::A_BYTES + h * C::B_BYTES) >> 4);
-          // operands and scales of the stage are in place; the three barriers are looked at together, since the
-          // answer of one takes as long as that of all
-          const uint32_t st_phase = (it / C::STAGES) & 1, m0 = n - back;
-          const bool s0 = mbar_test(smem_u32(&sf_full[s]), st_phase), s1 = mbar_test(smem_u32(&full_bar[s]), st_phase);
-          const bool s2 = n < back || mbar_test(smem_u32(&drained[m0 % C::RING]), (m0 / C::RING) & 1);
-          const uint32_t m1 = n + 1 - back;
-          const bool s3 = n + 1 < back || mbar_test(smem_u32(&drained[m1 % C::RING]), (m1 / C::RING) & 1);
-          bool ok = s0 || mbar_wait(&sf_full[s], st_phase, abort_flag, 25, args.wait_ns);
-          ok = ok && (s1 || mbar_wait(&full_bar[s], st_phase, abort_flag, 23, args.wait_ns));
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            if (2 * c >= n_mma) break;
-            // the chunk's accumulator is drained
-            if (n >= back && !(c == 0 ? s2 : s3)) {
-              const uint32_t m = n - back;
-              ok = ok && mbar_wait(&drained[m % C::RING], (m / C::RING) & 1, abort_flag, 22, args.wait_ns);
-            }
-            alive = __all_sync(0xFFFFFFFFu, ok);
-            if (!alive) break;
-            tc_fence_after();
-            if (elected) {
-              if (mine) {
-                const uint32_t acc_t = tmem_base + (C::OWN_BUFS ? 2 * (n % C::RING) + (uint32_t)h : (2 * n + (uint32_t)h) % 3u) * HN;
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                  if (2 * c + j < n_mma)
-                    tc_mma<KIND_MXF4>(acc_t, desc_of(DESC_SW128_HI, a_lo + 4 * c + 2 * j),
-                                      desc_of(DESC_SW128_HI, b_lo + 4 * c + 2 * j), args.idesc[j], (uint32_t)j,
-                                      sfa_t + c * 4, sfb_t + c * 4);
-                }
-              }
-              tc_commit(&my_full[n % C::RING]);
-            }
-            ++n;
-          }
+          const int c = (int)(odd ^ i);           // this issuer's chunk of the stage
+          const bool mine = 2 * c < n_mma;
+          // operands and scales of the stage are in place, the accumulator is drained
+          const uint32_t b0 = bar_sf + 8 * s, b1 = bar_full + 8 * s;
+          const uint32_t b2 = mine ? bar_acc + 8 * buf : b1, p2 = mine ? drained : st_phase;
+          alive = __all_sync(0xFFFFFFFFu, mbar_wait3_tight(b0, b1, st_phase, b2, p2, abort_addr, limit));
           if (!alive) break;
-          if (elected) tc_commit(&empty_bar[s]);   // both issuers
-          __syncwarp();
+          tc_fence_after();
+          const uint32_t sfa_t = tmem_base + C::TMEM_SF_BASE + s * C::STAGE_SF_COLS + c * 4;
+          const uint32_t sfb_t = tmem_base + C::TMEM_SF_BASE + s * C::STAGE_SF_COLS + C::SF_COLS + c * 4 * C::SFB_BLOCKS + sfb_off;
+          const uint32_t a_lo = (((smem_base + s * C::STAGE_BYTES) >> 4) | 0x10000u) + 4 * c;
+          const uint32_t b_lo = a_lo + (C::A_BYTES >> 4);
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            tc_mma_mxf4_if(elected && 2 * c + j < n_mma, tmem_base + buf * BN, desc_of(DESC_SW128_HI, a_lo + 2 * j),
+                           desc_of(DESC_SW128_HI, b_lo + 2 * j), args.idesc[j], (uint32_t)j, sfa_t, sfb_t);
+          tc_commit_if(elected && mine, smem_u32(p_full) + 8 * buf);
+          tc_commit_if(elected, smem_u32(empty_bar) + 8 * s);      // both issuers
+          if (mine) {                             // two chunks on
+            if (C::P_BUFS == 2 || buf != 0) drained ^= 1u;
+            if (C::P_BUFS == 3) buf = buf == 0 ? 2u : buf - 1;
+          }
+          odd ^= n_mma <= 2 ? 1u : 0u;
+          if (++s == C::STAGES) {
+            s = 0;
+            st_phase ^= 1u;
+          }
+        }
+      }
+      if (!alive) report_timeout(abort_flag, 22);
+    } else {
+      // ------------------------------ wait warp of the fold ------------------------------
+      // It waits for the finished chunks and releases the two groups of fold warps, each at its own named barrier of
+      // the accumulator: 20 cycles a chunk for a fold warp, where a look at an mbarrier and the branch on its answer
+      // took 75 of 260.  A barrier cannot be met twice ahead of the fold: the accumulator's next chunk is finished only
+      // after all fold warps have given it back.  After a failure the chunks left are handed over one by one without
+      // waiting for them, so that the fold warps come to their end (they store nothing then).
+      uint32_t buf = 0, phase = 0;
+      bool alive = true;
+      for (int tile = (int)blockIdx.x; tile < n_tiles; tile += (int)gridDim.x) {
+        const MacroTile mt = decode_macro_tile<C>(margs, (uint32_t)tile, k_stages);
+        int left = mt.t.skip ? 0 : mt.n_chunks;
+        for (; left > 0; --left) {
+          if (alive) {
+            alive = __all_sync(0xFFFFFFFFu, mbar_wait_tight(smem_u32(p_full) + 8 * buf, phase, abort_addr, limit));
+            if (!alive) report_timeout(abort_flag, 24);
+          }
+          if (alive) {
+            named_barrier_arrive(C::chunk_barrier(0, (int)buf), 160);
+            named_barrier_arrive(C::chunk_barrier(1, (int)buf), 160);
+          } else {
+            // (the fold is past the accumulator's chunk before: its barriers are free)
+            (void)mbar_wait_tight(smem_u32(p_empty) + 8 * buf, phase ^ 1u, smem_u32(const_cast<int*>(never)), limit);
+            __syncwarp();
+            named_barrier_sync(C::chunk_barrier(0, (int)buf), 160);
+            named_barrier_sync(C::chunk_barrier(1, (int)buf), 160);
+          }
+          if (++buf == C::P_BUFS) {
+            buf = 0;
+            phase ^= 1u;
+          }
         }
       }
     }
@@ -451,250 +554,259 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int quad = warp & 3;
     const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
     // factors: lane = (row of sixteen, chunk of the stage); the warp serves 32 rows of A and BN / 4 columns of B
-    const int fc = lane & 1, fr = lane >> 1;
-    uint32_t it = 0;
-    bool alive = true;
-    for (int tile = (int)blockIdx.x; tile < n_tiles && alive; tile += (int)gridDim.x) {
-      const MacroTile mt = decode_macro_tile<C>(margs, (uint32_t)tile, k_stages);
-      const TileInfo& ti = mt.t;
-      if (ti.skip) continue;
-      const int64_t m0 = ti.mb * BM, n0 = ti.nb * C::BN;
-      const uint8_t* pa = margs.ma.codes + (mt.chunk0 + fc) * margs.ma.chunk_stride +
-                          (m0 >> margs.ma.shift) * margs.ma.row_stride;
-      const uint8_t* pb = margs.mb.codes + (int64_t)mt.expert * margs.mb.expert_stride +
-                          (mt.chunk0 + fc) * margs.mb.chunk_stride + (n0 >> margs.mb.shift) * margs.mb.row_stride;
-      // offsets of the lane's rows from the tile's first (a row beyond the matrix reads the last one)
-      constexpr int NB = B_UNIFORM ? C::SFB_BLOCKS : C::BN / 64;
-      int64_t off_a[2], off_b[NB];
-      const uint32_t m_last = (uint32_t)(args.M - m0 < BM ? args.M - m0 : BM) - 1u;
-      const uint32_t n_last = (uint32_t)(args.N - n0 < C::BN ? args.N - n0 : C::BN) - 1u;
+    // (columns c, c + 4, c + 8 and c + 12 of a piece lie together, see Piece)
+    const int fc = lane & 1, fr = lane >> 1, fr_col = (fr & 3) * 4 + (fr >> 2) - fr;
+    constexpr int NB = B_UNIFORM ? C::SFB_BLOCKS : BN / 64;
+    struct Codes {
+      uint32_t a[2], b[NB];
+    };
+    // The codes of a stage are requested AHEAD stages before it: read one stage ahead, their latency was what a
+    // stage took (900 cycles, with no operand loaded, no MMA issued and nothing folded).
+    const uint8_t *pa[2], *pb[NB];
+    int next_tile = (int)blockIdx.x, stages_left = 0, chunks_left = 0;
+    auto request = [&](Codes& q) -> bool {
+      while (stages_left == 0) {
+        if (next_tile >= n_tiles) return false;
+        const MacroTile mt = decode_macro_tile<C>(margs, (uint32_t)next_tile, k_stages);
+        next_tile += (int)gridDim.x;
+        if (mt.t.skip) continue;
+        stages_left = mt.t.k_stages;
+        chunks_left = mt.n_chunks - fc;
+        const int64_t m0 = mt.t.mb * BM, n0 = mt.t.nb * BN;
+        const uint8_t* a0 = margs.ma.codes + (mt.chunk0 + fc) * margs.ma.chunk_stride + (m0 >> margs.ma.shift) * margs.ma.row_stride;
+        const uint8_t* b0 = margs.mb.codes + (int64_t)mt.expert * margs.mb.expert_stride +
+                            (mt.chunk0 + fc) * margs.mb.chunk_stride + (n0 >> margs.mb.shift) * margs.mb.row_stride;
+        // (a row beyond the matrix reads the last one)
+        const uint32_t m_last = (uint32_t)(args.M - m0 < BM ? args.M - m0 : BM) - 1u;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t r = (uint32_t)(quad * 32 + 16 * i + fr);
+          pa[i] = a0 + (int64_t)((r < m_last ? r : m_last) >> margs.ma.shift) * margs.ma.row_stride;
+        }
+        const uint32_t n_last = B_UNIFORM ? (uint32_t)(((args.N - 1) >> 7) - (n0 >> 7))   // of the 128-row blocks
+                                          : (uint32_t)(args.N - n0 < BN ? args.N - n0 : BN) - 1u;
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+          const uint32_t r = (uint32_t)(B_UNIFORM ? i : quad * (BN / 4) + 16 * i + fr);
+          pb[i] = b0 + (int64_t)(r < n_last ? r : n_last) * margs.mb.row_stride;
+        }
+      }
+      const bool have = chunks_left > 0;
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const uint32_t r = (uint32_t)(quad * 32 + 16 * i + fr);
-        off_a[i] = (int64_t)((r < m_last ? r : m_last) >> margs.ma.shift) * margs.ma.row_stride;
+        q.a[i] = have ? __ldg(pa[i]) : 0u;
+        pa[i] += 2 * margs.ma.chunk_stride;
       }
 #pragma unroll
       for (int i = 0; i < NB; ++i) {
-        const uint32_t r = (uint32_t)(B_UNIFORM ? 128 * i : quad * (C::BN / 4) + 16 * i + fr);
-        off_b[i] = (int64_t)((r < n_last ? r : n_last) >> (B_UNIFORM ? 7 : 0)) * margs.mb.row_stride;
+        q.b[i] = have ? __ldg(pb[i]) : 0u;
+        pb[i] += 2 * margs.mb.chunk_stride;
       }
-      uint32_t ca[2], cb[NB];
-      auto load_codes = [&](int ks) {
-        const bool have = 2 * ks + fc < mt.n_chunks;
+      --stages_left;
+      chunks_left -= 2;
+      return true;
+    };
+    uint32_t s = 0, phase = 0, slot = 0;          // operand stage and its phase, factor stage
+    auto transfer = [&](const Codes& q) -> bool {
+      if (!mbar_wait_tight(smem_u32(full_bar) + 8 * s, phase, abort_addr, limit)) return false;
+      const uint8_t* sf = smem + s * C::STAGE_BYTES + C::SF_OFF + lane * 16;
+      const uint32_t sf_t = tmem_base + lane_base + C::TMEM_SF_BASE + s * C::STAGE_SF_COLS;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) ca[i] = have ? __ldg(pa + off_a[i]) : 0u;
+      for (int t = 0; t < C::SF_TILES; ++t) {
+        const uint4 a = *reinterpret_cast<const uint4*>(sf + t * 512);
+        tc_st4(sf_t + t * 4, a.x, a.y, a.z, a.w);
 #pragma unroll
-        for (int i = 0; i < NB; ++i) cb[i] = have ? __ldg(pb + off_b[i]) : 0u;
-        pa += 2 * margs.ma.chunk_stride;
-        pb += 2 * margs.mb.chunk_stride;
-      };
-      load_codes(0);
-      for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
-        const int s = it % C::STAGES;
-        if (!mbar_wait(&full_bar[s], (it / C::STAGES) & 1, abort_flag, 26, args.wait_ns)) { alive = false; break; }
-        const uint8_t* sf = smem + s * C::STAGE_BYTES + C::SF_OFF + lane * 16;
-        const uint32_t sf_t = tmem_base + lane_base + C::TMEM_SF_BASE + s * C::STAGE_SF_COLS;
-#pragma unroll
-        for (int t = 0; t < (1 + C::SFB_BLOCKS) * C::SF_TILES; ++t) {
-          const uint4 a = *reinterpret_cast<const uint4*>(sf + t * 512);
-          tc_st4(sf_t + t * 4, a.x, a.y, a.z, a.w);
+        for (int h = 0; h < C::SFB_BLOCKS; ++h) {            // the blocks of a K tile lie together
+          const uint4 b = *reinterpret_cast<const uint4*>(sf + (1 + h) * C::SF_BYTES + t * 512);
+          tc_st4(sf_t + C::SF_COLS + (t * C::SFB_BLOCKS + h) * 4, b.x, b.y, b.z, b.w);
         }
-        float* dst = fac + (2 * (it % C::FAC_STAGES) + fc) * C::FAC_STRIDE + fr;
-        if (B_UNIFORM) {
+      }
+      float* dst = fac + (2 * slot + fc) * C::FAC_STRIDE + fr;
+      if (B_UNIFORM) {
 #pragma unroll
-          for (int j = 0; j < NB; ++j) {
-            const float rb = rcp_tab[cb[j]];
+        for (int j = 0; j < NB; ++j) {
+          const float rb = rcp_tab[q.b[j]];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) dst[BM * j + quad * 32 + 16 * i] = __fmul_rn(rcp_tab[ca[i]], rb);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 2; ++i) dst[quad * 32 + 16 * i] = rcp_tab[ca[i]];
-#pragma unroll
-          for (int i = 0; i < NB; ++i) dst[BM + quad * (C::BN / 4) + 16 * i] = rcp_tab[cb[i]];
+          for (int i = 0; i < 2; ++i) dst[BM * j + quad * 32 + 16 * i] = __fmul_rn(rcp_tab[q.a[i]], rb);
         }
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sf_full[s]);
-        if (ks + 1 < ti.k_stages) load_codes(ks + 1);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) dst[quad * 32 + 16 * i] = rcp_tab[q.a[i]];
+#pragma unroll
+        for (int i = 0; i < NB; ++i) dst[BM + quad * (BN / 4) + 16 * i + fr_col] = rcp_tab[q.b[i]];
+      }
+      tc_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      mbar_arrive_lane0(smem_u32(sf_full) + 8 * s, lane);
+      slot = (slot + 1) % C::FAC_STAGES;
+      if (++s == C::STAGES) {
+        s = 0;
+        phase ^= 1u;
+      }
+      return true;
+    };
+    constexpr int AHEAD = 3;
+    Codes q[AHEAD];
+    bool have[AHEAD];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) have[i] = request(q[i]);
+    bool alive = true;
+    while (alive && have[0]) {
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        if (alive && have[i]) {
+          alive = transfer(q[i]);
+          have[i] = request(q[i]);
+        }
       }
     }
+    if (!alive) report_timeout(abort_flag, 26);
   } else {
     // ------------------------------ fold + epilogue ------------------------------
     setmaxnreg_inc<C::REGS_FOLD>();
-    // Of the 200 registers, 160 are accumulators and pieces in flight: what else lives across the chunk loop is
-    // kept in 32 bits (shared-memory addresses, tile numbers).
+    // (What lives across the chunk loop beside the sums and the pieces is kept in 32 bits: local memory does not fit
+    // beside 230 KB of shared memory, a few spilled registers in this loop or the transfer's cost a tenth.)
     const int quad = warp & 3;                        // tensor-memory lane quarter this warp may read
-    const int half = (warp - 8) >> 2;                 // columns [HN half, HN half + HN) of the tile
-    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const int side = (warp - 8) >> 2;                 // columns [WN side, WN side + WN) of the tile
+    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(side * C::WN);
     // this lane's first row and column factor in a chunk's slot
-    const uint32_t fac_a = smem_u32(fac) + 4u * (uint32_t)((B_UNIFORM && C::SFB_BLOCKS == 2 ? half * BM : 0) + quad * 32 + (lane >> 2));
-    const uint32_t fac_b = smem_u32(fac) + 4u * (uint32_t)(BM + half * HN + 2 * (lane & 3));
-    const uint32_t my_full = smem_u32(p_full + half * C::RING), my_empty = smem_u32(p_empty + half * C::RING);
+    const uint32_t fac_a = smem_u32(fac) + 4u * (uint32_t)(quad * 32 + (B_UNIFORM ? lane : lane >> 2));
+    const uint32_t fac_b = smem_u32(fac) + 4u * (uint32_t)(BM + side * C::WN + 4 * (lane & 3));
+    const uint32_t bar_empty = smem_u32(p_empty);
     uint32_t store_it = 0;                            // store units so far
     uint32_t slot = 0;                                // byte offset of the chunk's factors, always of an even slot at a tile's start
-    // ring positions of the half's next chunk: its barriers (n % 3), their phase, its accumulator (see the issuers)
-    uint32_t ring = 0, phase = 0, acc_i = (uint32_t)half;
+    uint32_t ring = 0;                                // accumulator of the next chunk
     constexpr uint32_t SLOT_BYTES = C::FAC_STRIDE * 4, SLOTS_END = 2 * C::FAC_STAGES * SLOT_BYTES;
-    bool alive = true;
-    for (int tile = (int)blockIdx.x; tile < n_tiles && alive; tile += (int)gridDim.x) {
+    constexpr int PIECES = C::PIECES, FLIGHT = C::FLIGHT, RA = B_UNIFORM ? C::SFB_BLOCKS : 2;
+    for (int tile = (int)blockIdx.x; tile < n_tiles; tile += (int)gridDim.x) {
       int left, row0, col0, batch;                    // chunks left, this warp's part of the output
-      bool mine;
+      int split = PIECES;                             // B_UNIFORM: pieces under the first of the tile's 128-column blocks
       {
         const MacroTile mt = decode_macro_tile<C>(margs, (uint32_t)tile, k_stages);
         left = mt.t.skip ? 0 : mt.n_chunks;
-        mine = half < mt.halves;
         row0 = (int)mt.t.mb * BM + quad * 32;
-        col0 = (int)mt.t.nb * C::BN + half * HN;
+        col0 = (int)mt.t.nb * BN + side * C::WN;
         batch = mt.t.batch;
+        if (C::SFB_BLOCKS == 2) split = (128 - ((int)(mt.t.nb * BN) & 127) - side * C::WN) / 16;
       }
-      auto step = [&]() {
-        if (++ring == C::RING) {
-          ring = 0;
-          phase ^= 1u;
-        }
-        acc_i = C::OWN_BUFS ? 2u * ring + (uint32_t)half : acc_i == 0u ? 2u : acc_i - 1u;   // (+ 2 mod 3)
-        slot = slot + SLOT_BYTES == SLOTS_END ? 0u : slot + SLOT_BYTES;
-      };
-      float2 acc[HN / 2];                             // [PIECES][Piece]
+      float2 acc[C::WN / 2];                          // [PIECES][Piece]
 #pragma unroll
-      for (int j = 0; j < HN / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
+      for (int j = 0; j < C::WN / 2; ++j) acc[j] = make_float2(0.0f, 0.0f);
       const bool odd = (left & 1) != 0;
-      if (left > 0) {
-        alive = mbar_wait(generic_bar(my_full + 8 * ring), phase, abort_flag, 24, args.wait_ns);
-        if (!alive) break;
-      }
-      if (!mine) {                                    // nothing to read, only the hand-over
-        while (left > 0 && alive) {
-          __syncwarp();
-          if (lane == 0) mbar_arrive(generic_bar(my_empty + 8 * ring));
-          step();
-          if (--left > 0) alive = mbar_wait(generic_bar(my_full + 8 * ring), phase, abort_flag, 24, args.wait_ns);
-        }
-      } else if (left > 0) {
-        uint32_t t_acc = t_row + acc_i * HN;
+      for (; left > 0; --left) {
+        named_barrier_sync(C::chunk_barrier(side, (int)ring), 160);   // the chunk is finished
         tc_fence_after();
-        if constexpr (C::OWN_BUFS) {
-          // the whole chunk at once: a piece's registers take the next chunk's piece as soon as it is folded
-          Piece pc[C::PIECES];
+        // As much of the chunk as the registers take, so that its accumulator is given back before most of the
+        // multiply-adds.
+        Piece pc[FLIGHT];
+        const uint32_t t_acc = t_row + ring * BN;
 #pragma unroll
-          for (int p = 0; p < C::PIECES; ++p) tc_ld_piece(t_acc + 16 * p, pc[p]);
-          while (true) {
-            const uint32_t fb = fac_b + slot;
-            float ra[4];
+        for (int p = 0; p < FLIGHT; ++p) tc_ld_piece<B_UNIFORM>(t_acc + 16 * p, pc[p]);
+        const uint32_t fb = fac_b + slot;
+        float2 ra[RA];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) ra[q] = ld_shared_f32(fac_a + slot + 32 * q);
-            const uint32_t gone = my_empty + 8 * ring;
-            step();
-            const bool ready = __all_sync(0xFFFFFFFFu, mbar_test(my_full + 8 * ring, phase)) && left > 1;
-            tc_wait_piece(pc[0]);           // all of them
+        for (int q = 0; q < RA; ++q) {
+          if (B_UNIFORM) {
+            ra[q].x = ra[q].y = ld_shared_f32(fac_a + slot + 4 * BM * q);
+          } else {
+            ra[q].x = ld_shared_f32(fac_a + slot + 64 * q);
+            ra[q].y = ld_shared_f32(fac_a + slot + 64 * q + 32);
+          }
+        }
+        const uint32_t gone = bar_empty + 8 * ring;
+        if (++ring == C::P_BUFS) ring = 0;
+        slot = slot + SLOT_BYTES == SLOTS_END ? 0u : slot + SLOT_BYTES;
+        auto fold = [&](int p) {
+          if constexpr (B_UNIFORM) {
+            const float2 r[1] = {RA == 1 || p < split ? ra[0] : ra[RA - 1]};
+            fold_piece<true>(acc + 8 * p, pc[p % FLIGHT], r, 0u);
+          } else {
+            fold_piece<false>(acc + 8 * p, pc[p % FLIGHT], ra, fb + 64 * p);
+          }
+        };
+        auto landed = [&]() {
 #pragma unroll
-            for (int p = 1; p < C::PIECES; ++p) tc_landed_piece(pc[p]);
-            tc_fence_before();
-            if (lane == 0) mbar_arrive(generic_bar(gone));
-            t_acc = t_row + acc_i * HN;
-            if (ready) {
-              tc_fence_after();
+          for (int p = 0; p < FLIGHT; ++p) tc_landed_piece(pc[p]);
+        };
+        if (FLIGHT < PIECES) {
+          tc_wait_ld();
+          landed();
+        }
 #pragma unroll
-              for (int p = 0; p < C::PIECES; ++p) {
-                fold_piece<B_UNIFORM>(acc + 8 * p, pc[p], ra, fb + 64 * p);
-                tc_ld_piece(t_acc + 16 * p, pc[p]);
+        for (int p = FLIGHT; p < PIECES; ++p) {
+          fold(p - FLIGHT);
+          tc_ld_piece<B_UNIFORM>(t_acc + 16 * p, pc[p - FLIGHT]);
+        }
+        tc_wait_ld();
+        tc_fence_before();
+        mbar_arrive_lane0(gone, lane);
+        landed();                       // (after the arrival: no multiply-add moves in front of it)
+#pragma unroll
+        for (int p = PIECES - FLIGHT; p < PIECES; ++p) fold(p);
+      }
+      if (odd) slot = slot + SLOT_BYTES == SLOTS_END ? 0u : slot + SLOT_BYTES;   // a stage has two slots
+      // ---- epilogue of the tile: this warp's 32 rows x WN columns, in units of 32 columns ----
+      // (64 bytes a row of bf16 with the 64-byte swizzle, two buffers; 128 bytes of fp32, one)
+      const float os = margs.out_scale;
+      const bool out_bf16 = args.out_bf16 != 0, failed = *abort_flag != 0;
+      uint8_t* const epi_warp = epi + (warp - 8) * C::EPI_WARP_BYTES;
+#pragma unroll
+      for (int q = 0; q < C::WN / 32; ++q) {
+        if (lane == 0) {                                // the last store has finished reading this buffer
+          if (out_bf16) bulk_wait_read<1>();
+          else bulk_wait_read<0>();
+        }
+        __syncwarp();
+        uint8_t* const unit = epi_warp + (out_bf16 ? (store_it & 1u) * 2048u : 0u);
+        const uint32_t base = smem_u32(unit);
+        if constexpr (B_UNIFORM) {
+          const uint32_t row = (uint32_t)lane;
+          if (out_bf16) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+              uint32_t o[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const float2 v = acc[q * 16 + g * 4 + e];
+                const __nv_bfloat162 p2 = __floats2bfloat162_rn(__fmul_rn(v.x, os), __fmul_rn(v.y, os));
+                o[e] = *reinterpret_cast<const uint32_t*>(&p2);
               }
-              --left;
-              continue;
+              st_shared_v4(base + row * 64u + ((((uint32_t)g) ^ ((row >> 1) & 3u)) << 4), o[0], o[1], o[2], o[3]);
             }
+          } else {
 #pragma unroll
-            for (int p = 0; p < C::PIECES; ++p) fold_piece<B_UNIFORM>(acc + 8 * p, pc[p], ra, fb + 64 * p);
-            if (--left == 0) break;
-            alive = mbar_wait(generic_bar(my_full + 8 * ring), phase, abort_flag, 24, args.wait_ns);
-            if (!alive) break;
-            tc_fence_after();
-#pragma unroll
-            for (int p = 0; p < C::PIECES; ++p) tc_ld_piece(t_acc + 16 * p, pc[p]);
+            for (int g = 0; g < 8; ++g) {
+              const float2 v = acc[q * 16 + g * 2], w = acc[q * 16 + g * 2 + 1];
+              st_shared_v4(base + row * 128u + ((((uint32_t)g) ^ (row & 7u)) << 4), f2u(__fmul_rn(v.x, os)),
+                           f2u(__fmul_rn(v.y, os)), f2u(__fmul_rn(w.x, os)), f2u(__fmul_rn(w.y, os)));
+            }
           }
         } else {
-          Piece p0, p1;                                 // one arrives while the other is folded
-          tc_ld_piece(t_acc, p0);
-          while (true) {
-            const uint32_t fb = fac_b + slot;
-            float ra[4];
+          const uint32_t lr = (uint32_t)(lane >> 2), lc = (uint32_t)(lane & 3);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) ra[q] = ld_shared_f32(fac_a + slot + 32 * q);
-            const uint32_t gone = my_empty + 8 * ring;
-            step();
-            // the next chunk's barrier is looked at here, where the answer has time to arrive (a wait on a
-            // barrier that is already complete costs ~150 cycles when the code depends on it at once)
-            const bool ready = __all_sync(0xFFFFFFFFu, mbar_test(my_full + 8 * ring, phase));
+          for (int g = 0; g < 8; ++g) {                 // column lc + 4 g of the unit
 #pragma unroll
-            for (int p = 0; p < C::PIECES - 1; ++p) {
-              tc_wait_piece(p & 1 ? p1 : p0);
-              tc_ld_piece(t_acc + 16 * (p + 1), p & 1 ? p0 : p1);
-              fold_piece<B_UNIFORM>(acc + 8 * p, p & 1 ? p1 : p0, ra, fb + 64 * p);
+            for (int e = 0; e < 4; ++e) {               // row lr + 8 e
+              const float2 pair = acc[(q * 2 + (g >> 2)) * 8 + (e >> 1) * 4 + (g & 3)];
+              const float v = __fmul_rn((e & 1) != 0 ? pair.y : pair.x, os);
+              const uint32_t row = lr + 8u * e;
+              if (out_bf16)
+                st_shared_u16(base + row * 64u + ((((uint32_t)g >> 1) ^ ((row >> 1) & 3u)) << 4) + (g & 1) * 8u + lc * 2u,
+                              __bfloat16_as_ushort(__float2bfloat16_rn(v)));
+              else
+                st_shared_u32(base + row * 128u + ((((uint32_t)g) ^ (row & 7u)) << 4) + lc * 4u, f2u(v));
             }
-            static_assert(C::PIECES % 2 == 0, "the last piece is in p1");
-            tc_wait_piece(p1);              // the chunk has left tensor memory (a warp-wide wait)
-            tc_fence_before();
-            if (lane == 0) mbar_arrive(generic_bar(gone));
-            if (--left > 0) {
-              if (!ready) {
-                alive = mbar_wait(generic_bar(my_full + 8 * ring), phase, abort_flag, 24, args.wait_ns);
-                if (!alive) break;
-              }
-              t_acc = t_row + acc_i * HN;
-              tc_fence_after();
-              tc_ld_piece(t_acc, p0);
-            }
-            fold_piece<B_UNIFORM>(acc + 8 * (C::PIECES - 1), p1, ra, fb + 64 * (C::PIECES - 1));
-            if (left == 0) break;
           }
         }
-      }
-      if (!alive) break;
-      if (odd) slot = slot + SLOT_BYTES == SLOTS_END ? 0u : slot + SLOT_BYTES;   // a stage has two slots
-      if (!mine) continue;
-      // ---- epilogue of the tile: this warp's 32 rows x HN columns, in units of 16 rows x 128 bytes ----
-      const float os = margs.out_scale;
-      const bool out_bf16 = args.out_bf16 != 0;
-      uint8_t* epi_warp = epi + (warp - 8) * C::EPI_WARP_BYTES;
-      const int lr = lane >> 2, lc = lane & 3;
-#pragma unroll
-      for (int q = 0; q < HN / 32; ++q) {
-        if (out_bf16 && (q & 1) != 0) continue;
-#pragma unroll
-        for (int rh = 0; rh < 2; ++rh) {
-          if (lane == 0) bulk_wait_read<1>();  // the store issued two units ago has finished reading this buffer
-          __syncwarp();
-          uint8_t* unit = epi_warp + (store_it & 1u) * C::EPI_UNIT;
-          const uint32_t base = smem_u32(unit);
-#pragma unroll
-          for (int g = 0; g < 8; ++g) {                 // column groups of eight: 16 bytes of bf16, 32 of fp32
-            if (!out_bf16 && g >= 4) continue;
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {               // row lr + 8 e of the unit
-              const int cg = (q * 4 + g) & (HN / 8 - 1);   // (the mask keeps the unreachable fp32 case inside acc)
-              const float2 v = acc[(cg >> 1) * 8 + rh * 4 + (cg & 1) * 2 + e];
-              const uint32_t row = (uint32_t)(lr + 8 * e);
-              const float x = __fmul_rn(v.x, os), y = __fmul_rn(v.y, os);
-              if (out_bf16) {
-                const __nv_bfloat162 p2 = __floats2bfloat162_rn(x, y);
-                st_shared_u32(base + row * 128u + ((((uint32_t)g) ^ (row & 7u)) << 4) + lc * 4u,
-                              *reinterpret_cast<const uint32_t*>(&p2));
-              } else {
-                const uint32_t chunk = (uint32_t)(2 * g) + (uint32_t)(lc >> 1);
-                st_shared_v2(base + row * 128u + ((chunk ^ (row & 7u)) << 4) + (lc & 1) * 8u, f2u(x), f2u(y));
-              }
-            }
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          __syncwarp();
-          const int col = col0 + 32 * q, r0 = row0 + 16 * rh;
-          if (lane == 0) {
-            if (r0 < args.M && col < args.N) tma_store_3d(unit, &tmap_d, col, r0, batch);
-            bulk_commit();  // one group per unit, empty or not: the waits above count groups
-          }
-          ++store_it;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        const int col = col0 + 32 * q;
+        if (lane == 0) {
+          if (row0 < args.M && col < args.N && !failed) tma_store_3d(unit, &tmap_d, col, row0, batch);
+          bulk_commit();  // one group per unit, empty or not: the waits above count groups
         }
+        ++store_it;
       }
     }
     if (lane == 0) bulk_wait_all();

@@ -1541,11 +1541,11 @@ static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N,
 #undef LAUNCH
 }
 
-template <int HN, bool B_UNIFORM>
+template <int BN, bool B_UNIFORM>
 static int launch_gemm_macro(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td,
                              const MacroGemmArgs& margs, int64_t grid, cudaStream_t st) {
-  using C = CfgMacro<HN>;
-  auto kernel = gemm_macro_kernel<HN, B_UNIFORM>;
+  using C = CfgMacro<BN>;
+  auto kernel = gemm_macro_kernel<BN, B_UNIFORM>;
   static std::atomic<int> attr_set[MAX_DEVICES];
   const int rc = ensure_smem_attr(kernel, C::SMEM_BYTES, attr_set);
   if (rc != ALTOB200_OK) return rc;
@@ -1553,25 +1553,23 @@ static int launch_gemm_macro(const CUtensorMap& ta, const CUtensorMap& tb, const
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }
 
-// Columns of a half: 128 (tiles of 128 x 256) or 64 (128 x 128).  A wide tile takes less time per column of a
-// chunk, but there are half as many, so it loses where they leave SMs without work or a last wave nearly empty,
-// and its epilogue has nothing to overlap with, which counts where the K range is short.  The estimate is in chunk
-// times of a narrow tile (0.33 us with one B factor per tile, 0.37 with one per column), fitted to
-//                                      one B factor, us: narrow / wide     per column, us: narrow / wide
-//   320 x 288 x 14336 (9 / 6 tiles)            39.0 / 59.3                        43.9 / 83.8
-//   512 x 4096 x 4096 (one wave each)          14.7 / 21.4                        16.2 / 25.9
-//   2048^3 (two waves / one)                   15.6 / 14.3                        17.3 / 16.6
-//   4096^3 (seven / four)                      81.4 / 75.9                        91.6 / 94.2
-//   16 ranges of 128, 5760 x 2880                                                 188 / 213
-//   8 ranges of 384, 2880 x 2880                                                  70.3 / 68.8
-static int macro_half(int64_t row_tiles, int64_t N, int64_t chunks, bool b_uniform, int64_t* grid) {
+// Columns of a tile.  192 take 1.44 times as long as 128 per chunk, so a little less per column, which pays where there
+// are many tiles; 128 leave fewer SMs idle and have the better last wave.  With one B factor per column the wide
+// tile is the slower one everywhere (its chunk does not fit the registers beside the factors: 533 against 519 us at
+// 8192 x 4096 x 14336, 1514 / 1493 at 32 ranges of 2048, 5760 x 2880).  The estimate is in chunk times of a narrow
+// tile (0.2 us), fitted to (one B factor, us: narrow / wide)
+//   8192 x 4096 x 14336   363 / 349        2048^3                13.9 / 17.1
+//   8192 x 14336 x 4096   332 / 341        320 x 288 x 14336     26.5 / 36.5
+//   69 632 rows in groups, 2880 -> 5760   930 / 893              5760 -> 2880  847 / 805
+static int macro_tile_n(int64_t row_tiles, int64_t N, int64_t chunks, bool b_uniform, int64_t* grid) {
   const int64_t sms = sm_count_gemm();
-  const int64_t narrow = row_tiles * ceil_div(N, 128), wide = row_tiles * ceil_div(N, 256);
-  const double t_narrow = (double)ceil_div(narrow, sms) * (4.0 + (double)chunks);
-  const double t_wide = (double)ceil_div(wide, sms) * (9.0 + (b_uniform ? 1.56 : 1.77) * (double)chunks);
-  const int64_t tiles = t_narrow <= t_wide ? narrow : wide;
+  const int64_t narrow = row_tiles * ceil_div(N, 128), wide = row_tiles * ceil_div(N, 192);
+  const double t_narrow = (double)ceil_div(narrow, sms) * (4.3 + (double)chunks);
+  const double t_wide = (double)ceil_div(wide, sms) * (5.9 + 1.44 * (double)chunks);
+  const bool use_wide = b_uniform && t_wide < t_narrow;
+  const int64_t tiles = use_wide ? wide : narrow;
   *grid = tiles < sms ? tiles : sms;
-  return t_narrow <= t_wide ? 64 : 128;
+  return use_wide ? 192 : 128;
 }
 
 static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_experts, const void* a_codes,
@@ -1601,14 +1599,15 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   const bool b_uniform = b_macro->row_shift == 7;   // one B factor per 128 columns and chunk
   const int64_t batches = k_offs != nullptr ? num_experts : 1;
   int64_t grid = 0;
-  const int HN = macro_half(ceil_div(M, BM) * batches, N, ceil_div(K / batches, 128), b_uniform, &grid);
+  const int BN = macro_tile_n(ceil_div(M, BM) * batches, N, ceil_div(K / batches, 128), b_uniform, &grid);
 
   CUtensorMap ta, tb, td;
   int rc = make_tmap(&ta, a_codes, M, k_bytes, BM);
   if (rc != ALTOB200_OK) return rc;
-  rc = make_tmap(&tb, b_codes, b_rows, k_bytes, HN);
+  rc = make_tmap(&tb, b_codes, b_rows, k_bytes, BN);
   if (rc != ALTOB200_OK) return rc;
-  rc = make_tmap_out(&td, d, k_offs != nullptr ? num_experts : 1, M, N, ldd, out_dtype == ALTOB200_DT_BF16, 128, 16);
+  rc = make_tmap_out(&td, d, k_offs != nullptr ? num_experts : 1, M, N, ldd, out_dtype == ALTOB200_DT_BF16,
+                     out_dtype == ALTOB200_DT_BF16 ? 64 : 128);
   if (rc != ALTOB200_OK) return rc;
 
   MacroGemmArgs m;
@@ -1627,7 +1626,7 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
     if (gm > tiles_m) gm = tiles_m;
     const int64_t n_groups = ceil_div(tiles_m, gm);
     g.group_m = (int)ceil_div(tiles_m, n_groups);
-    const int64_t tiles_n = ceil_div(N, 2 * HN);
+    const int64_t tiles_n = ceil_div(N, BN);
     m.per_batch = make_tile_div(tiles_m * tiles_n);
     m.per_group = make_tile_div(g.group_m * tiles_n);
     m.rows_full = make_tile_div(g.group_m);
@@ -1635,7 +1634,7 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   }
   g.wait_ns = wait_limit_ns();
   for (int j = 0; j < 4; ++j)
-    g.idesc[j] = make_idesc(KIND_MXF4, ALTOB200_FMT_MXFP4, ALTOB200_FMT_MXFP4, BM, HN, (j & 1) * 2);
+    g.idesc[j] = make_idesc(KIND_MXF4, ALTOB200_FMT_MXFP4, ALTOB200_FMT_MXFP4, BM, BN, (j & 1) * 2);
 #ifdef ALTOB200_GEMM_PROFILE
   {
     const char* e = getenv("ALTOB200_GEMM_DEBUG");
@@ -1648,9 +1647,8 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   m.mb.expert_stride = row_groups ? b_macro->expert_stride : 0; m.mb.shift = b_macro->row_shift;
   m.out_scale = out_scale;
   cudaStream_t st = (cudaStream_t)stream;
-  if (HN == 64)
-    return b_uniform ? launch_gemm_macro<64, true>(ta, tb, td, m, grid, st) : launch_gemm_macro<64, false>(ta, tb, td, m, grid, st);
-  return b_uniform ? launch_gemm_macro<128, true>(ta, tb, td, m, grid, st) : launch_gemm_macro<128, false>(ta, tb, td, m, grid, st);
+  if (!b_uniform) return launch_gemm_macro<128, false>(ta, tb, td, m, grid, st);
+  return BN == 128 ? launch_gemm_macro<128, true>(ta, tb, td, m, grid, st) : launch_gemm_macro<192, true>(ta, tb, td, m, grid, st);
 }
 
 }  // namespace altob200

@@ -94,3 +94,22 @@ def test_row_groups(groups, n, k, tiles):
             assert (out[rows] == 0).all()
         else:
             _near(out[rows], a.values[rows], bs[e].values)
+
+
+@pytest.mark.parametrize("n", [2304 + 32, 2304 + 160])
+@pytest.mark.parametrize("k", [640, 2880])
+def test_wide_tiles_of_row_groups(n, k):
+    # 18 row tiles: tiles of 192 columns, whose scales of B begin on a block of 128 rows or in its middle; the last
+    # tile ends before its second block, or in it, and reads on into the next expert's rows
+    groups, n_exp = [0, 1] * 9, 2
+    a = Random(128 * len(groups), k, 15)
+    bs = [Random(n, k, 16 + e, True) for e in range(n_exp)]
+    macro = torch.stack([b.macro.codes for b in bs])
+    f = L.MacroScale(macro, bs[0].macro.row_stride, 1, 7, macro[0].numel())
+    out = torch.empty(128 * len(groups), n, dtype=torch.float32, device="cuda")
+    L.gemm_mxfp4_two_level(out.shape[0], n, k, a.codes, a.scales, a.macro, torch.cat([b.codes for b in bs]),
+                           torch.cat([b.scales for b in bs]), f, out,
+                           group_expert=torch.tensor(groups, dtype=torch.int32, device="cuda"), num_experts=n_exp)
+    for i, e in enumerate(groups):
+        rows = slice(128 * i, 128 * i + 128)
+        _near(out[rows], a.values[rows], bs[e].values)
