@@ -49,28 +49,9 @@ struct MacroSide {
   int shift;                // 0: one factor per row; 7: one factor per 128 rows (2-D macro blocks)
 };
 
-// Quotients of tile numbers by a divisor fixed per launch: t / d = t * m >> s for t < 2^31, with
-// s = 31 + ceil(log2 d) and m = floor(2^s / d) + 1.  A tile's coordinates are on the critical path of every role;
-// with three 64-bit divides a weight gradient of 128 rows per expert (one chunk per tile) took 26 % longer
-// (8 experts, 2880 x 2880: 64.5 us, now 51.4).
-struct TileDiv {
-  uint32_t d, m;
-  int s;
-  __device__ __forceinline__ uint32_t quotient(uint32_t t) const { return (uint32_t)(((uint64_t)t * m) >> s); }
-};
-static TileDiv make_tile_div(int64_t d) {
-  TileDiv v;
-  v.d = (uint32_t)d;
-  v.s = 31;
-  while ((1ll << (v.s - 31)) < d) ++v.s;
-  v.m = (uint32_t)(((unsigned __int128)1 << v.s) / (uint64_t)d + 1);
-  return v;
-}
-
 struct MacroGemmArgs {
   GemmArgs g;
   MacroSide ma, mb;
-  TileDiv per_batch, per_group, rows_full, rows_last;   // tiles per batch, per raster group; row tiles of a group
   float out_scale;
 };
 
@@ -138,21 +119,15 @@ struct MacroTile {
   int expert;
 };
 
-// (the raster of decode_tile: groups of `group_m` row tiles, each swept across all column tiles, row tile fastest)
 template <class C>
 __device__ __forceinline__ MacroTile decode_macro_tile(const MacroGemmArgs& margs, uint32_t tile, int k_stages_dense) {
   const GemmArgs& args = margs.g;
   MacroTile m;
   TileInfo& t = m.t;
-  const uint32_t e = args.k_offs != nullptr ? margs.per_batch.quotient(tile) : 0u;
-  const uint32_t rem = tile - e * margs.per_batch.d;
-  const uint32_t g = margs.per_group.quotient(rem);
-  const uint32_t in_group = rem - g * margs.per_group.d;
-  const bool last_group = (uint64_t)(g + 1) * margs.per_group.d >= margs.per_batch.d;
-  const TileDiv rows = last_group ? margs.rows_last : margs.rows_full;
-  const uint32_t nb = rows.quotient(in_group);
-  t.nb = nb;
-  t.mb = (int64_t)g * args.group_m + (in_group - nb * rows.d);
+  const TileCoord coord = tile_coord(args, tile);
+  const uint32_t e = coord.batch;
+  t.nb = coord.nb;
+  t.mb = coord.mb;
   t.batch = (int)e;
   t.k_byte0 = 0;
   t.sf_tile0 = 0;
@@ -243,74 +218,6 @@ __device__ __forceinline__ float4 ld_shared_f32x4(uint32_t addr) {
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
-// Bounded waits as one small loop each.  Two dozen warps' worth of different code share the instruction caches of an
-// SM, where every taken branch costs 30 to 40 cycles: a wait that is spread over inlined slow paths (mbar_wait) took
-// 200 cycles and more on a barrier that was already complete, and with it a chunk's way around the roles 1300.
-// Counted on the SM's cycle counter, as in mbar_wait; false when the limit has passed or another role has given up.
-#define ALTOB200_WAIT_LOOP(LOOK_AT)                                                                           \
-  "{\n\t.reg .pred p, q, r;\n\t.reg .u32 f, n;\n\t.reg .u64 t, t0;\n\t" LOOK_AT                                 \
-  "@p bra DONE;\n\t"                                                                                         \
-  "mov.u64 t0, %clock64;\n"                                                                                  \
-  "AGAIN:\n\t"                                                                                               \
-  "mov.u32 n, 64;\n"                                                                                         \
-  "LOOK:\n\t" LOOK_AT                                                                                        \
-  "@p bra DONE;\n\t"                                                                                         \
-  "sub.u32 n, n, 1;\n\t"                                                                                     \
-  "setp.ne.u32 q, n, 0;\n\t"                                                                                 \
-  "@q bra LOOK;\n\t"                                                                                         \
-  "ld.volatile.shared.u32 f, [%2];\n\t"                                                                      \
-  "mov.u64 t, %clock64;\n\t"                                                                                 \
-  "sub.u64 t, t, t0;\n\t"                                                                                    \
-  "setp.ne.u32 q, f, 0;\n\t"                                                                                 \
-  "setp.gt.or.u64 q, t, %1, q;\n\t"                                                                          \
-  "@!q bra AGAIN;\n"                                                                                         \
-  "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-__device__ __forceinline__ bool mbar_wait_tight(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint64_t limit_cycles) {
-  uint32_t ok;
-  asm volatile(ALTOB200_WAIT_LOOP("mbarrier.try_wait.parity.shared::cta.b64 p, [%3], %4;\n\t")
-               : "=r"(ok)
-               : "l"(limit_cycles), "r"(abort_addr), "r"(bar), "r"(parity)
-               : "memory");
-  return ok != 0;
-}
-// Three barriers at once (the first two at the same parity): their answers take as long as one.
-__device__ __forceinline__ bool mbar_wait3_tight(uint32_t b0, uint32_t b1, uint32_t parity01, uint32_t b2, uint32_t parity2,
-                                                 uint32_t abort_addr, uint64_t limit_cycles) {
-  uint32_t ok;
-  asm volatile(ALTOB200_WAIT_LOOP("mbarrier.test_wait.parity.shared::cta.b64 p, [%3], %5;\n\t"
-                                  "mbarrier.test_wait.parity.shared::cta.b64 q, [%4], %5;\n\t"
-                                  "mbarrier.test_wait.parity.shared::cta.b64 r, [%6], %7;\n\t"
-                                  "and.pred p, p, q;\n\tand.pred p, p, r;\n\t")
-               : "=r"(ok)
-               : "l"(limit_cycles), "r"(abort_addr), "r"(b0), "r"(b1), "r"(parity01), "r"(b2), "r"(parity2)
-               : "memory");
-  return ok != 0;
-}
-#undef ALTOB200_WAIT_LOOP
-// A role that gave up: the others learn of it, the first one's place is kept.
-__device__ __forceinline__ void report_timeout(volatile int* abort_flag, int site) {
-  if (*abort_flag != 0) return;
-  *abort_flag = 1;
-  if (atomicCAS(&g_status[0], 0, ALTOB200_ETIMEOUT_DEVICE) == 0) {
-    g_status[1] = 1;
-    g_status[2] = (int)blockIdx.x;
-    g_status[3] = site;
-  }
-}
-// An arrival by one lane, without a branch.
-__device__ __forceinline__ void mbar_arrive_lane0(uint32_t bar, int lane) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t"
-      "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
-      ::"r"(bar), "r"(lane)
-      : "memory");
-}
-__device__ __forceinline__ void named_barrier_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-__device__ __forceinline__ void named_barrier_arrive(int id, int count) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
 // tcgen05 instructions of one lane, without a branch around them
 __device__ __forceinline__ void tc_mma_mxf4_if(bool pred, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                uint32_t accumulate, uint32_t sfa, uint32_t sfb) {
@@ -375,7 +282,7 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // (an output of 2^31 tiles would not fit any memory)
-  const int n_tiles = (int)(margs.per_batch.d * (args.k_offs != nullptr ? args.num_batches : 1));
+  const int n_tiles = (int)(margs.g.per_batch.d * (args.k_offs != nullptr ? args.num_batches : 1));
   const int k_stages = (int)((args.k_bytes + STAGE_K_BYTES - 1) / STAGE_K_BYTES);
 
   if (threadIdx.x == 0) {

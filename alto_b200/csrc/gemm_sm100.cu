@@ -67,6 +67,24 @@ struct Kind<KIND_MXF8> {
   static constexpr int ELEMS_PER_BYTE = 1, BLOCK = 32;
 };
 
+// Quotients of tile numbers by a divisor fixed per launch: t / d = t * m >> s for t < 2^31, with
+// s = 31 + ceil(log2 d) and m = floor(2^s / d) + 1.  A tile's coordinates are on the critical path of every role;
+// with three 64-bit divides a weight gradient of 128 rows per expert (one chunk per tile) took 26 % longer
+// (8 experts, 2880 x 2880: 64.5 us, now 51.4).
+struct TileDiv {
+  uint32_t d, m;
+  int s;
+  __device__ __forceinline__ uint32_t quotient(uint32_t t) const { return (uint32_t)(((uint64_t)t * m) >> s); }
+};
+static TileDiv make_tile_div(int64_t d) {
+  TileDiv v;
+  v.d = (uint32_t)d;
+  v.s = 31;
+  while ((1ll << (v.s - 31)) < d) ++v.s;
+  v.m = (uint32_t)(((unsigned __int128)1 << v.s) / (uint64_t)d + 1);
+  return v;
+}
+
 struct GemmArgs {
   int64_t M, N, K;       // K in elements
   int64_t k_bytes;       // bytes per operand row
@@ -87,6 +105,7 @@ struct GemmArgs {
   const int32_t* k_offs;
   int num_batches;
   int group_m;           // row tiles per raster group (see decode_tile)
+  TileDiv per_batch, per_group, rows_full, rows_last;   // tiles per batch, per raster group; row tiles of a group
   uint32_t idesc[4];    // instruction descriptors of the four MMAs of a stage
   uint64_t wait_ns;     // limit of every mbarrier wait (wall clock)
 #ifdef ALTOB200_GEMM_PROFILE
@@ -167,6 +186,86 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// Bounded waits as one small loop each.  More than a dozen warps' worth of different code share the instruction caches of an
+// SM, where every taken branch costs 30 to 40 cycles: a wait that is spread over inlined slow paths (mbar_wait) took
+// 200 cycles and more on a barrier that was already complete, and with it a chunk's way around the roles 1300.
+// Counted on the SM's cycle counter, as in mbar_wait; false when the limit has passed or another role has given up.
+#define ALTOB200_WAIT_LOOP(LOOK_AT)                                                                           \
+  "{\n\t.reg .pred p, q, r;\n\t.reg .u32 f, n;\n\t.reg .u64 t, t0;\n\t" LOOK_AT                                 \
+  "@p bra DONE;\n\t"                                                                                         \
+  "mov.u64 t0, %clock64;\n"                                                                                  \
+  "AGAIN:\n\t"                                                                                               \
+  "mov.u32 n, 64;\n"                                                                                         \
+  "LOOK:\n\t" LOOK_AT                                                                                        \
+  "@p bra DONE;\n\t"                                                                                         \
+  "sub.u32 n, n, 1;\n\t"                                                                                     \
+  "setp.ne.u32 q, n, 0;\n\t"                                                                                 \
+  "@q bra LOOK;\n\t"                                                                                         \
+  "ld.volatile.shared.u32 f, [%2];\n\t"                                                                      \
+  "mov.u64 t, %clock64;\n\t"                                                                                 \
+  "sub.u64 t, t, t0;\n\t"                                                                                    \
+  "setp.ne.u32 q, f, 0;\n\t"                                                                                 \
+  "setp.gt.or.u64 q, t, %1, q;\n\t"                                                                          \
+  "@!q bra AGAIN;\n"                                                                                         \
+  "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+__device__ __forceinline__ bool mbar_wait_tight(uint32_t bar, uint32_t parity, uint32_t abort_addr, uint64_t limit_cycles) {
+  uint32_t ok;
+  asm volatile(ALTOB200_WAIT_LOOP("mbarrier.try_wait.parity.shared::cta.b64 p, [%3], %4;\n\t")
+               : "=r"(ok)
+               : "l"(limit_cycles), "r"(abort_addr), "r"(bar), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
+// Two barriers at once, at the same parity: their answers take as long as one.
+__device__ __forceinline__ bool mbar_wait2_tight(uint32_t b0, uint32_t b1, uint32_t parity, uint32_t abort_addr,
+                                                 uint64_t limit_cycles) {
+  uint32_t ok;
+  asm volatile(ALTOB200_WAIT_LOOP("mbarrier.test_wait.parity.shared::cta.b64 p, [%3], %5;\n\t"
+                                  "mbarrier.test_wait.parity.shared::cta.b64 q, [%4], %5;\n\t"
+                                  "and.pred p, p, q;\n\t")
+               : "=r"(ok)
+               : "l"(limit_cycles), "r"(abort_addr), "r"(b0), "r"(b1), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
+// Three barriers at once (the first two at the same parity): their answers take as long as one.
+__device__ __forceinline__ bool mbar_wait3_tight(uint32_t b0, uint32_t b1, uint32_t parity01, uint32_t b2, uint32_t parity2,
+                                                 uint32_t abort_addr, uint64_t limit_cycles) {
+  uint32_t ok;
+  asm volatile(ALTOB200_WAIT_LOOP("mbarrier.test_wait.parity.shared::cta.b64 p, [%3], %5;\n\t"
+                                  "mbarrier.test_wait.parity.shared::cta.b64 q, [%4], %5;\n\t"
+                                  "mbarrier.test_wait.parity.shared::cta.b64 r, [%6], %7;\n\t"
+                                  "and.pred p, p, q;\n\tand.pred p, p, r;\n\t")
+               : "=r"(ok)
+               : "l"(limit_cycles), "r"(abort_addr), "r"(b0), "r"(b1), "r"(parity01), "r"(b2), "r"(parity2)
+               : "memory");
+  return ok != 0;
+}
+#undef ALTOB200_WAIT_LOOP
+// A role that gave up: the others learn of it, the first one's place is kept.
+__device__ __forceinline__ void report_timeout(volatile int* abort_flag, int site) {
+  if (*abort_flag != 0) return;
+  *abort_flag = 1;
+  if (atomicCAS(&g_status[0], 0, ALTOB200_ETIMEOUT_DEVICE) == 0) {
+    g_status[1] = 1;
+    g_status[2] = (int)blockIdx.x;
+    g_status[3] = site;
+  }
+}
+// An arrival by one lane, without a branch.
+__device__ __forceinline__ void mbar_arrive_lane0(uint32_t bar, int lane) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}"
+      ::"r"(bar), "r"(lane)
+      : "memory");
+}
+__device__ __forceinline__ void named_barrier_sync(int id, int count) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+__device__ __forceinline__ void named_barrier_arrive(int id, int count) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
 // true in exactly one lane of a converged warp
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
@@ -470,22 +569,31 @@ struct TileInfo {
   bool skip;           // nothing to contract: the epilogue writes zeros
 };
 
+// Tile coordinates.  The raster: groups of `group_m` row tiles, each group swept across all column tiles with the row
+// tile running fastest, so that the group's A rows stay in L2 while B streams once per group.
+struct TileCoord {
+  uint32_t batch, mb, nb;
+};
+__device__ __forceinline__ TileCoord tile_coord(const GemmArgs& args, uint32_t tile) {
+  TileCoord t;
+  t.batch = args.k_offs != nullptr ? args.per_batch.quotient(tile) : 0u;
+  const uint32_t rem = tile - t.batch * args.per_batch.d;
+  const uint32_t g = args.per_group.quotient(rem);
+  const uint32_t in_group = rem - g * args.per_group.d;
+  const bool last_group = (uint64_t)(g + 1) * args.per_group.d >= args.per_batch.d;
+  const TileDiv rows = last_group ? args.rows_last : args.rows_full;
+  t.nb = rows.quotient(in_group);
+  t.mb = g * (uint32_t)args.group_m + (in_group - t.nb * rows.d);
+  return t;
+}
+
 template <int KIND, int BN>
-__device__ __forceinline__ TileInfo decode_tile(const GemmArgs& args, int64_t tile, int64_t tiles_m, int64_t tiles_n,
-                                                int k_stages_dense) {
+__device__ __forceinline__ TileInfo decode_tile(const GemmArgs& args, int tile, int k_stages_dense) {
   TileInfo t;
-  const int64_t per_batch = tiles_m * tiles_n;
-  const int64_t e = args.k_offs != nullptr ? tile / per_batch : 0;
-  const int64_t rem = tile - e * per_batch;
-  // raster: groups of `group_m` row tiles, each group swept across all column tiles with the row
-  // tile running fastest, so that the group's A rows stay in L2 while B streams once per group
-  const int64_t per_group = (int64_t)args.group_m * tiles_n;
-  const int64_t g = rem / per_group;
-  const int64_t r2 = rem - g * per_group;
-  const int64_t m0 = g * args.group_m;
-  const int64_t gsz = (tiles_m - m0) < args.group_m ? (tiles_m - m0) : (int64_t)args.group_m;
-  t.nb = r2 / gsz;
-  t.mb = m0 + (r2 - t.nb * gsz);
+  const TileCoord c = tile_coord(args, (uint32_t)tile);
+  const uint32_t e = c.batch;
+  t.nb = c.nb;
+  t.mb = c.mb;
   t.batch = (int)e;
   t.k_stages = k_stages_dense;
   t.last_mmas = 4;
@@ -535,9 +643,8 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t tiles_m = (args.M + BM - 1) / BM;
-  const int64_t tiles_n = (args.N + BN - 1) / BN;
-  const int64_t n_tiles = tiles_m * tiles_n * (args.k_offs != nullptr ? args.num_batches : 1);
+  // (an output of 2^31 tiles would not fit any memory)
+  const int n_tiles = (int)(args.per_batch.d * (args.k_offs != nullptr ? args.num_batches : 1));
   const int k_stages = (int)((args.k_bytes + STAGE_K_BYTES - 1) / STAGE_K_BYTES);
   const int64_t n_row_blocks = (args.N + 127) / 128;
 
@@ -570,6 +677,8 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
+  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see mbar_wait
   // barriers, tensor memory and the zeroed scale staging are set up: from here on global memory is read
   // and written, which has to wait for the kernel in front of this one (programmatic dependent launch)
   grid_dependency_wait();
@@ -580,8 +689,8 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     const bool elected = elect_one();
     uint32_t it = 0;
     bool alive = true;
-    for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+    for (int tile = (int)blockIdx.x; tile < n_tiles && alive; tile += (int)gridDim.x) {
+      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
       if (ti.skip) continue;  // nothing to load: the epilogue writes zeros
       const int64_t mb = ti.mb, nb = ti.nb;
       // 128-row blocks of B that exist (the last tile of a ragged N has fewer)
@@ -590,7 +699,7 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
       for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
         const int s = it % C::STAGES;
         alive = __all_sync(0xFFFFFFFFu,
-                           mbar_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1, abort_flag, 1, args.wait_ns));
+                           mbar_wait_tight(smem_u32(&empty_bar[s]), ((it / C::STAGES) & 1) ^ 1, abort_addr, limit));
         if (!alive) break;
         uint8_t* st = smem + s * C::STAGE_BYTES;
         const int64_t cb0 = ti.sf_tile0 + (int64_t)ks * C::SF_TILES;
@@ -616,6 +725,7 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         __syncwarp();
       }
     }
+    if (!alive) report_timeout(abort_flag, 1);
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     // Whole warp, elected lane issues; the shared-memory barriers are waited on by warp 10, which
@@ -624,8 +734,8 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     uint32_t it = 0, tile_it = 0;
     bool alive = true;
     const uint32_t smem_base = smem_u32(smem);
-    for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+    for (int tile = (int)blockIdx.x; tile < n_tiles && alive; tile += (int)gridDim.x) {
+      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
       if (ti.skip) continue;
       const int acc = tile_it % C::ACC_STAGES;
       const uint32_t d_tmem = tmem_base + acc * BN;
@@ -661,20 +771,20 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     // ------------------------------ wait warp ------------------------------
     uint32_t it = 0, tile_it = 0;
     bool alive = true;
-    for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+    for (int tile = (int)blockIdx.x; tile < n_tiles && alive; tile += (int)gridDim.x) {
+      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
       if (ti.skip) continue;
       const int acc = tile_it % C::ACC_STAGES;
-      bool ok = mbar_wait(&acc_empty[acc], ((tile_it / C::ACC_STAGES) & 1) ^ 1, abort_flag, 2, args.wait_ns);
+      const bool drained = mbar_wait_tight(smem_u32(&acc_empty[acc]), ((tile_it / C::ACC_STAGES) & 1) ^ 1, abort_addr, limit);
       for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
         const int s = it % C::STAGES;
-        ok = ok && mbar_wait(&full_bar[s], (it / C::STAGES) & 1, abort_flag, 3, args.wait_ns);
-        ok = ok && mbar_wait(&sf_full[s], (it / C::STAGES) & 1, abort_flag, 5, args.wait_ns);
-        const bool failed = !__all_sync(0xFFFFFFFFu, ok);
-        if (named_barrier_or(1 + s, 64, failed)) { alive = false; break; }
+        const bool full = mbar_wait_tight(smem_u32(&full_bar[s]), (it / C::STAGES) & 1, abort_addr, limit);
+        const bool ok = full && mbar_wait_tight(smem_u32(&sf_full[s]), (it / C::STAGES) & 1, abort_addr, limit);
+        if (named_barrier_or(1 + s, 64, !(ok && drained))) { alive = false; break; }
       }
       ++tile_it;
     }
+    if (!alive) report_timeout(abort_flag, 2);
   } else if (warp >= 6) {
     // ------------------------------ scale transfer (warps 6..9) ------------------------------
     // Tile t of A -> columns [4t, 4t+4) of the stage's A-scale area; tile t of B row block j ->
@@ -683,12 +793,12 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     uint32_t it = 0;
     bool alive = true;
-    for (int64_t tile = blockIdx.x; tile < n_tiles && alive; tile += gridDim.x) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+    for (int tile = (int)blockIdx.x; tile < n_tiles && alive; tile += (int)gridDim.x) {
+      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
       if (ti.skip) continue;
       for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
         const int s = it % C::STAGES;
-        if (!mbar_wait(&full_bar[s], (it / C::STAGES) & 1, abort_flag, 6, args.wait_ns)) { alive = false; break; }
+        if (!mbar_wait_tight(smem_u32(&full_bar[s]), (it / C::STAGES) & 1, abort_addr, limit)) { alive = false; break; }
         const uint8_t* sf = smem + s * C::STAGE_BYTES + C::A_BYTES + C::B_BYTES + lane * 16;
         const uint32_t sfa_t = tmem_base + lane_base + C::TMEM_SF_BASE + s * (C::SF_COLS_A + C::SF_COLS_B);
         const uint32_t sfb_t = sfa_t + C::SF_COLS_A;
@@ -707,9 +817,10 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sf_full[s]);
+        mbar_arrive_lane0(smem_u32(&sf_full[s]), lane);
       }
     }
+    if (!alive) report_timeout(abort_flag, 6);
   } else {
     // ------------------------------ epilogue ------------------------------
     const int quad = warp & 3;  // tensor-memory lane quarter this warp may read
@@ -717,14 +828,17 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
     if (args.alpha_a != nullptr) alpha = __fmul_rn(alpha, __ldg(args.alpha_a));
     if (args.alpha_b != nullptr) alpha = __fmul_rn(alpha, __ldg(args.alpha_b));
     uint32_t tile_it = 0, store_it = 0;
-    for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+    for (int tile = (int)blockIdx.x; tile < n_tiles; tile += (int)gridDim.x) {
+      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
       const int64_t mb = ti.mb, nb = ti.nb;
       const int64_t row0 = mb * BM + quad * 32;
       const bool pad_group = ti.skip;
       const int acc = tile_it % C::ACC_STAGES;
       if (!pad_group) {
-        if (!mbar_wait(&acc_full[acc], (tile_it / C::ACC_STAGES) & 1, abort_flag, 4, args.wait_ns)) break;
+        if (!mbar_wait_tight(smem_u32(&acc_full[acc]), (tile_it / C::ACC_STAGES) & 1, abort_addr, limit)) {
+          report_timeout(abort_flag, 4);
+          break;
+        }
         tc_fence_after();
       }
       const uint32_t t_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN;
@@ -901,10 +1015,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();      // 0 = leader
   const bool leader = rank == 0;
-  const int64_t pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int64_t tiles_m = (args.M + 2 * BM - 1) / (2 * BM);    // tiles of 256 rows
-  const int64_t tiles_n = (args.N + BN - 1) / BN;
-  const int64_t n_tiles = tiles_m * tiles_n * (args.k_offs != nullptr ? args.num_batches : 1);
+  const int pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
+  const int n_tiles = (int)(args.per_batch.d * (args.k_offs != nullptr ? args.num_batches : 1));   // of 256 rows
   const int k_stages = (int)((args.k_bytes + STAGE_K_BYTES - 1) / STAGE_K_BYTES);
   const int64_t n_row_blocks = (args.N + 127) / 128;
 
@@ -938,6 +1050,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
   cluster_sync_all();   // the peer's barriers are initialised before anything can arrive on them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
+  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see mbar_wait
   // barriers, tensor memory and the zeroed scale staging are set up: from here on global memory is read
   // and written, which has to wait for the kernel in front of this one (programmatic dependent launch)
   grid_dependency_wait();
@@ -952,8 +1066,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
       const bool elected = elect_one();
       uint32_t it = 0;
       bool alive = true;
-      for (int64_t tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-        const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+      for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
+        const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
         if (ti.skip) continue;
         const int64_t mb = ti.mb * 2 + rank;          // this CTA's 128-row block of A
         const int64_t sfb_blk0 = (ti.nb * BN) >> 7;   // first 128-row block of B scales under this tile
@@ -965,7 +1079,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
         for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
           const int s = it % C::STAGES;
           alive = __all_sync(0xFFFFFFFFu,
-                             mbar_wait(&empty_bar[s], ((it / C::STAGES) & 1) ^ 1, abort_flag, 11, args.wait_ns));
+                             mbar_wait_tight(smem_u32(&empty_bar[s]), ((it / C::STAGES) & 1) ^ 1, abort_addr, limit));
           if (!alive) break;
           uint8_t* st = smem + s * C::STAGE_BYTES;
           const int64_t cb0 = ti.sf_tile0 + (int64_t)ks * C::SF_TILES;
@@ -997,6 +1111,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
           __syncwarp();
         }
       }
+      if (!alive) report_timeout(abort_flag, 11);
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------
@@ -1012,8 +1127,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
       long long pk_mma = 0, pk_bar = 0, pk_n = 0;
       const long long pk_t0 = clock64();
 #endif
-      for (int64_t tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-        const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+      for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
+        const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
         if (ti.skip) continue;
         const uint32_t acc = tile_it % C::ACC_STAGES;
         const uint32_t d_tmem = tmem_base + acc * BN;
@@ -1069,20 +1184,19 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
     if (leader) {
       uint32_t it = 0, tile_it = 0;
       bool alive = true;
-      for (int64_t tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-        const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+      for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
+        const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
         if (ti.skip) continue;
-        bool ok = mbar_wait(&acc_empty[tile_it % C::ACC_STAGES], ((tile_it / C::ACC_STAGES) & 1) ^ 1, abort_flag, 12,
-                            args.wait_ns);
+        const bool drained = mbar_wait_tight(smem_u32(&acc_empty[tile_it % C::ACC_STAGES]),
+                                             ((tile_it / C::ACC_STAGES) & 1) ^ 1, abort_addr, limit);
         for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
           const int s = it % C::STAGES;
-          ok = ok && mbar_wait(&full_bar[s], (it / C::STAGES) & 1, abort_flag, 13, args.wait_ns);
-          ok = ok && mbar_wait(&sf_full[s], (it / C::STAGES) & 1, abort_flag, 15, args.wait_ns);
-          const bool failed = !__all_sync(0xFFFFFFFFu, ok);
-          if (named_barrier_or(1 + s, 64, failed)) { alive = false; break; }
+          const bool ok = mbar_wait2_tight(smem_u32(&full_bar[s]), smem_u32(&sf_full[s]), (it / C::STAGES) & 1, abort_addr, limit);
+          if (named_barrier_or(1 + s, 64, !(ok && drained))) { alive = false; break; }
         }
         ++tile_it;
       }
+      if (!alive) report_timeout(abort_flag, 12);
     }
   }  // warp 3 idles: it completes warpgroup 0
   } else if (warp < 8) {
@@ -1091,17 +1205,17 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
     uint32_t it = 0;
     bool alive = true;
-    for (int64_t tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+    for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
+      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
       if (ti.skip) continue;
       for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
         const int s = it % C::STAGES;
-        if (!mbar_wait(&sfs_full[s], (it / C::STAGES) & 1, abort_flag, 16, args.wait_ns)) { alive = false; break; }
+        if (!mbar_wait_tight(smem_u32(&sfs_full[s]), (it / C::STAGES) & 1, abort_addr, limit)) { alive = false; break; }
         if (C::SF_SLOTS < C::STAGES && it >= (uint32_t)C::SF_SLOTS) {
           // fewer scale slots than operand stages: the slot is free once the MMAs that read it have
           // completed, which is what frees the operand stage of that earlier step as well
           const uint32_t prev = it - C::SF_SLOTS;
-          if (!mbar_wait(&empty_bar[prev % C::STAGES], (prev / C::STAGES) & 1, abort_flag, 17, args.wait_ns)) {
+          if (!mbar_wait_tight(smem_u32(&empty_bar[prev % C::STAGES]), (prev / C::STAGES) & 1, abort_addr, limit)) {
             alive = false;
             break;
           }
@@ -1129,6 +1243,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
         }
       }
     }
+    if (!alive) report_timeout(abort_flag, 16);
   } else {
     // ------------------------------ epilogue (each CTA stores its own 128 rows) ------------------------------
     // Warps 8-11 drain the first half of the accumulator's columns, warps 12-15 the second half; a
@@ -1156,14 +1271,17 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
     const uint32_t my_row = smem_u32(epi_warp) + (uint32_t)lane * (uint32_t)UNIT_BYTES;
     const uint32_t sw = UNIT_BYTES == 128 ? (uint32_t)(lane & 7) : (uint32_t)((lane >> 1) & 3);
     uint32_t tile_it = 0, store_it = 0;
-    for (int64_t tile = pair; tile < n_tiles; tile += n_pairs) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, tiles_m, tiles_n, k_stages);
+    for (int tile = pair; tile < n_tiles; tile += n_pairs) {
+      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
       const int64_t row0 = (ti.mb * 2 + rank) * BM + quad * 32;
       const int64_t col_base = ti.nb * BN + half * HC;
       uint32_t r[HC];
       if (!ti.skip) {
         const uint32_t acc = tile_it % C::ACC_STAGES;
-        if (!mbar_wait(&acc_full[acc], (tile_it / C::ACC_STAGES) & 1, abort_flag, 14, args.wait_ns)) break;
+        if (!mbar_wait_tight(smem_u32(&acc_full[acc]), (tile_it / C::ACC_STAGES) & 1, abort_addr, limit)) {
+          report_timeout(abort_flag, 14);
+          break;
+        }
         tc_fence_after();
         if (!ALTOB200_DBG(args, 8)) {
           const uint32_t t_acc = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN + half * HC;
@@ -1429,6 +1547,17 @@ static int pair_tile_n() {
   return v;
 }
 
+// Raster of the tiles, `group` row tiles a group (at most all): same number of groups, near-equal sizes.
+static void set_raster(GemmArgs* g, int64_t tiles_m, int64_t tiles_n, int64_t group) {
+  const int64_t n_groups = ceil_div(tiles_m, group);
+  const int64_t gm = ceil_div(tiles_m, n_groups);
+  g->group_m = (int)gm;
+  g->per_batch = make_tile_div(tiles_m * tiles_n);
+  g->per_group = make_tile_div(gm * tiles_n);
+  g->rows_full = make_tile_div(gm);
+  g->rows_last = make_tile_div(tiles_m - (ceil_div(tiles_m, gm) - 1) * gm);
+}
+
 static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N, int64_t K, int32_t num_experts,
                        const void* a_codes, const void* a_scales, const void* b_codes, const void* b_scales,
                        const int32_t* group_expert, const float* alpha_a, const float* alpha_b,
@@ -1500,10 +1629,7 @@ static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N,
     if (gm_env > 0) gm = gm_env;
     if (gm < 1) gm = 1;
     if (gm > tiles_m) gm = tiles_m;
-    // even out the groups: same number of groups, near-equal sizes
-    const int64_t n_groups = ceil_div(tiles_m, gm);
-    gm = ceil_div(tiles_m, n_groups);
-    g.group_m = (int)gm;
+    set_raster(&g, tiles_m, ceil_div(N, BN), gm);
   }
   g.wait_ns = wait_limit_ns();
   for (int j = 0; j < 4; ++j) {
@@ -1622,15 +1748,7 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   g.k_offs = k_offs; g.num_batches = (int)batches;
   {
     const int64_t tiles_m = ceil_div(M, BM);
-    int64_t gm = 8;
-    if (gm > tiles_m) gm = tiles_m;
-    const int64_t n_groups = ceil_div(tiles_m, gm);
-    g.group_m = (int)ceil_div(tiles_m, n_groups);
-    const int64_t tiles_n = ceil_div(N, BN);
-    m.per_batch = make_tile_div(tiles_m * tiles_n);
-    m.per_group = make_tile_div(g.group_m * tiles_n);
-    m.rows_full = make_tile_div(g.group_m);
-    m.rows_last = make_tile_div(tiles_m - (ceil_div(tiles_m, g.group_m) - 1) * g.group_m);
+    set_raster(&g, tiles_m, ceil_div(N, BN), tiles_m < 8 ? tiles_m : 8);
   }
   g.wait_ns = wait_limit_ns();
   for (int j = 0; j < 4; ++j)
