@@ -57,6 +57,8 @@ EXPORTED_SYMBOLS = (
     "altob200_swiglu_backward",
     "altob200_dge_scale",
     "altob200_deosc_accumulate",
+    "altob200_linear_backward_work_bytes",
+    "altob200_linear_backward",
     "altob200_gemm_blockscaled",
     "altob200_grouped_gemm_blockscaled",
     "altob200_grouped_gemm_wgrad_blockscaled",
@@ -126,6 +128,15 @@ class MacroScaleDesc(C.Structure):
     ]
 
 
+class LinearBackwardArgs(C.Structure):
+    """``altob200_linear_backward_args`` of the header."""
+    _fields_ = [(n, C.c_int64) for n in ("M", "K", "N", "ld")] + [
+        (n, C.c_void_p) for n in ("dy", "xm_codes", "xm_scales", "wt_codes", "wt_scales", "xm_outer", "wt_outer", "dx", "dw",
+                                  "scratch")] + [
+        ("rht_perm", C.POINTER(C.c_int32)), ("rht_sign", C.POINTER(C.c_int32)), ("sr_words", C.c_uint64 * 4)] + [
+        (n, C.c_int32) for n in ("format", "dtype", "use_outer", "use_sr", "rht_n")]
+
+
 class Altob200Error(RuntimeError):
     def __init__(self, status: int, where: str):
         self.status = status
@@ -174,6 +185,10 @@ def _declare_more(lib):
     lib.altob200_grouped_gemm_wgrad_blockscaled.restype = C.c_int
     lib.altob200_grouped_gemm_wgrad_blockscaled.argtypes = [i32, i32, i64, i64, i64, i32, vp, vp, vp, vp, vp, vp, vp,
                                                             i32, vp, i64, vp]
+    lib.altob200_linear_backward_work_bytes.restype = i64
+    lib.altob200_linear_backward_work_bytes.argtypes = [C.POINTER(LinearBackwardArgs)]
+    lib.altob200_linear_backward.restype = C.c_int
+    lib.altob200_linear_backward.argtypes = [C.POINTER(LinearBackwardArgs), vp, vp]
     lib.altob200_macro_block_scaling.restype = C.c_int
     lib.altob200_macro_block_scaling.argtypes = [vp, i32, i64, i64, i64, i32, vp, vp, vp]
     lib.altob200_macro_block_descaling.restype = C.c_int
@@ -243,7 +258,7 @@ def _check(status: int, where: str) -> None:
 
 def _stream() -> int:
     # the handle alone: building a torch.cuda.Stream object per launch cost a fifth of a small step's host time
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -302,29 +317,40 @@ class Rht:
 CLIP_MODES = {"none": 0, "static": 1, "dynamic": 2}
 
 
-def _params(fmt, x, rounding, outer_scale, rand_bits, rht: Optional[Rht], flags, philox=(0, 0),
-            clip_mode: str = "none", use_uos: bool = False, rand_tile=(0, 0), macro_codes=None) -> QuantParams:
+@functools.lru_cache(maxsize=512)
+def _params_template(fmt: int, dtype: torch.dtype, rounding: int, flags: int, clip_mode: str, use_uos: bool,
+                     rand_tile: tuple) -> bytes:
+    """The fields that are neither pointers nor seeds; copying them takes half the time of setting them."""
     p = QuantParams()
-    p.macro_codes = _ptr(macro_codes)
-    if macro_codes is not None:
-        flags |= SCALE_MACRO
     p.clip_mode = CLIP_MODES[clip_mode]
     p.use_uos = 1 if use_uos else 0
     p.rand_tile_rows, p.rand_tile_pairs = int(rand_tile[0]), int(rand_tile[1])
     p.format = fmt
-    p.in_dtype = _dt(x.dtype)
+    p.in_dtype = _dt(dtype)
     p.rounding = rounding
     p.scale_flags = flags
-    p.outer_scale = _ptr(outer_scale)
-    p.rand_bits = _ptr(rand_bits)
-    p.philox_seed = int(philox[0]) & 0xFFFFFFFFFFFFFFFF
-    p.philox_offset = int(philox[1]) & 0xFFFFFFFFFFFFFFFF
+    return bytes(p)
+
+
+def _params(fmt, x, rounding, outer_scale, rand_bits, rht: Optional[Rht], flags, philox=(0, 0),
+            clip_mode: str = "none", use_uos: bool = False, rand_tile=(0, 0), macro_codes=None) -> QuantParams:
+    if macro_codes is not None:
+        flags |= SCALE_MACRO
+    p = QuantParams.from_buffer_copy(_params_template(fmt, x.dtype, rounding, flags, clip_mode, bool(use_uos),
+                                                      tuple(rand_tile)))
+    if macro_codes is not None:
+        p.macro_codes = macro_codes.data_ptr()
+    if outer_scale is not None:
+        p.outer_scale = outer_scale.data_ptr()
+    if rand_bits is not None:
+        p.rand_bits = rand_bits.data_ptr()
+    if philox != (0, 0):
+        p.philox_seed = int(philox[0]) & 0xFFFFFFFFFFFFFFFF
+        p.philox_offset = int(philox[1]) & 0xFFFFFFFFFFFFFFFF
     if rht is not None:
         p.rht_n = rht.n
         p.rht_perm = rht._perm_c
         p.rht_sign = rht._sign_c
-    else:
-        p.rht_n = 0
     return p
 
 
@@ -604,6 +630,37 @@ def gemm_blockscaled(fmt_a, fmt_b, M, N, K, a_codes, a_scales, b_codes, b_scales
                                            b_codes.data_ptr(), b_scales.data_ptr(), _ptr(alpha_a), _ptr(alpha_b),
                                            _dt(out.dtype), out.data_ptr(), out.stride(0), _stream()),
            "altob200_gemm_blockscaled")
+
+
+def linear_backward(fmt, dims, dy, xm, wt, need_dx: bool, need_dw: bool, scratch, words, rht: Optional[Rht]):
+    """(dX, dW) of a dense linear by ``altob200_linear_backward``: dy [M, N], xm / wt = (codes, scales, outer or None)
+    of X along M and W along N, ``scratch`` as in ``amax`` (None: no outer scales), ``words`` the seeds and offsets of
+    stochastic rounding (None: nearest)."""
+    _require_cuda(dy, *xm, *wt, scratch)
+    assert dy.dim() == 2 and dy.stride(1) == 1
+    M, K, N = dims
+    assert dy.shape[0] == M and dy.shape[1] == N
+    a = LinearBackwardArgs()
+    a.M, a.K, a.N, a.ld, a.format, a.dtype = M, K, N, dy.stride(0), fmt, _dt(dy.dtype)
+    a.dy = dy.data_ptr()
+    dx = dw = None
+    if need_dx:
+        dx = torch.empty(M, K, dtype=dy.dtype, device=dy.device)
+        a.dx, a.wt_codes, a.wt_scales, a.wt_outer = dx.data_ptr(), wt[0].data_ptr(), wt[1].data_ptr(), _ptr(wt[2])
+    if need_dw:
+        dw = torch.empty(N, K, dtype=dy.dtype, device=dy.device)
+        a.dw, a.xm_codes, a.xm_scales, a.xm_outer = dw.data_ptr(), xm[0].data_ptr(), xm[1].data_ptr(), _ptr(xm[2])
+    if scratch is not None:
+        a.use_outer, a.scratch = 1, scratch.data_ptr()
+    if words is not None:
+        a.use_sr = 1
+        a.sr_words[:] = words
+    if rht is not None:
+        a.rht_n, a.rht_perm, a.rht_sign = rht.n, rht._perm_c, rht._sign_c
+    handle = lib()
+    work = torch.empty(handle.altob200_linear_backward_work_bytes(a), dtype=torch.uint8, device=dy.device)
+    _check(handle.altob200_linear_backward(a, work.data_ptr(), _stream()), "altob200_linear_backward")
+    return dx, dw
 
 
 def grouped_gemm_blockscaled(fmt_a, fmt_b, M, N, K, num_experts, a_codes, a_scales, b_codes, b_scales,

@@ -90,7 +90,7 @@ def quantize(x: torch.Tensor, fmt: int, axis: int, is_2d: bool, *, outer_scale: 
         return codes.view(_CODE_DTYPE[fmt]), scales
 
     if a == -1:
-        x2 = x.reshape(-1, N)
+        x2 = x if x.dim() == 2 else x.reshape(-1, N)
         if x2.stride(-1) != 1 or (x2.stride(0) * x2.element_size()) % 16 != 0:
             x2 = x2.contiguous()
         R = x2.shape[0]
@@ -105,8 +105,11 @@ def quantize(x: torch.Tensor, fmt: int, axis: int, is_2d: bool, *, outer_scale: 
         else:
             L.quantize_rowwise(x2, fmt, codes, scales, None, rounding=rounding, outer_scale=outer_scale,
                                rand_bits=_rand_planes(rand_bits, R, N), philox=philox, **opts)
-        return (codes.reshape(*x.shape[:-1], codes.shape[-1]).view(_CODE_DTYPE[fmt]),
-                scales.reshape(*x.shape[:-1], N // block))
+        if not fp4:
+            codes = codes.view(_CODE_DTYPE[fmt])
+        if x.dim() == 2:
+            return codes, scales
+        return codes.reshape(*x.shape[:-1], codes.shape[-1]), scales.reshape(*x.shape[:-1], N // block)
 
     # axis = -2: blocks of consecutive rows; physical output is the transposed matrix
     x3 = x.reshape(-1, M, N)
@@ -149,6 +152,17 @@ def dequantize(codes: torch.Tensor, scales: torch.Tensor, fmt: int, axis: int, i
     block = L.block_of(fmt)
     fp4 = L.is_fp4(fmt)
     a = _norm_axis(axis, codes.dim())
+    osc = None if outer_scale is None else outer_scale.to(device=codes.device, dtype=torch.float32).reshape(1)
+    if a == -1 and codes.dim() == 2 and scales.dim() == 2:
+        # (a matrix as it is: the views below took two thirds of a small call's host time)
+        rows, cols = codes.shape[0], codes.shape[1] * (2 if fp4 else 1)
+        s2 = scales.reshape(rows // block if is_2d else rows, cols // block).contiguous()
+        if fmt == L.FMT_NVFP4:
+            s2 = s2.float()
+        c2 = codes.contiguous()
+        out = torch.empty(rows, cols, dtype=out_dtype, device=codes.device)
+        L.dequantize(c2, s2, fmt, is_2d, rows, cols, out, osc, static_clip)
+        return out
     c = codes.transpose(a, -1)
     s = scales.transpose(a, -1)
     shp = c.shape
@@ -162,7 +176,6 @@ def dequantize(codes: torch.Tensor, scales: torch.Tensor, fmt: int, axis: int, i
     if fmt == L.FMT_NVFP4:
         s3 = s3.float()
     out = torch.empty(c3.shape[0], c3.shape[1], cols, dtype=out_dtype, device=codes.device)
-    osc = None if outer_scale is None else outer_scale.to(device=codes.device, dtype=torch.float32).reshape(1)
     for b in range(c3.shape[0]):
         L.dequantize(c3[b], s3[b], fmt, is_2d, c3.shape[1], cols, out[b], osc, static_clip)
     return out.reshape(*shp[:-1], cols).transpose(a, -1)

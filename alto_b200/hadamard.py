@@ -85,6 +85,19 @@ def random_hadamard_matrix(size: int, dtype=torch.float32, device="cpu", gen: Op
     return Q.unsqueeze(1) * Ht
 
 
+_SIGNED_SYLVESTER = {}
+
+
+def _signed_sylvester_16() -> Optional[Tensor]:
+    """The first column of the base matrix of size 16 if its rows are those of the Sylvester matrix up to sign, else
+    None: what makes a row-signed base matrix fusable, and the signs its rows already have."""
+    base = _base_matrix_t(16)
+    if _SIGNED_SYLVESTER.get("base") is not base:
+        w = base.float()
+        _SIGNED_SYLVESTER.update(base=base, first=w[:, 0] if torch.equal(w[:, :1] * w, _SYLVESTER_16) else None)
+    return _SIGNED_SYLVESTER["first"]
+
+
 class HadamardFactory:
     """Class-level configuration and construction of :class:`HadamardTransform`."""
 
@@ -109,6 +122,12 @@ class HadamardFactory:
 
     @classmethod
     def create_transform(cls, device) -> "HadamardTransform":
+        if cls.randomized and cls._create_weight.__func__ is HadamardFactory._create_weight.__func__:
+            # the draws of random_hadamard_matrix; the product with the base matrix waits until it is asked for,
+            # since the fused kernels take the signs (32 us of a small linear's forward)
+            signs = torch.randint(low=0, high=2, size=(cls.block_size,), generator=cls.generator, dtype=cls.dtype) * 2 - 1
+            _base_matrix_t(cls.block_size)      # sizes that cannot be built are refused here
+            return HadamardTransform(None, cls._create_permutation(signs), signs)
         weight = cls._create_weight(device)
         perm = cls._create_permutation(weight) if cls.randomized else None
         return HadamardTransform(weight, perm)
@@ -125,18 +144,30 @@ class HadamardFactory:
 
 
 class HadamardTransform:
-    """``weight``: n x n (+-1) matrix; ``perm``: optional permutation applied to its rows and columns."""
+    """``weight``: n x n (+-1) matrix; ``perm``: optional permutation applied to its rows and columns.  ``signs``: in
+    the place of ``weight``, the signs of the rows of the base matrix of their number."""
 
-    def __init__(self, weight: Tensor, perm: Optional[Tensor]):
-        self.weight = weight
+    def __init__(self, weight: Optional[Tensor], perm: Optional[Tensor], signs: Optional[Tensor] = None):
+        self._weight = weight
+        self._signs = signs
         self.perm = perm
         self._rht: Optional[L.Rht] = None
         self._fusable: Optional[bool] = None
         self._dev = {}
 
     @property
+    def weight(self) -> Tensor:
+        if self._weight is None:
+            self._weight = self._signs.unsqueeze(1) * _base_matrix_t(self._signs.numel()).to(self._signs.dtype)
+        return self._weight
+
+    @weight.setter
+    def weight(self, value: Tensor) -> None:
+        self._weight = value
+
+    @property
     def n(self) -> int:
-        return int(self.weight.size(0))
+        return int(self._signs.numel() if self._weight is None else self._weight.size(0))
 
     def matrix(self) -> Tensor:
         w = self.weight
@@ -151,7 +182,9 @@ class HadamardTransform:
         goes through the dense transform kernel followed by a plain quantizer."""
         if self._fusable is None:
             ok = self.n == 16
-            if ok:
+            if ok and self._weight is None:
+                ok = _signed_sylvester_16() is not None
+            elif ok:
                 w = self.weight.detach().float().cpu()
                 ok = bool(torch.equal(w[:, :1] * w, _SYLVESTER_16))
             self._fusable = ok
@@ -164,9 +197,9 @@ class HadamardTransform:
                 raise NotImplementedError("this Hadamard matrix is not a row-signed Sylvester matrix of size 16; "
                                           "use the transform itself (dense kernel)")
             n = self.n
-            sign = self.weight.detach().float().cpu()[:, 0]
+            sign = self._signs * _signed_sylvester_16() if self._weight is None else self.weight.detach().float().cpu()[:, 0]
             perm = self.perm.cpu().tolist() if self.perm is not None else list(range(n))
-            self._rht = L.Rht(n, perm, [int(v) for v in sign.tolist()])
+            self._rht = L.Rht(n, perm, sign.tolist())
         return self._rht
 
     def device_matrix(self, device) -> Tensor:

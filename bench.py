@@ -240,13 +240,13 @@ class KernelTimer:
 
         setattr(mod, name, wrapped)
 
-    def count(self, mod, name):
-        """Counts launches of a wrapper whose kernel is too small to be worth timing."""
+    def count(self, mod, name, launches=lambda *a, **kw: 1):
+        """Counts the launches of a wrapper that is not timed: its kernel is too small, or it makes several."""
         orig = getattr(mod, name)
         timer = self
 
         def wrapped(*a, **kw):
-            timer.launches += 1
+            timer.launches += launches(*a, **kw)
             return orig(*a, **kw)
 
         setattr(mod, name, wrapped)
@@ -292,6 +292,9 @@ def run_ours(args):
     timer.wrap(L, "gemm_mxfp4_two_level", "gemm", lambda m, n, k, *a, **kw: 2.0 * m * n * k)
     timer.count(L, "philox_tile")   # the two 16 KB random-word tables of a step's stochastic-rounding quantizers
     timer.count(L, "philox_slots")
+    # a backward behind one call: amax with outer scales, per gradient a quantizer, its word table and a GEMM
+    timer.count(L, "linear_backward", lambda fmt, dims, dy, xm, wt, need_dx, need_dw, scratch, words, rht:
+                (scratch is not None) + (need_dx + need_dw) * (2 + (words is not None)))
 
     g = torch.Generator(device=dev).manual_seed(rank)
     gw = torch.Generator(device=dev).manual_seed(12345)  # identical weights on every rank
@@ -343,16 +346,17 @@ def run_ours(args):
     value = world * FLOPS_PER_STEP * args.steps / (ms * 1e-3) / 1e12
 
     # ---- per-kernel timing pass (events around every launch; not part of the headline) ----
-    # The quantizer/GEMM stream overlap is switched off here so that every kernel is timed alone.
+    # The quantizer/GEMM stream overlap and the backward behind one call are switched off here so that every kernel
+    # is timed alone.
     from alto_b200 import _linear as E
-    overlap = E.OVERLAP
-    E.OVERLAP = False
+    overlap, one_call = E.OVERLAP, E.one_call_backward
+    E.OVERLAP, E.one_call_backward = False, lambda *a: False
     timer.enabled = True
     for _ in range(args.steps):
         step()
     torch.cuda.synchronize()
     timer.enabled = False
-    E.OVERLAP = overlap
+    E.OVERLAP, E.one_call_backward = overlap, one_call
     fam = timer.summary()
     kernels = {}
     for name, d in fam.items():

@@ -428,6 +428,31 @@ int altob200_gemm_blockscaled(int32_t format_a, int32_t format_b, int64_t M, int
                               int32_t out_dtype, void* d, int64_t ldd, void* stream);
 
 /*
+ * Backward pass of a dense linear y = x w^T whose forward kept X along M and W along N, behind one call:
+ * amax of dY (use_outer), the two quantizers of dY with their tables of random words, dX = dYq Wq and
+ * dW = dYq^T Xq, in the order and with the arguments of the single entry points
+ * (alto/kernels/fp4/nvfp4/nvfp_linear.py:160-278, alto/kernels/fp4/mxfp4/mxfp_linear.py:431-570,
+ * alto/kernels/mxfp8/mxfp8_linear.py:378-439; 1-D activation blocks, no clip mode, upward scales or DGE factor).
+ * dY [M, N] with leading dimension ld; dX [M, K] and dW [N, K] contiguous, of dY's type; a NULL dx or dw
+ * leaves that gradient and the operand only it needs out.  `work`: device memory of
+ * altob200_linear_backward_work_bytes, 16-byte aligned.
+ */
+typedef struct altob200_linear_backward_args {
+  int64_t M, K, N, ld;
+  const void* dy;
+  const void *xm_codes, *xm_scales; /* [K, M] and its packed scales */
+  const void *wt_codes, *wt_scales; /* [K, N] and its packed scales */
+  const float *xm_outer, *wt_outer; /* use_outer: their outer scales */
+  void *dx, *dw;
+  void* scratch;                    /* use_outer: of altob200_amax */
+  const int32_t *rht_perm, *rht_sign;
+  uint64_t sr_words[4];             /* use_sr: seed and offset of dY along N, then along M */
+  int32_t format, dtype, use_outer, use_sr, rht_n;
+} altob200_linear_backward_args;
+int64_t altob200_linear_backward_work_bytes(const altob200_linear_backward_args* args);
+int altob200_linear_backward(const altob200_linear_backward_args* args, void* work, void* stream);
+
+/*
  * Grouped (MoE) variant: rows of A are grouped in runs of 128 that share one
  * expert; `group_expert[g]` (device int32, length ceil(M/128), -1 = padding rows that
  * produce zeros) selects B[e] of shape [N, K].  Replaces

@@ -1,0 +1,43 @@
+"""The drawn signs of a transform against the matrix they stand for."""
+import pytest
+import torch
+
+from alto_b200 import hadamard as H
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("size", [16, 32, 64])
+def test_signs_and_matrix_agree(size, dtype):
+    state = {k: getattr(H.HadamardFactory, k) for k in ("block_size", "randomized", "dtype", "seed")}
+    try:
+        H.HadamardFactory.configure(block_size=size, randomized=True, dtype=dtype, seed=11)
+        drawn = H.HadamardFactory.create_transform("cpu")
+        after = H.HadamardFactory.generator.get_state()
+        gen = torch.Generator().manual_seed(11)
+        weight = H.random_hadamard_matrix(size, dtype, "cpu", gen)
+        perm = torch.randperm(size, generator=gen)
+        assert torch.equal(gen.get_state(), after) and torch.equal(perm, drawn.perm)
+        plain = H.HadamardTransform(weight, perm)
+        assert drawn.n == plain.n == size and drawn.is_fused == plain.is_fused == (size == 16)
+        if drawn.is_fused:
+            a, b = drawn.device_params(), plain.device_params()
+            assert (a.n, a.perm, a.sign) == (b.n, b.perm, b.sign) and all(isinstance(v, int) for v in a.sign)
+        assert torch.equal(drawn.weight, weight) and drawn.weight.dtype == dtype
+        assert torch.equal(drawn.matrix(), plain.matrix())
+        drawn.weight = torch.ones(size, size)          # a matrix put in by hand counts
+        again = H.HadamardTransform(None, perm, torch.ones(size))
+        again.weight = torch.ones(size, size)
+        assert not again.is_fused and torch.equal(again.matrix(), torch.ones(size, size))
+    finally:
+        for k, v in state.items():
+            setattr(H.HadamardFactory, k, v)
+
+
+def test_sizes_that_cannot_be_built_are_refused_when_drawn():
+    state = H.HadamardFactory.block_size
+    try:
+        H.HadamardFactory.configure(block_size=6, randomized=True)
+        with pytest.raises(ValueError):
+            H.HadamardFactory.create_transform("cpu")
+    finally:
+        H.HadamardFactory.block_size = state
