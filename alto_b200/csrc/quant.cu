@@ -1041,9 +1041,10 @@ __global__ void __launch_bounds__(WARPS_2D * 32, ROUND == ALTOB200_ROUND_RTN ? 5
   constexpr int PER = MACRO ? 2 : 1;   // warp tiles per counted tile in either direction
   const int64_t tiles_c = (a.cols + TC * PER - 1) / (TC * PER), tiles_r = (a.rows + TR * PER - 1) / (TR * PER);
   const int64_t warp_all = (int64_t)blockIdx.x * WARPS_2D + (threadIdx.x >> 5);
-  const int64_t tile_all = MACRO ? warp_all >> 2 : warp_all;
+  // from the end, where the pass before (the maximum of the tensor) left what L2 holds
+  const int64_t tile_all = tiles_c * tiles_r * a.batch - 1 - (MACRO ? warp_all >> 2 : warp_all);
   // (whole warps leave, with MACRO whole CTAs)
-  if (tile_all >= tiles_c * tiles_r * a.batch) return;
+  if (tile_all < 0) return;
   // matrix `bi` of the batch: its outputs follow those of matrix bi - 1, so the batch index enters the
   // addresses as extra rows (bi * rows for the K packing, bi * cols for the transposed one)
   // (BATCHED is a template parameter so that the single-matrix kernel carries none of this arithmetic)
@@ -1319,6 +1320,7 @@ __global__ void __launch_bounds__(WARPS_2D * 32, ROUND == ALTOB200_ROUND_RTN ? 5
 // =======================================================================================
 struct AmaxArgs {
   const void* x;
+  int32_t steps;         // loads of a thread in a row, up to LOADS: as many as leave no block without work
   int64_t rows, cols, ld;
   uint32_t* amax_bits;   // [2], written by the last block
   float* outer_scale;    // [2] or NULL
@@ -1335,7 +1337,10 @@ __device__ __forceinline__ float outer_from_amax_bits(uint32_t bits) {
   return fmaxf(__fdiv_rn(amax, 2688.0f), 1.0e-30f);
 }
 
-template <bool IN_BF16, bool RHT>
+// LOADS: 16-byte loads of a thread in flight (without RHT).  Eight of them, neighbours of a block, where there is work
+// for all: 117 MB of bf16 24.0 us, 268 MB 54.9, where four a grid's width apart took 26.7 and 58.3.  Four where a
+// block has fewer, which leaves room for eight blocks on an SM: 4 MB 5.2 us, 6.9 with eight.
+template <bool IN_BF16, bool RHT, int LOADS = 1>
 __global__ void __launch_bounds__(256) amax_kernel(AmaxArgs a) {
   grid_dependency_wait();
   __shared__ uint32_t s_red[2][8];
@@ -1356,19 +1361,19 @@ __global__ void __launch_bounds__(256) amax_kernel(AmaxArgs a) {
       }
       return __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint8_t*>(a.x) + off * (IN_BF16 ? 2 : 4)));
     };
-    // four independent 16-byte loads are issued before any of them is consumed: the pass is a pure
-    // stream and needs bytes in flight, not arithmetic
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (; i0 < total; i0 += 4 * stride) {
-      uint4 wv[4];
+    // the loads are issued before any of them is consumed: the pass is a pure stream and needs bytes in flight,
+    // not arithmetic
+    constexpr int U = LOADS;
+    const int64_t chunk = a.steps * 256;
+    for (int64_t b = blockIdx.x * chunk + threadIdx.x; b < total; b += gridDim.x * chunk) {
+      uint4 wv[U];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t i = i0 + u * stride;
-        wv[u] = i < total ? load(i) : make_uint4(0u, 0u, 0u, 0u);
+      for (int u = 0; u < U; ++u) {
+        const int64_t i = b + u * 256;
+        wv[u] = u < a.steps && i < total ? load(i) : make_uint4(0u, 0u, 0u, 0u);
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < U; ++u) {
       const uint4 w = wv[u];
       if (IN_BF16) {
         const uint32_t acc = absmax2_bf16x2(absmax2_bf16x2(0, w.x, w.y), w.z, w.w);
@@ -2155,13 +2160,16 @@ int altob200_amax(const void* x, int32_t in_dtype, int64_t rows, int64_t cols, i
   int64_t blocks = work;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
+  const int64_t steps = ceil_div(rows * (cols * esz / 16), blocks * 256);
+  a.steps = (int32_t)(steps < 8 ? (steps < 4 ? steps : 4) : 8);
   const bool bf = in_dtype == ALTOB200_DT_BF16;
   if (rht_n) {
     if (bf) (void)launch_after(amax_kernel<true, true>, dim3((unsigned)blocks), dim3(256), 0, st, a);
     else (void)launch_after(amax_kernel<false, true>, dim3((unsigned)blocks), dim3(256), 0, st, a);
   } else {
-    if (bf) (void)launch_after(amax_kernel<true, false>, dim3((unsigned)blocks), dim3(256), 0, st, a);
-    else (void)launch_after(amax_kernel<false, false>, dim3((unsigned)blocks), dim3(256), 0, st, a);
+    const auto kernel = a.steps == 8 ? (bf ? amax_kernel<true, false, 8> : amax_kernel<false, false, 8>)
+                                     : (bf ? amax_kernel<true, false, 4> : amax_kernel<false, false, 4>);
+    (void)launch_after(kernel, dim3((unsigned)blocks), dim3(256), 0, st, a);
   }
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }

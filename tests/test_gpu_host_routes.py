@@ -1,4 +1,5 @@
-"""Routes that spare host work against the general ones: the backward behind one call, matrices dequantised as they are."""
+"""Routes that spare host work against the general ones: the backward behind one call, matrices dequantised as they are;
+the maximum of tensors at the sizes where its loads a thread change."""
 import pytest
 import torch
 
@@ -62,3 +63,16 @@ def test_a_matrix_is_dequantised_as_it_is(fmt, is_2d):
             got = Q.dequantize(c, s, fmt, -1, is_2d, dtype, outer)
             want = Q.dequantize(codes[None], scales[None], fmt, -1, is_2d, dtype, outer)[0]
             assert got.dtype == dtype and got.shape == (rows, cols) and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows,cols,pitch", [(1, 8, 8), (37, 2056, 2056), (1200, 8200, 8200), (1187, 8192, 8208), (2411, 8200, 8208),
+                                             (5000, 8200, 8200)])
+def test_maximum_wherever_it_lies(rows, cols, pitch, dtype):
+    # one load a thread, a few, four (1184 blocks of 256 threads and more), eight
+    x = torch.zeros(rows, pitch, dtype=dtype, device="cuda")[:, :cols]
+    bits, outer, scratch = torch.empty(2, dtype=torch.int32, device="cuda"), torch.empty(2, device="cuda"), E.amax_scratch(x.device)
+    for i, (r, c) in enumerate([(0, 0), (rows - 1, cols - 1), (rows // 2, cols // 3), (rows - 1, 0), (0, cols - 1)]):
+        x[r, c] = -(i + 1.5)
+        L.amax(x, bits, outer, scratch)
+        assert bits.view(torch.float32)[0].item() == i + 1.5
