@@ -989,11 +989,92 @@ struct CfgPair {
   static constexpr int HALF_COLS = BN / 2;                    // columns drained by one epilogue warp
   static constexpr int NUM_BARS = 4 * STAGES + 2 * ACC_STAGES;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+  static constexpr int SMEM_BYTES_GROUPED = SMEM_BYTES + 2048 * 4;   // and the list of units
   static_assert(NUM_BARS * 8 + 16 <= 512, "barrier area");
-  static_assert(SMEM_BYTES <= 232448, "shared memory budget");
+  static_assert(SMEM_BYTES_GROUPED <= 232448, "shared memory budget");
 };
 
-template <int KIND, bool OUT_BF16, int BN_>
+// Rows grouped by expert in runs of 128 (GROUPED): a tile of 256 rows can hold rows of two experts.  A unit is 256 rows
+// with one expert's weights; a pair of groups of two experts makes two units, and each CTA stores in the one that is
+// its rows' own (in the other it loads no rows of A; what the MMA makes of the stale ones stays in its own tensor-memory
+// lanes and is dropped).  Word of a unit: pair of groups, CTAs that store the product, CTAs that store zeros (their
+// group has no expert), expert; no CTA that stores the product: nothing is loaded or multiplied.
+struct PairUnit {
+  static constexpr int MAX = 2048;                    // units of a launch (one per group and one more at most)
+  static constexpr int PAIR_BITS = 11, EXPERT_SHIFT = PAIR_BITS + 4, EXPERT_BITS = 16;
+  uint32_t w;
+  __device__ __forceinline__ uint32_t pair() const { return w & ((1u << PAIR_BITS) - 1); }
+  __device__ __forceinline__ uint32_t stores() const { return (w >> PAIR_BITS) & 3u; }
+  __device__ __forceinline__ uint32_t zeros() const { return (w >> (PAIR_BITS + 2)) & 3u; }
+  __device__ __forceinline__ uint32_t expert() const { return w >> EXPERT_SHIFT; }
+  static __device__ __forceinline__ uint32_t make(uint32_t pair, uint32_t stores, uint32_t zeros, uint32_t expert) {
+    return pair | (stores << PAIR_BITS) | (zeros << (PAIR_BITS + 2)) | (expert << EXPERT_SHIFT);
+  }
+};
+
+// The units of a launch in order, by one warp; returns their number.
+__device__ __forceinline__ int list_units(const GemmArgs& args, int lane, uint32_t* units) {
+  const int n_groups = (int)((args.M + 127) >> 7), n_pairs = (n_groups + 1) >> 1;
+  int base = 0;
+  for (int p0 = 0; p0 < n_pairs; p0 += 32) {
+    const int p = p0 + lane;
+    const bool valid = p < n_pairs;
+    const int e0 = valid ? __ldg(args.group_expert + 2 * p) : -1;
+    const int e1 = valid && 2 * p + 1 < n_groups ? __ldg(args.group_expert + 2 * p + 1) : -1;
+    const bool two = e0 >= 0 && e1 >= 0 && e0 != e1;
+    const uint32_t m_two = __ballot_sync(0xFFFFFFFFu, two), below = (1u << lane) - 1;
+    if (valid) {
+      const int at = base + lane + __popc(m_two & below);
+      if (two) {
+        units[at] = PairUnit::make((uint32_t)p, 1u, 0u, (uint32_t)e0);
+        units[at + 1] = PairUnit::make((uint32_t)p, 2u, 0u, (uint32_t)e1);
+      } else {
+        const uint32_t stores = (e0 >= 0 ? 1u : 0u) | (e1 >= 0 ? 2u : 0u);
+        units[at] = PairUnit::make((uint32_t)p, stores, stores ^ 3u, (uint32_t)(e0 >= 0 ? e0 : e1 >= 0 ? e1 : 0));
+      }
+    }
+    const int n_valid = n_pairs - p0 < 32 ? n_pairs - p0 : 32;
+    base += n_valid + __popc(m_two);
+  }
+  return base;
+}
+
+struct PairTile {
+  TileInfo t;
+  uint32_t stores, zeros;   // CTAs (bit = rank)
+};
+template <int KIND, int BN, bool GROUPED>
+__device__ __forceinline__ PairTile decode_pair_tile(const GemmArgs& args, int tile, int k_stages, const uint32_t* units, int n_units) {
+  PairTile p;
+  if constexpr (!GROUPED) {
+    p.t = decode_tile<KIND, BN>(args, tile, k_stages);
+    p.stores = p.t.skip ? 0u : 3u;
+    p.zeros = p.stores ^ 3u;
+  } else {
+    // the raster of tile_coord over units instead of row tiles
+    const uint32_t g = args.per_group.quotient((uint32_t)tile), first = g * (uint32_t)args.group_m;
+    const uint32_t in_group = (uint32_t)tile - g * args.per_group.d, left = (uint32_t)n_units - first;
+    const uint32_t rows = left < (uint32_t)args.group_m ? left : (uint32_t)args.group_m;
+    const uint32_t nb = in_group / rows;
+    const PairUnit u{units[first + in_group - nb * rows]};
+    p.stores = u.stores();
+    p.zeros = u.zeros();
+    p.t.nb = nb;
+    p.t.mb = u.pair();
+    p.t.batch = 0;
+    p.t.k_stages = k_stages;
+    const int64_t tail = args.k_bytes - (int64_t)(k_stages - 1) * STAGE_K_BYTES;
+    p.t.last_mmas = (int)((tail + 31) / 32);
+    p.t.k_byte0 = 0;
+    p.t.sf_tile0 = 0;
+    p.t.b_row0 = (int64_t)nb * BN + (int64_t)u.expert() * args.N;
+    p.t.sfb = args.sfb + (int64_t)u.expert() * args.sfb_expert_stride;
+    p.t.skip = p.stores == 0;
+  }
+  return p;
+}
+
+template <int KIND, bool OUT_BF16, int BN_, bool GROUPED>
 __global__ void __launch_bounds__(NUM_THREADS_PAIR, 1)
 gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                              const __grid_constant__ CUtensorMap tmap_d, const GemmArgs args) {
@@ -1016,7 +1097,9 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
   const uint32_t rank = cluster_ctarank();      // 0 = leader
   const bool leader = rank == 0;
   const int pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
-  const int n_tiles = (int)(args.per_batch.d * (args.k_offs != nullptr ? args.num_batches : 1));   // of 256 rows
+  int n_tiles = (int)(args.per_batch.d * (args.k_offs != nullptr ? args.num_batches : 1));   // of 256 rows
+  uint32_t* const units = reinterpret_cast<uint32_t*>(epi + C::EPI_BYTES + 512);   // GROUPED
+  int n_units = 0;
   const int k_stages = (int)((args.k_bytes + STAGE_K_BYTES - 1) / STAGE_K_BYTES);
   const int64_t n_row_blocks = (args.N + 127) / 128;
 
@@ -1055,6 +1138,16 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
   // barriers, tensor memory and the zeroed scale staging are set up: from here on global memory is read
   // and written, which has to wait for the kernel in front of this one (programmatic dependent launch)
   grid_dependency_wait();
+  if constexpr (GROUPED) {
+    volatile uint32_t* const count = tmem_slot + 2;
+    if (warp == 0) {
+      const int n = list_units(args, lane, units);
+      if (lane == 0) *count = (uint32_t)n;
+    }
+    __syncthreads();
+    n_units = (int)*count;
+    n_tiles = n_units * (int)((args.N + BN - 1) / BN);
+  }
 
   if (warp < 4) {
   setmaxnreg_dec<C::REGS_SMALL>();
@@ -1067,14 +1160,17 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
       uint32_t it = 0;
       bool alive = true;
       for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-        const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
+        const PairTile pt = decode_pair_tile<KIND, BN, GROUPED>(args, tile, k_stages, units, n_units);
+        const TileInfo& ti = pt.t;
         if (ti.skip) continue;
         const int64_t mb = ti.mb * 2 + rank;          // this CTA's 128-row block of A
         const int64_t sfb_blk0 = (ti.nb * BN) >> 7;   // first 128-row block of B scales under this tile
         int nb_valid = (int)(n_row_blocks - sfb_blk0);
         if (nb_valid > C::NB) nb_valid = C::NB;
         // a CTA whose rows of A lie past M has no scale row block to load; its rows are never stored
-        const bool sfa_exists = mb * BM < args.M;
+        const bool own = !GROUPED || ((pt.stores >> rank) & 1u) != 0;
+        const bool sfa_exists = own && mb * BM < args.M;
+        const uint32_t operand_bytes = (GROUPED ? (uint32_t)__popc(pt.stores) : 2u) * C::A_BYTES + 2 * C::B_BYTES;
         const uint8_t* sfa_row = args.sfa + mb * args.nct * 512;
         for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
           const int s = it % C::STAGES;
@@ -1096,10 +1192,10 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
             continue;
           }
           if (elected) {
-            if (leader) mbar_expect_tx(&full_bar[s], 2 * (C::A_BYTES + C::B_BYTES));
+            if (leader) mbar_expect_tx(&full_bar[s], operand_bytes);
             mbar_expect_tx(&sfs_full[s], sf_bytes * ((sfa_exists ? 1 : 0) + nb_valid));
             const uint32_t full_leader = mapa_u32(smem_u32(&full_bar[s]), 0);
-            tma_load_2d_pair(st, &tmap_a, kx, (int32_t)(mb * BM), full_leader);
+            if (own) tma_load_2d_pair(st, &tmap_a, kx, (int32_t)(mb * BM), full_leader);
             tma_load_2d_pair(st + C::A_BYTES, &tmap_b, kx, (int32_t)(ti.b_row0 + rank * (BN / 2)), full_leader);
             if (sfa_exists) bulk_load(st + C::A_BYTES + C::B_BYTES, sfa_row + cb0 * 512, sf_bytes, &sfs_full[s]);
 #pragma unroll
@@ -1128,7 +1224,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
       const long long pk_t0 = clock64();
 #endif
       for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-        const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
+        const PairTile pt = decode_pair_tile<KIND, BN, GROUPED>(args, tile, k_stages, units, n_units);
+        const TileInfo& ti = pt.t;
         if (ti.skip) continue;
         const uint32_t acc = tile_it % C::ACC_STAGES;
         const uint32_t d_tmem = tmem_base + acc * BN;
@@ -1185,7 +1282,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
       uint32_t it = 0, tile_it = 0;
       bool alive = true;
       for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-        const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
+        const PairTile pt = decode_pair_tile<KIND, BN, GROUPED>(args, tile, k_stages, units, n_units);
+        const TileInfo& ti = pt.t;
         if (ti.skip) continue;
         const bool drained = mbar_wait_tight(smem_u32(&acc_empty[tile_it % C::ACC_STAGES]),
                                              ((tile_it / C::ACC_STAGES) & 1) ^ 1, abort_addr, limit);
@@ -1206,7 +1304,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
     uint32_t it = 0;
     bool alive = true;
     for (int tile = pair; tile < n_tiles && alive; tile += n_pairs) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
+      const PairTile pt = decode_pair_tile<KIND, BN, GROUPED>(args, tile, k_stages, units, n_units);
+      const TileInfo& ti = pt.t;
       if (ti.skip) continue;
       for (int ks = 0; ks < ti.k_stages; ++ks, ++it) {
         const int s = it % C::STAGES;
@@ -1272,7 +1371,8 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
     const uint32_t sw = UNIT_BYTES == 128 ? (uint32_t)(lane & 7) : (uint32_t)((lane >> 1) & 3);
     uint32_t tile_it = 0, store_it = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs) {
-      const TileInfo ti = decode_tile<KIND, BN>(args, tile, k_stages);
+      const PairTile pt = decode_pair_tile<KIND, BN, GROUPED>(args, tile, k_stages, units, n_units);
+      const TileInfo& ti = pt.t;
       const int64_t row0 = (ti.mb * 2 + rank) * BM + quad * 32;
       const int64_t col_base = ti.nb * BN + half * HC;
       uint32_t r[HC];
@@ -1297,9 +1397,16 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
         }
         ++tile_it;
         if (ALTOB200_DBG(args, 8)) continue;
-      } else {
+      } else if (!GROUPED) {
 #pragma unroll
         for (int q = 0; q < HC; ++q) r[q] = 0u;
+      }
+      if constexpr (GROUPED) {
+        if ((((pt.stores | pt.zeros) >> rank) & 1u) == 0) continue;   // the rows belong to another unit
+        if (((pt.zeros >> rank) & 1u) != 0) {
+#pragma unroll
+          for (int q = 0; q < HC; ++q) r[q] = 0u;
+        }
       }
 #pragma unroll
       for (int u = 0; u < N_UNITS; ++u) {
@@ -1493,10 +1600,11 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
 }
 
 // CTA-pair kernel: clusters of two CTAs, as many clusters as the device can hold at once.
-template <int KIND, bool OUT_BF16, int BN_>
+template <int KIND, bool OUT_BF16, int BN_, bool GROUPED>
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const GemmArgs& args,
                             cudaStream_t st) {
   using C = CfgPair<KIND, BN_>;
+  constexpr int SMEM = GROUPED ? C::SMEM_BYTES_GROUPED : C::SMEM_BYTES;
   static std::atomic<int> clusters_of[MAX_DEVICES];  // 0 = not asked yet, < 0 = the device cannot run the pair kernel
   const int dev = current_device();
   int max_clusters = dev >= 0 ? clusters_of[dev].load(std::memory_order_relaxed) : 0;
@@ -1509,16 +1617,16 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // see launch_after()
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.blockDim = dim3(NUM_THREADS_PAIR, 1, 1);
-  cfg.dynamicSmemBytes = C::SMEM_BYTES;
+  cfg.dynamicSmemBytes = SMEM;
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
   if (max_clusters == 0) {
-    ALTOB200_CUDA_CHECK(cudaFuncSetAttribute(gemm_blockscaled_pair_kernel<KIND, OUT_BF16, BN_>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    ALTOB200_CUDA_CHECK(cudaFuncSetAttribute(gemm_blockscaled_pair_kernel<KIND, OUT_BF16, BN_, GROUPED>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     cfg.gridDim = dim3(2 * (unsigned)sm_count_gemm(), 1, 1);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_blockscaled_pair_kernel<KIND, OUT_BF16, BN_>, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_blockscaled_pair_kernel<KIND, OUT_BF16, BN_, GROUPED>, &cfg) != cudaSuccess || n <= 0) {
       (void)cudaGetLastError();
       max_clusters = -1;
     } else {
@@ -1528,11 +1636,11 @@ static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const 
   }
   if (max_clusters < 0) return ALTOB200_EUNSUPPORTED;
   const int64_t tiles =
-      ceil_div(args.M, 2 * BM) * ceil_div(args.N, C::BN) * (args.k_offs != nullptr ? args.num_batches : 1);
+      (GROUPED ? ceil_div(args.M, BM) + 1 : ceil_div(args.M, 2 * BM)) * ceil_div(args.N, C::BN) * (args.k_offs != nullptr ? args.num_batches : 1);
   int64_t clusters = max_clusters;
   if (clusters > tiles) clusters = tiles;
   cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_blockscaled_pair_kernel<KIND, OUT_BF16, BN_>, ta, tb, td, args);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_blockscaled_pair_kernel<KIND, OUT_BF16, BN_, GROUPED>, ta, tb, td, args);
   return e == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }
 
@@ -1586,16 +1694,22 @@ static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N,
     return ALTOB200_ELIMIT;
 
   int BN = N <= 128 ? 128 : 256;
-  // The CTA-pair kernel serves dense and K-range problems; rows grouped by expert in runs of 128
-  // could put two experts' rows into one 256-row pair tile, so that mode stays on the single-CTA
-  // kernel.  ALTOB200_GEMM_PAIR=0 forces the single-CTA kernel everywhere.
+  // The CTA-pair kernel takes dense and K-range problems, and rows grouped by expert where an expert has enough of
+  // them (counted with the buffer's padding: 512 a piece).  Pairs of groups with two experts are multiplied twice there:
+  // with 256 rows an expert every second pair is, and the single-CTA kernel is the faster one.
+  // us, pair / single CTA, forward of MXFP8 experts 2880 -> 2880 (and NVFP4), 32 of them: 256 rows an expert 88 / 81
+  // (55 / 50), 384 116 / 118 (72 / 72), 512 136 / 148 (84 / 94); 69 632 rows, 2880 -> 5760: MXFP8 944 / 1144, MXFP4
+  // 518 / 635, NVFP4 562 / 677.  ALTOB200_GEMM_PAIR=0 forces the single-CTA kernel everywhere.
   static int pair_env = -1;
   if (pair_env < 0) {
     const char* e = getenv("ALTOB200_GEMM_PAIR");
     pair_env = e ? atoi(e) : 1;
   }
-  const bool use_pair = pair_env != 0 && num_experts == 0 && N > 128 && M > 128;
-  if (use_pair && pair_tile_n() == 192) BN = 192;
+  const bool grouped = num_experts > 0;
+  const bool units_fit = !grouped || (M >= 512 * (int64_t)num_experts && ceil_div(M, BM) < PairUnit::MAX &&
+                                      num_experts < (1 << PairUnit::EXPERT_BITS));
+  const bool use_pair = pair_env != 0 && units_fit && N > 128 && M > 128;
+  if (use_pair && !grouped && pair_tile_n() == 192) BN = 192;
   const int64_t b_rows = N * (num_experts > 0 ? num_experts : 1);
   CUtensorMap ta, tb;
   int rc = make_tmap(&ta, a_codes, M, k_bytes, BM);
@@ -1646,10 +1760,13 @@ static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N,
   if (use_pair) {
     const bool obf = g.out_bf16 != 0;
 #define LAUNCH_PAIR(KD)                                                                                        \
-  return BN == 192 ? (obf ? launch_gemm_pair<KD, true, 192>(ta, tb, td, g, st)                                \
-                          : launch_gemm_pair<KD, false, 192>(ta, tb, td, g, st))                              \
-                   : (obf ? launch_gemm_pair<KD, true, 256>(ta, tb, td, g, st)                                \
-                          : launch_gemm_pair<KD, false, 256>(ta, tb, td, g, st))
+  if (grouped)                                                                                                 \
+    return obf ? launch_gemm_pair<KD, true, 256, true>(ta, tb, td, g, st)                                      \
+               : launch_gemm_pair<KD, false, 256, true>(ta, tb, td, g, st);                                    \
+  return BN == 192 ? (obf ? launch_gemm_pair<KD, true, 192, false>(ta, tb, td, g, st)                          \
+                          : launch_gemm_pair<KD, false, 192, false>(ta, tb, td, g, st))                        \
+                   : (obf ? launch_gemm_pair<KD, true, 256, false>(ta, tb, td, g, st)                          \
+                          : launch_gemm_pair<KD, false, 256, false>(ta, tb, td, g, st))
     switch (kind) {
       case KIND_NVF4: LAUNCH_PAIR(KIND_NVF4);
       case KIND_MXF4: LAUNCH_PAIR(KIND_MXF4);
