@@ -78,7 +78,9 @@ struct CfgMacro {
   static constexpr int WN = BN / 2;                             // columns of a fold warp
   static constexpr int PIECES = WN / 16;
   static constexpr int FLIGHT = 4;                              // pieces in registers at a time
-  static constexpr int EPI_WARP_BYTES = 4096;                   // 32 rows x 32 columns: two units of bf16, one of fp32
+  // staged units of 32 rows: 64 columns of bf16 where they divide a warp's, else 32; 32 of fp32
+  static constexpr int EPI_COLS = WN % 64 == 0 ? 64 : 32;
+  static constexpr int EPI_WARP_BYTES = 4096;
   static constexpr int EPI_BYTES = FOLD_WARPS * EPI_WARP_BYTES;
   // Ring of reciprocal factors, per chunk 128 rows and BN columns (B_UNIFORM: the products of both, 128 rows per
   // 128 columns).  No barrier guards its reuse: a slot is rewritten FAC_STAGES stages after its last use, once
@@ -653,56 +655,75 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         for (int p = PIECES - FLIGHT; p < PIECES; ++p) fold(p);
       }
       if (odd) slot = slot + SLOT_BYTES == SLOTS_END ? 0u : slot + SLOT_BYTES;   // a stage has two slots
-      // ---- epilogue of the tile: this warp's 32 rows x WN columns, in units of 32 columns ----
-      // (64 bytes a row of bf16 with the 64-byte swizzle, two buffers; 128 bytes of fp32, one)
-      const float os = margs.out_scale;
+      // ---- epilogue of the tile: this warp's 32 rows x WN columns ----
+      // Units of 128 bytes a row in one buffer, or of 64 (32 columns of bf16) in two.  A unit costs 600 cycles beside its
+      // conversions, for the wait for the last store and the proxy fence, so it is as wide as it can be (a warp's 64
+      // columns as two: wgrad of 69 632 rows, 5760 x 2880, in 32 ranges 1508 us).  A row per lane straight to global
+      // memory was slower yet: 378 us for 356, forward at 8192 x 4096 x 14336.
+      // Executed once a tile, this code is not in the instruction caches: its instructions count (1400 to 2500 cycles,
+      // in which the MMAs get no further than the free accumulators).
+      if (margs.out_scale != 1.0f) {
+        const float2 os = make_float2(margs.out_scale, margs.out_scale);
+#pragma unroll
+        for (int j = 0; j < C::WN / 2; ++j) acc[j] = __fmul2_rn(acc[j], os);
+      }
       const bool out_bf16 = args.out_bf16 != 0, failed = *abort_flag != 0;
       uint8_t* const epi_warp = epi + (warp - 8) * C::EPI_WARP_BYTES;
+      constexpr bool NARROW = C::EPI_COLS == 32;          // bf16 units of 64 bytes a row
 #pragma unroll
-      for (int q = 0; q < C::WN / 32; ++q) {
-        if (lane == 0) {                                // the last store has finished reading this buffer
-          if (out_bf16) bulk_wait_read<1>();
+      for (int q = 0; q < C::WN / 32; ++q) {              // 32 columns
+        if (!NARROW && out_bf16 && (q & 1) != 0) continue;
+        if (lane == 0) {                                  // the last store has finished reading this buffer
+          if (NARROW && out_bf16) bulk_wait_read<1>();
           else bulk_wait_read<0>();
         }
         __syncwarp();
-        uint8_t* const unit = epi_warp + (out_bf16 ? (store_it & 1u) * 2048u : 0u);
+        uint8_t* const unit = epi_warp + (NARROW && out_bf16 ? (store_it & 1u) * 2048u : 0u);
         const uint32_t base = smem_u32(unit);
         if constexpr (B_UNIFORM) {
           const uint32_t row = (uint32_t)lane;
           if (out_bf16) {
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
+            for (int g = 0; g < C::EPI_COLS / 8; ++g) {
               uint32_t o[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const float2 v = acc[q * 16 + g * 4 + e];
-                const __nv_bfloat162 p2 = __floats2bfloat162_rn(__fmul_rn(v.x, os), __fmul_rn(v.y, os));
+                const float2 v = acc[(q * 16 + g * 4 + e) % (C::WN / 2)];   // (never beyond: an even q where units have 64)
+                const __nv_bfloat162 p2 = __floats2bfloat162_rn(v.x, v.y);
                 o[e] = *reinterpret_cast<const uint32_t*>(&p2);
               }
-              st_shared_v4(base + row * 64u + ((((uint32_t)g) ^ ((row >> 1) & 3u)) << 4), o[0], o[1], o[2], o[3]);
+              const uint32_t at = NARROW ? row * 64u + ((((uint32_t)g) ^ ((row >> 1) & 3u)) << 4)
+                                         : row * 128u + ((((uint32_t)g) ^ (row & 7u)) << 4);
+              st_shared_v4(base + at, o[0], o[1], o[2], o[3]);
             }
           } else {
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
               const float2 v = acc[q * 16 + g * 2], w = acc[q * 16 + g * 2 + 1];
-              st_shared_v4(base + row * 128u + ((((uint32_t)g) ^ (row & 7u)) << 4), f2u(__fmul_rn(v.x, os)),
-                           f2u(__fmul_rn(v.y, os)), f2u(__fmul_rn(w.x, os)), f2u(__fmul_rn(w.y, os)));
+              st_shared_v4(base + row * 128u + ((((uint32_t)g) ^ (row & 7u)) << 4), f2u(v.x), f2u(v.y), f2u(w.x), f2u(w.y));
             }
           }
         } else {
+          static_assert(B_UNIFORM || !NARROW, "units of per-column factors");
           const uint32_t lr = (uint32_t)(lane >> 2), lc = (uint32_t)(lane & 3);
 #pragma unroll
-          for (int g = 0; g < 8; ++g) {                 // column lc + 4 g of the unit
+          for (int g = 0; g < 16; ++g) {                // column lc + 4 g of the unit
+            if (!out_bf16 && g >= 8) continue;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {               // row lr + 8 e
-              const float2 pair = acc[(q * 2 + (g >> 2)) * 8 + (e >> 1) * 4 + (g & 3)];
-              const float v = __fmul_rn((e & 1) != 0 ? pair.y : pair.x, os);
-              const uint32_t row = lr + 8u * e;
-              if (out_bf16)
-                st_shared_u16(base + row * 64u + ((((uint32_t)g >> 1) ^ ((row >> 1) & 3u)) << 4) + (g & 1) * 8u + lc * 2u,
-                              __bfloat16_as_ushort(__float2bfloat16_rn(v)));
-              else
-                st_shared_u32(base + row * 128u + ((((uint32_t)g) ^ (row & 7u)) << 4) + lc * 4u, f2u(v));
+            for (int h = 0; h < 2; ++h) {               // rows lr + 16 h and + 8
+              const float2 v = acc[((q * 2 + (g >> 2)) * 8 + h * 4 + (g & 3)) % (C::WN / 2)];
+              const uint32_t row_at = base + (lr + 16u * h) * 128u;   // (the swizzle of both rows is that of lr)
+              if (out_bf16) {
+                const __nv_bfloat162 p2 = __floats2bfloat162_rn(v.x, v.y);
+                const uint32_t w = *reinterpret_cast<const uint32_t*>(&p2);
+                const uint32_t at = row_at + ((((uint32_t)g >> 1) ^ lr) << 4) + (g & 1) * 8u + lc * 2u;
+                st_shared_u16(at, (unsigned short)w);
+                st_shared_u16(at + 8u * 128u, (unsigned short)(w >> 16));
+              } else {
+                const uint32_t at = row_at + ((((uint32_t)g) ^ lr) << 4) + lc * 4u;
+                st_shared_u32(at, f2u(v.x));
+                st_shared_u32(at + 8u * 128u, f2u(v.y));
+              }
             }
           }
         }

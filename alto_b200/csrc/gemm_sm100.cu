@@ -1850,7 +1850,7 @@ static int gemm_macro_common(int64_t M, int64_t N, int64_t K, int32_t num_expert
   rc = make_tmap(&tb, b_codes, b_rows, k_bytes, BN);
   if (rc != ALTOB200_OK) return rc;
   rc = make_tmap_out(&td, d, k_offs != nullptr ? num_experts : 1, M, N, ldd, out_dtype == ALTOB200_DT_BF16,
-                     out_dtype == ALTOB200_DT_BF16 ? 64 : 128);
+                     out_dtype == ALTOB200_DT_BF16 && BN == 192 ? 64 : 128);
   if (rc != ALTOB200_OK) return rc;
 
   MacroGemmArgs m;
