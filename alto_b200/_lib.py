@@ -23,7 +23,7 @@ LIB_PATH = _PKG / "libaltob200.so"
 # enums of include/altob200.h
 FMT_NVFP4, FMT_MXFP4, FMT_MXFP8_E4M3, FMT_MXFP8_E5M2 = 0, 1, 2, 3
 DT_BF16, DT_F32 = 0, 1
-SCALE_PLAIN, SCALE_PACKED, SCALE_MACRO = 1, 2, 4
+SCALE_PLAIN, SCALE_PACKED, SCALE_MACRO, RHT_DENSE32 = 1, 2, 4, 8
 ROUND_RTN, ROUND_SR_BITS, ROUND_SR_PHILOX, ROUND_SR_SLOTS = 0, 1, 2, 3
 AMAX_SCRATCH_BYTES = 16
 
@@ -88,6 +88,7 @@ class QuantParams(C.Structure):
         ("rand_tile_rows", C.c_int64),
         ("rand_tile_pairs", C.c_int64),
         ("macro_codes", C.c_void_p),
+        ("rht_dense", C.c_void_p),
     ]
 
 
@@ -430,12 +431,18 @@ def quantize_rowwise(x, fmt, codes, scale_plain=None, scale_packed=None, *, roun
 
 def quantize_colwise(x, fmt, codes, scale_plain=None, scale_packed=None, *, rounding=ROUND_RTN,
                      outer_scale=None, rand_bits=None, rht: Optional[Rht] = None, philox=(0, 0),
-                     clip_mode="none", use_uos=False, rand_tile=(0, 0), macro_codes=None) -> None:
-    _require_cuda(x, codes, scale_plain, scale_packed, outer_scale, rand_bits, macro_codes)
+                     clip_mode="none", use_uos=False, rand_tile=(0, 0), macro_codes=None, dense=None) -> None:
+    """``dense``: the fp32 [32, 32] matrix of a dense transform of the rows (``ALTOB200_RHT_DENSE32``)."""
+    _require_cuda(x, codes, scale_plain, scale_packed, outer_scale, rand_bits, macro_codes, dense)
     assert x.dim() == 2 and x.stride(1) == 1
     flags = (SCALE_PLAIN if scale_plain is not None else 0) | (SCALE_PACKED if scale_packed is not None else 0)
+    if dense is not None:
+        assert dense.dtype == torch.float32 and dense.shape == (32, 32) and dense.is_contiguous()
+        flags |= RHT_DENSE32
     p = _params(fmt, x, rounding, outer_scale, rand_bits, rht, flags, philox, clip_mode, use_uos, rand_tile,
                 macro_codes)
+    if dense is not None:
+        p.rht_dense = dense.data_ptr()
     _check(lib().altob200_quantize_colwise(x.data_ptr(), x.shape[0], x.shape[1], x.stride(0), C.byref(p),
                                            codes.data_ptr(), _ptr(scale_plain), _ptr(scale_packed), _stream()),
            "altob200_quantize_colwise")

@@ -68,6 +68,14 @@ def cols_operand(t2: torch.Tensor, use_uos: bool, clip_mode: str = "none", sr: O
     applies it (``_fusable_cols``), else without."""
     rht = rht_of(hadamard_transform)
     sr = sr or E.RTN
+    if rht is None and hadamard_transform is not None and _fusable_cols(t2, None, clip_mode):
+        matrix = E.dense_in_quantizer(t2, hadamard_transform, MX, sr)
+        if matrix is not None:
+            R, Cc = t2.shape
+            mbs = torch.empty(Cc, _chunks(R), dtype=torch.uint8, device=t2.device)
+            op = E.quant_cols(t2, MX, None, None, sr, use_uos, clip_mode, macro_codes=mbs, dense=matrix)
+            op.macro = L.MacroScale(mbs, mbs.shape[-1], 1, 0)
+            return op
     if rht is None:
         t2 = _rotate(t2, hadamard_transform)
     if _fusable_cols(t2, rht, clip_mode) and sr["rounding"] in (L.ROUND_RTN, L.ROUND_SR_SLOTS):

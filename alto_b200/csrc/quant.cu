@@ -557,7 +557,76 @@ struct ColwiseArgs {
   RhtParams rht;
   MxOpts mx;
   uint8_t* macro_codes;  // MACRO: [cols, ceil(rows / 128)] factor codes, written
+  const float* dense;    // DENSE: the 32 x 32 matrix
+  float dense_scale;     // DENSE: 1 / sqrt(32)
 };
+
+// A warp's 32 rows x 64 columns times the 32 x 32 matrix of +-1, as bf16 words of a lane's two columns by row.  The
+// matrix is not of Sylvester type, so there is no butterfly: mma.sync on a tile in shared memory, as in
+// csrc/rht_dense.cu and with its roundings.  Here it spares that kernel's pass over memory.  Bound by issue slots
+// behind the loads, which is why all of them are asked for before anything else (176 us without).  With macro blocks:
+// 69 632 x 2880 RTN 167 + 110 us (transform, then quantizer) -> 165 us, 5760 columns with random words 329 + 366 -> 508.
+constexpr int DENSE_PITCH = 64 * 2 + 16;   // bytes per tile row: rows 16 bytes apart modulo 128
+__device__ __forceinline__ void dense32_words(const uint8_t* src, int64_t pitch, int n_cols, bool rows_ok, const float* w,
+                                              float scale, uint8_t* tile, int lane, uint32_t* words) {
+  uint4 raw[8];
+  {
+    const bool ok = rows_ok && (lane & 7) * 8 < n_cols;
+    const uint8_t* p = src + (lane >> 3) * pitch + (lane & 7) * 16;
+#pragma unroll
+    for (int i = 0; i < 8; ++i, p += 4 * pitch) raw[i] = ok ? __ldg(reinterpret_cast<const uint4*>(p)) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  uint32_t fa[2][2][4];   // A fragments of the matrix (16 x 16 tiles)
+  {
+    const int r = lane >> 2, c2 = 2 * (lane & 3);
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int kt = 0; kt < 2; ++kt)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 f = __ldg(reinterpret_cast<const float2*>(w + (mt * 16 + r + 8 * (q & 1)) * 32 + kt * 16 + c2 + 8 * (q >> 1)));
+          const __nv_bfloat162 p2 = __floats2bfloat162_rn(f.x, f.y);
+          fa[mt][kt][q] = *reinterpret_cast<const uint32_t*>(&p2);
+        }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(tile + (i * 4 + (lane >> 3)) * DENSE_PITCH + (lane & 7) * 16) = raw[i];
+  __syncwarp();
+  const uint32_t tile_s = (uint32_t)__cvta_generic_to_shared(tile);
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {                // 8 columns
+    uint32_t b[4];                             // rows 0-15, 16-31
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(tile_s + (uint32_t)lane * DENSE_PITCH + t * 16)
+                 : "memory");
+    float acc[2][4];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+      acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.0f;
+#pragma unroll
+      for (int kt = 0; kt < 2; ++kt)
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                     : "+f"(acc[mt][0]), "+f"(acc[mt][1]), "+f"(acc[mt][2]), "+f"(acc[mt][3])
+                     : "r"(fa[mt][kt][0]), "r"(fa[mt][kt][1]), "r"(fa[mt][kt][2]), "r"(fa[mt][kt][3]),
+                       "r"(b[2 * kt]), "r"(b[2 * kt + 1]));
+    }
+    __syncwarp();   // every lane's fragment of these columns has been read
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        // the fused +0 turns the product of a -0 sum into +0, as the matmul's accumulation from zero does
+        const float2 y = __ffma2_rn(make_float2(acc[mt][2 * h], acc[mt][2 * h + 1]), make_float2(scale, scale), make_float2(0.0f, 0.0f));
+        const __nv_bfloat162 p2 = __floats2bfloat162_rn(y.x, y.y);
+        *reinterpret_cast<uint32_t*>(tile + (mt * 16 + (lane >> 2) + 8 * h) * DENSE_PITCH + t * 16 + (lane & 3) * 4) =
+            *reinterpret_cast<const uint32_t*>(&p2);
+      }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 32; ++k) words[k] = *reinterpret_cast<const uint32_t*>(tile + k * DENSE_PITCH + lane * 4);
+}
 
 // Threads per CTA = rows per CTA tile.  128 rather than 256: more, smaller CTAs per SM, so that the start-up
 // loads and the barrier of one overlap the arithmetic of the others.
@@ -572,7 +641,8 @@ constexpr int COL_TN = 64;   // columns per CTA tile
 // be made in slot order and neighbouring lanes read neighbouring words.
 // MACRO (MXFP4 from bf16): the two-level recipe's scaling runs in front of the quantisation - a CTA tile is one
 // macro block of 128 rows per column, so its maxima only have to cross the four warps.
-template <int FMT, bool IN_BF16, int ROUND, bool RHT, bool MACRO>
+// DENSE (MXFP4 from bf16, no RHT): the dense transform of 32 rows runs in front of all that.
+template <int FMT, bool IN_BF16, int ROUND, bool RHT, bool MACRO, bool DENSE = false>
 // (fp32 blocks of 32 with words by position are held to the 128 registers of four CTAs an SM: 63 -> 58 us for
 // 8192 x 4096; drawn in the kernel, only behind the transform, 24.0 -> 22.6 us for 4096 x 2880 (without it 5.2 -> 5.4
 // for 512 x 4096); 0 leaves the others to the compiler)
@@ -590,6 +660,8 @@ quantize_colwise_kernel(ColwiseArgs a) {
   constexpr int ROW_BYTES = F::FP4 ? COL_TM / 2 : COL_TM;  // bytes per output row per tile
   constexpr int BLK_BYTES = F::FP4 ? B / 2 : B;            // bytes per block per column
   static_assert(!MACRO || (FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && COL_TM == 128 && ITERS == 1), "macro blocks");
+  static_assert(!DENSE || (IN_BF16 && B == 32 && ITERS == 1 && !RHT && COL_TN == 64), "a warp's rows are a block of the transform");
+  __shared__ __align__(16) uint8_t s_dense[DENSE ? WARPS : 1][DENSE ? 32 * DENSE_PITCH : 16];
   // codes staged as [block][column][BLK_BYTES]; scales as [column][NBLK]
   __shared__ __align__(16) uint8_t s_codes[COL_TN * ROW_BYTES];
   __shared__ __align__(16) uint8_t s_sf[COL_TN * NBLK];
@@ -619,7 +691,12 @@ quantize_colwise_kernel(ColwiseArgs a) {
   constexpr int ESZ = IN_BF16 ? 2 : 4;
   const int64_t half_blk = 16 * a.ld * ESZ;  // second 16-row group of a 32-row block
   uint32_t pre[IN_BF16 ? ITERS : 1][IN_BF16 ? B : 1];
-  if (IN_BF16) {
+  if constexpr (DENSE) {
+    const int64_t mb = m0 + (int64_t)warp * B;
+    const int64_t n_cols = a.cols - n0;
+    dense32_words(reinterpret_cast<const uint8_t*>(a.x) + (mb * a.ld + n0) * ESZ, a.ld * ESZ,
+                  (int)(n_cols < COL_TN ? n_cols : COL_TN), mb < a.rows, a.dense, a.dense_scale, s_dense[warp], lane, pre[0]);
+  } else if (IN_BF16) {
 #pragma unroll
     for (int it = 0; it < ITERS; ++it) {
       const int64_t mb = m0 + (int64_t)(warp + WARPS * it) * B;
@@ -1795,6 +1872,13 @@ template <int FMT, bool IN_BF16, int ROUND, bool RHT>
 static void launch_colwise_kernel(const ColwiseArgs& a, cudaStream_t st) {
   const dim3 grid((unsigned)ceil_div(a.cols, COL_TN), (unsigned)ceil_div(a.rows, COL_NT)), block(COL_NT);
   constexpr bool CAN_MACRO = FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && (ROUND == ALTOB200_ROUND_RTN || ROUND == ALTOB200_ROUND_SR_SLOTS);
+  if constexpr (CAN_MACRO && !RHT) {
+    if (a.dense != nullptr) {
+      if (a.macro_codes != nullptr) (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, ROUND, false, true, true>, grid, block, 0, st, a);
+      else (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, ROUND, false, false, true>, grid, block, 0, st, a);
+      return;
+    }
+  }
   if (CAN_MACRO && a.macro_codes != nullptr)
     (void)launch_after(quantize_colwise_kernel<FMT, IN_BF16, ROUND, RHT, CAN_MACRO>, grid, block, 0, st, a);
   else
@@ -2060,6 +2144,15 @@ int altob200_quantize_colwise(const void* x, int64_t rows, int64_t cols, int64_t
       (p->format != ALTOB200_FMT_MXFP4 || p->in_dtype != ALTOB200_DT_BF16 ||
        (p->rounding != ALTOB200_ROUND_RTN && p->rounding != ALTOB200_ROUND_SR_SLOTS)))
     return ALTOB200_EUNSUPPORTED;
+  a.dense = (p->scale_flags & ALTOB200_RHT_DENSE32) != 0 ? p->rht_dense : nullptr;
+  a.dense_scale = 1.0f / (float)sqrt(32.0);
+  if ((p->scale_flags & ALTOB200_RHT_DENSE32) != 0) {
+    if (a.dense == nullptr || p->rht_n != 0) return ALTOB200_EINVAL_SHAPE;
+    if (p->format != ALTOB200_FMT_MXFP4 || p->in_dtype != ALTOB200_DT_BF16 ||
+        (p->rounding != ALTOB200_ROUND_RTN && p->rounding != ALTOB200_ROUND_SR_SLOTS))
+      return ALTOB200_EUNSUPPORTED;
+    if (!aligned16(a.dense)) return ALTOB200_EINVAL_ALIGN;
+  }
   a.x = x; a.rows = rows; a.cols = cols; a.ld = ld;
   a.codes = (uint8_t*)codes; a.scale_plain = scale_plain; a.scale_packed = (uint8_t*)scale_packed;
   a.ncol_tiles = ceil_div(rows / B, 4);

@@ -58,6 +58,7 @@ extern "C" {
 #define ALTOB200_SCALE_PLAIN 1
 #define ALTOB200_SCALE_PACKED 2
 #define ALTOB200_SCALE_MACRO 4  /* altob200_quant_params.macro_codes is set (the field is not read otherwise) */
+#define ALTOB200_RHT_DENSE32 8  /* altob200_quant_params.rht_dense is set (the field is not read otherwise) */
 /* rounding */
 #define ALTOB200_ROUND_RTN 0
 #define ALTOB200_ROUND_SR_BITS 1   /* stochastic rounding, caller supplies 32 random bits per element */
@@ -136,6 +137,10 @@ typedef struct altob200_quant_params {
    * periodic table) / SR_SLOTS (column-wise).  The column-wise quantizer applies the Hadamard transform before
    * it; with CLIP_DYNAMIC and a transform it sums a block's statistics in the order of the transform's slots. */
   uint8_t* macro_codes;
+  /* Column-wise quantizer, MXFP4 from bf16, RTN or SR_SLOTS, only read with ALTOB200_RHT_DENSE32 in scale_flags
+   * (rht_n must be 0): device fp32 [32][32] of +-1, 16-byte aligned; every block of 32 rows is first transformed as
+   * altob200_rht_dense does it with n = 32, rounding to bf16 included. */
+  const float* rht_dense;
 } altob200_quant_params;
 
 /*
