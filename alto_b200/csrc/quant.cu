@@ -203,6 +203,58 @@ __device__ __forceinline__ uint32_t fp4_octet(const float* x, const BlockScale& 
   return word;
 }
 
+// Two values that are bf16 numbers as one word.
+__device__ __forceinline__ uint32_t pack_bf16_bits(float lo, float hi) { return __byte_perm(f2u(lo), f2u(hi), 0x7632); }
+
+// The random words of eight elements in the forms that e2m1_sr_value takes from a word: -RU(word) * 2^-33 and the
+// low 22 bits.  Elements that share words (rows a table's period apart) share these.
+struct SrOctet {
+  float nu[8];
+  uint32_t m[8];
+};
+__device__ __forceinline__ SrOctet sr_octet(const uint4& even, const uint4& odd) {
+  const uint32_t w[8] = {even.x, odd.x, even.y, odd.y, even.z, odd.z, even.w, odd.w};
+  SrOctet o;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    o.nu[j] = __fmul_rn(__uint2float_ru(w[j]), -1.16415321826934814453125e-10f);
+    o.m[j] = w[j] & 0x3FFFFFu;
+  }
+  return o;
+}
+
+// fp4_octet<FAST> with such words: the steps of e2m1_sr_value, two elements to an instruction where there is one, and
+// the sign from the element itself.
+template <int FMT, bool IN_BF16>
+__device__ __forceinline__ uint32_t fp4_octet_sr(const float* x, const BlockScale& s, const SrOctet& o) {
+  float c[8];
+#pragma unroll
+  for (int j = 0; j < 8; j += 2) {
+    float2 v = make_float2(x[j], x[j + 1]);
+    const float2 r = make_float2(s.r, s.r);
+    if (Fmt<FMT>::MX) {
+      v = __fmul2_rn(v, r);
+    } else if (IN_BF16) {   // div_bf16_num up to the sign of a zero
+      const float2 y = __fmul2_rn(v, r), nq = make_float2(-s.q, -s.q);
+      v = __ffma2_rn(__ffma2_rn(y, nq, v), r, y);
+    } else {
+      v = make_float2(div_f32_num(v.x, s.q, s.r), div_f32_num(v.y, s.q, s.r));
+    }
+    const float2 t = make_float2(__fadd_rz(fabsf(v.x), o.nu[j]), __fadd_rz(fabsf(v.y), o.nu[j + 1]));
+    const float2 g = __ffma2_rd(t, make_float2(2.0f, 2.0f), make_float2(12582912.0f, 12582912.0f));
+    float2 below, above;
+    asm("fma.rn.sat.f32 %0, %1, 0f3F000000, %2;" : "=f"(below.x) : "f"(g.x), "f"(-6291455.5f));
+    asm("fma.rn.sat.f32 %0, %1, 0f3F000000, %2;" : "=f"(below.y) : "f"(g.y), "f"(-6291455.5f));
+    const uint32_t n0 = (f2u(v.x) + o.m[j]) & 0x7FC00000u, n1 = (f2u(v.y) + o.m[j + 1]) & 0x7FC00000u;
+    asm("fma.rn.sat.f32 %0, %1, 0f3E000000, 0fBE000000;" : "=f"(above.x) : "f"(u2f(n0)));
+    asm("fma.rn.sat.f32 %0, %1, 0f3E000000, 0fBE000000;" : "=f"(above.y) : "f"(u2f(n1)));
+    const float2 w = __ffma2_rn(above, make_float2(8.0f, 8.0f), below);
+    c[j] = u2f(f2u(w.x) | (f2u(x[j]) & 0x80000000u));
+    c[j + 1] = u2f(f2u(w.y) | (f2u(x[j + 1]) & 0x80000000u));
+  }
+  return e2m1x8_rtn_hw(c);
+}
+
 // Whether a block may take the reciprocal forms: with stochastic rounding only without infinities and NaNs.
 template <bool IN_BF16, int ROUND>
 __device__ __forceinline__ bool block_fast(const BlockScale& s, uint32_t amax_abs_bits) {
@@ -275,15 +327,28 @@ struct RowwiseArgs {
 // loads of all four rows are issued before the first is consumed (128 bytes per lane in flight), and
 // the index arithmetic of a task (row and chunk, pointers, position in the periodic random table) is
 // paid once per 64 elements of a lane.
-// Three resident blocks per SM (at most 85 registers per thread): other block sizes and counts measured within
-// 3 %, although the stochastic-rounding variants spill (NVFP4 bf16 72 bytes, fp32 428); all of them are faster
-// than the body that spilled less (8192 x 4096 NVFP4 from a table: bf16 38 -> 33 us, fp32 70 -> 53).
+// Three resident blocks of 256 threads per SM (at most 85 registers per thread): other block sizes and counts
+// measured within 3 %.
+//
+// With words from memory the four rows are a period of the table apart: they meet the same words, which are loaded
+// and converted once, behind the scales of all four rows.  Bound by the instructions of the rounding (26 an element
+// with macro factors, 20 without, the scheduler 64 % busy).  Four blocks of 128 threads (128 registers) keep bf16 rows
+// free of spills; five, or three of 256, spill and are slower than words loaded by row.  8192 x 14336 from bf16, words by
+// row -> shared: MXFP4 119 -> 106 us, with macro factors 141 -> 133, NVFP4 125 -> 113; fp32 141 -> 131 and 178 -> 147.
 constexpr int ROW_R = 4;
+
+constexpr int rowwise_threads(int round) { return round == ALTOB200_ROUND_SR_BITS ? 128 : 256; }
+
+// Rows of a task: neighbours, or a period of the random table apart, so that the four rows share their words.
+__host__ __device__ __forceinline__ int64_t rowwise_row_step(const RowwiseArgs& a) { return a.tile_rows != 0 ? a.tile_rows : 1; }
+__host__ __device__ __forceinline__ int64_t rowwise_row_groups(const RowwiseArgs& a, int64_t step) {
+  return (a.rows + ROW_R * step - 1) / (ROW_R * step) * step;
+}
 
 // MACRO (MXFP4 from bf16): the two-level recipe's scaling runs in front of the quantisation; a macro block of
 // 128 columns is eight neighbouring lanes.
 template <int FMT, bool IN_BF16, int ROUND, bool MACRO>
-__global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a) {
+__global__ void __launch_bounds__(rowwise_threads(ROUND), ROUND == ALTOB200_ROUND_SR_BITS ? 4 : 3) quantize_rowwise_kernel(RowwiseArgs a) {
   grid_dependency_wait();
   using F = Fmt<FMT>;
   static_assert(!MACRO || (FMT == ALTOB200_FMT_MXFP4 && IN_BF16), "macro blocks");
@@ -293,7 +358,9 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
   constexpr int NV = IN_BF16 ? 2 : 4;  // 16-byte vectors per lane and row
   const int lane = threadIdx.x & 31;
   const int64_t chunks_per_row = (a.cols + 511) >> 9;
-  const int64_t n_tasks = ((a.rows + ROW_R - 1) / ROW_R) * chunks_per_row;
+  constexpr bool WORDS = ROUND == ALTOB200_ROUND_SR_BITS;
+  const int64_t step = WORDS ? rowwise_row_step(a) : 1;
+  const int64_t n_tasks = rowwise_row_groups(a, step) * chunks_per_row;
   const int64_t warp0 = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t n_warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const OuterScale os = make_outer_scale((!F::MX) && a.outer != nullptr, a.outer);
@@ -305,56 +372,50 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
   for (int64_t task = warp0; task < n_tasks; task += n_warps) {
     int64_t rg, chunk;
     divmod_fast(task, chunks_per_row, &rg, &chunk);
-    const int64_t row0 = rg * ROW_R;
+    int64_t row0 = rg * ROW_R;
+    if (WORDS && step != 1) {
+      int64_t period, first;
+      divmod_fast(rg, step, &period, &first);
+      row0 = period * (ROW_R * step) + first;
+    }
     const int64_t col = (chunk << 9) + lane * 16;
     const bool col_ok = col < a.cols;
     const uint8_t* src = reinterpret_cast<const uint8_t*>(a.x) + (row0 * a.ld + col) * ESZ;
-    const int64_t pitch = a.ld * ESZ;
+    const int64_t pitch = a.ld * ESZ * step;
+    // rows of the task that exist, and the place of their codes, from a count and a pitch where registers are left for them
+    constexpr bool COUNTED = IN_BF16 || WORDS;
+    constexpr int EPB = F::FP4 ? 2 : 1;   // elements per byte of codes
+    int n_ok = 0;
+#pragma unroll
+    for (int i = 0; COUNTED && i < ROW_R; ++i) n_ok += row0 + i * step < a.rows ? 1 : 0;
+    uint8_t* const dst0 = a.codes + (row0 * a.cols + col) / EPB;
+    const int64_t dst_pitch = step * (a.cols / EPB);
+    const auto row_ok = [&](int i) { return COUNTED ? i < n_ok : row0 + i * step < a.rows; };
+    const auto dst = [&](int i) { return COUNTED ? dst0 + i * dst_pitch : a.codes + ((row0 + i * step) * a.cols + col) / EPB; };
 
     // ---- all loads of the task ----
     uint4 raw[ROW_R][NV];
 #pragma unroll
     for (int i = 0; i < ROW_R; ++i) {
-      const bool ok = col_ok && row0 + i < a.rows;
+      const bool ok = col_ok && row_ok(i);
 #pragma unroll
       for (int q = 0; q < NV; ++q)
         raw[i][q] = ok ? __ldg(reinterpret_cast<const uint4*>(src + i * pitch) + q) : make_uint4(0u, 0u, 0u, 0u);
-    }
-    // position of the task in the periodic random table (32-bit: the host refuses larger extents)
-    uint32_t rr0 = 0, pp = 0;
-    if (ROUND == ALTOB200_ROUND_SR_BITS && tiled) {
-      rr0 = (uint32_t)row0 % t_rows;
-      pp = (uint32_t)(col >> 1) % t_pairs;
     }
     const int64_t kb = (chunk << 9) / F::B + lane / LPB;  // scale column of this lane
     const bool holder = col_ok && (lane % LPB == 0);
     static_assert(ROW_R == 4, "the packed scales are transposed four rows at a time");
     uint32_t scale_bytes = 0;   // byte i: scale of row i
 
+    BlockScale scales[WORDS ? ROW_R : 1];
+    bool all_fast = true;
 #pragma unroll
     for (int i = 0; i < ROW_R; ++i) {
-      const int64_t row = row0 + i;
-      const bool active = col_ok && row < a.rows;
-      // random words first: their (cache-resident) loads overlap the scale arithmetic below
+      const int64_t row = row0 + i * step;
+      if (WORDS && !row_ok(i)) break;   // the whole warp
+      const bool active = col_ok && row_ok(i);
       uint32_t r0[8], r1[8];
-      if (ROUND == ALTOB200_ROUND_SR_BITS) {
-        // full planes [2][rows][cols/2], or a [2][tile_rows][tile_pairs] table repeated over the matrix
-        // (the 8 pairs of a lane never straddle a tile: tile_pairs is a multiple of 8)
-        uint32_t rr = rr0 + (uint32_t)i;
-        while (tiled && rr >= t_rows) rr -= t_rows;
-        const int64_t off = tiled ? (int64_t)(rr * t_pairs + pp) : row * half_cols + (col >> 1);
-        const int64_t plane = tiled ? (int64_t)(t_rows * t_pairs) : a.rows * half_cols;
-        uint4 a0 = make_uint4(0u, 0u, 0u, 0u), a1 = a0, b0 = a0, b1 = a0;
-        if (active) {
-          const uint4* p0 = reinterpret_cast<const uint4*>(a.rand_bits + off);
-          const uint4* p1 = reinterpret_cast<const uint4*>(a.rand_bits + plane + off);
-          a0 = __ldg(p0); a1 = __ldg(p0 + 1); b0 = __ldg(p1); b1 = __ldg(p1 + 1);
-        }
-        r0[0] = a0.x; r0[1] = a0.y; r0[2] = a0.z; r0[3] = a0.w;
-        r0[4] = a1.x; r0[5] = a1.y; r0[6] = a1.z; r0[7] = a1.w;
-        r1[0] = b0.x; r1[1] = b0.y; r1[2] = b0.z; r1[3] = b0.w;
-        r1[4] = b1.x; r1[5] = b1.y; r1[6] = b1.z; r1[7] = b1.w;
-      } else if (ROUND == ALTOB200_ROUND_SR_PHILOX) {
+      if (ROUND == ALTOB200_ROUND_SR_PHILOX) {
         // one Philox call feeds two element pairs: call index = pair index / 2
         const uint64_t q0 = a.philox_offset + (uint64_t)((row * half_cols + (col >> 1)) >> 1);
 #pragma unroll
@@ -446,12 +507,28 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
       }
 
       // ---- encode and store ----
+      if constexpr (WORDS) {   // behind the loop; what clip and factors made of the elements goes back into their words
+        scales[i] = s;
+        all_fast = all_fast && block_fast<IN_BF16, ROUND>(s, amax_bits);
+        if (MACRO || (F::MX && a.mx.clip == 1)) {
+          if (IN_BF16) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+              raw[i][q] = make_uint4(pack_bf16_bits(v[8 * q], v[8 * q + 1]), pack_bf16_bits(v[8 * q + 2], v[8 * q + 3]),
+                                     pack_bf16_bits(v[8 * q + 4], v[8 * q + 5]), pack_bf16_bits(v[8 * q + 6], v[8 * q + 7]));
+          } else {
+#pragma unroll
+            for (int q = 0; q < NV; ++q)
+              raw[i][q] = make_uint4(f2u(v[(4 * q) & 15]), f2u(v[(4 * q + 1) & 15]), f2u(v[(4 * q + 2) & 15]), f2u(v[(4 * q + 3) & 15]));
+          }
+        }
+      } else
       with_uniform_fast(block_fast<IN_BF16, ROUND>(s, amax_bits), [&](auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
         if (F::FP4) {
           const uint32_t lo = fp4_octet<FMT, IN_BF16, ROUND, FAST>(v, s, r0, r1);
           const uint32_t hi = fp4_octet<FMT, IN_BF16, ROUND, FAST>(v + 8, s, r0 + 4, r1 + 4);
-          if (active) *reinterpret_cast<uint2*>(a.codes + row * half_cols + (col >> 1)) = make_uint2(lo, hi);
+          if (active) *reinterpret_cast<uint2*>(dst(i)) = make_uint2(lo, hi);
         } else {
           uint32_t o[4];
 #pragma unroll
@@ -461,16 +538,70 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
             for (int c = 0; c < 4; ++c) q[c] = scale_elem<FMT, IN_BF16, FAST>(v[4 * j + c], s);
             o[j] = fp8x2_rtn_hw<F::E5M2>(q[0], q[1]) | (fp8x2_rtn_hw<F::E5M2>(q[2], q[3]) << 16);
           }
-          if (active) *reinterpret_cast<uint4*>(a.codes + row * a.cols + col) = make_uint4(o[0], o[1], o[2], o[3]);
+          if (active) *reinterpret_cast<uint4*>(dst(i)) = make_uint4(o[0], o[1], o[2], o[3]);
         }
       });
 
       // ---- scales ----
-      if (a.scale_plain != nullptr && holder && row < a.rows) {
+      if (a.scale_plain != nullptr && holder && row_ok(i)) {
         if (F::MX) reinterpret_cast<uint8_t*>(a.scale_plain)[row * nkb + kb] = (uint8_t)s.byte;
         else reinterpret_cast<float*>(a.scale_plain)[row * nkb + kb] = s.plain;
       }
-      scale_bytes = merge_shifted((holder && row < a.rows) ? s.byte : 0u, 8 * i, scale_bytes);
+      scale_bytes = merge_shifted((holder && row_ok(i)) ? s.byte : 0u, 8 * i, scale_bytes);
+    }
+    if constexpr (WORDS) {
+      // position of the task in the periodic table (32-bit: the host refuses larger extents), or in full planes
+      // [2][rows][cols/2] (the 8 pairs of a lane never straddle a tile: tile_pairs is a multiple of 8)
+      int64_t off = row0 * half_cols + (col >> 1), plane = a.rows * half_cols;
+      if (tiled) {
+        off = (int64_t)(((uint32_t)row0 % t_rows) * t_pairs + (uint32_t)(col >> 1) % t_pairs);
+        plane = (int64_t)(t_rows * t_pairs);
+      }
+      with_uniform_fast(all_fast, [&](auto fast_tag) {
+        constexpr bool FAST = decltype(fast_tag)::value;
+        uint32_t first[ROW_R];
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+          uint4 even = make_uint4(0u, 0u, 0u, 0u), odd = even;
+          SrOctet words;
+#pragma unroll
+          for (int i = 0; i < ROW_R; ++i) {
+            if (!row_ok(i)) break;
+            if (i == 0 || !tiled) {
+              if (col_ok) {
+                const uint32_t* p = a.rand_bits + off + (tiled ? 0 : i * half_cols);
+                even = __ldg(reinterpret_cast<const uint4*>(p) + o);
+                odd = __ldg(reinterpret_cast<const uint4*>(p + plane) + o);
+              }
+              if (FAST) words = sr_octet(even, odd);
+            }
+            float v[8];
+            if (IN_BF16) {
+              const uint32_t w[4] = {raw[i][o].x, raw[i][o].y, raw[i][o].z, raw[i][o].w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                v[2 * j] = bf16lo_to_f32(w[j]);
+                v[2 * j + 1] = bf16hi_to_f32(w[j]);
+              }
+            } else {
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                const uint4 w = raw[i][(2 * o + q) % NV];
+                v[4 * q] = u2f(w.x); v[4 * q + 1] = u2f(w.y); v[4 * q + 2] = u2f(w.z); v[4 * q + 3] = u2f(w.w);
+              }
+            }
+            uint32_t code;
+            if constexpr (FAST) {
+              code = fp4_octet_sr<FMT, IN_BF16>(v, scales[i], words);
+            } else {
+              const uint32_t r0[4] = {even.x, even.y, even.z, even.w}, r1[4] = {odd.x, odd.y, odd.z, odd.w};
+              code = fp4_octet<FMT, IN_BF16, ROUND, false>(v, scales[i], r0, r1);
+            }
+            if (o == 0) first[i] = code;
+            else if (col_ok) *reinterpret_cast<uint2*>(dst(i)) = make_uint2(first[i], code);
+          }
+        }
+      });
     }
     // ---- packed scales: four lanes hold four rows of four scale columns each; a 4 x 4 byte transpose in two
     // exchanges leaves each of them one row's word (a word is four scale columns of one row) ----
@@ -481,8 +612,9 @@ __global__ void __launch_bounds__(256, 3) quantize_rowwise_kernel(RowwiseArgs a)
       o = __shfl_xor_sync(0xFFFFFFFFu, scale_bytes, LPB);
       scale_bytes = __byte_perm(scale_bytes, o, (h & 1) ? 0x3715 : 0x6240);
       const int64_t kb4 = kb - h;
-      if (lane % LPB == 0 && kb4 < a.ncol_tiles * 4 && row0 + h < a.rows)
-        *reinterpret_cast<uint32_t*>(a.scale_packed + packed_scale_offset(row0 + h, kb4, a.ncol_tiles)) = scale_bytes;
+      const int64_t row = row0 + h * step;
+      if (lane % LPB == 0 && kb4 < a.ncol_tiles * 4 && row_ok(h))
+        *reinterpret_cast<uint32_t*>(a.scale_packed + packed_scale_offset(row, kb4, a.ncol_tiles)) = scale_bytes;
     }
   }
 }
@@ -1842,16 +1974,17 @@ static void fill_rht_row_offsets(RhtParams* r, int64_t ld, int esz) {
 
 template <int FMT, bool IN_BF16, int ROUND>
 static void launch_rowwise_kernel(const RowwiseArgs& a, cudaStream_t st) {
-  const int64_t tasks = ceil_div(a.rows, ROW_R) * ((a.cols + 511) >> 9);
-  int64_t blocks = ceil_div(tasks, 8);
-  const int64_t cap = (int64_t)sm_count() * 8;
+  const int64_t tasks = rowwise_row_groups(a, ROUND == ALTOB200_ROUND_SR_BITS ? rowwise_row_step(a) : 1) * ((a.cols + 511) >> 9);
+  constexpr int NT = rowwise_threads(ROUND);
+  int64_t blocks = ceil_div(tasks, NT / 32);
+  const int64_t cap = (int64_t)sm_count() * (2048 / NT);
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   constexpr bool CAN_MACRO = FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && ROUND != ALTOB200_ROUND_SR_PHILOX;
   if (CAN_MACRO && a.macro_codes != nullptr)
-    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, CAN_MACRO>, dim3((unsigned)blocks), dim3(256), 0, st, a);
+    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, CAN_MACRO>, dim3((unsigned)blocks), dim3(NT), 0, st, a);
   else
-    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, false>, dim3((unsigned)blocks), dim3(256), 0, st, a);
+    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, false>, dim3((unsigned)blocks), dim3(NT), 0, st, a);
 }
 
 template <int FMT, bool IN_BF16>
