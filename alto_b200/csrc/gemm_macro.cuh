@@ -85,12 +85,14 @@ struct CfgMacro {
   // Ring of reciprocal factors, per chunk 128 rows and BN columns (B_UNIFORM: the products of both, 128 rows per
   // 128 columns).  No barrier guards its reuse: a slot is rewritten FAC_STAGES stages after its last use, once
   // that stage's operands have landed, so the MMAs of the stage STAGES earlier are done, and with them every chunk
-  // up to P_BUFS before has been read out, in order - all but the latest of these have therefore been folded.
-  static constexpr int FAC_STAGES = 8;
+  // up to P_BUFS before has been read out, in order - all but the latest of these have therefore been folded (that
+  // one's column factors are read after its accumulator was given back).  A stage may hold a single chunk (K ranges of
+  // 128), so P_BUFS chunks are as many stages.
+  static constexpr int FAC_STAGES = BN == 192 ? 8 : 9;
   static constexpr int FAC_STRIDE = BM + (BN == 192 ? 192 : 128) + 4;   // floats per chunk; + 4 spreads the banks
   static_assert(FAC_STRIDE >= SFB_BLOCKS * BM && FAC_STRIDE >= BM + BN, "factors of a chunk");
   static constexpr int FAC_BYTES = 2 * FAC_STAGES * FAC_STRIDE * 4;
-  static_assert(FAC_STAGES >= STAGES + 1 + (P_BUFS + 1) / 2, "factors are overwritten while they are in use");
+  static_assert(FAC_STAGES >= STAGES + P_BUFS + 1, "factors are overwritten while they are in use");
   static constexpr int RCP_BYTES = 256 * 4;                     // 1 / factor for every code
   static constexpr int TMEM_SF_BASE = P_BUFS * BN;
   static constexpr int TMEM_COLS_USED = TMEM_SF_BASE + STAGES * STAGE_SF_COLS;
@@ -548,7 +550,7 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       tc_fence_before();
       __syncwarp();
       mbar_arrive_lane0(smem_u32(sf_full) + 8 * s, lane);
-      slot = (slot + 1) % C::FAC_STAGES;
+      if (++slot == C::FAC_STAGES) slot = 0;
       if (++s == C::STAGES) {
         s = 0;
         phase ^= 1u;

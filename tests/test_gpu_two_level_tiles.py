@@ -113,3 +113,28 @@ def test_wide_tiles_of_row_groups(n, k):
     for i, e in enumerate(groups):
         rows = slice(128 * i, 128 * i + 128)
         _near(out[rows], a.values[rows], bs[e].values)
+
+
+@pytest.mark.parametrize("shape,counts", [((2304, 2336), [128] * 16), ((2304, 2336), [128, 128, 256, 128, 384, 128, 128, 0] * 3),
+                                          ((5760, 2880), [128] * 16)])
+def test_single_chunk_stages(shape, counts):
+    # dozens of tiles a CTA, most of them one chunk in a stage of its own: the ring of factors is reused at its closest
+    m, n = shape
+    total, ends = sum(counts), torch.tensor(counts).cumsum(0).to(torch.int32).cuda()
+    a, b = Random(m, total, 31), Random(n, total, 32)
+    out = torch.full((len(counts), m, n), 7.0, dtype=torch.float32, device="cuda")
+    L.gemm_mxfp4_two_level(m, n, total, a.codes, a.scales, a.macro, b.codes, b.scales, b.macro, out, k_offs=ends,
+                           num_experts=len(counts))
+    start = 0
+    for e, end in enumerate(ends.tolist()):
+        _near(out[e], a.values[:, start:end], b.values[:, start:end])
+        start = end
+
+
+@pytest.mark.parametrize("k", [32, 128])
+def test_single_chunk_stages_dense(k):
+    m, n = 9216, 2592                              # ten tiles a CTA
+    a, b = Random(m, k, 33), Random(n, k, 34)
+    out = torch.empty(m, n, dtype=torch.float32, device="cuda")
+    L.gemm_mxfp4_two_level(m, n, k, a.codes, a.scales, a.macro, b.codes, b.scales, b.macro, out)
+    _near(out, a.values, b.values)
