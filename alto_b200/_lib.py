@@ -749,5 +749,5 @@ def set_wait_limit_ns(limit_ns: int) -> None:
 
 
 def selftest_wait_timeout(limit_ns: int = 1_000_000) -> None:
-    """Launches the kernel whose only wait cannot be satisfied; ``status_read`` then reports the timeout."""
+    """Launches the kernel whose waits cannot be satisfied; ``status_read`` then reports the timeout."""
     _check(lib().altob200_selftest_wait_timeout(int(limit_ns), _stream()), "altob200_selftest_wait_timeout")

@@ -321,7 +321,7 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
-  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see mbar_wait
+  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see the waits
   grid_dependency_wait();   // set-up done; global memory from here on (programmatic dependent launch)
 
   if (warp < 4) {

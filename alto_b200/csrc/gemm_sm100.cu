@@ -137,59 +137,18 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-#ifdef ALTOB200_WAIT_SPIN
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-#else
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-#endif
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-// Bounded wait.  Returns false (and raises the abort flag) when the limit passes or when
-// another role already aborted.  The limit is counted on the SM's cycle counter (a register
-// read); %globaltimer is far too slow to read inside a wait that is on the critical path of
-// every pipeline stage.  `limit_ns` is converted at 2 cycles per nanosecond, the most an SM of
-// this part runs at, so the wait gives up no earlier than limit_ns and no later than about
-// twice that at the lowest sustained clocks.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          int site, uint64_t limit_ns, int kernel_id = 1) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  const long long limit_cycles = (long long)(limit_ns * 2ull);
-  uint32_t spins = 0;
-  while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((++spins & 0x1Fu) == 0) {
-      if (*abort_flag != 0) return false;
-      if (clock64() - t0 > limit_cycles) {
-        *abort_flag = 1;
-        if (atomicCAS(&g_status[0], 0, ALTOB200_ETIMEOUT_DEVICE) == 0) {
-          g_status[1] = kernel_id;  // 1 = a GEMM kernel, 9 = the wait self-test
-          g_status[2] = (int)blockIdx.x;
-          g_status[3] = site;
-        }
-        return false;
-      }
-    }
-  }
-}
-
 // Bounded waits as one small loop each.  More than a dozen warps' worth of different code share the instruction caches of an
-// SM, where every taken branch costs 30 to 40 cycles: a wait that is spread over inlined slow paths (mbar_wait) took
+// SM, where every taken branch costs 30 to 40 cycles: a wait that is spread over inlined slow paths took
 // 200 cycles and more on a barrier that was already complete, and with it a chunk's way around the roles 1300.
-// Counted on the SM's cycle counter, as in mbar_wait; false when the limit has passed or another role has given up.
+// False when the limit has passed or another role has given up.  The limit is counted on the SM's cycle counter (a
+// register read; %globaltimer is far too slow inside a wait on the critical path of every stage): nanoseconds are taken
+// as two cycles each, the most an SM of this part runs at, so a wait gives up no earlier than its limit and no later
+// than about twice that at the lowest sustained clocks.  wait_selftest_kernel runs every form into its limit.
 #define ALTOB200_WAIT_LOOP(LOOK_AT)                                                                           \
   "{\n\t.reg .pred p, q, r;\n\t.reg .u32 f, n;\n\t.reg .u64 t, t0;\n\t" LOOK_AT                                 \
   "@p bra DONE;\n\t"                                                                                         \
@@ -242,12 +201,12 @@ __device__ __forceinline__ bool mbar_wait3_tight(uint32_t b0, uint32_t b1, uint3
   return ok != 0;
 }
 #undef ALTOB200_WAIT_LOOP
-// A role that gave up: the others learn of it, the first one's place is kept.
-__device__ __forceinline__ void report_timeout(volatile int* abort_flag, int site) {
+// A role that gave up: the others learn of it, the first one's place is kept.  kernel_id: 1 = a GEMM, 9 = the self-test.
+__device__ __forceinline__ void report_timeout(volatile int* abort_flag, int site, int kernel_id = 1) {
   if (*abort_flag != 0) return;
   *abort_flag = 1;
   if (atomicCAS(&g_status[0], 0, ALTOB200_ETIMEOUT_DEVICE) == 0) {
-    g_status[1] = 1;
+    g_status[1] = kernel_id;
     g_status[2] = (int)blockIdx.x;
     g_status[3] = site;
   }
@@ -678,7 +637,7 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
-  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see mbar_wait
+  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see the waits
   // barriers, tensor memory and the zeroed scale staging are set up: from here on global memory is read
   // and written, which has to wait for the kernel in front of this one (programmatic dependent launch)
   grid_dependency_wait();
@@ -1134,7 +1093,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
-  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see mbar_wait
+  const uint64_t limit = args.wait_ns * 2ull;   // cycles, see the waits
   // barriers, tensor memory and the zeroed scale staging are set up: from here on global memory is read
   // and written, which has to wait for the kernel in front of this one (programmatic dependent launch)
   grid_dependency_wait();
@@ -1458,21 +1417,55 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
 #include "gemm_macro.cuh"
 
 // ---------------------------------------------------------------------------------------
-// self-test of the bounded wait: one CTA, one thread waits on an mbarrier nobody arrives on
+// self-test of the bounded waits: every form on barriers that are complete and on one that nobody arrives on
 // ---------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(32, 1) wait_selftest_kernel(uint64_t limit_ns) {
-  __shared__ uint64_t bar;
-  __shared__ int abort_flag;
+__global__ void __launch_bounds__(256, 1) wait_selftest_kernel(uint64_t limit_ns) {
+  __shared__ uint64_t done_bar, never_bar;      // phase 0 of the second one never completes
+  __shared__ int lowered, raised, abort_flag, other_flag;
+  __shared__ unsigned bad;
   if (threadIdx.x == 0) {
-    mbar_init(&bar, 1);
-    abort_flag = 0;
+    mbar_init(&done_bar, 1);
+    mbar_init(&never_bar, 1);
+    lowered = abort_flag = other_flag = 0;
+    raised = 1;
+    bad = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_arrive(&done_bar);
   }
   __syncthreads();
-  // phase 0 never completes (no arrival is ever made): the wait runs into its limit, records
-  // {kernel 9, block, site 99} in the status word and returns false; the kernel then ends normally
-  if (threadIdx.x == 0) (void)mbar_wait(&bar, 0, &abort_flag, 99, limit_ns, 9);
+  const int warp = threadIdx.x >> 5;
+  const uint32_t done = smem_u32(&done_bar), never = smem_u32(&never_bar), down = smem_u32(&lowered), up = smem_u32(&raised);
+  const uint64_t limit = limit_ns * 2ull;
+  const long long t0 = clock64();
+  bool ok = true;
+  if (warp == 0) {          // nothing to wait for (parity 1: the phase before the first)
+    ok = mbar_wait_tight(done, 0, down, limit) && mbar_wait_tight(never, 1, down, limit) &&
+         mbar_wait2_tight(done, done, 0, down, limit) && mbar_wait3_tight(done, done, 0, never, 1, down, limit);
+  } else if (warp == 1) {   // run into the limit: alone, then in each place
+    ok = !mbar_wait_tight(never, 0, down, limit);
+  } else if (warp == 2) {
+    ok = !mbar_wait2_tight(never, done, 0, down, limit);
+  } else if (warp == 3) {
+    ok = !mbar_wait2_tight(done, never, 0, down, limit);
+  } else if (warp == 4) {
+    ok = !mbar_wait3_tight(never, done, 0, done, 0, down, limit);
+  } else if (warp == 5) {
+    ok = !mbar_wait3_tight(done, never, 0, done, 0, down, limit);
+  } else if (warp == 6) {
+    ok = !mbar_wait3_tight(done, done, 0, never, 0, down, limit);
+  } else {                  // another role has given up: no need to wait for the limit
+    ok = !mbar_wait_tight(never, 0, up, limit) && !mbar_wait2_tight(never, done, 0, up, limit) &&
+         !mbar_wait3_tight(done, done, 0, never, 0, up, limit);
+  }
+  const bool whole_limit = (uint64_t)(clock64() - t0) > limit;
+  if (!ok || whole_limit != (warp >= 1 && warp <= 6)) atomicOr(&bad, 1u << warp);
   __syncthreads();
+  // the status word keeps the first report: {9, block, 99}, or 100 + the first warp whose wait was not as it should be
+  if (threadIdx.x == 0) {
+    report_timeout(&abort_flag, bad == 0 ? 99 : 99 + __ffs((int)bad), 9);
+    report_timeout(&abort_flag, 98, 9);
+    report_timeout(&other_flag, 97, 9);
+  }
 }
 
 // ---------------------------------------------------------------------------------------
@@ -1958,7 +1951,7 @@ int altob200_set_wait_limit_ns(uint64_t limit_ns) {
 
 int altob200_selftest_wait_timeout(uint64_t limit_ns, void* stream) {
   if (limit_ns == 0 || limit_ns > 1000000000ull) return ALTOB200_EINVAL_SHAPE;  // at most one second
-  wait_selftest_kernel<<<1, 32, 0, (cudaStream_t)stream>>>(limit_ns);
+  wait_selftest_kernel<<<1, 256, 0, (cudaStream_t)stream>>>(limit_ns);
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;
 }
 

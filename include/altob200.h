@@ -565,11 +565,12 @@ int altob200_grouped_gemm_wgrad_mxfp4_two_level(int64_t M, int64_t N, int64_t K,
 int altob200_set_wait_limit_ns(uint64_t limit_ns);
 
 /*
- * Launches one small kernel whose single wait can never be satisfied (an mbarrier on which nobody
- * arrives) with the given limit (at most 1e9 ns).  Nothing faults and nothing is left running: the
- * wait gives up after `limit_ns`, and the next altob200_status_read on the stream returns
- * ALTOB200_ETIMEOUT_DEVICE with detail {9, 0, 99, 0}, the one after that 0.  For tests of the
- * host-side handling of a device timeout.  No counterpart in the reference.
+ * Launches one small kernel that runs each form of the GEMMs' bounded waits on complete barriers, on one on
+ * which nobody arrives with the given limit (at most 1e9 ns), and on that one with the abort flag raised.
+ * Nothing faults and nothing is left running: the waits give up after `limit_ns` (or at once), and the next
+ * altob200_status_read on the stream returns ALTOB200_ETIMEOUT_DEVICE with detail {9, 0, 99, 0}, the one after
+ * that 0; a third word of 100 or more names a wait that did not do what it should.  For tests of the waits and of
+ * the host-side handling of a device timeout.  No counterpart in the reference.
  */
 int altob200_selftest_wait_timeout(uint64_t limit_ns, void* stream);
 
