@@ -424,7 +424,7 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           }
         }
       }
-      if (!alive) report_timeout(abort_flag, 22);
+      if (!alive) report_timeout(abort_flag, !mbar_complete(bar_full + 8 * s, st_phase) ? 23 : !mbar_complete(bar_sf + 8 * s, st_phase) ? 25 : 22);
     } else {
       // ------------------------------ wait warp of the fold ------------------------------
       // It waits for the finished chunks and releases the two groups of fold warps, each at its own named barrier of

@@ -201,6 +201,15 @@ __device__ __forceinline__ bool mbar_wait3_tight(uint32_t b0, uint32_t b1, uint3
   return ok != 0;
 }
 #undef ALTOB200_WAIT_LOOP
+// Whether a phase is complete, without waiting: which barrier of a failed wait it was (asked behind a role's loop).
+__device__ __forceinline__ bool mbar_complete(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
 // A role that gave up: the others learn of it, the first one's place is kept.  kernel_id: 1 = a GEMM, 9 = the self-test.
 __device__ __forceinline__ void report_timeout(volatile int* abort_flag, int site, int kernel_id = 1) {
   if (*abort_flag != 0) return;
@@ -743,7 +752,11 @@ gemm_blockscaled_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid
       }
       ++tile_it;
     }
-    if (!alive) report_timeout(abort_flag, 2);
+    if (!alive) {
+      const int s = it % C::STAGES;
+      const uint32_t phase = (it / C::STAGES) & 1;
+      report_timeout(abort_flag, !mbar_complete(smem_u32(&full_bar[s]), phase) ? 3 : !mbar_complete(smem_u32(&sf_full[s]), phase) ? 5 : 2);
+    }
   } else if (warp >= 6) {
     // ------------------------------ scale transfer (warps 6..9) ------------------------------
     // Tile t of A -> columns [4t, 4t+4) of the stage's A-scale area; tile t of B row block j ->
@@ -1253,7 +1266,11 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
         }
         ++tile_it;
       }
-      if (!alive) report_timeout(abort_flag, 12);
+      if (!alive) {
+        const int s = it % C::STAGES;
+        const uint32_t phase = (it / C::STAGES) & 1;
+        report_timeout(abort_flag, !mbar_complete(smem_u32(&full_bar[s]), phase) ? 13 : !mbar_complete(smem_u32(&sf_full[s]), phase) ? 15 : 12);
+      }
     }
   }  // warp 3 idles: it completes warpgroup 0
   } else if (warp < 8) {
@@ -1301,7 +1318,7 @@ gemm_blockscaled_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const _
         }
       }
     }
-    if (!alive) report_timeout(abort_flag, 16);
+    if (!alive) report_timeout(abort_flag, !mbar_complete(smem_u32(&sfs_full[it % C::STAGES]), (it / C::STAGES) & 1) ? 16 : 17);
   } else {
     // ------------------------------ epilogue (each CTA stores its own 128 rows) ------------------------------
     // Warps 8-11 drain the first half of the accumulator's columns, warps 12-15 the second half; a

@@ -74,7 +74,9 @@ size_t altob200_packed_scale_bytes(int64_t rows, int64_t ncols);
 /* Reads (and clears) the sticky device-side status word written by kernels
  * whose bounded waits gave up.  Synchronises `stream`.  Returns 0 or
  * ALTOB200_ETIMEOUT_DEVICE; `detail` (host, may be NULL) receives
- * {kernel id, block id, wait site, 0}. */
+ * {kernel id, block id, wait site, 0}.  Kernel 1 is a GEMM; its wait sites are, for one CTA / a CTA pair / the
+ * two-level kernel: free stage 1 / 11 / 21, drained accumulator 2 / 12 / 22, operands 3 / 13 / 23, finished
+ * accumulator 4 / 14 / 24, scales in tensor memory 5 / 15 / 25, landed scales 6 / 16 / 26, free scale slot 17. */
 int altob200_status_read(void* stream, int32_t detail[4]);
 
 #define ALTOB200_CLIP_NONE 0
