@@ -163,7 +163,8 @@ class HadamardTransform:
 
     @weight.setter
     def weight(self, value: Tensor) -> None:
-        self._weight = value
+        self._weight, self._signs = value, None
+        self._rht, self._fusable, self._dev = None, None, {}     # what was derived from the matrix before
 
     @property
     def n(self) -> int:

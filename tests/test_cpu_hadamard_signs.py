@@ -9,6 +9,7 @@ from alto_b200 import hadamard as H
 @pytest.mark.parametrize("size", [16, 32, 64])
 def test_signs_and_matrix_agree(size, dtype):
     state = {k: getattr(H.HadamardFactory, k) for k in ("block_size", "randomized", "dtype", "seed")}
+    generator = H.HadamardFactory.generator.get_state()
     try:
         H.HadamardFactory.configure(block_size=size, randomized=True, dtype=dtype, seed=11)
         drawn = H.HadamardFactory.create_transform("cpu")
@@ -24,13 +25,22 @@ def test_signs_and_matrix_agree(size, dtype):
             assert (a.n, a.perm, a.sign) == (b.n, b.perm, b.sign) and all(isinstance(v, int) for v in a.sign)
         assert torch.equal(drawn.weight, weight) and drawn.weight.dtype == dtype
         assert torch.equal(drawn.matrix(), plain.matrix())
-        drawn.weight = torch.ones(size, size)          # a matrix put in by hand counts
         again = H.HadamardTransform(None, perm, torch.ones(size))
-        again.weight = torch.ones(size, size)
-        assert not again.is_fused and torch.equal(again.matrix(), torch.ones(size, size))
+        for t in (drawn, again):                       # a matrix put in by hand counts, whatever was derived before
+            t.device_matrix("cpu")
+            t.weight = torch.ones(size, size)
+            assert not t.is_fused and t.n == size and torch.equal(t.matrix(), torch.ones(size, size))
+            assert torch.equal(t.device_matrix("cpu"), torch.ones(size, size))
+            t.weight = weight
+            assert t.is_fused == (size == 16) and torch.equal(t.device_matrix("cpu"), plain.device_matrix("cpu"))
+            if size == 16:
+                assert t.device_params().sign == plain.device_params().sign
+            t.weight = torch.ones(2, 2)
+            assert t.n == 2
     finally:
         for k, v in state.items():
             setattr(H.HadamardFactory, k, v)
+        H.HadamardFactory.generator.set_state(generator)
 
 
 def test_sizes_that_cannot_be_built_are_refused_when_drawn():
