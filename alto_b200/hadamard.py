@@ -122,7 +122,8 @@ class HadamardFactory:
 
     @classmethod
     def create_transform(cls, device) -> "HadamardTransform":
-        if cls.randomized and cls._create_weight.__func__ is HadamardFactory._create_weight.__func__:
+        if cls.randomized and getattr(cls._create_weight, "__func__", None) is _CREATE_WEIGHT \
+                and getattr(cls._create_permutation, "__func__", None) is _CREATE_PERMUTATION:
             # the draws of random_hadamard_matrix; the product with the base matrix waits until it is asked for,
             # since the fused kernels take the signs (32 us of a small linear's forward)
             signs = torch.randint(low=0, high=2, size=(cls.block_size,), generator=cls.generator, dtype=cls.dtype) * 2 - 1
@@ -141,6 +142,10 @@ class HadamardFactory:
     @classmethod
     def _create_permutation(cls, weight: Tensor) -> Tensor:
         return torch.randperm(weight.size(0), generator=cls.generator)
+
+
+# what create_transform may shorten: neither replaced nor overridden
+_CREATE_WEIGHT, _CREATE_PERMUTATION = HadamardFactory._create_weight.__func__, HadamardFactory._create_permutation.__func__
 
 
 class HadamardTransform:

@@ -51,3 +51,32 @@ def test_sizes_that_cannot_be_built_are_refused_when_drawn():
             H.HadamardFactory.create_transform("cpu")
     finally:
         H.HadamardFactory.block_size = state
+
+
+def test_a_factory_of_its_own_is_asked_for_both_parts(monkeypatch):
+    generator = H.HadamardFactory.generator.get_state()
+
+    class Sorted(H.HadamardFactory):
+        block_size, randomized = 16, True
+
+        @classmethod
+        def _create_permutation(cls, weight):
+            assert weight.shape == (16, 16)            # the matrix, whose rows it may look at
+            return torch.argsort(weight[:, 0], stable=True)
+
+    class Negated(H.HadamardFactory):
+        block_size, randomized = 16, True
+
+        @classmethod
+        def _create_weight(cls, device):
+            return -H.deterministic_hadamard_matrix(16)
+
+    try:
+        drawn = Sorted.create_transform("cpu")
+        assert torch.equal(drawn.perm, torch.argsort(drawn.weight[:, 0], stable=True))
+        assert torch.equal(Negated.create_transform("cpu").weight, -H.deterministic_hadamard_matrix(16))
+        monkeypatch.setattr(H.HadamardFactory, "block_size", 16)
+        monkeypatch.setattr(H.HadamardFactory, "_create_weight", lambda device: torch.ones(16, 16))
+        assert torch.equal(H.HadamardFactory.create_transform("cpu").weight, torch.ones(16, 16))
+    finally:
+        H.HadamardFactory.generator.set_state(generator)
