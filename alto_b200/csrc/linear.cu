@@ -67,6 +67,9 @@ extern "C" int altob200_linear_backward(const altob200_linear_backward_args* arg
       (a.dw != nullptr && (a.xm_codes == nullptr || a.xm_scales == nullptr)) || a.M <= 0 || a.K <= 0 || a.N <= 0 ||
       a.M % 32 != 0 || a.N % 32 != 0 || a.K % 32 != 0)
     return ALTOB200_EINVAL_SHAPE;
+  // (the GEMMs would take a missing outer scale for 1)
+  if (a.use_outer && ((a.dx != nullptr && a.wt_outer == nullptr) || (a.dw != nullptr && a.xm_outer == nullptr)))
+    return ALTOB200_EINVAL_SHAPE;
   if (reinterpret_cast<uintptr_t>(work) & 15) return ALTOB200_EINVAL_ALIGN;
   Work w = {};
   carve(a, (uint8_t*)work, &w);
