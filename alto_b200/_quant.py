@@ -156,7 +156,15 @@ def dequantize(codes: torch.Tensor, scales: torch.Tensor, fmt: int, axis: int, i
     if a == -1 and codes.dim() == 2 and scales.dim() == 2:
         # (a matrix as it is: the views below took two thirds of a small call's host time)
         rows, cols = codes.shape[0], codes.shape[1] * (2 if fp4 else 1)
-        s2 = scales.reshape(rows // block if is_2d else rows, cols // block).contiguous()
+        s_rows, s_cols = rows // block if is_2d else rows, cols // block
+        if scales.shape == (s_rows, s_cols):
+            s2 = scales.contiguous()
+        elif is_2d:     # more scales than codes (padding): the first ones count
+            s2 = scales.reshape(-1, s_rows, s_cols)[0].contiguous()
+        else:
+            s2 = scales.reshape(-1, s_cols)[:rows].contiguous()
+        if s2.shape[0] != s_rows:
+            raise RuntimeError(f"scales of shape {tuple(scales.shape)} for codes of shape {tuple(codes.shape)}")
         if fmt == L.FMT_NVFP4:
             s2 = s2.float()
         c2 = codes.contiguous()

@@ -76,3 +76,19 @@ def test_maximum_wherever_it_lies(rows, cols, pitch, dtype):
         x[r, c] = -(i + 1.5)
         L.amax(x, bits, outer, scratch)
         assert bits.view(torch.float32)[0].item() == i + 1.5
+
+
+@pytest.mark.parametrize("fmt", [L.FMT_NVFP4, L.FMT_MXFP4, L.FMT_MXFP8_E4M3])
+@pytest.mark.parametrize("is_2d,pad", [(False, 91), (True, 6)])
+def test_scales_with_rows_behind_the_codes(fmt, is_2d, pad):
+    # buffers of scales are padded by some callers; too few are refused
+    rows, cols, block = (96 if is_2d else 37), 160, L.block_of(fmt)
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(2)).cuda()
+    codes, scales = Q.quantize(x, fmt, -1, is_2d)
+    want = Q.dequantize(codes, scales, fmt, -1, is_2d, torch.float32)
+    more = torch.cat([scales, torch.ones(pad, scales.shape[1], device="cuda").to(scales.dtype)])
+    if is_2d:
+        more = more[:2 * scales.shape[0]]
+    assert torch.equal(Q.dequantize(codes, more, fmt, -1, is_2d, torch.float32), want)
+    with pytest.raises(RuntimeError):
+        Q.dequantize(codes, scales[:-1], fmt, -1, is_2d, torch.float32)
