@@ -1529,7 +1529,7 @@ __global__ void __launch_bounds__(WARPS_2D * 32, ROUND == ALTOB200_ROUND_RTN ? 5
 // =======================================================================================
 struct AmaxArgs {
   const void* x;
-  int32_t steps;         // loads of a thread in a row, up to LOADS: as many as leave no block without work
+  int32_t steps;         // loads of a thread in a row, up to LOADS
   int64_t rows, cols, ld;
   uint32_t* amax_bits;   // [2], written by the last block
   float* outer_scale;    // [2] or NULL
@@ -1546,9 +1546,11 @@ __device__ __forceinline__ float outer_from_amax_bits(uint32_t bits) {
   return fmaxf(__fdiv_rn(amax, 2688.0f), 1.0e-30f);
 }
 
-// LOADS: 16-byte loads of a thread in flight (without RHT).  Eight of them, neighbours of a block, where there is work
-// for all: 117 MB of bf16 24.0 us, 268 MB 54.9, where four a grid's width apart took 26.7 and 58.3.  Four where a
-// block has fewer, which leaves room for eight blocks on an SM: 4 MB 5.2 us, 6.9 with eight.
+// LOADS: 16-byte loads of a thread in flight (without RHT).  Eight of them, neighbours of a block, from nine for each
+// thread of the grid on: 117 MB of bf16 24.0 us, 268 MB 54.9, where four a grid's width apart took 26.7 and 58.3.  Below
+// that four, which leaves room for eight blocks on an SM: 4 MB 5.2 us, 6.9 with eight; 36.4 MB (7.5 a thread) 9.4 and
+// 10.6, 38.9 MB 10.3 and 11.0 (43.7 MB, nine: 11.2 with eight, 11.8 with those four).  Just above a multiple of the grid a part of the blocks has
+// nothing to do, which costs nothing: 4.86 MB, one load a thread and a little, 5.0 us in half of the blocks, 5.8 spread out.
 template <bool IN_BF16, bool RHT, int LOADS = 1>
 __global__ void __launch_bounds__(256) amax_kernel(AmaxArgs a) {
   grid_dependency_wait();
@@ -2386,8 +2388,8 @@ int altob200_amax(const void* x, int32_t in_dtype, int64_t rows, int64_t cols, i
   int64_t blocks = work;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  const int64_t steps = ceil_div(rows * (cols * esz / 16), blocks * 256);
-  a.steps = (int32_t)(steps < 8 ? (steps < 4 ? steps : 4) : 8);
+  const int64_t vecs = rows * (cols * esz / 16), steps = ceil_div(vecs, blocks * 256);
+  a.steps = (int32_t)(vecs >= 9 * blocks * 256 ? 8 : steps < 4 ? steps : 4);
   const bool bf = in_dtype == ALTOB200_DT_BF16;
   if (rht_n) {
     if (bf) (void)launch_after(amax_kernel<true, true>, dim3((unsigned)blocks), dim3(256), 0, st, a);

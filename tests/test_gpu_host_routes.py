@@ -92,3 +92,16 @@ def test_scales_with_rows_behind_the_codes(fmt, is_2d, pad):
     assert torch.equal(Q.dequantize(codes, more, fmt, -1, is_2d, torch.float32), want)
     with pytest.raises(RuntimeError):
         Q.dequantize(codes, scales[:-1], fmt, -1, is_2d, torch.float32)
+
+
+@pytest.mark.parametrize("dtype,cols", [(torch.bfloat16, 2048), (torch.float32, 1024)])      # 256 loads a row
+@pytest.mark.parametrize("steps,more", [(1, 1), (4, 0), (4, 1), (9, -1), (9, 0)])
+def test_maximum_where_the_loads_of_a_thread_change(dtype, cols, steps, more):
+    blocks = torch.cuda.get_device_properties(0).multi_processor_count * 8
+    rows = blocks * steps + more
+    x = torch.zeros(rows, cols, dtype=dtype, device="cuda")
+    bits, outer, scratch = torch.empty(2, dtype=torch.int32, device="cuda"), torch.empty(2, device="cuda"), E.amax_scratch(x.device)
+    for i, (r, c) in enumerate([(0, 0), (rows - 1, cols - 1), (rows - 1, 0), (blocks * 8 % rows, cols // 2), (blocks * 4 % rows, 3)]):
+        x[r, c] = -(i + 1.5)
+        L.amax(x, bits, outer, scratch)
+        assert bits.view(torch.float32)[0].item() == i + 1.5
