@@ -330,25 +330,27 @@ struct RowwiseArgs {
 // Three resident blocks of 256 threads per SM (at most 85 registers per thread): other block sizes and counts
 // measured within 3 %.
 //
-// With words from memory the four rows are a period of the table apart: they meet the same words, which are loaded
-// and converted once, behind the scales of all four rows.  Bound by the instructions of the rounding (26 an element
+// SHARED, words from a table: the four rows are a period of the table apart, so that they meet the same words, which are
+// loaded and converted once, behind the scales of all four rows.  Bound by the instructions of the rounding (26 an element
 // with macro factors, 20 without, the scheduler 64 % busy).  Four blocks of 128 threads (128 registers) keep bf16 rows
 // free of spills; five, or three of 256, spill and are slower than words loaded by row.  8192 x 14336 from bf16, words by
 // row -> shared: MXFP4 119 -> 106 us, with macro factors 141 -> 133, NVFP4 125 -> 113; fp32 141 -> 131 and 178 -> 147.
 constexpr int ROW_R = 4;
 
-constexpr int rowwise_threads(int round) { return round == ALTOB200_ROUND_SR_BITS ? 128 : 256; }
+// Words by row (full planes, or few rows: `rowwise_shares_words`) are loaded in front of a row's scale arithmetic, which
+// hides them.  Asked for behind it, in the registers of SHARED, 8192 x 14336 from bf16 took MXFP4 172 us for 150, with
+// macro factors 193 for 156, NVFP4 180 for 151.
+constexpr int rowwise_threads(bool shared) { return shared ? 128 : 256; }
 
-// Rows of a task: neighbours, or a period of the random table apart, so that the four rows share their words.
-__host__ __device__ __forceinline__ int64_t rowwise_row_step(const RowwiseArgs& a) { return a.tile_rows != 0 ? a.tile_rows : 1; }
-__host__ __device__ __forceinline__ int64_t rowwise_row_groups(const RowwiseArgs& a, int64_t step) {
-  return (a.rows + ROW_R * step - 1) / (ROW_R * step) * step;
+// Groups of rows that tasks take, rows `step` apart: neighbours, or a period of the random table (SHARED).
+__host__ __device__ __forceinline__ int64_t rowwise_row_groups(int64_t rows, int64_t step) {
+  return (rows + ROW_R * step - 1) / (ROW_R * step) * step;
 }
 
 // MACRO (MXFP4 from bf16): the two-level recipe's scaling runs in front of the quantisation; a macro block of
 // 128 columns is eight neighbouring lanes.
-template <int FMT, bool IN_BF16, int ROUND, bool MACRO>
-__global__ void __launch_bounds__(rowwise_threads(ROUND), ROUND == ALTOB200_ROUND_SR_BITS ? 4 : 3) quantize_rowwise_kernel(RowwiseArgs a) {
+template <int FMT, bool IN_BF16, int ROUND, bool MACRO, bool SHARED>
+__global__ void __launch_bounds__(rowwise_threads(SHARED), SHARED ? 4 : 3) quantize_rowwise_kernel(RowwiseArgs a) {
   grid_dependency_wait();
   using F = Fmt<FMT>;
   static_assert(!MACRO || (FMT == ALTOB200_FMT_MXFP4 && IN_BF16), "macro blocks");
@@ -358,9 +360,9 @@ __global__ void __launch_bounds__(rowwise_threads(ROUND), ROUND == ALTOB200_ROUN
   constexpr int NV = IN_BF16 ? 2 : 4;  // 16-byte vectors per lane and row
   const int lane = threadIdx.x & 31;
   const int64_t chunks_per_row = (a.cols + 511) >> 9;
-  constexpr bool WORDS = ROUND == ALTOB200_ROUND_SR_BITS;
-  const int64_t step = WORDS ? rowwise_row_step(a) : 1;
-  const int64_t n_tasks = rowwise_row_groups(a, step) * chunks_per_row;
+  static_assert(!SHARED || ROUND == ALTOB200_ROUND_SR_BITS, "words from a table");
+  const int64_t step = SHARED ? a.tile_rows : 1;
+  const int64_t n_tasks = rowwise_row_groups(a.rows, step) * chunks_per_row;
   const int64_t warp0 = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int64_t n_warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const OuterScale os = make_outer_scale((!F::MX) && a.outer != nullptr, a.outer);
@@ -373,7 +375,7 @@ __global__ void __launch_bounds__(rowwise_threads(ROUND), ROUND == ALTOB200_ROUN
     int64_t rg, chunk;
     divmod_fast(task, chunks_per_row, &rg, &chunk);
     int64_t row0 = rg * ROW_R;
-    if (WORDS && step != 1) {
+    if (SHARED) {
       int64_t period, first;
       divmod_fast(rg, step, &period, &first);
       row0 = period * (ROW_R * step) + first;
@@ -383,7 +385,7 @@ __global__ void __launch_bounds__(rowwise_threads(ROUND), ROUND == ALTOB200_ROUN
     const uint8_t* src = reinterpret_cast<const uint8_t*>(a.x) + (row0 * a.ld + col) * ESZ;
     const int64_t pitch = a.ld * ESZ * step;
     // rows of the task that exist, and the place of their codes, from a count and a pitch where registers are left for them
-    constexpr bool COUNTED = IN_BF16 || WORDS;
+    constexpr bool COUNTED = IN_BF16 || SHARED;
     constexpr int EPB = F::FP4 ? 2 : 1;   // elements per byte of codes
     int n_ok = 0;
 #pragma unroll
@@ -402,20 +404,44 @@ __global__ void __launch_bounds__(rowwise_threads(ROUND), ROUND == ALTOB200_ROUN
       for (int q = 0; q < NV; ++q)
         raw[i][q] = ok ? __ldg(reinterpret_cast<const uint4*>(src + i * pitch) + q) : make_uint4(0u, 0u, 0u, 0u);
     }
+    // position of the task in the periodic random table (32-bit: the host refuses larger extents)
+    uint32_t rr0 = 0, pp = 0;
+    if (ROUND == ALTOB200_ROUND_SR_BITS && !SHARED && tiled) {
+      rr0 = (uint32_t)row0 % t_rows;
+      pp = (uint32_t)(col >> 1) % t_pairs;
+    }
     const int64_t kb = (chunk << 9) / F::B + lane / LPB;  // scale column of this lane
     const bool holder = col_ok && (lane % LPB == 0);
     static_assert(ROW_R == 4, "the packed scales are transposed four rows at a time");
     uint32_t scale_bytes = 0;   // byte i: scale of row i
 
-    BlockScale scales[WORDS ? ROW_R : 1];
+    BlockScale scales[SHARED ? ROW_R : 1];
     bool all_fast = true;
 #pragma unroll
     for (int i = 0; i < ROW_R; ++i) {
       const int64_t row = row0 + i * step;
-      if (WORDS && !row_ok(i)) break;   // the whole warp
+      if (SHARED && !row_ok(i)) break;   // the whole warp
       const bool active = col_ok && row_ok(i);
       uint32_t r0[8], r1[8];
-      if (ROUND == ALTOB200_ROUND_SR_PHILOX) {
+      if (ROUND == ALTOB200_ROUND_SR_BITS && !SHARED) {
+        // random words first: their loads overlap the scale arithmetic below.  Full planes [2][rows][cols/2], or a
+        // [2][tile_rows][tile_pairs] table repeated over the matrix (the 8 pairs of a lane never straddle a tile:
+        // tile_pairs is a multiple of 8)
+        uint32_t rr = rr0 + (uint32_t)i;
+        while (tiled && rr >= t_rows) rr -= t_rows;
+        const int64_t off = tiled ? (int64_t)(rr * t_pairs + pp) : row * half_cols + (col >> 1);
+        const int64_t plane = tiled ? (int64_t)(t_rows * t_pairs) : a.rows * half_cols;
+        uint4 a0 = make_uint4(0u, 0u, 0u, 0u), a1 = a0, b0 = a0, b1 = a0;
+        if (active) {
+          const uint4* p0 = reinterpret_cast<const uint4*>(a.rand_bits + off);
+          const uint4* p1 = reinterpret_cast<const uint4*>(a.rand_bits + plane + off);
+          a0 = __ldg(p0); a1 = __ldg(p0 + 1); b0 = __ldg(p1); b1 = __ldg(p1 + 1);
+        }
+        r0[0] = a0.x; r0[1] = a0.y; r0[2] = a0.z; r0[3] = a0.w;
+        r0[4] = a1.x; r0[5] = a1.y; r0[6] = a1.z; r0[7] = a1.w;
+        r1[0] = b0.x; r1[1] = b0.y; r1[2] = b0.z; r1[3] = b0.w;
+        r1[4] = b1.x; r1[5] = b1.y; r1[6] = b1.z; r1[7] = b1.w;
+      } else if (ROUND == ALTOB200_ROUND_SR_PHILOX) {
         // one Philox call feeds two element pairs: call index = pair index / 2
         const uint64_t q0 = a.philox_offset + (uint64_t)((row * half_cols + (col >> 1)) >> 1);
 #pragma unroll
@@ -507,7 +533,7 @@ __global__ void __launch_bounds__(rowwise_threads(ROUND), ROUND == ALTOB200_ROUN
       }
 
       // ---- encode and store ----
-      if constexpr (WORDS) {   // behind the loop; what clip and factors made of the elements goes back into their words
+      if constexpr (SHARED) {   // behind the loop; what clip and factors made of the elements goes back into their words
         scales[i] = s;
         all_fast = all_fast && block_fast<IN_BF16, ROUND>(s, amax_bits);
         if (MACRO || (F::MX && a.mx.clip == 1)) {
@@ -549,32 +575,23 @@ __global__ void __launch_bounds__(rowwise_threads(ROUND), ROUND == ALTOB200_ROUN
       }
       scale_bytes = merge_shifted((holder && row_ok(i)) ? s.byte : 0u, 8 * i, scale_bytes);
     }
-    if constexpr (WORDS) {
-      // position of the task in the periodic table (32-bit: the host refuses larger extents), or in full planes
-      // [2][rows][cols/2] (the 8 pairs of a lane never straddle a tile: tile_pairs is a multiple of 8)
-      int64_t off = row0 * half_cols + (col >> 1), plane = a.rows * half_cols;
-      if (tiled) {
-        off = (int64_t)(((uint32_t)row0 % t_rows) * t_pairs + (uint32_t)(col >> 1) % t_pairs);
-        plane = (int64_t)(t_rows * t_pairs);
-      }
+    if constexpr (SHARED) {
+      const uint32_t* const at = a.rand_bits + (int64_t)(((uint32_t)row0 % t_rows) * t_pairs + (uint32_t)(col >> 1) % t_pairs);
       with_uniform_fast(all_fast, [&](auto fast_tag) {
         constexpr bool FAST = decltype(fast_tag)::value;
         uint32_t first[ROW_R];
 #pragma unroll
         for (int o = 0; o < 2; ++o) {
           uint4 even = make_uint4(0u, 0u, 0u, 0u), odd = even;
+          if (col_ok) {
+            even = __ldg(reinterpret_cast<const uint4*>(at) + o);
+            odd = __ldg(reinterpret_cast<const uint4*>(at + (int64_t)(t_rows * t_pairs)) + o);
+          }
           SrOctet words;
+          if (FAST) words = sr_octet(even, odd);
 #pragma unroll
           for (int i = 0; i < ROW_R; ++i) {
             if (!row_ok(i)) break;
-            if (i == 0 || !tiled) {
-              if (col_ok) {
-                const uint32_t* p = a.rand_bits + off + (tiled ? 0 : i * half_cols);
-                even = __ldg(reinterpret_cast<const uint4*>(p) + o);
-                odd = __ldg(reinterpret_cast<const uint4*>(p + plane) + o);
-              }
-              if (FAST) words = sr_octet(even, odd);
-            }
             float v[8];
             if (IN_BF16) {
               const uint32_t w[4] = {raw[i][o].x, raw[i][o].y, raw[i][o].z, raw[i][o].w};
@@ -1974,30 +1991,43 @@ static void fill_rht_row_offsets(RhtParams* r, int64_t ld, int esz) {
   for (int k = 0; k < 16; ++k) r->row_off[k] = (int64_t)r->pinv[k] * ld * esz;
 }
 
-template <int FMT, bool IN_BF16, int ROUND>
+// Whether the rows of a task are taken a period of the table apart.  There are up to four times as many tasks then where
+// rows are few, each with fewer loads in flight: faster while one wave of warps holds them (64 x 14336 6.4 -> 5.0 us) and
+// with three rows or more in a task (192 x 65536 17.4 -> 16.2, 512 x 65536 33.5 -> 31.9), not below (64 x 131072
+// 13.2 -> 17.7; 320 x 131072, five rows in eight places, 46.9 -> 49.7; NVFP4 from bf16).  fp32 rows are twice as long and
+// the body with words by row spills: from three rows in two tasks on (96 x 65536 15.1 -> 14.3, 64 x 131072 18.8 -> 20.4).
+static bool rowwise_shares_words(const RowwiseArgs& a, bool in_bf16) {
+  if (a.tile_rows == 0 || a.tile_rows >= (1ll << 32)) return false;
+  const int64_t groups = rowwise_row_groups(a.rows, a.tile_rows);
+  return groups * ((a.cols + 511) >> 9) <= (int64_t)sm_count() * 16 || 2 * a.rows >= (in_bf16 ? 6 : 3) * groups;
+}
+
+template <int FMT, bool IN_BF16, int ROUND, bool SHARED>
 static void launch_rowwise_kernel(const RowwiseArgs& a, cudaStream_t st) {
-  const int64_t tasks = rowwise_row_groups(a, ROUND == ALTOB200_ROUND_SR_BITS ? rowwise_row_step(a) : 1) * ((a.cols + 511) >> 9);
-  constexpr int NT = rowwise_threads(ROUND);
+  const int64_t tasks = rowwise_row_groups(a.rows, SHARED ? a.tile_rows : 1) * ((a.cols + 511) >> 9);
+  constexpr int NT = rowwise_threads(SHARED);
   int64_t blocks = ceil_div(tasks, NT / 32);
   const int64_t cap = (int64_t)sm_count() * (2048 / NT);
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   constexpr bool CAN_MACRO = FMT == ALTOB200_FMT_MXFP4 && IN_BF16 && ROUND != ALTOB200_ROUND_SR_PHILOX;
   if (CAN_MACRO && a.macro_codes != nullptr)
-    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, CAN_MACRO>, dim3((unsigned)blocks), dim3(NT), 0, st, a);
+    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, CAN_MACRO, SHARED>, dim3((unsigned)blocks), dim3(NT), 0, st, a);
   else
-    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, false>, dim3((unsigned)blocks), dim3(NT), 0, st, a);
+    (void)launch_after(quantize_rowwise_kernel<FMT, IN_BF16, ROUND, false, SHARED>, dim3((unsigned)blocks), dim3(NT), 0, st, a);
 }
 
 template <int FMT, bool IN_BF16>
 static int launch_rowwise(const RowwiseArgs& a, int rounding, cudaStream_t st) {
   constexpr bool FP4 = Fmt<FMT>::FP4;
   if (rounding == ALTOB200_ROUND_RTN)
-    launch_rowwise_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN>(a, st);
+    launch_rowwise_kernel<FMT, IN_BF16, ALTOB200_ROUND_RTN, false>(a, st);
+  else if (rounding == ALTOB200_ROUND_SR_BITS && FP4 && rowwise_shares_words(a, IN_BF16))
+    launch_rowwise_kernel<FMT, IN_BF16, FP4 ? ALTOB200_ROUND_SR_BITS : ALTOB200_ROUND_RTN, FP4>(a, st);
   else if (rounding == ALTOB200_ROUND_SR_BITS && FP4)
-    launch_rowwise_kernel<FMT, IN_BF16, FP4 ? ALTOB200_ROUND_SR_BITS : ALTOB200_ROUND_RTN>(a, st);
+    launch_rowwise_kernel<FMT, IN_BF16, FP4 ? ALTOB200_ROUND_SR_BITS : ALTOB200_ROUND_RTN, false>(a, st);
   else if (rounding == ALTOB200_ROUND_SR_PHILOX && FP4)
-    launch_rowwise_kernel<FMT, IN_BF16, FP4 ? ALTOB200_ROUND_SR_PHILOX : ALTOB200_ROUND_RTN>(a, st);
+    launch_rowwise_kernel<FMT, IN_BF16, FP4 ? ALTOB200_ROUND_SR_PHILOX : ALTOB200_ROUND_RTN, false>(a, st);
   else
     return ALTOB200_EUNSUPPORTED;
   return cudaGetLastError() == cudaSuccess ? ALTOB200_OK : ALTOB200_ECUDA;

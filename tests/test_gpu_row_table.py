@@ -38,3 +38,26 @@ def test_equals_words_for_every_element(rows, cols, fmt, dtype, macro, special):
     one = _quantise(x, fmt, outer, macro, rand_bits=table, rand_tile=tile)
     two = _quantise(x, fmt, outer, macro, rand_bits=planes)
     assert all(torch.equal(a, b) for a, b in zip(one, two))
+
+
+@pytest.mark.parametrize("rows,cols,tile", [(96, 65536, None), (31, 131072, None), (321, 65536 + 32, None), (40, 544, (200_000, 8)),
+                                            (5, 4128, (3, 16))])
+@pytest.mark.parametrize("fmt,dtype,macro", [(L.FMT_MXFP4, torch.bfloat16, False), (L.FMT_MXFP4, torch.bfloat16, True),
+                                             (L.FMT_MXFP4, torch.float32, False), (L.FMT_NVFP4, torch.bfloat16, False),
+                                             (L.FMT_NVFP4, torch.float32, False)])
+@pytest.mark.parametrize("special", [False, True])
+def test_few_rows_equal_words_for_every_element(rows, cols, tile, fmt, dtype, macro, special):
+    # wide enough that the rows of a task are neighbours, each with words of its own; a table far longer than the rows
+    tile = tile or L.sr_tile_dims(rows, cols)
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = torch.randn(rows, cols, generator=g, device="cuda") * torch.logspace(-6, 6, cols, device="cuda")
+    if special:
+        x[rows - 1, 0], x[rows // 3, 1], x[0, 2] = float("nan"), float("inf"), -0.0
+    x = x.to(dtype)
+    table = torch.randint(-2 ** 31, 2 ** 31, (2, *tile), generator=g, device="cuda", dtype=torch.int64).to(torch.int32)
+    r, c = torch.arange(rows, device="cuda") % tile[0], torch.arange(cols // 2, device="cuda") % tile[1]
+    planes = table[:, r][:, :, c].contiguous()
+    outer = torch.tensor([0.37], device="cuda") if fmt == L.FMT_NVFP4 else None
+    one = _quantise(x, fmt, outer, macro, rand_bits=table, rand_tile=tile)
+    two = _quantise(x, fmt, outer, macro, rand_bits=planes)
+    assert all(torch.equal(a, b) for a, b in zip(one, two))
