@@ -1676,6 +1676,25 @@ static void set_raster(GemmArgs* g, int64_t tiles_m, int64_t tiles_n, int64_t gr
   g->rows_last = make_tile_div(tiles_m - (ceil_div(tiles_m, gm) - 1) * gm);
 }
 
+// Whether rows grouped by expert go to CTA pairs.  Pairs of groups with two experts are multiplied twice there, so an
+// expert needs enough rows (counted with the buffer's padding: 512 a piece; 32 experts, 2880 -> 2880, us for the pair / the
+// single-CTA kernel, MXFP8 and NVFP4: 256 rows an expert 88 / 81 and 55 / 50, 384 116 / 118 and 72 / 72, 512 136 / 148 and
+// 84 / 94).  And a launch of few tiles is bound by their waves and its start: us per launch, fitted within 6 % on average over 520
+// launches of 2 to 64 experts, 256 to 5760 columns, K of 256 to 4096,
+//   single CTA  3.6 + waves of 148 x (2.1  + 0.5   x stages)
+//   pairs       5.6 + waves of  74 x (1.17 + 0.425 x stages)
+// where the host does not know the experts' rows: faster with groups that pair up, and not much slower with half an expert
+// more in units.  MXFP8, all experts of an odd number of groups, pair / single: 16 experts of 512 rows, 512 x 2048
+// 18.4 / 12.8, 1024 x 512 13.3 / 11.8; even numbers, 4 experts of 512, 512 x 512 8.5 / 7.3, 8 of 512, 5760 x 256 14.8 / 18.3.
+// Large ones: 69 632 rows, 2880 -> 5760: MXFP8 944 / 1144, MXFP4 518 / 635, NVFP4 562 / 677.
+static bool grouped_pairs_pay(int64_t M, int64_t experts, int64_t tiles_n, int64_t stages) {
+  if (M < 512 * experts) return false;
+  const int64_t groups = ceil_div(M, BM), sms = sm_count_gemm(), pairs = sms / 2 > 0 ? sms / 2 : 1;
+  const auto with_units = [&](int64_t units) { return 5.6 + (double)ceil_div(units * tiles_n, pairs) * (1.17 + 0.425 * (double)stages); };
+  const double single = 3.6 + (double)ceil_div(groups * tiles_n, sms) * (2.1 + 0.5 * (double)stages);
+  return with_units(ceil_div(groups, 2)) < 0.97 * single && with_units(ceil_div(groups, 2) + experts / 2) < 1.2 * single;
+}
+
 static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N, int64_t K, int32_t num_experts,
                        const void* a_codes, const void* a_scales, const void* b_codes, const void* b_scales,
                        const int32_t* group_expert, const float* alpha_a, const float* alpha_b,
@@ -1704,20 +1723,16 @@ static int gemm_common(int32_t format_a, int32_t format_b, int64_t M, int64_t N,
     return ALTOB200_ELIMIT;
 
   int BN = N <= 128 ? 128 : 256;
-  // The CTA-pair kernel takes dense and K-range problems, and rows grouped by expert where an expert has enough of
-  // them (counted with the buffer's padding: 512 a piece).  Pairs of groups with two experts are multiplied twice there:
-  // with 256 rows an expert every second pair is, and the single-CTA kernel is the faster one.
-  // us, pair / single CTA, forward of MXFP8 experts 2880 -> 2880 (and NVFP4), 32 of them: 256 rows an expert 88 / 81
-  // (55 / 50), 384 116 / 118 (72 / 72), 512 136 / 148 (84 / 94); 69 632 rows, 2880 -> 5760: MXFP8 944 / 1144, MXFP4
-  // 518 / 635, NVFP4 562 / 677.  ALTOB200_GEMM_PAIR=0 forces the single-CTA kernel everywhere.
+  // The CTA-pair kernel takes dense and K-range problems, and rows grouped by expert where `grouped_pairs_pay` says so.
+  // ALTOB200_GEMM_PAIR=0 forces the single-CTA kernel everywhere.
   static int pair_env = -1;
   if (pair_env < 0) {
     const char* e = getenv("ALTOB200_GEMM_PAIR");
     pair_env = e ? atoi(e) : 1;
   }
   const bool grouped = num_experts > 0;
-  const bool units_fit = !grouped || (M >= 512 * (int64_t)num_experts && ceil_div(M, BM) < PairUnit::MAX &&
-                                      num_experts < (1 << PairUnit::EXPERT_BITS));
+  const bool units_fit = !grouped || (ceil_div(M, BM) < PairUnit::MAX && num_experts < (1 << PairUnit::EXPERT_BITS) &&
+                                      grouped_pairs_pay(M, num_experts, ceil_div(N, 256), ceil_div(k_bytes, STAGE_K_BYTES)));
   const bool use_pair = pair_env != 0 && units_fit && N > 128 && M > 128;
   if (use_pair && !grouped && pair_tile_n() == 192) BN = 192;
   const int64_t b_rows = N * (num_experts > 0 ? num_experts : 1);

@@ -41,3 +41,11 @@ def test_groups_equal_their_rows_alone(groups, n, k, fmt):
             L.gemm_blockscaled(fmt, fmt, 128, n, k, a.codes[rows], a.scales[block * i:block * (i + 1)], bs[e].codes,
                                bs[e].scales, want, outer, outer)
             assert torch.equal(out[rows], want)
+
+
+# the same over as many tiles as make pairs the faster ones, whatever the runs; 17 experts of an odd number of groups
+@pytest.mark.parametrize("fmt", [L.FMT_NVFP4, L.FMT_MXFP4, L.FMT_MXFP8_E4M3])
+@pytest.mark.parametrize("k", [96, 1056])
+@pytest.mark.parametrize("groups", [g * (-(-160 // len(g))) for g in GROUPS] + [[i // 9 for i in range(153)]])
+def test_many_groups_equal_their_rows_alone(groups, k, fmt):
+    test_groups_equal_their_rows_alone(groups, 1056, k, fmt)
