@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(rowwise_threads(SHARED), SHARED ? 4 : 3) quant
     const uint8_t* src = reinterpret_cast<const uint8_t*>(a.x) + (row0 * a.ld + col) * ESZ;
     const int64_t pitch = a.ld * ESZ * step;
     // rows of the task that exist, and the place of their codes, from a count and a pitch where registers are left for them
-    constexpr bool COUNTED = IN_BF16 || SHARED;
+    constexpr bool COUNTED = SHARED || (IN_BF16 && ROUND == ALTOB200_ROUND_RTN);
     constexpr int EPB = F::FP4 ? 2 : 1;   // elements per byte of codes
     int n_ok = 0;
 #pragma unroll
