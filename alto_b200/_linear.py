@@ -25,6 +25,7 @@ import torch
 
 from . import _lib as L
 from . import dge
+from .hadamard import HadamardTransform
 
 # ---------------------------------------------------------------------------------------
 # scratch and random-bit plumbing
@@ -146,9 +147,9 @@ def quant_rows(x2, fmt, outer, sr: dict, use_uos: bool = False, macro_codes=None
 
 def dense_in_quantizer(t2, transform, fmt: int, sr: dict) -> Optional[torch.Tensor]:
     """The matrix of a dense transform that the column-wise quantizer applies itself (32 x 32, MXFP4 from bf16 with
-    words in slot order or none, rows that can be read as they are), else None: the transform's own kernel runs
-    first.  69 632 x 2880 with macro blocks: 165 us in one kernel, 277 in two."""
-    if (transform.n != 32 or fmt != L.FMT_MXFP4 or t2.dtype != torch.bfloat16 or t2.dim() != 2 or t2.shape[0] % 32 != 0
+    words in slot order or none, rows that can be read as they are), else None: the transform is called first, as is
+    one that has a call of its own.  69 632 x 2880 with macro blocks: 165 us in one kernel, 277 in two."""
+    if (getattr(type(transform), "__call__", None) is not HadamardTransform.__call__ or transform.n != 32 or fmt != L.FMT_MXFP4 or t2.dtype != torch.bfloat16 or t2.dim() != 2 or t2.shape[0] % 32 != 0
             or t2.stride(1) != 1 or t2.stride(0) < t2.shape[1] or t2.stride(0) % 8 != 0 or t2.data_ptr() % 16 != 0
             or sr["rounding"] not in (L.ROUND_RTN, L.ROUND_SR_SLOTS) or not t2.is_cuda):
         return None

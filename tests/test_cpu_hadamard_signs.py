@@ -80,3 +80,27 @@ def test_a_factory_of_its_own_is_asked_for_both_parts(monkeypatch):
         assert torch.equal(H.HadamardFactory.create_transform("cpu").weight, torch.ones(16, 16))
     finally:
         H.HadamardFactory.generator.set_state(generator)
+
+
+def test_a_transform_with_a_call_of_its_own_is_called():
+    from alto_b200 import _lib as L
+    from alto_b200 import _linear as E
+
+    class Rows:                                        # what a bf16 matrix on a GPU answers
+        dtype, shape, device, is_cuda = torch.bfloat16, (64, 128), torch.device("cpu"), True
+        dim = lambda self: 2
+        stride = lambda self, axis: (128, 1)[axis]
+        data_ptr = lambda self: 0
+
+    class Halved(H.HadamardTransform):
+        def __call__(self, value, **options):
+            return super().__call__(value, **options) / 2
+
+    class Other:                                       # no matrix to ask for
+        is_fused = False
+        __call__ = lambda self, value, left_mul: value
+
+    weight = H.deterministic_hadamard_matrix(32)
+    ask = lambda transform: E.dense_in_quantizer(Rows(), transform, L.FMT_MXFP4, E.RTN)
+    assert torch.equal(ask(H.HadamardTransform(weight, None)), weight)
+    assert ask(Halved(weight, None)) is None and ask(Other()) is None
