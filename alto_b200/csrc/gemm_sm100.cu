@@ -137,11 +137,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ uint64_t globaltimer_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
 // Bounded waits as one small loop each.  More than a dozen warps' worth of different code share the instruction caches of an
 // SM, where every taken branch costs 30 to 40 cycles: a wait that is spread over inlined slow paths took
 // 200 cycles and more on a barrier that was already complete, and with it a chunk's way around the roles 1300.
@@ -285,11 +280,6 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
       : "memory");
 }
 
-__device__ __forceinline__ void tma_store_2d(const void* smem_src, const CUtensorMap* map, int32_t x, int32_t y) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-               ::"l"(map), "r"(smem_u32(smem_src)), "r"(x), "r"(y)
-               : "memory");
-}
 __device__ __forceinline__ void tma_store_3d(const void* smem_src, const CUtensorMap* map, int32_t x, int32_t y,
                                              int32_t z) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
@@ -308,9 +298,6 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t
 
 __device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t a) {
   asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(a) : "memory");
-}
-__device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t a, uint32_t b) {
-  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -354,21 +341,6 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-#define ALTOB200_R8(r, o) "=r"(r[o]), "=r"(r[o + 1]), "=r"(r[o + 2]), "=r"(r[o + 3]), "=r"(r[o + 4]), "=r"(r[o + 5]), \
-                         "=r"(r[o + 6]), "=r"(r[o + 7])
-__device__ __forceinline__ void tc_ld64(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x64.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, "
-      "%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, "
-      "%48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-      : ALTOB200_R8(r, 0), ALTOB200_R8(r, 8), ALTOB200_R8(r, 16), ALTOB200_R8(r, 24), ALTOB200_R8(r, 32),
-        ALTOB200_R8(r, 40), ALTOB200_R8(r, 48), ALTOB200_R8(r, 56)
-      : "r"(taddr)
-      : "memory");
-}
-#undef ALTOB200_R8
 __device__ __forceinline__ void tc_st4(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c),
                "r"(d)
@@ -383,16 +355,6 @@ __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sy
 constexpr uint32_t DESC_SW128_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint64_t desc_of(uint32_t hi, uint32_t lo) { return ((uint64_t)hi << 32) | lo; }
 
-// Shared-memory matrix descriptor, K-major, 128-byte swizzle, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t make_desc_sw128(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3FFFu);      // start address
-  d |= (uint64_t)1 << 16;                       // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;             // stride byte offset
-  d |= (uint64_t)1 << 46;                       // descriptor version (Blackwell)
-  d |= (uint64_t)2 << 61;                       // SWIZZLE_128B
-  return d;
-}
 // ---------------------------------------------------------------------------------------
 // epilogue of one tile for one warp (its 32 accumulator rows), shared by both kernels
 // ---------------------------------------------------------------------------------------
@@ -868,9 +830,6 @@ __device__ __forceinline__ uint32_t mapa_u32(uint32_t local_addr, uint32_t rank)
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank));
   return r;
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // Arrival without a cluster-scope release.  What the waiting side consumes after these arrivals
 // is tensor memory, whose writes (tcgen05.st) and reads (tcgen05.ld) the arriving warp has already
@@ -1511,13 +1470,13 @@ static EncodeTiledFn get_encode_fn() {
 // the 128-byte swizzle, or x 64 bytes with the 64-byte swizzle (epilogues whose column share is not
 // a multiple of 128 bytes).  The batch coordinate keeps a ragged tile of one batch entry out of the next.
 static int make_tmap_out(CUtensorMap* m, void* base, int64_t batches, int64_t M, int64_t N, int64_t ldd, bool bf16,
-                         int row_bytes = 128, int box_rows = 32) {
+                         int row_bytes) {
   EncodeTiledFn fn = get_encode_fn();
   if (fn == nullptr) return ALTOB200_ECUDA;
   const int esz = bf16 ? 2 : 4;
   cuuint64_t dims[3] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)batches};
   cuuint64_t strides[2] = {(cuuint64_t)(ldd * esz), (cuuint64_t)(M * ldd * esz)};
-  cuuint32_t box[3] = {(cuuint32_t)(row_bytes / esz), (cuuint32_t)box_rows, 1u};
+  cuuint32_t box[3] = {(cuuint32_t)(row_bytes / esz), 32u, 1u};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(m, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
