@@ -577,7 +577,7 @@ gemm_macro_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // ------------------------------ fold + epilogue ------------------------------
     setmaxnreg_inc<C::REGS_FOLD>();
     // (What lives across the chunk loop beside the sums and the pieces is kept in 32 bits: local memory does not fit
-    // beside 230 KB of shared memory, a few spilled registers in this loop or the transfer's cost a tenth.)
+    // beside 228 128 bytes of shared memory (232 192 with 192 columns), a few spilled registers in this loop or the transfer's cost a tenth.)
     const int quad = warp & 3;                        // tensor-memory lane quarter this warp may read
     const int side = (warp - 8) >> 2;                 // columns [WN side, WN side + WN) of the tile
     const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(side * C::WN);
